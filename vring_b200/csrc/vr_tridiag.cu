@@ -11,31 +11,202 @@
 
 namespace vr {
 
-// One thread per system, the reference's recurrence verbatim
-// (beta(k) = bb(k) - cc(k-1)*aa(k)/beta(k-1), ...); beta is kept in sol and
-// gamm in a scratch row so nothing is allocated per thread.
-__global__ void k_thomas(const double *__restrict__ rhs, double *__restrict__ sol, const double *__restrict__ aa,
-                         const double *__restrict__ bb, const double *__restrict__ cc, double *__restrict__ gamm,
-                         int n, int nbatch) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbatch) return;
-  size_t o = (size_t)b * n;
-  const double *r = rhs + o, *a = aa + o, *d = bb + o, *c = cc + o;
-  double *beta = sol + o, *gm = gamm + o;
-  beta[0] = d[0];
-  gm[0] = r[0] / d[0];
-  for (int k = 1; k < n; k++) {
-    beta[k] = d[k] - c[k - 1] * a[k] / beta[k - 1];
-    gm[k] = (r[k] - a[k] * gm[k - 1]) / beta[k];
+// Batched Thomas solve (beta(k) = bb(k) - cc(k-1)*aa(k)/beta(k-1),
+// gamm(k) = (rhs(k) - aa(k) gamm(k-1)) / beta(k), sol(k) = gamm(k) -
+// cc(k)/beta(k) sol(k+1)) of S systems per CTA.
+//
+// A system is a chain of n dependent steps, so the time is the chain's
+// latency and not its bytes: 10.5 MB at 257 x 1024 would take 1.6 us, a
+// division per step alone 10 us.  The chain is therefore taken apart:
+// - beta is carried as a ratio u(k) / u(k-1) of the leading minors,
+//   u(k) = bb(k) u(k-1) - cc(k-1) aa(k) u(k-2), one fused multiply-add per
+//   step on the critical path and no division.  The ratio of the two stored
+//   numbers is the beta that the next step continues from, so the rounding of
+//   a step enters as it does in the recurrence above; the pair is scaled by a
+//   power of two per step (exact), so the minors neither overflow nor vanish.
+// - the divisions 1 / beta(k) of a tile are independent of each other and run
+//   on all 32 lanes of a warp of their own.
+// - three warps work on three consecutive tiles of KT positions at a time:
+//   the minors of one, the divisions of the one before, gamm of the one
+//   before that, while a fourth brings the next tile from memory (8-byte
+//   asynchronous copies, lanes along a system: full sectors) and stores the
+//   tile that is done.  cc/beta goes to the gamm scratch and gamm to sol; the
+//   back substitution streams both backwards the same way.
+// The positions past n of the last tile, and systems past nbatch, are rows of
+// the identity.  aa(1) and cc(n) are not used: they are taken as 0.
+//
+// 257 x 1024 (us per call): one thread per system with its loads a system
+// apart 241, this form 18.4.
+constexpr int kThomKT = 16;    // positions per tile
+constexpr int kThomRing = 6;   // tiles in flight
+
+// 2^-e of x = m 2^e, 1 <= |m| < 2 (0 for an infinity or a NaN: the product is then no number either)
+__device__ __forceinline__ double pow2_inv(double x) {
+  const int e = (__double2hiint(x) >> 20) & 0x7ff;
+  return __hiloint2double(max(2046 - e, 0) << 20, 0);
+}
+
+template <int S>
+__global__ void __launch_bounds__(128) k_thomas(const double *__restrict__ rhs, double *sol,
+                                              const double *__restrict__ aa, const double *__restrict__ bb,
+                                              const double *__restrict__ cc, double *gamm, int n, int nbatch) {
+  constexpr int KT = kThomKT, LD = S + 1, AR = KT * LD, R = kThomRing;
+  constexpr int TR = 0, TA = 1, TB = 2, TC = 3, TX = 4;  // arrays of a tile: rhs, aa, bb, cc, u(k-1)
+  extern __shared__ double sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s0 = blockIdx.x * S, ns = min(S, nbatch - s0);
+  const int nt = (n + KT - 1) / KT;
+  auto tile = [&](int t, int arr) { return sm + ((size_t)(t % R) * 5 + arr) * AR; };
+  const size_t base = (size_t)s0 * n;
+  double x = 1.0, y = 1.0, cprev = 0.0;  // warp 1: u(k-1), u(k-2), cc(k-1)
+  double g = 0.0;                        // warp 3: gamm(k-1)
+  for (int i = 0; i < nt + 5; i++) {
+    if (warp == 0) {
+      if (i < nt) {
+        double *r = tile(i, TR), *a = tile(i, TA), *b = tile(i, TB), *c = tile(i, TC);
+#pragma unroll
+        for (int e = lane; e < KT * S; e += 32) {
+          const int kk = e % KT, s = e / KT, k = i * KT + kk, o = kk * LD + s;
+          const size_t q = base + (size_t)s * n + k;
+          if (s < ns && k < n) {
+            cp_async8(r + o, rhs + q);
+            cp_async8(b + o, bb + q);
+            if (k > 0) cp_async8(a + o, aa + q); else a[o] = 0.0;
+            if (k < n - 1) cp_async8(c + o, cc + q); else c[o] = 0.0;
+          } else {
+            r[o] = 0.0;
+            a[o] = 0.0;
+            b[o] = 1.0;
+            c[o] = 0.0;
+          }
+        }
+      }
+      cp_async_commit();
+      const int t = i - 5;  // this tile is done: cc/beta and gamm to memory
+      if (t >= 0) {
+        const double *f = tile(t, TC), *gm = tile(t, TR);
+#pragma unroll
+        for (int e = lane; e < KT * S; e += 32) {
+          const int kk = e % KT, s = e / KT, k = t * KT + kk;
+          const size_t q = base + (size_t)s * n + k;
+          if (s < ns && k < n) {
+            gamm[q] = f[kk * LD + s];
+            sol[q] = gm[kk * LD + s];
+          }
+        }
+      }
+      cp_async_wait<1>();  // tile i - 1 has landed
+    } else if (warp == 1) {
+      const int t = i - 2;
+      if (t >= 0 && t < nt && lane < S) {
+        const double *a = tile(t, TA) + lane, *c = tile(t, TC) + lane;
+        double *b = tile(t, TB) + lane, *xo = tile(t, TX) + lane;
+#pragma unroll
+        for (int kk = 0; kk < KT; kk++) {
+          const double s = pow2_inv(y), p = (cprev * a[kk * LD]) * s;
+          cprev = c[kk * LD];
+          const double z = fma(b[kk * LD] * s, x, -(p * y));
+          y = x * s;
+          b[kk * LD] = z;
+          xo[kk * LD] = y;
+          x = z;
+        }
+      }
+    } else if (warp == 2) {
+      const int t = i - 3;
+      if (t >= 0 && t < nt) {
+        const double *b = tile(t, TB);
+        double *c = tile(t, TC), *xo = tile(t, TX);
+#pragma unroll
+        for (int e = lane; e < KT * S; e += 32) {
+          const int o = (e / S) * LD + e % S;
+          const double ib = xo[o] / b[o];
+          xo[o] = ib;
+          c[o] = c[o] * ib;
+        }
+      }
+    } else {
+      const int t = i - 4;
+      if (t >= 0 && t < nt && lane < S) {
+        const double *a = tile(t, TA) + lane, *xo = tile(t, TX) + lane;
+        double *r = tile(t, TR) + lane;
+#pragma unroll
+        for (int kk = 0; kk < KT; kk++) {
+          g = fma(-a[kk * LD], g, r[kk * LD]) * xo[kk * LD];
+          r[kk * LD] = g;
+        }
+      }
+    }
+    __syncthreads();
   }
-  // back substitution overwrites beta with the solution from the end
-  double x = gm[n - 1];
-  beta[n - 1] = x;
-  for (int k = n - 2; k >= 0; k--) {
-    double bk = beta[k];
-    x = gm[k] - c[k] * x / bk;
-    beta[k] = x;
+  // back substitution, last tile first: arrays 0 gamm, 1 cc/beta, 2 the solution
+  double xn = 0.0;
+  for (int i = 0; i < nt + 3; i++) {
+    if (warp == 0) {
+      if (i < nt) {
+        const int t = nt - 1 - i;
+        double *gm = tile(i, 0), *f = tile(i, 1);
+#pragma unroll
+        for (int e = lane; e < KT * S; e += 32) {
+          const int kk = e % KT, s = e / KT, k = t * KT + kk, o = kk * LD + s;
+          const size_t q = base + (size_t)s * n + k;
+          if (s < ns && k < n) {
+            cp_async8(gm + o, sol + q);
+            cp_async8(f + o, gamm + q);
+          } else {
+            gm[o] = 0.0;
+            f[o] = 0.0;
+          }
+        }
+      }
+      cp_async_commit();
+      cp_async_wait<1>();
+    } else if (warp == 1) {
+      if (i >= 2 && i - 2 < nt && lane < S) {
+        const double *gm = tile(i - 2, 0) + lane, *f = tile(i - 2, 1) + lane;
+        double *o = tile(i - 2, 2) + lane;
+#pragma unroll
+        for (int kk = KT - 1; kk >= 0; kk--) {
+          xn = fma(-f[kk * LD], xn, gm[kk * LD]);
+          o[kk * LD] = xn;
+        }
+      }
+    } else if (warp == 2) {
+      if (i >= 3) {
+        const int t = nt - 1 - (i - 3);
+        const double *o = tile(i - 3, 2);
+#pragma unroll
+        for (int e = lane; e < KT * S; e += 32) {
+          const int kk = e % KT, s = e / KT, k = t * KT + kk;
+          if (s < ns && k < n) sol[base + (size_t)s * n + k] = o[kk * LD + s];
+        }
+      }
+    }
+    __syncthreads();
   }
+}
+
+// S systems per CTA: 8 keeps a batch of up to 2 x 148 x 8 systems on CTAs of
+// their own (the chain's length sets the time, so more systems per CTA gain
+// nothing there); larger batches are bound by throughput and take 16.
+static const void *thomas_kernel(int nbatch, int *s, size_t *smem) {
+  *s = nbatch <= 2 * 148 * 8 ? 8 : 16;
+  *smem = sizeof(double) * kThomRing * 5 * kThomKT * (*s + 1);
+  return *s == 8 ? (const void *)k_thomas<8> : (const void *)k_thomas<16>;
+}
+
+// returns the error of this launch alone: one that an earlier, unrelated
+// launch left pending on the thread is neither reported nor cleared
+static cudaError_t launch_thomas(const double *rhs, double *sol, const double *aa, const double *bb, const double *cc,
+                                 double *gamm, int n, int nbatch, cudaStream_t st) {
+  int s;
+  size_t smem;
+  const void *kern = thomas_kernel(nbatch, &s, &smem);
+  cudaError_t e = allow_dyn_smem(kern, smem);
+  if (e) return e;
+  void *args[] = {(void *)&rhs, (void *)&sol, (void *)&aa, (void *)&bb, (void *)&cc, (void *)&gamm,
+                  (void *)&n, (void *)&nbatch};
+  return cudaLaunchKernel(kern, dim3((nbatch + s - 1) / s), dim3(128), args, smem, st);
 }
 
 cudaError_t launch_thomas_batched(const double *rhs, double *sol, const double *aa, const double *bb,
@@ -43,8 +214,7 @@ cudaError_t launch_thomas_batched(const double *rhs, double *sol, const double *
   double *gamm = nullptr;
   cudaError_t e = cudaMallocAsync(&gamm, sizeof(double) * (size_t)n * nbatch, s);
   if (e) return e;
-  k_thomas<<<(nbatch + 127) / 128, 128, 0, s>>>(rhs, sol, aa, bb, cc, gamm, n, nbatch);
-  e = cudaGetLastError();
+  e = launch_thomas(rhs, sol, aa, bb, cc, gamm, n, nbatch, s);
   cudaFreeAsync(gamm, s);
   return e;
 }
@@ -220,15 +390,9 @@ extern "C" int vr_solve_lap_thom_noalloc(const double *rhs, double *sol, const d
     gamm = static_cast<double *>(addr);
     g_thom_scratch_ptr[dev].store(gamm, std::memory_order_release);
   }
-  // cudaLaunchKernel returns the error of this launch alone; an error that an
-  // earlier, unrelated launch left pending on the thread is neither reported
-  // here nor cleared
-  cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-  int n_ = n, nb_ = nbatch;
-  void *args[] = {(void *)&rhs, (void *)&sol, (void *)&aa, (void *)&bb, (void *)&cc, (void *)&gamm,
-                  (void *)&n_, (void *)&nb_};
-  cudaError_t e = cudaLaunchKernel((const void *)k_thomas, dim3((nbatch + 127) / 128), dim3(128), args, 0, s);
-  return e == cudaSuccess ? VR_OK : VR_ERR_CUDA;
+  return launch_thomas(rhs, sol, aa, bb, cc, gamm, n, nbatch, static_cast<cudaStream_t>(cuda_stream)) == cudaSuccess
+             ? VR_OK
+             : VR_ERR_CUDA;
 }
 
 extern "C" int vr_solve_lap_bthom(const double *rhs, double *sol, const double *b1, const double *b2,

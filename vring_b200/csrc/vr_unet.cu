@@ -160,18 +160,6 @@ __global__ void __launch_bounds__(256) k_conv3(const TI *__restrict__ in, int H,
   }
 }
 
-// 16-byte asynchronous global -> shared copy; bytes < 16 zero-fills the rest
-// (0: no global read, the destination becomes zeros)
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, unsigned bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // The same 3x3 convolution on the tensor cores (BF16 in, FP32 accumulate):
 // an implicit GEMM over a patch of 8 (r) x 16 (z) output pixels per CTA,
 // M = 128 pixels (row m = r + 8 z), N = NOUT output channels, K = 9 CINP
