@@ -12,6 +12,7 @@
 #include <utility>
 #include <vector>
 
+#include "vr_fold.cuh"
 #include "vr_internal.cuh"
 
 using vr::Geo;
@@ -304,7 +305,7 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
   if (d.abi_version != VR_ABI_VERSION) return VR_ERR_DESC;
   // theta <= 1024 (warp-per-line theta solve holds <= 32 unknowns per lane);
   // r, z <= 2048 (one line tile in 227 KB of shared memory); a z length that
-  // is not a power of two uses the direct DCT, written for nz <= 512.
+  // is not a power of two: up to 512.
   bool nz_pow2 = (d.nz & (d.nz - 1)) == 0;
   if (d.ntheta < 3 || d.ntheta > 1024 || d.nr < 4 || d.nz < 4 || d.nr > 2048 || d.nz > 2048 ||
       (!nz_pow2 && d.nz > 512))
@@ -475,6 +476,15 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
     }
   }
   size_t o_twt = blob.add(twt), o_twz = blob.add(twz);
+  const bool th_fold = !fft_theta_length(N), z_fold = !fft_z_length(d.nz);
+  size_t o_fold[4] = {};
+  for (int kind = 0; kind < 2; kind++) {
+    if (!(kind == kFoldZ ? z_fold : th_fold)) continue;
+    std::vector<double> f, i;
+    fold_tables(kind, kind == kFoldZ ? d.nz : N, f, i);
+    o_fold[2 * kind] = blob.add(f);
+    o_fold[2 * kind + 1] = blob.add(i);
+  }
 
   c->dcoef_len = blob.v.size();
   if (cudaMalloc(&c->dcoef, sizeof(double) * c->dcoef_len) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -504,6 +514,10 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
   c->pois_ib = D + o_pib;
   c->tw_th = D + o_twt;
   c->tw_z = D + o_twz;
+  for (int i = 0; i < 2; i++) {
+    c->fold_z[i] = z_fold ? D + o_fold[2 * kFoldZ + i] : nullptr;
+    c->fold_th[i] = th_fold ? D + o_fold[2 * kFoldTh + i] : nullptr;
+  }
   // host copies for the hdnbc scalars
   c->h_rc = new double[m.rc.size()];
   c->h_rm = new double[m.rm.size()];
@@ -535,6 +549,7 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
     if (cudaMemsetAsync(*o.p, 0, o.w * o.n, c->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
     c->state.emplace_back(*o.p, o.w * o.n);
   }
+  if (z_fold && cudaMalloc(&c->spec2, sizeof(double) * nrs) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&c->d_count, sizeof(unsigned long long) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMemsetAsync(c->d_count, 0, sizeof(unsigned long long) * 4, c->stream) != cudaSuccess)
     return fail(VR_ERR_CUDA);
@@ -552,7 +567,7 @@ extern "C" int vr_destroy(vr_ctx *c) {
   for (int i = 0; i < 4; i++)
     if (c->graph_ok[i]) cudaGraphExecDestroy(c->graph[i]);
   double *ptrs[] = {c->q[0], c->q[1], c->q[2], c->dq[0], c->dq[1], c->dq[2], c->ru[0], c->ru[1],
-                    c->ru[2], c->qrhs[0], c->qrhs[1], c->qrhs[2], c->pres, c->prg, c->rhs, c->spec,
+                    c->ru[2], c->qrhs[0], c->qrhs[1], c->qrhs[2], c->pres, c->prg, c->rhs, c->spec, c->spec2,
                     c->dph, c->csort, c->dq3no, c->corr3n, c->corr3s, c->tconv, c->dcoef, c->d_red};
   for (double *p : ptrs)
     if (p) cudaFree(p);

@@ -147,6 +147,7 @@ struct vr_ctx {
   // device fields
   double *q[3], *dq[3], *ru[3], *qrhs[3];
   double *prg, *pres, *rhs, *dph, *spec;
+  double *spec2;  // second spectral buffer (z lengths without an FFT), or null
   double *csort, *dq3no, *corr3n, *corr3s, *tconv;
   // device coefficient storage (one allocation) and family tables
   double *dcoef;
@@ -156,6 +157,7 @@ struct vr_ctx {
   const double *pois_ib;                   // (nth/2+1, nr, nz) -> [kz][j][mm]
   const double *pois_a, *pois_c;           // aa/cc with aa(1)=0, cc(nr)=0
   const double *tw_th;                     // theta twiddles (cos, sin) 2*nth
+  const double *fold_th[2], *fold_z[2];    // forward, inverse tables of lengths without an FFT (vr_fold.cuh), or null
   const double *tw_z;                      // z twiddles for FFT (cos,sin) n and DCT shifts
   // host-side copies needed for hdnbc scalars
   double *h_rc, *h_rm, *h_da, *h_qc;
@@ -304,6 +306,8 @@ cudaError_t launch_divq(vr_ctx *c, const Rk &rk);
 // poisson_takes_dq
 cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk = nullptr);
 bool poisson_takes_dq(const vr_ctx *c);
+bool fft_theta_length(int n);
+bool fft_z_length(int n);
 cudaError_t launch_upsol(vr_ctx *c, const Rk &rk);
 cudaError_t launch_uppres(vr_ctx *c, const Rk &rk);
 cudaError_t launch_upsol_uppres(vr_ctx *c, const Rk &rk);

@@ -5,8 +5,8 @@
 //   r:     one tridiagonal solve per (theta mode, z mode) (poisson_solve.F90:270-323)
 //   back:  DCT-III along z, inverse packed DFT along theta, copied into dph.
 //
-// Power-of-two lengths run radix-2 FFTs in shared memory (twiddles computed
-// on the host in double); other lengths use the direct sums.  The radial
+// Power-of-two lengths from 32 run FFTs (twiddles computed on the host in
+// double); the other lengths are folded matrix products (vr_fold.cuh).  The radial
 // factorisation depends only on (theta mode, z mode) and is built once at
 // vr_create; the solve streams the right-hand side through a shared-memory
 // tile and runs the two substitutions chunk-parallel (see vr_momentum.cu).
@@ -15,6 +15,7 @@
 
 #include "vr_chunk.cuh"
 #include "vr_fft.cuh"
+#include "vr_fold.cuh"
 #include "vr_internal.cuh"
 
 namespace vr {
@@ -51,114 +52,6 @@ __device__ void smem_fft(double *re, double *im, int n, int lpb, const double *_
     __syncthreads();
   }
 }
-
-// ---------------------------------------------------------------------------
-// theta transforms on lines of nth contiguous values
-// ---------------------------------------------------------------------------
-__global__ void k_fft_fwd(const double *__restrict__ in, double *__restrict__ out, int N, int logn,
-                          int lpb, int nlines, const double *__restrict__ tw) {
-  extern __shared__ double sm[];
-  double *re = sm, *im = sm + lpb * N;
-  int line0 = blockIdx.x * lpb;
-  int nl = min(lpb, nlines - line0);
-  for (int idx = threadIdx.x; idx < lpb * N; idx += blockDim.x) {
-    int l = idx / N, n = idx % N;
-    double v = l < nl ? in[(size_t)(line0 + l) * N + n] : 0.0;
-    re[l * N + brev(n, logn)] = v;
-    im[l * N + brev(n, logn)] = 0.0;
-  }
-  __syncthreads();
-  smem_fft(re, im, N, lpb, tw, -1);
-  for (int idx = threadIdx.x; idx < nl * N; idx += blockDim.x) {
-    int l = idx / N, s = idx % N;  // output slot s (0-based)
-    double v;
-    if (s == 0) {
-      v = re[l * N] / N;
-    } else if (s & 1) {  // a_k, k = (s+1)/2
-      int k = (s + 1) >> 1;
-      v = 2.0 * re[l * N + k] / N;
-    } else {  // b_k, k = s/2 (k < N/2)
-      int k = s >> 1;
-      v = -2.0 * im[l * N + k] / N;
-    }
-    out[(size_t)(line0 + l) * N + s] = v;
-  }
-}
-
-// inverse: packed -> values; writes into dph(i, j, k) (j = 1..nr, k = 1..nz)
-__global__ void k_fft_bwd(const double *__restrict__ in, double *__restrict__ dph, Geo g, int logn, int lpb,
-                          int nlines, const double *__restrict__ tw) {
-  extern __shared__ double sm[];
-  const int N = g.nth;
-  double *re = sm, *im = sm + lpb * N;
-  int line0 = blockIdx.x * lpb;
-  int nl = min(lpb, nlines - line0);
-  for (int idx = threadIdx.x; idx < lpb * N; idx += blockDim.x) {
-    int l = idx / N, k = idx % N;
-    double fr = 0.0, fi = 0.0;
-    if (l < nl) {
-      const double *p = in + (size_t)(line0 + l) * N;
-      int kk = k <= N / 2 ? k : N - k;  // Hermitian extension
-      if (kk == 0) {
-        fr = p[0];
-      } else {
-        fr = p[2 * kk - 1] / 2.0;
-        fi = (2 * kk < N) ? -1.0 * p[2 * kk] / 2.0 : 0.0;
-      }
-      if (k > N / 2) fi = -fi;
-      if (2 * kk == N) fi = 0.0;
-    }
-    re[l * N + brev(k, logn)] = fr;
-    im[l * N + brev(k, logn)] = fi;
-  }
-  __syncthreads();
-  smem_fft(re, im, N, lpb, tw, +1);
-  for (int idx = threadIdx.x; idx < nl * N; idx += blockDim.x) {
-    int l = idx / N, n = idx % N;
-    int L = line0 + l;  // L = (j-1) + nr*(k-1)
-    int j = 1 + L % g.nr, k = 1 + L / g.nr;
-    dph[IDP(g, n + 1, j, k)] = re[l * N + n];
-  }
-}
-
-// direct sums for lengths that are not powers of two
-__global__ void k_dft_fwd_direct(const double *__restrict__ in, double *__restrict__ out, int N, int nlines) {
-  int L = blockIdx.x;
-  if (L >= nlines) return;
-  const double *x = in + (size_t)L * N;
-  for (int s = threadIdx.x; s < N; s += blockDim.x) {
-    int k = (s + 1) >> 1;
-    double acc = 0.0;
-    for (int j = 0; j < N; j++) {
-      double sn, cs;
-      sincospi(2.0 * (double)(((long long)j * k) % N) / N, &sn, &cs);
-      acc += x[j] * ((s == 0 || (s & 1)) ? cs : -sn);
-    }
-    out[(size_t)L * N + s] = (s == 0) ? acc / N : (s & 1) ? 2.0 * acc / N : -2.0 * acc / N;
-  }
-}
-
-__global__ void k_dft_bwd_direct(const double *__restrict__ in, double *__restrict__ dph, Geo g, int nlines) {
-  int L = blockIdx.x;
-  if (L >= nlines) return;
-  const int N = g.nth;
-  const double *p = in + (size_t)L * N;
-  int j = 1 + L % g.nr, k = 1 + L / g.nr;
-  for (int n = threadIdx.x; n < N; n += blockDim.x) {
-    double s = p[0];
-    for (int kk = 1; kk <= N / 2; kk++) {
-      double sn, cs;
-      sincospi(2.0 * (double)(((long long)n * kk) % N) / N, &sn, &cs);
-      double fr = p[2 * kk - 1] / 2.0, fi = (2 * kk < N) ? -1.0 * p[2 * kk] / 2.0 : 0.0;
-      if (2 * kk == N)
-        s += fr * cs;
-      else
-        s += 2.0 * (fr * cs - fi * sn);
-    }
-    dph[IDP(g, n + 1, j, k)] = s;
-  }
-}
-
 
 // ---------------------------------------------------------------------------
 // warp-register transforms (power-of-two lengths >= 32)
@@ -1463,32 +1356,6 @@ __global__ void k_dct(double *__restrict__ a, Geo g, int logn, int dir, const do
   }
 }
 
-__global__ void k_dct_direct(double *__restrict__ a, Geo g, int dir) {
-  extern __shared__ double sm[];
-  const int n = g.nz;
-  const int slot = blockIdx.x, j = blockIdx.y;
-  const size_t s2 = (size_t)g.nth * g.nr;
-  double *x = sm;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) x[k] = a[slot + (size_t)g.nth * j + s2 * k];
-  __syncthreads();
-  double y[8];
-  int cnt = 0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    double s = 0.0;
-    if (dir > 0) {
-      for (int p = 0; p < n; p++) s += x[p] * cospi((double)(((long long)(2 * p + 1) * k) % (4 * n)) / (2.0 * n));
-      s = 2.0 * s / (2.0 * n * 1);
-    } else {
-      s = x[0];
-      for (int p = 1; p < n; p++) s += 2.0 * x[p] * cospi((double)(((long long)p * (2 * k + 1)) % (4 * n)) / (2.0 * n));
-    }
-    y[cnt++] = s;
-  }
-  __syncthreads();
-  cnt = 0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) a[slot + (size_t)g.nth * j + s2 * k] = y[cnt++];
-}
-
 // ---------------------------------------------------------------------------
 // radial solves: lines (slot, kz) along j, per-line factorisation from the
 // (kz, j, mode) table; slot s (1-based) carries mode m = s/2.
@@ -1656,6 +1523,10 @@ static cudaError_t run_dct(vr_ctx *c, int dir) {
   return cudaGetLastError();
 }
 
+// the theta transforms' side of the spectrum: the folded z transforms are not
+// in place, so theirs is the second buffer
+static double *theta_spec(vr_ctx *c) { return c->fold_z[0] ? c->spec2 : c->spec; }
+
 template <int E>
 static cudaError_t run_fft_w(vr_ctx *c, int dir) {
   const Geo &g = c->geo;
@@ -1667,10 +1538,10 @@ static cudaError_t run_fft_w(vr_ctx *c, int dir) {
   LaunchScope ls(c, PK_FFT);
   if (dir > 0) {
     if ((e = allow_dyn_smem(k_fft_fwd_w<E>, sm))) return e;
-    k_fft_fwd_w<E><<<blocks, 256, sm, c->stream>>>(c->rhs, c->spec, nlines, c->tw_th);
+    k_fft_fwd_w<E><<<blocks, 256, sm, c->stream>>>(c->rhs, theta_spec(c), nlines, c->tw_th);
   } else {
     if ((e = allow_dyn_smem(k_fft_bwd_w<E>, sm))) return e;
-    k_fft_bwd_w<E><<<blocks, 256, sm, c->stream>>>(c->spec, c->dph, g, nlines, c->tw_th);
+    k_fft_bwd_w<E><<<blocks, 256, sm, c->stream>>>(theta_spec(c), c->dph, g, nlines, c->tw_th);
   }
   return cudaGetLastError();
 }
@@ -1691,19 +1562,19 @@ static cudaError_t run_fft_s(vr_ctx *c, int dir, const Rk *div_rk = nullptr) {
       if ((e = allow_dyn_smem(kern, sm))) return e;
       DivSrc<float> dv{g, inv_adt, reinterpret_cast<const float *>(c->dq[0]),
                        reinterpret_cast<const float *>(c->dq[1]), reinterpret_cast<const float *>(c->dq[2])};
-      kern<<<blocks, 128, sm, c->stream>>>(nullptr, c->spec, nlines, c->tw_th, dv);
+      kern<<<blocks, 128, sm, c->stream>>>(nullptr, theta_spec(c), nlines, c->tw_th, dv);
     } else {
       auto kern = k_fft_fwd_s<T, double, true>;
       if ((e = allow_dyn_smem(kern, sm))) return e;
       DivSrc<double> dv{g, inv_adt, c->dq[0], c->dq[1], c->dq[2]};
-      kern<<<blocks, 128, sm, c->stream>>>(nullptr, c->spec, nlines, c->tw_th, dv);
+      kern<<<blocks, 128, sm, c->stream>>>(nullptr, theta_spec(c), nlines, c->tw_th, dv);
     }
   } else if (dir > 0) {
     if ((e = allow_dyn_smem(k_fft_fwd_s<T>, sm))) return e;
-    k_fft_fwd_s<T><<<blocks, 128, sm, c->stream>>>(c->rhs, c->spec, nlines, c->tw_th, DivSrc<double>{});
+    k_fft_fwd_s<T><<<blocks, 128, sm, c->stream>>>(c->rhs, theta_spec(c), nlines, c->tw_th, DivSrc<double>{});
   } else {
     if ((e = allow_dyn_smem(k_fft_bwd_s<T>, sm))) return e;
-    k_fft_bwd_s<T><<<blocks, 128, sm, c->stream>>>(c->spec, c->dph, g, nlines, c->tw_th);
+    k_fft_bwd_s<T><<<blocks, 128, sm, c->stream>>>(theta_spec(c), c->dph, g, nlines, c->tw_th);
   }
   return cudaGetLastError();
 }
@@ -1814,6 +1685,24 @@ static bool slab_tmap(vr_ctx *c, CUtensorMap *tm) {
 
 static cudaError_t radial_solves(vr_ctx *c);
 
+// the lengths with an FFT of their own (2048 along z: radix 2 in shared memory)
+bool fft_theta_length(int n) { return is_pow2(n) && n >= 32 && n <= 1024; }
+bool fft_z_length(int n) { return is_pow2(n) && n >= 32 && n <= 2048; }
+
+// the z transforms of every (slot, r) column
+static cudaError_t run_z(vr_ctx *c, int dir) {
+  const Geo &g = c->geo;
+  if (c->fold_z[0]) {
+    const int M = g.nth * g.nr;
+    LaunchScope ls(c, PK_DCT);
+    return dir > 0 ? fold_run<kFoldZ, +1>(c->spec2, c->spec, c->fold_z[0], g.nz, M, 0, c->nsm, c->stream)
+                   : fold_run<kFoldZ, -1>(c->spec, c->spec2, c->fold_z[1], g.nz, M, 0, c->nsm, c->stream);
+  }
+  bool done = false;
+  cudaError_t e = dct_warp_dispatch(c, dir, &done);
+  return done || e ? e : run_dct<4>(c, dir);
+}
+
 cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk) {
   const Geo &g = c->geo;
   cudaError_t e;
@@ -1825,57 +1714,24 @@ cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk) {
     if ((e = radial_solves(c))) return e;
     return run_slab_bwd(c, stm);
   }
-  // theta forward: rhs (or divq of dq) -> spec
+  // theta forward: rhs (or divq of dq) -> spectrum
   bool done = false;
-  if ((e = fft_warp_dispatch(c, +1, &done, div_rk))) return e;
-  if (done) {
-  } else if (is_pow2(N)) {
-    int lpb = N >= 1024 ? 1 : 1024 / N;
-    size_t sm = sizeof(double) * 2 * lpb * N;
-    if ((e = allow_dyn_smem(k_fft_fwd, sm))) return e;
+  if (c->fold_th[0]) {
     LaunchScope ls(c, PK_FFT);
-    k_fft_fwd<<<(nlines + lpb - 1) / lpb, 256, sm, c->stream>>>(c->rhs, c->spec, N, ilog2(N), lpb, nlines,
-                                                                c->tw_th);
+    e = fold_run<kFoldTh, +1>(c->rhs, theta_spec(c), c->fold_th[0], N, nlines, 0, c->nsm, c->stream);
   } else {
-    LaunchScope ls(c, PK_FFT);
-    k_dft_fwd_direct<<<nlines, 64, 0, c->stream>>>(c->rhs, c->spec, N, nlines);
+    e = fft_warp_dispatch(c, +1, &done, div_rk);
   }
-  if ((e = cudaGetLastError())) return e;
-  // z forward DCT
-  if ((e = dct_warp_dispatch(c, +1, &done))) return e;
-  if (done) {
-  } else if (is_pow2(g.nz)) {
-    if ((e = g.nz <= 1024 ? run_dct<8>(c, +1) : run_dct<4>(c, +1))) return e;
-  } else {
-    LaunchScope ls(c, PK_DCT);
-    k_dct_direct<<<dim3(N, g.nr), 64, sizeof(double) * g.nz, c->stream>>>(c->spec, g, +1);
-  }
-  if ((e = cudaGetLastError())) return e;
+  if (e) return e;
+  if ((e = run_z(c, +1))) return e;
   if ((e = radial_solves(c))) return e;
-  // z backward
-  if ((e = dct_warp_dispatch(c, -1, &done))) return e;
-  if (done) {
-  } else if (is_pow2(g.nz)) {
-    if ((e = g.nz <= 1024 ? run_dct<8>(c, -1) : run_dct<4>(c, -1))) return e;
-  } else {
-    LaunchScope ls(c, PK_DCT);
-    k_dct_direct<<<dim3(N, g.nr), 64, sizeof(double) * g.nz, c->stream>>>(c->spec, g, -1);
-  }
-  if ((e = cudaGetLastError())) return e;
+  if ((e = run_z(c, -1))) return e;
   // theta backward -> dph
-  if ((e = fft_warp_dispatch(c, -1, &done))) return e;
-  if (done) {
-  } else if (is_pow2(N)) {
-    int lpb = N >= 1024 ? 1 : 1024 / N;
-    size_t sm = sizeof(double) * 2 * lpb * N;
-    if ((e = allow_dyn_smem(k_fft_bwd, sm))) return e;
+  if (c->fold_th[0]) {
     LaunchScope ls(c, PK_FFT);
-    k_fft_bwd<<<(nlines + lpb - 1) / lpb, 256, sm, c->stream>>>(c->spec, c->dph, g, ilog2(N), lpb, nlines, c->tw_th);
-  } else {
-    LaunchScope ls(c, PK_FFT);
-    k_dft_bwd_direct<<<nlines, 64, 0, c->stream>>>(c->spec, c->dph, g, nlines);
+    return fold_run<kFoldTh, -1>(theta_spec(c), c->dph, c->fold_th[1], N, nlines, g.nr, c->nsm, c->stream);
   }
-  return cudaGetLastError();
+  return fft_warp_dispatch(c, -1, &done);
 }
 
 // the radial tridiagonal lines of every (theta mode, z mode)
