@@ -1,5 +1,6 @@
-"""The folded transforms (lengths without an FFT) at the lengths where a tile, a
-coefficient stage or the choice of form ends.
+"""The folded transforms (lengths without an FFT) and the axisymmetric direct
+solve, at the lengths where a tile, a coefficient stage or the choice of form
+ends.
 
 Tolerances: a transform of N terms and the substitutions of nr rows each add
 rounding of a few eps per operation, well conditioned except for the
@@ -46,3 +47,42 @@ def test_folded_columns_above_two_ctas_per_sm():
     g = gpu.get("dph")[:, 1:nr + 1, 1:nz + 1]
     r = orc.field("dph")[:, 1:nr + 1, 1:nz + 1]
     assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
+
+
+def _direct(faces, nz, zmax, f):
+    """The direct solve in plain numpy: z cosine products, a Thomas solve per mode."""
+    nr = faces.size - 1
+    dz, rm, dr = zmax / nz, 0.5 * (faces[:-1] + faces[1:]), np.diff(faces)
+    c = faces[1:-1] * dz / np.diff(rm)
+    vol = rm * dr * dz
+    lo, up = -np.concatenate([[0.0], c]) / vol, -np.concatenate([c, [0.0]]) / vol
+    q = np.arange(nz)
+    C = np.cos(np.pi * ((np.outer(q, 2 * q + 1)) % (4 * nz)) / (2 * nz))
+    fh = f @ C.T / nz
+    d = (-(lo + up))[:, None] + 2.0 / dz ** 2 * (1.0 - np.cos(q * np.pi / nz))
+    d[-1, 0] += 2.0 * faces[-1] * dz / dr[-1] / vol[-1]
+    for j in range(1, nr):
+        w = lo[j] / d[j - 1]
+        d[j] -= w * up[j - 1]
+        fh[j] -= w * fh[j - 1]
+    fh[-1] /= d[-1]
+    for j in range(nr - 2, -1, -1):
+        fh[j] = (fh[j] - up[j] * fh[j + 1]) / d[j]
+    C[1:] *= 2.0
+    return fh @ C
+
+
+# z: FFT (32 .. 1024), folded (other lengths up to 1453), full products above;
+# r: below a lane's 16 positions, around a segment of 512
+@pytest.mark.parametrize("nr,nz", [(4, 4), (5, 7), (16, 16), (17, 31), (33, 32), (100, 33), (511, 64), (512, 97),
+                                   (513, 128), (64, 180), (30, 256), (40, 512), (1025, 40), (512, 1024), (20, 1000),
+                                   (18, 1453), (18, 1454), (12, 2048)])
+def test_axisymmetric_direct_solve(nr, nz):
+    import vring_b200 as V
+    from vring_b200.learned import tanh_faces
+    faces = tanh_faces(nr)
+    k = V.K2d(faces, nz, 15.0)
+    f = np.random.default_rng(nr * 10007 + nz).standard_normal((nr, nz))
+    x = k.direct(f)
+    r = _direct(faces, nz, 15.0, f)
+    assert np.abs(x - r).max() <= 1e-11 * np.abs(r).max()

@@ -308,6 +308,10 @@ cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk = nullptr);
 bool poisson_takes_dq(const vr_ctx *c);
 bool fft_theta_length(int n);
 bool fft_z_length(int n);
+// the z transform of ncol columns outside a context (twz: cos, sin of
+// 2 pi n / nz, then of pi k / (2 nz)); lengths dct_columns_length takes
+bool dct_columns_length(int n);
+cudaError_t dct_columns(const double *in, double *out, int ncol, int nz, int dir, const double *twz, cudaStream_t s);
 cudaError_t launch_upsol(vr_ctx *c, const Rk &rk);
 cudaError_t launch_uppres(vr_ctx *c, const Rk &rk);
 cudaError_t launch_upsol_uppres(vr_ctx *c, const Rk &rk);

@@ -37,6 +37,7 @@
 #include <string>
 #include <vector>
 
+#include "vr_fold.cuh"
 #include "vr_internal.cuh"
 #include "vr_learned.cuh"
 
@@ -62,10 +63,12 @@ enum K2dScal {
 // partial-sum slots
 enum K2dPart { PT_A = 0, PT_B, PT_C, PT_D, PT_N };
 // flags: [0] done, [1] iterations
+// how the direct solve's z transforms run
+enum K2dZ { K2D_Z_FFT = 0, K2D_Z_FOLD, K2D_Z_GEMM };
 }  // namespace vr
 
 struct vr_k2d {
-  int nr = 0, nz = 0, n = 0, dev = 0, nb = 0;
+  int nr = 0, nz = 0, n = 0, dev = 0, nb = 0, nsm = 148;
   cudaStream_t stream = nullptr;
   double *coef = nullptr;  // aw, ae, az, vol (per j), then per cell 1/diag(S) and diag(S)^-1/2
   double gam = 0.0;
@@ -77,8 +80,10 @@ struct vr_k2d {
   int cg_parity = 0;        // direction buffer of the next CG iteration being captured
   int bi_parity = 0;        // p and v buffers of the next BiCGSTAB iteration being captured
   int nb_cg = 1;            // grid of the CG iteration kernels
-  // direct solve: forward / inverse z transforms (nz x nz, row-major [kz][k]
-  // and [k][kz]) and the radial Thomas factorisation per z mode
+  // direct solve: the z transforms' tables (dct_f, dct_i: folded matrices, or
+  // nz x nz ones, row-major [kz][k] and [k][kz], for long lines; or the FFT's
+  // twiddles in dct_f alone) and the radial Thomas factorisation per z mode
+  int zform = 0;  // K2D_Z_*
   double *dct_f = nullptr, *dct_i = nullptr, *tlo = nullptr, *tup = nullptr, *tib = nullptr;
   double *tmp = nullptr;
   cudaGraphExec_t graph[5] = {};  // CG, Jacobi CG, BiCGSTAB, learned FCG, Jacobi-only FCG
@@ -737,23 +742,104 @@ __global__ void __launch_bounds__(256) k2d_gemm_abt(int m, int n, int kk, const 
     }
 }
 
-// one thread per z mode: the radial tridiagonal of that mode (contiguous in j)
-__global__ void k2d_radial_thomas(int nr, int nz, double *__restrict__ a, const double *__restrict__ lo,
-                                  const double *__restrict__ up, const double *__restrict__ ib) {
-  const int kz = blockIdx.x * blockDim.x + threadIdx.x;
+// The radial tridiagonal of each z mode, a warp per mode (contiguous in j).
+// The pivots are fixed, so both substitutions are first-order recurrences: a
+// lane composes the affine map of its kRadCH positions, a shuffle scan chains
+// the maps, and the lane re-runs its positions from its exact input.  The
+// line and its pivots come in with lanes along j and are re-read by chunk
+// (rows of kRadCH padded to an odd stride); longer lines go in segments with a
+// carry.  512 x 1024 (us): one thread per mode, its loads a line apart, 575;
+// this form 7.4.
+constexpr int kRadCH = 16, kRadSeg = 32 * kRadCH, kRadLD = kRadSeg + 32, kRadWarps = 4;
+
+__global__ void __launch_bounds__(32 * kRadWarps) k2d_radial_thomas(int nr, int nz, double *__restrict__ a,
+                                                                  const double *__restrict__ lo,
+                                                                  const double *__restrict__ up,
+                                                                  const double *__restrict__ ib) {
+  constexpr int CH = kRadCH, SEG = kRadSeg, LD = kRadLD;
+  extern __shared__ double sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kz = blockIdx.x * kRadWarps + warp;
+  double *sx = sm + (size_t)warp * 4 * LD, *sp = sx + LD, *sl = sp + LD, *su = sl + LD;
   if (kz >= nz) return;
   double *x = a + (size_t)nr * kz;
   const double *piv = ib + (size_t)nr * kz;
-  double g = x[0] * piv[0];
-  x[0] = g;
-  for (int j = 1; j < nr; j++) {
-    g = (x[j] - lo[j] * g) * piv[j];
-    x[j] = g;
+  const int nseg = (nr + SEG - 1) / SEG;
+  auto at = [](int j) { return j + (j / CH); };
+  const int o = lane * (CH + 1);
+  auto load = [&](int j0) {  // positions past the line: pivot 0, so they carry 0
+    __syncwarp();
+    for (int j = lane; j < SEG; j += 32) {
+      if (j0 + j < nr) {
+        cp_async8(sx + at(j), x + j0 + j);
+        cp_async8(sp + at(j), piv + j0 + j);
+        cp_async8(sl + at(j), lo + j0 + j);
+        cp_async8(su + at(j), up + j0 + j);
+      } else {
+        sx[at(j)] = sp[at(j)] = sl[at(j)] = su[at(j)] = 0.0;
+      }
+    }
+    cp_async_wait_all();
+    __syncwarp();
+  };
+  double carry = 0.0;
+  for (int s = 0; s < nseg; s++) {
+    load(s * SEG);
+    double m = 1.0, c = 0.0;
+#pragma unroll
+    for (int u = 0; u < CH; u++) {
+      const double p = sp[o + u], f = -sl[o + u] * p;
+      c = fma(f, c, sx[o + u] * p);
+      m *= f;
+    }
+    // (m, c) of lanes 0 .. lane; the input of this lane's chunk
+    for (int d = 1; d < 32; d <<= 1) {
+      const double mp = __shfl_up_sync(0xffffffffu, m, d), cp = __shfl_up_sync(0xffffffffu, c, d);
+      if (lane >= d) {
+        c = fma(m, cp, c);
+        m *= mp;
+      }
+    }
+    const double mp = __shfl_up_sync(0xffffffffu, m, 1), cp = __shfl_up_sync(0xffffffffu, c, 1);
+    double g = lane == 0 ? carry : fma(mp, carry, cp);
+#pragma unroll
+    for (int u = 0; u < CH; u++) {
+      g = (sx[o + u] - sl[o + u] * g) * sp[o + u];
+      sx[o + u] = g;
+    }
+    carry = __shfl_sync(0xffffffffu, g, 31);
+    if (nseg > 1) {
+      __syncwarp();
+      for (int j = lane; j < SEG && s * SEG + j < nr; j += 32) x[s * SEG + j] = sx[at(j)];
+    }
   }
-  double xn = x[nr - 1];
-  for (int j = nr - 2; j >= 0; j--) {
-    xn = x[j] - up[j] * piv[j] * xn;
-    x[j] = xn;
+  carry = 0.0;
+  for (int s = nseg - 1; s >= 0; s--) {
+    if (nseg > 1) load(s * SEG);
+    double m = 1.0, c = 0.0;
+#pragma unroll
+    for (int u = CH - 1; u >= 0; u--) {
+      const double f = -su[o + u] * sp[o + u];
+      c = fma(f, c, sx[o + u]);
+      m *= f;
+    }
+    for (int d = 1; d < 32; d <<= 1) {
+      const double mp = __shfl_down_sync(0xffffffffu, m, d), cp = __shfl_down_sync(0xffffffffu, c, d);
+      if (lane + d < 32) {
+        c = fma(m, cp, c);
+        m *= mp;
+      }
+    }
+    const double mp = __shfl_down_sync(0xffffffffu, m, 1), cp = __shfl_down_sync(0xffffffffu, c, 1);
+    double xn = lane == 31 ? carry : fma(mp, carry, cp);
+#pragma unroll
+    for (int u = CH - 1; u >= 0; u--) {
+      xn = sx[o + u] - su[o + u] * sp[o + u] * xn;
+      sx[o + u] = xn;
+    }
+    carry = __shfl_sync(0xffffffffu, xn, 0);
+    __syncwarp();
+    for (int j = lane; j < SEG && s * SEG + j < nr; j += 32) x[s * SEG + j] = sx[at(j)];
   }
 }
 
@@ -800,8 +886,8 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
   k->h_faces.assign(f, f + nr + 1);
   if (cudaSetDevice(k->dev) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&k->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VR_ERR_CUDA);
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, k->dev);
+  cudaDeviceGetAttribute(&k->nsm, cudaDevAttrMultiProcessorCount, k->dev);
+  const int nsm = k->nsm;
   k->nb = std::min(kK2dMaxBlocks, std::max(1, std::min(2 * nsm, (k->n + kK2dThreads - 1) / kK2dThreads)));
   k->nb_cg = std::min(kK2dMaxBlocks,
                       std::max(1, std::min(kK2dCgBlocksPerSm * nsm, (k->n + kK2dThreads - 1) / kK2dThreads)));
@@ -834,15 +920,34 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
       coef[4 * nr + j + (size_t)nr * kk] = 1.0 / dg;
       coef[4 * nr + (size_t)nr * nz + j + (size_t)nr * kk] = 1.0 / std::sqrt(dg);
     }
-  // direct solve tables: DCT-II scaled 1/(2 nz) (REDFT10) and DCT-III (REDFT01)
+  // z transforms of the direct solve: DCT-II scaled 1/(2 nz) (REDFT10) and
+  // DCT-III (REDFT01), by FFT, as folded products, or as full products where
+  // the folded form's columns do not fit shared memory
   const double pi = std::acos(-1.0);
-  std::vector<double> cf((size_t)nz * nz), ci((size_t)nz * nz);
-  for (int q = 0; q < nz; q++)
-    for (int kk = 0; kk < nz; kk++) {
-      const double c = std::cos(pi * q * (2.0 * kk + 1.0) / (2.0 * nz));
-      cf[(size_t)q * nz + kk] = c / nz;                 // [kz][k]
-      ci[(size_t)kk * nz + q] = q == 0 ? 1.0 : 2.0 * c;  // [k][kz]
+  std::vector<double> cf, ci;
+  if (dct_columns_length(nz)) {
+    k->zform = K2D_Z_FFT;
+    cf.resize((size_t)4 * nz);
+    for (int q = 0; q < nz; q++) {
+      cf[2 * q] = std::cos(2.0 * pi * q / nz);
+      cf[2 * q + 1] = std::sin(2.0 * pi * q / nz);
+      cf[2 * nz + 2 * q] = std::cos(pi * q / (2.0 * nz));
+      cf[2 * nz + 2 * q + 1] = std::sin(pi * q / (2.0 * nz));
     }
+  } else if (fold_fits(nz)) {
+    k->zform = K2D_Z_FOLD;
+    fold_tables(kFoldZ, nz, cf, ci);
+  } else {
+    k->zform = K2D_Z_GEMM;
+    cf.resize((size_t)nz * nz);
+    ci.resize((size_t)nz * nz);
+    for (int q = 0; q < nz; q++)
+      for (int kk = 0; kk < nz; kk++) {
+        const double c = std::cos(pi * q * (2.0 * kk + 1.0) / (2.0 * nz));
+        cf[(size_t)q * nz + kk] = c / nz;                  // [kz][k]
+        ci[(size_t)kk * nz + q] = q == 0 ? 1.0 : 2.0 * c;  // [k][kz]
+      }
+  }
   // radial Thomas per z mode on K rows: lo = -aw/V, up = -ae/V
   std::vector<double> lo(nr), up(nr), ib((size_t)nr * nz);
   for (int j = 0; j < nr; j++) {
@@ -870,7 +975,7 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
   if (cudaMalloc(&k->cnt, sizeof(unsigned) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMemset(k->cnt, 0, sizeof(unsigned) * 4) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaMalloc(&k->dct_f, sizeof(double) * cf.size()) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMalloc(&k->dct_i, sizeof(double) * ci.size()) != cudaSuccess) return fail(VR_ERR_OOM);
+  if (!ci.empty() && cudaMalloc(&k->dct_i, sizeof(double) * ci.size()) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->tlo, sizeof(double) * nr) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->tup, sizeof(double) * nr) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->tib, sizeof(double) * ib.size()) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -880,7 +985,8 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
     const std::vector<double> *h;
   } up_[] = {{k->coef, &coef}, {k->dct_f, &cf}, {k->dct_i, &ci}, {k->tlo, &lo}, {k->tup, &up}, {k->tib, &ib}};
   for (auto &u : up_)
-    if (cudaMemcpy(u.d, u.h->data(), sizeof(double) * u.h->size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (!u.h->empty() &&
+        cudaMemcpy(u.d, u.h->data(), sizeof(double) * u.h->size(), cudaMemcpyHostToDevice) != cudaSuccess)
       return fail(VR_ERR_CUDA);
   if (cudaMemset(k->part, 0, sizeof(double) * PT_N * kK2dMaxBlocks) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaMemset(k->flags, 0, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_CUDA);
@@ -958,13 +1064,24 @@ extern "C" int vr_k2d_apply(vr_k2d *k, const double *x, double *y) {
 // direct solve K x = f on device arrays (x may alias f)
 static cudaError_t k2d_direct_dev(vr_k2d *k, const double *f, double *x) {
   const int nr = k->nr, nz = k->nz;
-  dim3 g1((nr + 63) / 64, (nz + 63) / 64);
-  // fh(j, kz) = sum_k f(j, k) cf[kz][k]
-  k2d_gemm_abt<<<g1, 256, 0, k->stream>>>(nr, nz, nz, f, k->dct_f, k->tmp);
-  k2d_radial_thomas<<<(nz + 127) / 128, 128, 0, k->stream>>>(nr, nz, k->tmp, k->tlo, k->tup, k->tib);
-  // x(j, k) = sum_kz sol(j, kz) ci[k][kz]
-  k2d_gemm_abt<<<g1, 256, 0, k->stream>>>(nr, nz, nz, k->tmp, k->dct_i, x);
-  return cudaGetLastError();
+  // fh(j, kz) = sum_k f(j, k) cf[kz][k], or x(j, k) = sum_kz sol(j, kz) ci[k][kz]
+  auto transform = [&](const double *in, double *out, bool fwd) {
+    if (k->zform == K2D_Z_FFT) return dct_columns(in, out, nr, nz, fwd ? 1 : -1, k->dct_f, k->stream);
+    if (k->zform == K2D_Z_FOLD)
+      return fwd ? fold_run<kFoldZ, +1>(in, out, k->dct_f, nz, nr, 0, k->nsm, k->stream)
+                 : fold_run<kFoldZ, -1>(in, out, k->dct_i, nz, nr, 0, k->nsm, k->stream);
+    k2d_gemm_abt<<<dim3((nr + 63) / 64, (nz + 63) / 64), 256, 0, k->stream>>>(nr, nz, nz, in,
+                                                                            fwd ? k->dct_f : k->dct_i, out);
+    return cudaGetLastError();
+  };
+  cudaError_t e = transform(f, k->tmp, true);
+  if (e) return e;
+  const size_t sm = sizeof(double) * kRadWarps * 4 * kRadLD;
+  if ((e = allow_dyn_smem(k2d_radial_thomas, sm))) return e;
+  k2d_radial_thomas<<<(nz + kRadWarps - 1) / kRadWarps, 32 * kRadWarps, sm, k->stream>>>(nr, nz, k->tmp, k->tlo, k->tup,
+                                                                                         k->tib);
+  if ((e = cudaGetLastError())) return e;
+  return transform(k->tmp, x, false);
 }
 
 extern "C" int vr_k2d_direct_dev(vr_k2d *k, const double *f, double *x) {

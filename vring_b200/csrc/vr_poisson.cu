@@ -632,7 +632,7 @@ __device__ __forceinline__ void warp_fft512(double (&re)[16], double (&im)[16], 
 // as one complex sequence (Makhoul's even/odd reordering turns the DCT into
 // an N-point FFT plus a quarter-wave shift).
 template <int E, int LT>
-__global__ void __launch_bounds__(LT * 16) k_dct_w(double *__restrict__ a, Geo g, int dir,
+__global__ void __launch_bounds__(LT * 16) k_dct_w(const double *in, double *out, Geo g, int dir,
                                                    const double *__restrict__ twz) {
   constexpr int N = 32 * E, LOGN = Log2N<E>::v, LD = LT + 1;
   // row k of the tile starts at k*LD + k/16: the bit-reversed scatter of the
@@ -643,7 +643,8 @@ __global__ void __launch_bounds__(LT * 16) k_dct_w(double *__restrict__ a, Geo g
   const int i0 = blockIdx.x * LT, j = blockIdx.y;  // j 0-based radial index
   const int nl = min(LT, g.nth - i0);
   const size_t s2 = (size_t)g.nth * g.nr;
-  double *base = a + i0 + (size_t)g.nth * j;
+  const double *base = in + i0 + (size_t)g.nth * j;
+  double *dest = out + i0 + (size_t)g.nth * j;  // in place when in == out: the CTA holds its whole columns
   for (int idx = threadIdx.x; idx < N * LT; idx += LT * 16) {
     int k = idx / LT, l = idx % LT;
     if (l < nl)
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(LT * 16) k_dct_w(double *__restrict__ a, Geo g
   __syncthreads();
   for (int idx = threadIdx.x; idx < N * LT; idx += LT * 16) {
     int k = idx / LT, l = idx % LT;
-    if (l < nl) base[l + s2 * k] = tile[row(k) + l];
+    if (l < nl) dest[l + s2 * k] = tile[row(k) + l];
   }
 }
 
@@ -1605,8 +1606,38 @@ static cudaError_t run_dct_w(vr_ctx *c, int dir) {
   cudaError_t e = allow_dyn_smem(k_dct_w<E, LT>, sm);
   if (e) return e;
   LaunchScope ls(c, PK_DCT);
-  k_dct_w<E, LT><<<dim3((g.nth + LT - 1) / LT, g.nr), LT * 16, sm, c->stream>>>(c->spec, g, dir, c->tw_z);
+  k_dct_w<E, LT><<<dim3((g.nth + LT - 1) / LT, g.nr), LT * 16, sm, c->stream>>>(c->spec, c->spec, g, dir, c->tw_z);
   return cudaGetLastError();
+}
+
+// The z transform of ncol columns (entry k of column c at in[c + ncol k]) for
+// the axisymmetric direct solve, whose few columns (its radial cells) want
+// small tiles: 4 columns per CTA put 512 columns on 128 CTAs.  NotSupported
+// for lengths that have no FFT here.
+template <int E>
+static cudaError_t dct_cols(const double *in, double *out, int ncol, int dir, const double *twz, cudaStream_t s) {
+  constexpr int N = 32 * E, LT = 4;
+  Geo g{};
+  g.nth = ncol;
+  g.nr = 1;
+  g.nz = N;
+  const size_t sm = sizeof(double) * ((size_t)N * (LT + 1) + N / 16 + 1);
+  cudaError_t e = allow_dyn_smem(k_dct_w<E, LT>, sm);
+  if (e) return e;
+  k_dct_w<E, LT><<<dim3((ncol + LT - 1) / LT, 1), LT * 16, sm, s>>>(in, out, g, dir, twz);
+  return cudaGetLastError();
+}
+bool dct_columns_length(int n) { return is_pow2(n) && n >= 32 && n <= 1024; }
+cudaError_t dct_columns(const double *in, double *out, int ncol, int nz, int dir, const double *twz, cudaStream_t s) {
+  switch (nz) {
+    case 32: return dct_cols<1>(in, out, ncol, dir, twz, s);
+    case 64: return dct_cols<2>(in, out, ncol, dir, twz, s);
+    case 128: return dct_cols<4>(in, out, ncol, dir, twz, s);
+    case 256: return dct_cols<8>(in, out, ncol, dir, twz, s);
+    case 512: return dct_cols<16>(in, out, ncol, dir, twz, s);
+    case 1024: return dct_cols<32>(in, out, ncol, dir, twz, s);
+    default: return cudaErrorNotSupported;
+  }
 }
 
 // the TMA-streamed 512-point transform; NotSupported when the shape or the
