@@ -87,6 +87,29 @@ def test_gradients_match_oracle(pool):
     net.close()
 
 
+# channels that fill 16-channel tiles partly, grids beside the gradient kernels'
+# patches (33 x 16 and 12 x 64 pixels, 32 x 16 and 8 x 16 tiles), levels of one pixel
+@pytest.mark.parametrize("nr,nz,ch,pool", [(8, 8, (8, 8, 8, 8), 2), (64, 64, (8, 16, 24, 64), 4),
+                                           (72, 40, (24, 40, 16, 64), 2), (32, 136, (64, 64, 64, 64), 2),
+                                           (264, 104, (16, 8, 48, 40), 2), (192, 320, (16, 32, 48, 64), 4)])
+def test_gradients_at_tile_edges(nr, nz, ch, pool):
+    import vring_b200 as V
+    from oracle import unet_ref as U
+    net = V.UNet(nr, nz, ch, seed=8, pool=pool)
+    w = net.get_params()
+    rng = np.random.default_rng(nr + nz)
+    x, g = rng.standard_normal((nr, nz)), rng.standard_normal((nr, nz))
+    dw, dx = net.backward(x, g)
+    dwo, dxo = U.backward(w, ch, x, g, F=pool)
+    off = 0
+    for i, (ci, co, _) in enumerate(U.layers(ch) + [(ch[0], 1, 0)]):
+        n = ci * co * (9 if i < 14 else 1)
+        assert _rel(dw[off:off + n], dwo[off:off + n]) <= 5e-3, i
+        off += n
+    assert _rel(dx, dxo) <= 5e-3
+    net.close()
+
+
 def test_training_reduces_the_loss():
     import torch
     import vring_b200 as V

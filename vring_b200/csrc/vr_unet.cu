@@ -15,13 +15,11 @@
 //   e_l (upsampled channels first), two 3x3 convs (-> c_l -> c_l);
 //   head: 1x1 conv c_0 -> 1, FP32 output.
 //
-// Convolutions (forward and data gradient) run one output pixel per thread
-// over 16 x 16 pixel tiles: the input tile (18 x 18 pixels x 16 channels) and
-// the weights of those 16 input channels are staged in shared memory as FP32,
-// and each thread keeps all of its pixel's output channels in registers.  The
-// data gradient is the same convolution with the weights flipped and
-// transposed ([cin][8 - tap][cout]).  Weight gradients reduce over pixels per
-// 16 x 16 (cout, cin) tile and are added with FP32 atomics.
+// The forward convolutions run on the tensor cores (k_conv3_tc) or, by flag, on
+// the CUDA cores (k_conv3).  The gradients are FP32 throughout, on the CUDA
+// cores: the data gradient is the convolution with the flipped weights
+// (k_dgrad3), the weight gradient an outer product per pixel (k_wgrad3), added
+// with FP32 atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -47,15 +45,15 @@ struct UnetLayer {
 }  // namespace vr
 
 struct vr_unet {
-  int nr = 0, nz = 0, dev = 0;
+  int nr = 0, nz = 0, dev = 0, nsm = 148;
   int ch[4] = {};
   int pool = 2;  // pooling factor between levels
   std::string err;
   vr::UnetLayer L[vr::kUnetLayers];
   size_t nparam = 0;
-  // parameters: FP32 master, BF16 copy, FP32 copy for the kernels, flipped
-  // copy for the data gradient, gradient, Adam moments
-  float *w32 = nullptr, *wk = nullptr, *wflip = nullptr, *gw = nullptr, *m1 = nullptr, *m2 = nullptr;
+  // parameters: FP32 master, BF16 copy, FP32 copy for the kernels, gradient,
+  // Adam moments
+  float *w32 = nullptr, *wk = nullptr, *gw = nullptr, *m1 = nullptr, *m2 = nullptr;
   __nv_bfloat16 *w16 = nullptr;
   __nv_bfloat16 *wpk = nullptr;  // per 3x3 layer [nout][9][cinp] BF16, zero padded (tensor-core form)
   size_t wpk_off[14] = {};
@@ -75,24 +73,12 @@ struct vr_unet {
 
 namespace vr {
 
-__device__ __forceinline__ float tof(float v) { return v; }
 __device__ __forceinline__ float tof(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <class T>
-__device__ __forceinline__ T fromf(float v);
-template <>
-__device__ __forceinline__ float fromf<float>(float v) {
-  return v;
-}
-template <>
-__device__ __forceinline__ __nv_bfloat16 fromf<__nv_bfloat16>(float v) {
-  return __float2bfloat16_rn(v);
-}
 
-// out[p][co] (=|+=) sum_{tap, ci} in[p + off(tap)][ci] w[co][tap][ci]
-template <class TI, class TO, int CO>
-__global__ void __launch_bounds__(256) k_conv3(const TI *__restrict__ in, int H, int W, int cin,
-                                             const float *__restrict__ w, int cout, TO *__restrict__ out,
-                                             int accumulate) {
+// out[p][co] = sum_{tap, ci} in[p + off(tap)][ci] w[co][tap][ci]
+template <int CO>
+__global__ void __launch_bounds__(256) k_conv3(const __nv_bfloat16 *__restrict__ in, int H, int W, int cin,
+                                             const float *__restrict__ w, int cout, __nv_bfloat16 *__restrict__ out) {
   extern __shared__ float sm[];
   float *tin = sm;                 // [18*18][17]
   float *tw = sm + 18 * 18 * 17;   // [CO][9][16]
@@ -153,10 +139,10 @@ __global__ void __launch_bounds__(256) k_conv3(const TI *__restrict__ in, int H,
   }
   const int gj = j0 + tj, gk = k0 + tk;
   if (gj < H && gk < W) {
-    TO *op = out + ((size_t)gj + (size_t)H * gk) * cout;
+    __nv_bfloat16 *op = out + ((size_t)gj + (size_t)H * gk) * cout;
 #pragma unroll
     for (int co = 0; co < CO; co++)
-      if (co < cout) op[co] = fromf<TO>(accumulate ? acc[co] + tof(op[co]) : acc[co]);
+      if (co < cout) op[co] = __float2bfloat16_rn(acc[co]);
   }
 }
 
@@ -316,48 +302,262 @@ __global__ void k_wpack(const float *__restrict__ w, int cin, int cout, int cinp
   }
 }
 
-// dw[co][tap][ci] += sum_p dout[p][co] in[p + off(tap)][ci]; one block per
-// (16-channel cin group, 16-channel cout group, pixel range)
-template <class TI>
-__global__ void __launch_bounds__(256) k_wgrad3(const float *__restrict__ dout, int H, int W, int cout,
-                                              const TI *__restrict__ in, int cin, float *__restrict__ dw,
-                                              int pix_per_block) {
-  __shared__ float sd[32][17];       // dout rows of 32 pixels
-  __shared__ float si[9][32][17];    // in at the 9 taps of those pixels
-  const int ci = threadIdx.x & 15, co = threadIdx.x >> 4;
-  const int ci0 = blockIdx.x * 16, co0 = blockIdx.y * 16;
-  const int P = H * W;
-  const int pbeg = blockIdx.z * pix_per_block, pend = min(P, pbeg + pix_per_block);
-  float acc[9];
-#pragma unroll
-  for (int t = 0; t < 9; t++) acc[t] = 0.f;
-  for (int pb = pbeg; pb < pend; pb += 32) {
-    for (int e = threadIdx.x; e < 32 * 16; e += 256) {
-      const int pl = e >> 4, c = e & 15, p = pb + pl;
-      sd[pl][c] = (p < pend && co0 + c < cout) ? dout[(size_t)p * cout + co0 + c] : 0.f;
-    }
-    for (int e = threadIdx.x; e < 9 * 32 * 16; e += 256) {
-      const int c = e & 15, pl = (e >> 4) & 31, t = e >> 9;
-      const int p = pb + pl;
-      float v = 0.f;
-      if (p < pend && ci0 + c < cin) {
-        const int j = p % H + t / 3 - 1, k = p / H + t % 3 - 1;
-        if (j >= 0 && j < H && k >= 0 && k < W) v = tof(in[((size_t)j + (size_t)H * k) * cin + ci0 + c]);
+// A 3x3 layer's input: channels [0, ca) from a and, when b is set, [ca, ca + cb)
+// from b at full resolution with a one level down (nearest upsampling by F):
+// the decoder's concatenation where it lies
+struct ConvIn {
+  const __nv_bfloat16 *a;
+  int ca;
+  const __nv_bfloat16 *b;
+  int cb, F;
+  __device__ __forceinline__ const __nv_bfloat16 *at(int j, int k, int H, int ci) const {
+    if (!b) return a + ((size_t)j + (size_t)H * k) * ca + ci;
+    if (ci < ca) return a + ((size_t)(j / F) + (size_t)(H / F) * (k / F)) * ca + ci;
+    return b + ((size_t)j + (size_t)H * k) * cb + (ci - ca);
+  }
+};
+
+// dw[co][tap][ci] += sum_p dout[p][co] in[p + off(tap)][ci]: an outer product
+// per pixel, summed over the grid.  What bounds it is the FP32 pipe (6.1 G
+// multiply-adds per sample at 512 x 1024), as long as the sums stay in
+// registers and shared memory feeds them seldom: a thread holds 4 output x CIT
+// input channels x 9 taps (CIT 4: 144 sums) and walks a line of pixels along
+// r, so of the 3 x 3 input values only the three of the new column are loaded
+// per pixel, with one load of the 4 gradients.  A CTA takes 16 output x 16
+// input channels (CIT 1, the first layer: 16 x 1) of patches of R x NS
+// pixels, one of its NS threads of equal channels per line, brought in by
+// 16-byte asynchronous copies two patches ahead of each other (zero outside the
+// grid).  It walks every gridDim.y-th patch and only then adds its threads'
+// sums (shuffle, shared memory) and the result to dw by FP32 atomics.
+// us at 512 x 1024, against one (output, input) pair per thread and ten
+// scalar loads per nine multiply-adds: WGTAB.
+template <int CIT>
+struct WgShape {
+  static constexpr int OT = CIT == 4 ? 16 : 4;  // threads that share a line
+  static constexpr int NS = 256 / OT;           // lines of a patch
+  static constexpr int R = CIT == 4 ? 33 : 12;  // pixels of a line (a multiple of the window's 3 phases)
+  static constexpr int IC = CIT == 4 ? 16 : 1;  // input channels of a CTA
+  // floats between lines of the gradient tile: 16 beyond the line, so that two lines fill the banks
+  static constexpr int DP = R * 16 + 16;
+  static constexpr int IN_BYTES = CIT == 4 ? (NS + 2) * (R + 2) * 32 : (NS + 2) * (R + 3) * 4;
+  static constexpr int STAGE = ((IN_BYTES + 15) & ~15) + NS * DP * 4;
+};
+
+template <int CIT>
+__global__ void __launch_bounds__(256, 1) k_wgrad3(const float *__restrict__ dout, int H, int W, int cout, ConvIn in,
+                                                 int cin, float *__restrict__ dw, int npr, int npatch) {
+  using S = WgShape<CIT>;
+  constexpr int NS = S::NS, R = S::R, DP = S::DP, NA = 4 * 9 * CIT;
+  extern __shared__ uint8_t smraw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nci = (cin + S::IC - 1) / S::IC;
+  const int ci0 = (blockIdx.x % nci) * S::IC, co0 = (blockIdx.x / nci) * 16;
+  const int cig = CIT == 4 ? tid & 3 : 0, cog = CIT == 4 ? (tid >> 2) & 3 : tid & 3, line = tid / S::OT;
+  auto stage_in = [&](int s) { return smraw + (size_t)s * S::STAGE; };
+  auto stage_d = [&](int s) { return (float *)(smraw + (size_t)s * S::STAGE + ((S::IN_BYTES + 15) & ~15)); };
+  auto fetch = [&](int patch, int s) {
+    const int j0 = (patch % npr) * R, k0 = (patch / npr) * NS;
+    if (CIT == 4) {
+      uint8_t *si = stage_in(s);
+      for (int e = tid; e < (NS + 2) * (R + 2) * 2; e += 256) {
+        const int q = e & 1, pix = e >> 1, hr = pix % (R + 2), hz = pix / (R + 2);
+        const int j = j0 + hr - 1, k = k0 + hz - 1, ci = ci0 + 8 * q;
+        const bool live = j >= 0 && j < H && k >= 0 && k < W && ci < cin;
+        cp_async16(si + (size_t)e * 16, live ? in.at(j, k, H, ci) : in.a, live ? 16u : 0u);
       }
-      si[t][pl][c] = v;
+    } else {  // one channel: plain loads, widened
+      float *si = (float *)stage_in(s);
+      for (int e = tid; e < (NS + 2) * (R + 2); e += 256) {
+        const int hr = e % (R + 2), hz = e / (R + 2), j = j0 + hr - 1, k = k0 + hz - 1;
+        const bool live = j >= 0 && j < H && k >= 0 && k < W;
+        si[hz * (R + 3) + hr] = live ? tof(*in.at(j, k, H, 0)) : 0.f;
+      }
+    }
+    float *sd = stage_d(s);
+    for (int e = tid; e < NS * R * 4; e += 256) {
+      const int q = e & 3, pix = e >> 2, hr = pix % R, hz = pix / R;
+      const int j = j0 + hr, k = k0 + hz, co = co0 + 4 * q;
+      const bool live = j < H && k < W && co < cout;
+      cp_async16(sd + hz * DP + hr * 16 + 4 * q, live ? dout + ((size_t)j + (size_t)H * k) * cout + co : dout,
+                 live ? 16u : 0u);
+    }
+    cp_async_commit();
+  };
+  float acc[4][9][CIT];
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+      for (int c = 0; c < CIT; c++) acc[a][t][c] = 0.f;
+  int s = 0, p = blockIdx.y;
+  if (p < npatch) fetch(p, 0);
+  for (; p < npatch; p += gridDim.y, s ^= 1) {
+    const int nx = p + gridDim.y;
+    if (nx < npatch) {
+      fetch(nx, s ^ 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
     }
     __syncthreads();
-#pragma unroll 4
-    for (int pl = 0; pl < 32; pl++) {
-      const float d = sd[pl][co];
+    const float *sd = stage_d(s) + line * DP + 4 * cog;
+    // column hr (0 .. R + 1) of the halo rows line .. line + 2
+    float w[3][3][CIT];  // [column mod 3][dz]
+    auto column = [&](int hr, float (&v)[3][CIT]) {
 #pragma unroll
-      for (int t = 0; t < 9; t++) acc[t] = fmaf(d, si[t][pl][ci], acc[t]);
+      for (int dz = 0; dz < 3; dz++) {
+        if constexpr (CIT == 4) {
+          const uint2 u = *reinterpret_cast<const uint2 *>(stage_in(s) + ((size_t)(line + dz) * (R + 2) + hr) * 32 +
+                                                           8 * cig);
+          v[dz][0] = __uint_as_float(u.x << 16);
+          v[dz][1] = __uint_as_float(u.x & 0xffff0000u);
+          v[dz][2] = __uint_as_float(u.y << 16);
+          v[dz][3] = __uint_as_float(u.y & 0xffff0000u);
+        } else {
+          v[dz][0] = ((const float *)stage_in(s))[(line + dz) * (R + 3) + hr];
+        }
+      }
+    };
+    column(0, w[0]);
+    column(1, w[1]);
+    const int rend = min(R, H - (p % npr) * R);  // pixels of the line inside the grid
+#pragma unroll 1
+    for (int r = 0; r < rend; r += 3) {
+#pragma unroll
+      for (int u = 0; u < 3; u++) {  // pixel r + u; past the line its gradient is 0
+        column(r + u + 2, w[(u + 2) % 3]);
+        const float4 d = *reinterpret_cast<const float4 *>(sd + (r + u) * 16);
+        const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int dr = 0; dr < 3; dr++)
+#pragma unroll
+          for (int dz = 0; dz < 3; dz++)
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+              for (int c = 0; c < CIT; c++)
+                acc[a][3 * dr + dz][c] = fmaf(dd[a], w[(u + dr) % 3][dz][c], acc[a][3 * dr + dz][c]);
+      }
+    }
+    __syncthreads();  // the stage is refilled
+  }
+  // the lines' sums: lanes of a warp that differ in the line, then the warps
+  float *red = (float *)smraw;  // [warp][sum][OT]
+  constexpr int OT = S::OT;
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+      for (int c = 0; c < CIT; c++) {
+        float v = acc[a][t][c];
+#pragma unroll
+        for (int o = 16; o >= OT; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane < OT) red[((size_t)warp * NA + (a * 9 + t) * CIT + c) * OT + lane] = v;
+      }
+  __syncthreads();
+  for (int e = tid; e < NA * OT; e += 256) {
+    float v = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) v += red[(size_t)q * NA * OT + e];
+    const int l = e % OT, i = e / OT, c = i % CIT, t = (i / CIT) % 9, a = i / (CIT * 9);
+    const int ci = ci0 + (CIT == 4 ? 4 * (l & 3) : 0) + c, co = co0 + 4 * (CIT == 4 ? l >> 2 : l) + a;
+    if (ci < cin && co < cout) atomicAdd(dw + ((size_t)co * 9 + t) * cin + ci, v);
+  }
+}
+
+// Data gradient: gin[p][ci] = sum_{tap, co} gout[p - off(tap)][co] w[co][tap][ci],
+// the convolution with the flipped weights w[co][8 - tap], in FP32.
+// Bound by the FP32 pipe once the sums sit in registers: a thread holds PX
+// pixels along r x 8 channels; per output channel and row of taps it loads
+// PX + 2 gradients (the channel's plane in shared memory, 16 bytes at a time)
+// and 24 weights that its whole warp shares, for 24 PX multiply-adds.  A CTA
+// takes 4 PX x 16 pixels x up to 48 channels (64 threads per 8 channels); the
+// gradients of 16 channels at a time come from memory channels-last and are
+// stored as planes.  PX = 2 where PX = 8 would leave SMs idle (the coarse
+// levels).  us at 512 x 1024, against one pixel x all channels per thread:
+// DGTAB.
+template <int PX>
+__global__ void __launch_bounds__(384) k_dgrad3(const float *__restrict__ gout, int H, int W, int cout,
+                                              const float *__restrict__ w, int cin, float *__restrict__ gin) {
+  constexpr int KC = 16, TR = 4 * PX, PITCH = TR + 4, ZR = 18, PLANE = ZR * PITCH;
+  extern __shared__ float smf[];
+  float *sg = smf;                // [KC][ZR][PITCH]: pixel r at column r + 1
+  float *sw = smf + KC * PLANE;   // [KC][dz][dr][channels of the CTA]
+  const int tid = threadIdx.x, nth = blockDim.x, nch = nth / 8;
+  const int strip = tid & 63, grp = tid >> 6, ci0 = blockIdx.z * nch;
+  const int sr = (strip & 3) * PX, sz = strip >> 2;
+  const int j0 = blockIdx.x * TR, k0 = blockIdx.y * 16;
+  float acc[PX][8];
+#pragma unroll
+  for (int p = 0; p < PX; p++)
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[p][c] = 0.f;
+  for (int c0 = 0; c0 < cout; c0 += KC) {
+    const int kc = min(KC, cout - c0);  // a multiple of 8
+    for (int e = tid; e < (TR + 2) * ZR * (KC / 4); e += nth) {
+      const int pix = e % ((TR + 2) * ZR), q = e / ((TR + 2) * ZR), hr = pix % (TR + 2), hz = pix / (TR + 2);
+      const int j = j0 + hr - 1, k = k0 + hz - 1;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (4 * q < kc && j >= 0 && j < H && k >= 0 && k < W)
+        v = *reinterpret_cast<const float4 *>(gout + ((size_t)j + (size_t)H * k) * cout + c0 + 4 * q);
+      float *d = sg + (4 * q) * PLANE + hz * PITCH + hr;
+      d[0] = v.x;
+      d[PLANE] = v.y;
+      d[2 * PLANE] = v.z;
+      d[3 * PLANE] = v.w;
+    }
+    for (int e = tid; e < kc * 9 * nch; e += nth) {
+      const int c = e % nch, t = (e / nch) % 9, co = e / (9 * nch);  // t = 3 dz + dr here
+      const float v = ci0 + c < cin ? w[((size_t)(c0 + co) * 9 + 8 - 3 * (t % 3) - t / 3) * cin + ci0 + c] : 0.f;
+      sw[e] = v;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int co = 0; co < kc; co++) {
+#pragma unroll
+      for (int dz = 0; dz < 3; dz++) {
+        const float *gp = sg + co * PLANE + (sz + dz) * PITCH + sr;
+        const float *wp = sw + (co * 9 + 3 * dz) * nch + 8 * grp;
+        float g[PX + 2];
+        if constexpr (PX == 8) {
+          const float4 a = *reinterpret_cast<const float4 *>(gp), b = *reinterpret_cast<const float4 *>(gp + 4);
+          const float2 c = *reinterpret_cast<const float2 *>(gp + 8);
+          g[0] = a.x, g[1] = a.y, g[2] = a.z, g[3] = a.w, g[4] = b.x, g[5] = b.y, g[6] = b.z, g[7] = b.w;
+          g[8] = c.x, g[9] = c.y;
+        } else {
+#pragma unroll
+          for (int i = 0; i < PX + 2; i++) g[i] = gp[i];
+        }
+#pragma unroll
+        for (int dr = 0; dr < 3; dr++) {
+          const float4 a = *reinterpret_cast<const float4 *>(wp + dr * nch);
+          const float4 b = *reinterpret_cast<const float4 *>(wp + dr * nch + 4);
+          const float wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+          for (int p = 0; p < PX; p++)
+#pragma unroll
+            for (int c = 0; c < 8; c++) acc[p][c] = fmaf(g[p + dr], wv[c], acc[p][c]);
+        }
+      }
     }
     __syncthreads();
   }
-  if (co0 + co < cout && ci0 + ci < cin)
+  const int ci = ci0 + 8 * grp, k = k0 + sz;
+  if (ci >= cin || k >= W) return;
 #pragma unroll
-    for (int t = 0; t < 9; t++) atomicAdd(dw + ((size_t)(co0 + co) * 9 + t) * cin + ci0 + ci, acc[t]);
+  for (int p = 0; p < PX; p++) {
+    const int j = j0 + sr + p;
+    if (j >= H) continue;
+    float *o = gin + ((size_t)j + (size_t)H * k) * cin + ci;
+    if (cin >= 8) {  // a multiple of 8
+      *reinterpret_cast<float4 *>(o) = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
+      *reinterpret_cast<float4 *>(o + 4) = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
+    } else {
+      for (int c = 0; c < 8 && ci + c < cin; c++) o[c] = acc[p][c];
+    }
+  }
 }
 
 // F x F average pooling (children summed in FP32, r fastest, then scaled by
@@ -401,7 +601,8 @@ __global__ void k_upcat(const __nv_bfloat16 *__restrict__ coarse, int ca, const 
     out[e] = ch < ca ? coarse[((size_t)(j / F) + (size_t)H2 * (k / F)) * ca + ch] : skip[p * cb + ch - ca];
   }
 }
-// gradient of k_upcat: gcoarse = sum over the F^2 children, gskip += the skip part
+// gradient of k_upcat: gcoarse = sum over the F^2 children, gskip = the skip part
+// (its first contribution)
 __global__ void k_upcat_bwd(const float *__restrict__ gout, int ca, int cb, int H, int W, int F,
                             float *__restrict__ gcoarse, float *__restrict__ gskip) {
   const int c = ca + cb, H2 = H / F, W2 = W / F;
@@ -419,7 +620,7 @@ __global__ void k_upcat_bwd(const float *__restrict__ gout, int ca, int cb, int 
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < ns; e += (size_t)gridDim.x * blockDim.x) {
     const int ch = (int)(e % cb);
     const size_t p = e / cb;
-    gskip[e] += gout[p * c + ca + ch];
+    gskip[e] = gout[p * c + ca + ch];
   }
 }
 // head: y[p] = sum_c in[p][c] w[c]
@@ -431,29 +632,30 @@ __global__ void k_head(const __nv_bfloat16 *__restrict__ in, int P, int c, const
     y[p] = s;
   }
 }
-// head gradient: gin[p][c] = gy[p] w[c]; gw[c] += sum_p gy[p] in[p][c]
+// head gradient: gin[p][c] = gy[p] w[c]; gw[c] += sum_p gy[p] in[p][c]; a
+// thread keeps four channels, so a warp writes whole pixels side by side
 __global__ void __launch_bounds__(256) k_head_bwd(const __nv_bfloat16 *__restrict__ in, int P, int c,
                                                 const float *__restrict__ w, const float *__restrict__ gy,
                                                 float *__restrict__ gin, float *__restrict__ gw) {
-  __shared__ float red[8][64];
-  float acc[64];
-  for (int ch = 0; ch < 64; ch++) acc[ch] = 0.f;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-    const float g = gy[p];
-    for (int ch = 0; ch < c; ch++) {
-      gin[(size_t)p * c + ch] = g * w[ch];
-      acc[ch] = fmaf(g, tof(in[(size_t)p * c + ch]), acc[ch]);
+  __shared__ float4 red[256];
+  const int nq = c / 4, per = 256 / nq, q = threadIdx.x % nq, lp = threadIdx.x / nq;
+  const float4 wq = *reinterpret_cast<const float4 *>(w + 4 * q);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (lp < per)
+    for (int p = blockIdx.x * per + lp; p < P; p += gridDim.x * per) {
+      const float g = gy[p];
+      const uint2 u = *reinterpret_cast<const uint2 *>(in + (size_t)p * c + 4 * q);
+      *reinterpret_cast<float4 *>(gin + (size_t)p * c + 4 * q) = make_float4(g * wq.x, g * wq.y, g * wq.z, g * wq.w);
+      acc.x = fmaf(g, __uint_as_float(u.x << 16), acc.x);
+      acc.y = fmaf(g, __uint_as_float(u.x & 0xffff0000u), acc.y);
+      acc.z = fmaf(g, __uint_as_float(u.y << 16), acc.z);
+      acc.w = fmaf(g, __uint_as_float(u.y & 0xffff0000u), acc.w);
     }
-  }
-  for (int ch = 0; ch < c; ch++) {
-    float v = acc[ch];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][ch] = v;
-  }
+  red[threadIdx.x] = acc;
   __syncthreads();
   if (threadIdx.x < c) {
     float s = 0.f;
-    for (int i = 0; i < 8; i++) s += red[i][threadIdx.x];
+    for (int i = 0; i < per; i++) s += reinterpret_cast<const float *>(&red[i * nq + threadIdx.x / 4])[threadIdx.x % 4];
     atomicAdd(gw + threadIdx.x, s);
   }
 }
@@ -476,21 +678,13 @@ __global__ void k_out(const float *__restrict__ y, int n, const double *__restri
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     z[i] = s * (double)y[i] * (dscale ? dscale[i] : 1.0);
 }
-// weights: bf16 copy, the rounded FP32 copy used by the kernels, the flipped
-// transposed copy for the data gradient of every 3x3 layer
+// weights: bf16 copy and the rounded FP32 copy used by the kernels
 __global__ void k_wprep(const float *__restrict__ w32, size_t n, __nv_bfloat16 *__restrict__ w16,
                         float *__restrict__ wk) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const __nv_bfloat16 b = __float2bfloat16_rn(w32[i]);
     w16[i] = b;
     wk[i] = __bfloat162float(b);
-  }
-}
-__global__ void k_wflip(const float *__restrict__ w, int cin, int cout, float *__restrict__ wf) {
-  const int n = cin * cout * 9;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const int co = e % cout, t = (e / cout) % 9, ci = e / (9 * cout);
-    wf[e] = w[((size_t)co * 9 + (8 - t)) * cin + ci];  // wf[ci][t][co]
   }
 }
 // Adam (Kingma & Ba 2015) on the FP32 master weights, gradient scaled by gs
@@ -506,8 +700,7 @@ __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float
   }
 }
 
-template <class TI, class TO>
-static cudaError_t conv3(const TI *in, int H, int W, int cin, const float *w, int cout, TO *out, int acc,
+static cudaError_t conv3(const __nv_bfloat16 *in, int H, int W, int cin, const float *w, int cout, __nv_bfloat16 *out,
                          cudaStream_t s) {
   const size_t smb = sizeof(float) * (18 * 18 * 17);
   dim3 g((H + 15) / 16, (W + 15) / 16);
@@ -515,8 +708,8 @@ static cudaError_t conv3(const TI *in, int H, int W, int cin, const float *w, in
 #define VR_CONV_CASE(C)                                                                  \
   if (cout <= C) {                                                                       \
     const size_t sm = smb + sizeof(float) * C * 9 * 16;                                  \
-    if ((e = allow_dyn_smem(k_conv3<TI, TO, C>, sm))) return e;                          \
-    k_conv3<TI, TO, C><<<g, 256, sm, s>>>(in, H, W, cin, w, cout, out, acc);             \
+    if ((e = allow_dyn_smem(k_conv3<C>, sm))) return e;                                  \
+    k_conv3<C><<<g, 256, sm, s>>>(in, H, W, cin, w, cout, out);                          \
     return cudaGetLastError();                                                           \
   }
   VR_CONV_CASE(8)
@@ -524,10 +717,6 @@ static cudaError_t conv3(const TI *in, int H, int W, int cin, const float *w, in
   VR_CONV_CASE(32)
   VR_CONV_CASE(48)
   VR_CONV_CASE(64)
-  VR_CONV_CASE(80)
-  VR_CONV_CASE(96)
-  VR_CONV_CASE(112)
-  VR_CONV_CASE(128)
 #undef VR_CONV_CASE
   return cudaErrorInvalidValue;
 }
@@ -581,14 +770,45 @@ static cudaError_t conv3_tc(const __nv_bfloat16 *in, int H, int W, int cin, cons
 
 static int round16(int x) { return (x + 15) / 16 * 16; }
 
-template <class TI>
-static cudaError_t wgrad3(const float *dout, int H, int W, int cout, const TI *in, int cin, float *dw,
-                          cudaStream_t s) {
-  const int P = H * W;
-  const int ppb = 4096;
-  dim3 g((cin + 15) / 16, (cout + 15) / 16, (P + ppb - 1) / ppb);
-  k_wgrad3<TI><<<g, 256, 0, s>>>(dout, H, W, cout, in, cin, dw, ppb);
+// One CTA per SM: as many patch walkers per channel tile as fill the chip
+template <int CIT>
+static cudaError_t wgrad3_n(const float *dout, int H, int W, int cout, const ConvIn &in, int cin, float *dw, int nsm,
+                            cudaStream_t s) {
+  using S = WgShape<CIT>;
+  const int npr = (H + S::R - 1) / S::R, npatch = npr * ((W + S::NS - 1) / S::NS);
+  const int nt = ((cin + S::IC - 1) / S::IC) * ((cout + 15) / 16);
+  const size_t sm = std::max((size_t)2 * S::STAGE, (size_t)8 * 4 * 9 * CIT * S::OT * sizeof(float));
+  cudaError_t e = allow_dyn_smem(k_wgrad3<CIT>, sm);
+  if (e) return e;
+  k_wgrad3<CIT><<<dim3(nt, std::min(npatch, std::max(1, nsm / nt))), 256, sm, s>>>(dout, H, W, cout, in, cin, dw, npr,
+                                                                                  npatch);
   return cudaGetLastError();
+}
+static cudaError_t wgrad3(const float *dout, int H, int W, int cout, const ConvIn &in, int cin, float *dw, int nsm,
+                          cudaStream_t s) {
+  return cin == 1 ? wgrad3_n<1>(dout, H, W, cout, in, cin, dw, nsm, s)
+                  : wgrad3_n<4>(dout, H, W, cout, in, cin, dw, nsm, s);
+}
+
+template <int PX>
+static cudaError_t dgrad3_n(const float *gout, int H, int W, int cout, const float *w, int cin, float *gin, int grp,
+                            int nz, cudaStream_t s) {
+  const size_t sm = sizeof(float) * (16 * 18 * (4 * PX + 4) + (size_t)16 * 9 * 8 * grp);
+  cudaError_t e = allow_dyn_smem(k_dgrad3<PX>, sm);
+  if (e) return e;
+  k_dgrad3<PX><<<dim3((H + 4 * PX - 1) / (4 * PX), (W + 15) / 16, nz), 64 * grp, sm, s>>>(gout, H, W, cout, w, cin,
+                                                                                          gin);
+  return cudaGetLastError();
+}
+static cudaError_t dgrad3(const float *gout, int H, int W, int cout, const float *w, int cin, float *gin, int nsm,
+                          cudaStream_t s) {
+  const int groups = (cin + 7) / 8;  // of 8 channels
+  const int tiles8 = ((H + 31) / 32) * ((W + 15) / 16);
+  int grp = std::min(groups, 6), nz = (groups + grp - 1) / grp;
+  if (tiles8 * nz >= nsm) return dgrad3_n<8>(gout, H, W, cout, w, cin, gin, (groups + nz - 1) / nz, nz, s);
+  grp = std::min(groups, 2);
+  nz = (groups + grp - 1) / grp;
+  return dgrad3_n<2>(gout, H, W, cout, w, cin, gin, grp, nz, s);
 }
 
 static int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 8); }
@@ -682,6 +902,7 @@ extern "C" int vr_unet_create(const vr_unet_desc *d, uint64_t seed, vr_unet **ou
   u->dev = d->device;
   for (int l = 0; l < 4; l++) u->ch[l] = d->ch[l];
   if (cudaSetDevice(u->dev) != cudaSuccess) return fail(VR_ERR_CUDA);
+  if (cudaDeviceGetAttribute(&u->nsm, cudaDevAttrMultiProcessorCount, u->dev) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&u->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VR_ERR_CUDA);
   const UnetShapes sh = shapes_of(u);
   size_t off = 0;
@@ -714,12 +935,9 @@ extern "C" int vr_unet_create(const vr_unet_desc *d, uint64_t seed, vr_unet **ou
       w[u->L[i].woff + e] = (float)(sd * std::sqrt(-2.0 * std::log(unif())) * std::cos(2.0 * pi * unif()));
   }
   const size_t P0 = (size_t)u->nr * u->nz;
-  size_t maxflip = 0;
-  for (int i = 0; i < 14; i++) maxflip = std::max(maxflip, (size_t)u->L[i].cin * u->L[i].cout * 9);
   float **fp[] = {&u->w32, &u->wk, &u->gw, &u->m1, &u->m2};
   for (float **p : fp)
     if (cudaMalloc(p, sizeof(float) * u->nparam) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMalloc(&u->wflip, sizeof(float) * maxflip) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&u->w16, sizeof(__nv_bfloat16) * u->nparam) != cudaSuccess) return fail(VR_ERR_OOM);
   size_t npk = 0;
   for (int i = 0; i < 14; i++) {
@@ -740,7 +958,9 @@ extern "C" int vr_unet_create(const vr_unet_desc *d, uint64_t seed, vr_unet **ou
     size_t div = 1;
     for (int l = 0; l < sh.lev[i]; l++) div *= (size_t)u->pool * u->pool;
     const size_t n = (P0 / div) * sh.ch[i];
-    if (cudaMalloc(&x->a[i], sizeof(__nv_bfloat16) * n) != cudaSuccess) return fail(VR_ERR_OOM);
+    const bool cat = i == S_U2 || i == S_U1 || i == S_U0;  // copied by the CUDA-core form only
+    if ((!cat || u->cuda_cores) && cudaMalloc(&x->a[i], sizeof(__nv_bfloat16) * n) != cudaSuccess)
+      return fail(VR_ERR_OOM);
     if (cudaMalloc(&x->g[i], sizeof(float) * n) != cudaSuccess) return fail(VR_ERR_OOM);
   }
   if (cudaMalloc(&x->gx0, sizeof(float) * P0) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -763,7 +983,7 @@ extern "C" int vr_unet_destroy(vr_unet *u) {
     if (u->g[i]) cudaFree(u->g[i]);
   }
   if (u->gx0) cudaFree(u->gx0);
-  float *fp[] = {u->w32, u->wk, u->gw, u->m1, u->m2, u->wflip, u->y, u->gy};
+  float *fp[] = {u->w32, u->wk, u->gw, u->m1, u->m2, u->y, u->gy};
   for (float *p : fp)
     if (p) cudaFree(p);
   if (u->w16) cudaFree(u->w16);
@@ -803,11 +1023,10 @@ extern "C" int vr_unet_set_params(vr_unet *u, const float *w) {
 
 namespace vr {
 
-// forward from u->x0 (bf16 input) to u->y (fp32)
-// infer: the decoder's concatenations are read by the tensor-core
-// convolutions where they lie (no upsampled copy); training keeps the copies,
-// which the backward pass reads
-static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, bool infer = false) {
+// forward from u->x0 (bf16 input) to u->y (fp32); the tensor-core
+// convolutions (and the weight gradients) read the decoder's concatenations
+// where they lie, only the CUDA-core form copies them
+static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s) {
   const UnetShapes sh = shapes_of(u);
   const vr_unet *x = u;
   cudaError_t e;
@@ -817,13 +1036,13 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, bool infer = false
     for (int l = 0; l < lev; l++) H /= u->pool, W /= u->pool;
   };
   int H, W;
-  const bool fuse = infer && !u->cuda_cores;
+  const bool fuse = !u->cuda_cores;
   auto conv = [&](int li) -> cudaError_t {
     const UnetLayer &L = u->L[li];
     HW(L.level, H, W);
     const __nv_bfloat16 *in = kConvIn[li] < 0 ? u->x0 : x->a[kConvIn[li]];
     if (u->cuda_cores)
-      return conv3<__nv_bfloat16, __nv_bfloat16>(in, H, W, L.cin, u->wk + L.woff, L.cout, x->a[kConvOut[li]], 0, s);
+      return conv3(in, H, W, L.cin, u->wk + L.woff, L.cout, x->a[kConvOut[li]], s);
     return conv3_tc(in, H, W, L.cin, u->wpk + u->wpk_off[li], L.cout, x->a[kConvOut[li]], u->status, s);
   };
   // the first convolution of a decoder level, on concat(upsample(coarse), skip)
@@ -876,27 +1095,23 @@ static cudaError_t unet_bwd(const vr_unet *u, bool want_dx, cudaStream_t s) {
     W = u->nz;
     for (int l = 0; l < lev; l++) H /= u->pool, W /= u->pool;
   };
-  for (int i = 0; i < S_NSLOT; i++) {
-    HW(sh.lev[i]);
-    if ((e = cudaMemsetAsync(x->g[i], 0, sizeof(float) * (size_t)H * W * sh.ch[i], s))) return e;
-  }
   const int P0 = u->nr * u->nz;
   k_head_bwd<<<std::min(P0 / 256 + 1, 148 * 4), 256, 0, s>>>(x->a[S_D0], P0, u->ch[0], u->wk + u->L[14].woff, u->gy,
                                                             x->g[S_D0], u->gw + u->L[14].woff);
   if ((e = cudaGetLastError())) return e;
-  // conv layer li: gradient of its output is in g[out]; adds the input
-  // gradient into g[in] (or gx0) and the weight gradient into gw
-  auto conv_bwd = [&](int li) -> cudaError_t {
+  // conv layer li: gradient of its output is in g[out]; writes the input
+  // gradient to g[in] (or gx0: each has one writer, the skip tensors get their
+  // pooling part after it) and adds the weight gradient to gw
+  auto conv_bwd = [&](int li, int coarse = -1, int skip = -1) -> cudaError_t {
     const UnetLayer &L = u->L[li];
     HW(L.level);
     const int so = kConvOut[li], si = kConvIn[li];
-    const __nv_bfloat16 *in = si < 0 ? u->x0 : x->a[si];
-    cudaError_t er = wgrad3<__nv_bfloat16>(x->g[so], H, W, L.cout, in, L.cin, u->gw + L.woff, s);
+    const ConvIn in = coarse < 0 ? ConvIn{si < 0 ? u->x0 : x->a[si], L.cin, nullptr, 0, 1}
+                                 : ConvIn{x->a[coarse], sh.ch[coarse], x->a[skip], sh.ch[skip], u->pool};
+    cudaError_t er = wgrad3(x->g[so], H, W, L.cout, in, L.cin, u->gw + L.woff, u->nsm, s);
     if (er) return er;
     if (si < 0 && !want_dx) return cudaSuccess;
-    k_wflip<<<grid_for((size_t)L.cin * L.cout * 9), 256, 0, s>>>(u->wk + L.woff, L.cin, L.cout, u->wflip);
-    float *gin = si < 0 ? x->gx0 : x->g[si];
-    return conv3<float, float>(x->g[so], H, W, L.cout, u->wflip, L.cin, gin, si < 0 ? 0 : 1, s);
+    return dgrad3(x->g[so], H, W, L.cout, u->wk + L.woff, L.cin, si < 0 ? x->gx0 : x->g[si], u->nsm, s);
   };
   auto upcat_bwd = [&](int coarse, int skip, int dst) {
     HW(sh.lev[skip]);
@@ -911,9 +1126,9 @@ static cudaError_t unet_bwd(const vr_unet *u, bool want_dx, cudaStream_t s) {
     k_pool_bwd<<<grid_for(n), 256, 0, s>>>(x->g[dst], H, W, sh.ch[src], u->pool, x->g[src]);
     return cudaGetLastError();
   };
-  if ((e = conv_bwd(13)) || (e = conv_bwd(12)) || (e = upcat_bwd(S_D1, S_E0, S_U0))) return e;
-  if ((e = conv_bwd(11)) || (e = conv_bwd(10)) || (e = upcat_bwd(S_D2, S_E1, S_U1))) return e;
-  if ((e = conv_bwd(9)) || (e = conv_bwd(8)) || (e = upcat_bwd(S_B3, S_E2, S_U2))) return e;
+  if ((e = conv_bwd(13)) || (e = conv_bwd(12, S_D1, S_E0)) || (e = upcat_bwd(S_D1, S_E0, S_U0))) return e;
+  if ((e = conv_bwd(11)) || (e = conv_bwd(10, S_D2, S_E1)) || (e = upcat_bwd(S_D2, S_E1, S_U1))) return e;
+  if ((e = conv_bwd(9)) || (e = conv_bwd(8, S_B3, S_E2)) || (e = upcat_bwd(S_B3, S_E2, S_U2))) return e;
   if ((e = conv_bwd(7)) || (e = conv_bwd(6)) || (e = pool_bwd(S_E2, S_P3))) return e;
   if ((e = conv_bwd(5)) || (e = conv_bwd(4)) || (e = pool_bwd(S_E1, S_P2))) return e;
   if ((e = conv_bwd(3)) || (e = conv_bwd(2)) || (e = pool_bwd(S_E0, S_P1))) return e;
@@ -931,7 +1146,7 @@ int unet_precondition(const vr_unet *u, const double *r, double *z, const double
   const int n = u->nr * u->nz;
   k_in<<<grid_for(n), 256, 0, s>>>(r, n, ss, 0.0, dscale, u->x0, flags);
   if (cudaGetLastError() != cudaSuccess) return VR_ERR_CUDA;
-  if (unet_fwd(u, s, true) != cudaSuccess) return VR_ERR_CUDA;
+  if (unet_fwd(u, s) != cudaSuccess) return VR_ERR_CUDA;
   k_out<<<grid_for(n), 256, 0, s>>>(u->y, n, ss, 0.0, dscale, z, flags);
   return cudaGetLastError() == cudaSuccess ? VR_OK : VR_ERR_CUDA;
 }
@@ -948,7 +1163,7 @@ extern "C" int vr_unet_forward(vr_unet *u, const double *xh, double *yh) {
   U_CUDA(u, cudaMemcpyAsync(u->xs, xh, sizeof(double) * n, cudaMemcpyHostToDevice, u->stream));
   k_in<<<grid_for(n), 256, 0, u->stream>>>(u->xs, n, nullptr, s > 0 ? 1.0 / s : 0.0, nullptr, u->x0, nullptr);
   U_CUDA(u, cudaGetLastError());
-  U_CUDA(u, unet_fwd(u, u->stream, true));
+  U_CUDA(u, unet_fwd(u, u->stream));
   k_out<<<grid_for(n), 256, 0, u->stream>>>(u->y, n, nullptr, s, nullptr, u->xs, nullptr);
   U_CUDA(u, cudaGetLastError());
   U_CUDA(u, cudaMemcpyAsync(yh, u->xs, sizeof(double) * n, cudaMemcpyDeviceToHost, u->stream));
