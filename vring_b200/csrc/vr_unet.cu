@@ -75,6 +75,24 @@ namespace vr {
 
 __device__ __forceinline__ float tof(__nv_bfloat16 v) { return __bfloat162float(v); }
 
+// two FP32 values in a 64-bit register pair; fma2 is one fused multiply-add
+// (rounded to nearest) in each half.  Its rate is that of two scalar ones (an
+// outer product in registers runs at 29 T multiply-adds per second either
+// way); it leaves half of the issue slots to the loads and conversions.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+  return c;
+}
+
 // out[p][co] = sum_{tap, ci} in[p + off(tap)][ci] w[co][tap][ci]
 template <int CO>
 __global__ void __launch_bounds__(256) k_conv3(const __nv_bfloat16 *__restrict__ in, int H, int W, int cin,
@@ -329,8 +347,10 @@ struct ConvIn {
 // 16-byte asynchronous copies two patches ahead of each other (zero outside the
 // grid).  It walks every gridDim.y-th patch and only then adds its threads'
 // sums (shuffle, shared memory) and the result to dw by FP32 atomics.
-// us at 512 x 1024, against one (output, input) pair per thread and ten
-// scalar loads per nine multiply-adds: WGTAB.
+// us at 512 x 1024 for 16 -> 16, 48 -> 16 and 1 -> 16 channels: 62, 185 and 23
+// (19.5 T multiply-adds per second in the first two); one (output, input) pair
+// per thread with ten scalar loads per nine multiply-adds, 4096 pixels per CTA:
+// 830, 1350 and 830, and 410 to 950 on the coarser levels (now 8 to 49).
 template <int CIT>
 struct WgShape {
   static constexpr int OT = CIT == 4 ? 16 : 4;  // threads that share a line
@@ -383,13 +403,17 @@ __global__ void __launch_bounds__(256, 1) k_wgrad3(const float *__restrict__ dou
     }
     cp_async_commit();
   };
-  float acc[4][9][CIT];
+  // CIT 4: output channel a, input channels 2 c, 2 c + 1 (the widened input
+  // comes in pairs, only the four gradients are copied into both halves);
+  // CIT 1: output channels 2 a, 2 a + 1
+  constexpr int PA = CIT == 4 ? 4 : 2, PC = CIT == 4 ? 2 : 1;
+  f32x2 acc[PA][9][PC];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < PA; a++)
 #pragma unroll
     for (int t = 0; t < 9; t++)
 #pragma unroll
-      for (int c = 0; c < CIT; c++) acc[a][t][c] = 0.f;
+      for (int c = 0; c < PC; c++) acc[a][t][c] = 0ull;
   int s = 0, p = blockIdx.y;
   if (p < npatch) fetch(p, 0);
   for (; p < npatch; p += gridDim.y, s ^= 1) {
@@ -403,19 +427,18 @@ __global__ void __launch_bounds__(256, 1) k_wgrad3(const float *__restrict__ dou
     __syncthreads();
     const float *sd = stage_d(s) + line * DP + 4 * cog;
     // column hr (0 .. R + 1) of the halo rows line .. line + 2
-    float w[3][3][CIT];  // [column mod 3][dz]
-    auto column = [&](int hr, float (&v)[3][CIT]) {
+    f32x2 w[3][3][PC];  // [column mod 3][dz]
+    auto column = [&](int hr, f32x2 (&v)[3][PC]) {
 #pragma unroll
       for (int dz = 0; dz < 3; dz++) {
         if constexpr (CIT == 4) {
           const uint2 u = *reinterpret_cast<const uint2 *>(stage_in(s) + ((size_t)(line + dz) * (R + 2) + hr) * 32 +
                                                            8 * cig);
-          v[dz][0] = __uint_as_float(u.x << 16);
-          v[dz][1] = __uint_as_float(u.x & 0xffff0000u);
-          v[dz][2] = __uint_as_float(u.y << 16);
-          v[dz][3] = __uint_as_float(u.y & 0xffff0000u);
+          v[dz][0] = pack2(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u));
+          v[dz][1] = pack2(__uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
         } else {
-          v[dz][0] = ((const float *)stage_in(s))[(line + dz) * (R + 3) + hr];
+          const float f = ((const float *)stage_in(s))[(line + dz) * (R + 3) + hr];
+          v[dz][0] = pack2(f, f);
         }
       }
     };
@@ -427,17 +450,23 @@ __global__ void __launch_bounds__(256, 1) k_wgrad3(const float *__restrict__ dou
 #pragma unroll
       for (int u = 0; u < 3; u++) {  // pixel r + u; past the line its gradient is 0
         column(r + u + 2, w[(u + 2) % 3]);
-        const float4 d = *reinterpret_cast<const float4 *>(sd + (r + u) * 16);
-        const float dd[4] = {d.x, d.y, d.z, d.w};
+        f32x2 dd[PA];
+        if constexpr (CIT == 4) {
+          const float4 d = *reinterpret_cast<const float4 *>(sd + (r + u) * 16);
+          dd[0] = pack2(d.x, d.x), dd[1] = pack2(d.y, d.y), dd[2] = pack2(d.z, d.z), dd[3] = pack2(d.w, d.w);
+        } else {
+          const ulonglong2 d = *reinterpret_cast<const ulonglong2 *>(sd + (r + u) * 16);
+          dd[0] = d.x, dd[1] = d.y;
+        }
 #pragma unroll
         for (int dr = 0; dr < 3; dr++)
 #pragma unroll
           for (int dz = 0; dz < 3; dz++)
 #pragma unroll
-            for (int a = 0; a < 4; a++)
+            for (int a = 0; a < PA; a++)
 #pragma unroll
-              for (int c = 0; c < CIT; c++)
-                acc[a][3 * dr + dz][c] = fmaf(dd[a], w[(u + dr) % 3][dz][c], acc[a][3 * dr + dz][c]);
+              for (int c = 0; c < PC; c++)
+                acc[a][3 * dr + dz][c] = fma2(dd[a], w[(u + dr) % 3][dz][c], acc[a][3 * dr + dz][c]);
       }
     }
     __syncthreads();  // the stage is refilled
@@ -451,7 +480,9 @@ __global__ void __launch_bounds__(256, 1) k_wgrad3(const float *__restrict__ dou
     for (int t = 0; t < 9; t++)
 #pragma unroll
       for (int c = 0; c < CIT; c++) {
-        float v = acc[a][t][c];
+        float v, v0, v1;
+        unpack2(CIT == 4 ? acc[a][t][c / 2] : acc[a / 2][t][0], v0, v1);
+        v = ((CIT == 4 ? c : a) & 1) ? v1 : v0;
 #pragma unroll
         for (int o = 16; o >= OT; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane < OT) red[((size_t)warp * NA + (a * 9 + t) * CIT + c) * OT + lane] = v;
@@ -468,95 +499,144 @@ __global__ void __launch_bounds__(256, 1) k_wgrad3(const float *__restrict__ dou
 }
 
 // Data gradient: gin[p][ci] = sum_{tap, co} gout[p - off(tap)][co] w[co][tap][ci],
-// the convolution with the flipped weights w[co][8 - tap], in FP32.
-// Bound by the FP32 pipe once the sums sit in registers: a thread holds PX
-// pixels along r x 8 channels; per output channel and row of taps it loads
-// PX + 2 gradients (the channel's plane in shared memory, 16 bytes at a time)
-// and 24 weights that its whole warp shares, for 24 PX multiply-adds.  A CTA
-// takes 4 PX x 16 pixels x up to 48 channels (64 threads per 8 channels); the
-// gradients of 16 channels at a time come from memory channels-last and are
-// stored as planes.  PX = 2 where PX = 8 would leave SMs idle (the coarse
-// levels).  us at 512 x 1024, against one pixel x all channels per thread:
-// DGTAB.
+// the convolution with the flipped weights w[co][8 - tap], in FP32.  Bound by
+// the FP32 pipe once the sums sit in registers: a thread holds PX pixels along
+// r x 8 channels; per four output channels and row of taps it loads PX + 2
+// pixels of 4 gradients, and per output channel 24 weights that its whole warp
+// shares, for 24 PX multiply-adds (packed, two channels each).  A CTA takes
+// tiles of 4 PX x 16 pixels x up to 48 channels (64 threads per 8 channels) in
+// turn, 16 output channels at a time; gradients (channels-last as they lie,
+// 4 floats after every PX pixels so that the strips of a quarter warp meet
+// different banks) and weights of the next 16 arrive by asynchronous copies
+// meanwhile.  PX = 2 where PX = 8 would leave SMs idle (the coarse levels).
+// us at 512 x 1024 for 16 -> 16 and 16 -> 48 channels: 77 and 187; one pixel x
+// all channels per thread: 139 and 373, and 47 to 180 on the coarser levels
+// (now 15 to 57).
+template <int PX>
+struct DgShape {
+  static constexpr int TR = 4 * PX, KC = 16;
+  // floats of a halo row: pixels of KC, a gap of 4 after every PX, and 16
+  // floats modulo 32 in all, so that two rows fill the banks
+  static constexpr int RAW = (TR + 2) * KC + ((TR + 2) / PX) * 4;
+  static constexpr int ROW = RAW + (48 - RAW % 32) % 32;
+  static constexpr int GF = 18 * ROW;  // floats of a stage's gradients
+};
+
 template <int PX>
 __global__ void __launch_bounds__(384) k_dgrad3(const float *__restrict__ gout, int H, int W, int cout,
-                                              const float *__restrict__ w, int cin, float *__restrict__ gin) {
-  constexpr int KC = 16, TR = 4 * PX, PITCH = TR + 4, ZR = 18, PLANE = ZR * PITCH;
+                                              const float *__restrict__ w, int cin, float *__restrict__ gin, int ntr,
+                                              int ntiles) {
+  using S = DgShape<PX>;
+  constexpr int KC = S::KC, TR = S::TR, ROW = S::ROW;
   extern __shared__ float smf[];
-  float *sg = smf;                // [KC][ZR][PITCH]: pixel r at column r + 1
-  float *sw = smf + KC * PLANE;   // [KC][dz][dr][channels of the CTA]
   const int tid = threadIdx.x, nth = blockDim.x, nch = nth / 8;
-  const int strip = tid & 63, grp = tid >> 6, ci0 = blockIdx.z * nch;
+  const int strip = tid & 63, grp = tid >> 6, ci0 = blockIdx.y * nch;
   const int sr = (strip & 3) * PX, sz = strip >> 2;
-  const int j0 = blockIdx.x * TR, k0 = blockIdx.y * 16;
-  float acc[PX][8];
-#pragma unroll
-  for (int p = 0; p < PX; p++)
-#pragma unroll
-    for (int c = 0; c < 8; c++) acc[p][c] = 0.f;
-  for (int c0 = 0; c0 < cout; c0 += KC) {
-    const int kc = min(KC, cout - c0);  // a multiple of 8
-    for (int e = tid; e < (TR + 2) * ZR * (KC / 4); e += nth) {
-      const int pix = e % ((TR + 2) * ZR), q = e / ((TR + 2) * ZR), hr = pix % (TR + 2), hz = pix / (TR + 2);
+  const int nk = (cout + KC - 1) / KC, stage_f = S::GF + KC * 9 * nch;
+  auto goff = [](int hr) { return hr * KC + (hr / PX) * 4; };
+  // stage s: the gradients of item (tile, 16 output channels) [18][ROW] and its weights [KC][dz][dr][nch]
+  auto fetch = [&](int tile, int kch, int s) {
+    float *sg = smf + (size_t)s * stage_f, *sw = sg + S::GF;
+    const int j0 = (tile % ntr) * TR, k0 = (tile / ntr) * 16, c0 = kch * KC, kc = min(KC, cout - c0);
+    for (int e = tid; e < 18 * (TR + 2) * (KC / 4); e += nth) {
+      const int q = e & 3, pix = e >> 2, hr = pix % (TR + 2), hz = pix / (TR + 2);
       const int j = j0 + hr - 1, k = k0 + hz - 1;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (4 * q < kc && j >= 0 && j < H && k >= 0 && k < W)
-        v = *reinterpret_cast<const float4 *>(gout + ((size_t)j + (size_t)H * k) * cout + c0 + 4 * q);
-      float *d = sg + (4 * q) * PLANE + hz * PITCH + hr;
-      d[0] = v.x;
-      d[PLANE] = v.y;
-      d[2 * PLANE] = v.z;
-      d[3 * PLANE] = v.w;
+      const bool live = 4 * q < kc && j >= 0 && j < H && k >= 0 && k < W;
+      cp_async16(sg + hz * ROW + goff(hr) + 4 * q,
+                 live ? gout + ((size_t)j + (size_t)H * k) * cout + c0 + 4 * q : gout, live ? 16u : 0u);
     }
-    for (int e = tid; e < kc * 9 * nch; e += nth) {
-      const int c = e % nch, t = (e / nch) % 9, co = e / (9 * nch);  // t = 3 dz + dr here
-      const float v = ci0 + c < cin ? w[((size_t)(c0 + co) * 9 + 8 - 3 * (t % 3) - t / 3) * cin + ci0 + c] : 0.f;
-      sw[e] = v;
+    if (cin >= 8) {
+      const int n4 = nch / 4;
+      for (int e = tid; e < KC * 9 * n4; e += nth) {
+        const int c = (e % n4) * 4, r = e / n4, t = r % 9, co = r / 9;  // t = 3 dz + dr
+        const bool live = co < kc && ci0 + c < cin;
+        cp_async16(sw + r * nch + c,
+                   live ? w + ((size_t)(c0 + co) * 9 + 8 - 3 * (t % 3) - t / 3) * cin + ci0 + c : w, live ? 16u : 0u);
+      }
+    } else {  // one channel
+      for (int e = tid; e < KC * 9 * nch; e += nth) {
+        const int c = e % nch, r = e / nch, t = r % 9, co = r / 9;
+        sw[e] = c < cin && co < kc ? w[((size_t)(c0 + co) * 9 + 8 - 3 * (t % 3) - t / 3) * cin + c] : 0.f;
+      }
+    }
+    cp_async_commit();
+  };
+  f32x2 acc[PX][4];
+  int s = 0, tile = blockIdx.x, kch = 0;
+  if (tile < ntiles) fetch(tile, 0, 0);
+  for (; tile < ntiles; s ^= 1) {
+    int ntile = tile, nkch = kch + 1;
+    if (nkch == nk) {
+      nkch = 0;
+      ntile += gridDim.x;
+    }
+    if (ntile < ntiles) {
+      fetch(ntile, nkch, s ^ 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
     }
     __syncthreads();
+    if (kch == 0) {
+#pragma unroll
+      for (int p = 0; p < PX; p++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[p][c] = 0ull;
+    }
+    const float *sg = smf + (size_t)s * stage_f, *sw = sg + S::GF;
+    const int kq = min(KC, cout - kch * KC) / 4;
 #pragma unroll 1
-    for (int co = 0; co < kc; co++) {
-#pragma unroll
+    for (int cq = 0; cq < kq; cq++) {
+#pragma unroll 1
       for (int dz = 0; dz < 3; dz++) {
-        const float *gp = sg + co * PLANE + (sz + dz) * PITCH + sr;
-        const float *wp = sw + (co * 9 + 3 * dz) * nch + 8 * grp;
-        float g[PX + 2];
-        if constexpr (PX == 8) {
-          const float4 a = *reinterpret_cast<const float4 *>(gp), b = *reinterpret_cast<const float4 *>(gp + 4);
-          const float2 c = *reinterpret_cast<const float2 *>(gp + 8);
-          g[0] = a.x, g[1] = a.y, g[2] = a.z, g[3] = a.w, g[4] = b.x, g[5] = b.y, g[6] = b.z, g[7] = b.w;
-          g[8] = c.x, g[9] = c.y;
-        } else {
+        const float *gp = sg + (sz + dz) * ROW + 4 * cq;
+        float g[PX + 2][4];
 #pragma unroll
-          for (int i = 0; i < PX + 2; i++) g[i] = gp[i];
+        for (int i = 0; i < PX + 2; i++) {
+          const float4 v = *reinterpret_cast<const float4 *>(gp + goff(sr) + i * KC + (i / PX) * 4);
+          g[i][0] = v.x, g[i][1] = v.y, g[i][2] = v.z, g[i][3] = v.w;
         }
 #pragma unroll
-        for (int dr = 0; dr < 3; dr++) {
-          const float4 a = *reinterpret_cast<const float4 *>(wp + dr * nch);
-          const float4 b = *reinterpret_cast<const float4 *>(wp + dr * nch + 4);
-          const float wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        for (int co = 0; co < 4; co++) {
+          const float *wp = sw + ((4 * cq + co) * 9 + 3 * dz) * nch + 8 * grp;
+          f32x2 g2[PX + 2];
 #pragma unroll
-          for (int p = 0; p < PX; p++)
+          for (int i = 0; i < PX + 2; i++) g2[i] = pack2(g[i][co], g[i][co]);
 #pragma unroll
-            for (int c = 0; c < 8; c++) acc[p][c] = fmaf(g[p + dr], wv[c], acc[p][c]);
+          for (int dr = 0; dr < 3; dr++) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(wp + dr * nch);
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(wp + dr * nch + 4);
+            const f32x2 wv[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+            for (int p = 0; p < PX; p++)
+#pragma unroll
+              for (int c = 0; c < 4; c++) acc[p][c] = fma2(g2[p + dr], wv[c], acc[p][c]);
+          }
         }
       }
     }
-    __syncthreads();
-  }
-  const int ci = ci0 + 8 * grp, k = k0 + sz;
-  if (ci >= cin || k >= W) return;
+    __syncthreads();  // the stage is refilled
+    if (nkch == 0) {
+      const int ci = ci0 + 8 * grp, j0 = (tile % ntr) * TR + sr, k = (tile / ntr) * 16 + sz;
+      if (ci < cin && k < W) {
 #pragma unroll
-  for (int p = 0; p < PX; p++) {
-    const int j = j0 + sr + p;
-    if (j >= H) continue;
-    float *o = gin + ((size_t)j + (size_t)H * k) * cin + ci;
-    if (cin >= 8) {  // a multiple of 8
-      *reinterpret_cast<float4 *>(o) = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
-      *reinterpret_cast<float4 *>(o + 4) = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
-    } else {
-      for (int c = 0; c < 8 && ci + c < cin; c++) o[c] = acc[p][c];
+        for (int p = 0; p < PX; p++) {
+          const int j = j0 + p;
+          if (j >= H) continue;
+          float *o = gin + ((size_t)j + (size_t)H * k) * cin + ci;
+          if (cin >= 8) {  // a multiple of 8
+            *reinterpret_cast<ulonglong2 *>(o) = make_ulonglong2(acc[p][0], acc[p][1]);
+            *reinterpret_cast<ulonglong2 *>(o + 4) = make_ulonglong2(acc[p][2], acc[p][3]);
+          } else {  // one channel
+            float v, rest;
+            unpack2(acc[p][0], v, rest);
+            o[0] = v;
+          }
+        }
+      }
     }
+    tile = ntile;
+    kch = nkch;
   }
 }
 
@@ -792,23 +872,27 @@ static cudaError_t wgrad3(const float *dout, int H, int W, int cout, const ConvI
 
 template <int PX>
 static cudaError_t dgrad3_n(const float *gout, int H, int W, int cout, const float *w, int cin, float *gin, int grp,
-                            int nz, cudaStream_t s) {
-  const size_t sm = sizeof(float) * (16 * 18 * (4 * PX + 4) + (size_t)16 * 9 * 8 * grp);
+                            int ny, int nsm, cudaStream_t s) {
+  using S = DgShape<PX>;
+  const int ntr = (H + S::TR - 1) / S::TR, ntiles = ntr * ((W + 15) / 16);
+  const size_t sm = 2 * sizeof(float) * (S::GF + (size_t)S::KC * 9 * 8 * grp);
   cudaError_t e = allow_dyn_smem(k_dgrad3<PX>, sm);
   if (e) return e;
-  k_dgrad3<PX><<<dim3((H + 4 * PX - 1) / (4 * PX), (W + 15) / 16, nz), 64 * grp, sm, s>>>(gout, H, W, cout, w, cin,
-                                                                                          gin);
+  // resident CTAs per SM by shared memory; each then takes its share of the tiles
+  const int per = std::max(1, (int)((size_t)(220 * 1024) / sm));
+  k_dgrad3<PX><<<dim3(std::min(ntiles, std::max(1, nsm * per / ny)), ny), 64 * grp, sm, s>>>(gout, H, W, cout, w, cin,
+                                                                                            gin, ntr, ntiles);
   return cudaGetLastError();
 }
 static cudaError_t dgrad3(const float *gout, int H, int W, int cout, const float *w, int cin, float *gin, int nsm,
                           cudaStream_t s) {
   const int groups = (cin + 7) / 8;  // of 8 channels
   const int tiles8 = ((H + 31) / 32) * ((W + 15) / 16);
-  int grp = std::min(groups, 6), nz = (groups + grp - 1) / grp;
-  if (tiles8 * nz >= nsm) return dgrad3_n<8>(gout, H, W, cout, w, cin, gin, (groups + nz - 1) / nz, nz, s);
+  int grp = std::min(groups, 6), ny = (groups + grp - 1) / grp;
+  if (tiles8 * ny >= nsm) return dgrad3_n<8>(gout, H, W, cout, w, cin, gin, (groups + ny - 1) / ny, ny, nsm, s);
   grp = std::min(groups, 2);
-  nz = (groups + grp - 1) / grp;
-  return dgrad3_n<2>(gout, H, W, cout, w, cin, gin, grp, nz, s);
+  ny = (groups + grp - 1) / grp;
+  return dgrad3_n<2>(gout, H, W, cout, w, cin, gin, grp, ny, nsm, s);
 }
 
 static int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 8); }
