@@ -22,8 +22,8 @@
 // Every reduction is deterministic: vector kernels write one partial sum per
 // block, and the partials are added in block order into the scalars the next
 // kernel reads -- by the block that finishes last (a ticket counter after a
-// memory fence) in the CG and BiCGSTAB kernels, which also take the scalar
-// steps there, and by a one-block kernel in the setup and the flexible CG.
+// memory fence) in the iteration kernels, which also take the scalar steps
+// there, and by a one-block kernel in the setup.
 // Grids whose vectors fit the chip run CG and BiCGSTAB in resident kernels
 // (vr_krylov_res.cuh).  The others stream them:
 // CG runs two kernels per iteration and BiCGSTAB three: each operator
@@ -80,7 +80,7 @@ struct vr_k2d {
   double *part = nullptr;   // PT_N x kK2dMaxBlocks
   double *sc = nullptr;     // SC_N
   int *flags = nullptr;     // done, iterations
-  unsigned *cnt = nullptr;  // arrival counters of the CG and BiCGSTAB kernels' last-block reductions
+  unsigned *cnt = nullptr;  // arrival counters of the last-block reductions (CG, BiCGSTAB, flexible CG)
   int cg_parity = 0;        // direction buffer of the next CG iteration being captured
   int bi_parity = 0;        // p and v buffers of the next BiCGSTAB iteration being captured
   int nb_cg = 1;            // grid of the CG iteration kernels
@@ -104,6 +104,7 @@ struct vr_k2d {
   // the flexible CG's kept directions p_i and q_i = S p_i (a ring of
   // kFcgKeep slots each), their p_i . q_i, the betas, and partial sums
   double *fp = nullptr, *fq = nullptr, *fpq = nullptr, *fbeta = nullptr, *fpart = nullptr;
+  double *frow = nullptr;  // last-radial-row arrays of nz: z0, diag(S)^-1/2, p, the network's output (float)
   // weight of the damped-Jacobi steps around the network (0: the network alone)
   double omega = 2.0 / 3.0;
 };
@@ -153,17 +154,21 @@ __device__ double last_row_mean(const K2dOp &o, const double *__restrict__ x, do
   return sh[32];
 }
 
-__device__ __forceinline__ double apply_S_at(const K2dOp &o, const double *__restrict__ x, int i, double mean) {
+// (S x)(i) with x given as a function of the index, xc its value at i
+template <class F>
+__device__ __forceinline__ double apply_S_fn(const K2dOp &o, const F &x, double xc, int i, double mean) {
   const int j = i % o.nr, k = i / o.nr;
-  const double xc = x[i];
   double y = 0.0;
-  if (j > 0) y += o.aw[j] * (xc - x[i - 1]);
-  if (j < o.nr - 1) y += o.ae[j] * (xc - x[i + 1]);
+  if (j > 0) y += o.aw[j] * (xc - x(i - 1));
+  if (j < o.nr - 1) y += o.ae[j] * (xc - x(i + 1));
   else y += o.gam * mean;
   const double az = o.az[j];
-  if (k > 0) y += az * (xc - x[i - o.nr]);
-  if (k < o.nz - 1) y += az * (xc - x[i + o.nr]);
+  if (k > 0) y += az * (xc - x(i - o.nr));
+  if (k < o.nz - 1) y += az * (xc - x(i + o.nr));
   return y;
+}
+__device__ __forceinline__ double apply_S_at(const K2dOp &o, const double *__restrict__ x, int i, double mean) {
+  return apply_S_fn(o, [&](int e) { return x[e]; }, x[i], i, mean);
 }
 
 // y = S x (form 0) or K x (form 1); with part, part[b] = sum over the block of w . y
@@ -217,10 +222,8 @@ __device__ __forceinline__ double sum_part(const double *p, int nb, double *sh) 
 enum K2dScalarOp {
   SO_CG_INIT = 0,   // bb, rz, rr from partials A (b.b), B (r.z), C (r.r)
   SO_BI_INIT,       // bb [A], rho_new = rh.r [B], rr [C]
-  SO_FCG_CONV,      // rr [A]
   SO_NORM,          // rr [A] only (sc[SC_RR])
-  SO_NORM_BB,       // bb [A] only (sc[SC_BB])
-  SO_SS             // (D r).(D r) [A] into sc[SC_SS] (the preconditioner's input scale)
+  SO_NORM_BB        // bb [A] only (sc[SC_BB])
 };
 
 __global__ void __launch_bounds__(1024) k2d_scalar(int op, const double *part, int nb, double *sc, int *flags) {
@@ -250,23 +253,13 @@ __global__ void __launch_bounds__(1024) k2d_scalar(int op, const double *part, i
       flags[0] = (c <= sc[SC_TOL2] * a) ? 1 : 0;
       flags[1] = 0;
       break;
-    case SO_FCG_CONV:
-      sc[SC_RR] = a;
-      flags[1] += 1;
-      if (a <= sc[SC_TOL2] * sc[SC_BB]) flags[0] = 1;
-      break;
     case SO_NORM:
       sc[SC_RR] = a;
       break;
     case SO_NORM_BB:
       sc[SC_BB] = a;
       break;
-    case SO_SS:
-      sc[SC_SS] = a;
-      break;
   }
-  // iteration cap (flags[2]): stop as not converged
-  if (op == SO_FCG_CONV && !flags[0] && flags[1] >= flags[2]) flags[0] = 2;
 }
 
 // A CG iteration is two kernels.  Each ends with a reduction of its blocks'
@@ -540,88 +533,172 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_bi_xr3(K2dOp o, double *__res
   if (threadIdx.x == 0) *counter = 0;
 }
 
-// partial sum of (D r)^2 [A] (the learned preconditioner's input scale)
-__global__ void __launch_bounds__(kK2dThreads) k2d_dscaled(int n, const double *__restrict__ r,
-                                                         const double *__restrict__ dh, double *part,
-                                                         const int *flags) {
-  __shared__ double sh[40];
-  if (flags[0]) return;
-  double a = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double x = dh[i] * r[i];
-    a += x * x;
-  }
-  double t = block_sum(a, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
 // ---- truncated flexible CG with kFcgKeep directions ---------------------------
 // kept = min(iteration, kFcgKeep); the new direction goes to slot iteration % kFcgKeep
 __device__ __forceinline__ int fcg_kept(const int *flags) { return min(flags[1], kFcgKeep); }
 __device__ __forceinline__ int fcg_slot(const int *flags) { return flags[1] % kFcgKeep; }
 
-// partials of z . q_i for the kept directions
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_zq(int n, const double *__restrict__ z,
-                                                        const double *__restrict__ fq, double *fpart,
-                                                        const int *flags) {
+// Five kernels per iteration beside the network, the scalar steps in the block
+// that arrives last, as for CG.  A stencil's argument that is a pointwise
+// function of stored vectors is formed where the stencil reads it, and the
+// values of the last radial row, whose mean over z the wall term needs, are
+// also kept side by side (row arrays of nz), so that every block of the next
+// kernel takes their mean from a few KB instead of one word per plane.  The
+// separate steps took 14 kernels of 2 blocks per SM: 0.11 of the 0.35 ms of a
+// learned iteration at 512 x 1024; these take FCGUS.
+__device__ __forceinline__ double row_mean(const K2dOp &o, const double *__restrict__ row, double *sh) {
+  double v = 0.0;
+  for (int k = threadIdx.x; k < o.nz; k += blockDim.x) v += row[k];
+  const double s = block_sum(v, sh);
+  __syncthreads();
+  if (threadIdx.x == 0) sh[32] = s / o.nz;
+  __syncthreads();
+  return sh[32];
+}
+
+// the first iteration's row arrays: z0 = omega D^-1 r, and D^-1/2
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_first(K2dOp o, double omega, const double *__restrict__ r,
+                                                           const double *__restrict__ dh, double *z0l, double *dhl) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < o.nz; k += gridDim.x * blockDim.x) {
+    const int i = o.nr - 1 + o.nr * k;
+    z0l[k] = omega * o.dinv[i] * r[i];
+    dhl[k] = dh[i];
+  }
+}
+
+// the network's input t = r - S z0, z0 = omega D^-1 r; the last block: the sum
+// of (D^-1/2 t)^2, its scale
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pre(K2dOp o, double omega, const double *__restrict__ r,
+                                                         const double *__restrict__ z0l, double *__restrict__ t,
+                                                         const double *__restrict__ dh, double *sc, double *part,
+                                                         unsigned *counter, const int *flags) {
+  __shared__ double sh[40];
+  if (flags[0]) return;
+  const double mean = row_mean(o, z0l, sh);
+  auto z0 = [&](int e) { return omega * o.dinv[e] * r[e]; };
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x) {
+    const double v = r[i] - apply_S_fn(o, z0, z0(i), i, mean);
+    t[i] = v;
+    const double x = dh[i] * v;
+    acc += x * x;
+  }
+  const double s = block_sum(acc, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  if (!arrived_last(counter)) return;
+  const double ss = sum_part_l2(part, gridDim.x, sh);
+  if (threadIdx.x == 0) {
+    sc[SC_SS] = ss;
+    *counter = 0;
+  }
+}
+
+// z = N + z0 (N = s D^-1/2 y, the network's correction; y null: none), with
+// omega > 0 also z += omega D^-1 (r - S z); partials of z . q_i for the kept
+// directions; the last block: beta_i = (z . q_i) / (p_i . q_i)
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_post(K2dOp o, double omega, const double *__restrict__ r,
+                                                          const float *__restrict__ y, const float *__restrict__ yl,
+                                                          const double *__restrict__ dh,
+                                                          const double *__restrict__ dhl,
+                                                          const double *__restrict__ z0l, double *__restrict__ z,
+                                                          const double *__restrict__ fq, const double *sc,
+                                                          double *fpart, const double *fpq, double *fbeta,
+                                                          unsigned *counter, const int *flags) {
   __shared__ double sh[40];
   if (flags[0]) return;
   const int kept = fcg_kept(flags);
+  const double s = y ? sqrt(sc[SC_SS] / o.n) : 0.0;
+  double mean = 0.0;
+  if (omega > 0.0) {
+    double v = 0.0;
+    for (int k = threadIdx.x; k < o.nz; k += blockDim.x) v += y ? s * (double)yl[k] * dhl[k] + z0l[k] : z0l[k];
+    const double ms = block_sum(v, sh);
+    __syncthreads();
+    if (threadIdx.x == 0) sh[32] = ms / o.nz;
+    __syncthreads();
+    mean = sh[32];
+  }
+  auto zn = [&](int e) {
+    const double z0 = omega * o.dinv[e] * r[e];
+    return y ? s * (double)y[e] * dh[e] + z0 : z0;
+  };
   double acc[kFcgKeep];
 #pragma unroll
   for (int i = 0; i < kFcgKeep; i++) acc[i] = 0.0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const double zi = z[e];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < o.n; e += gridDim.x * blockDim.x) {
+    double v = zn(e);
+    if (omega > 0.0) v += omega * o.dinv[e] * (r[e] - apply_S_fn(o, zn, v, e, mean));
+    z[e] = v;
 #pragma unroll
     for (int i = 0; i < kFcgKeep; i++)
-      if (i < kept) acc[i] += zi * fq[(size_t)i * n + e];
+      if (i < kept) acc[i] += v * fq[(size_t)i * o.n + e];
   }
-  for (int i = 0; i < kept; i++) {
-    const double t = block_sum(acc[i], sh);
-    if (threadIdx.x == 0) fpart[(size_t)i * kK2dMaxBlocks + blockIdx.x] = t;
-    __syncthreads();
+  // all kept sums at once: a warp's in registers, then a thread per direction;
+  // in the last block a warp per direction
+  __shared__ double sw[kK2dThreads / 32][kFcgKeep];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+    for (int i = 0; i < kFcgKeep; i++) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], d);
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < kFcgKeep; i++) sw[warp][i] = acc[i];
+  __syncthreads();
+  if (threadIdx.x < kept) {
+    double t = 0.0;
+    for (int w = 0; w < kK2dThreads / 32; w++) t += sw[w][threadIdx.x];
+    fpart[(size_t)threadIdx.x * kK2dMaxBlocks + blockIdx.x] = t;
   }
-}
-
-// beta_i = (z . q_i) / (p_i . q_i)
-__global__ void __launch_bounds__(1024) k2d_fcg_betas(const double *fpart, int nb, const double *fpq, double *fbeta,
-                                                    const int *flags) {
-  __shared__ double sh[40];
-  if (flags[0]) return;
-  const int kept = fcg_kept(flags);
-  for (int i = 0; i < kept; i++) {
-    const double a = sum_part(fpart + (size_t)i * kK2dMaxBlocks, nb, sh);
-    if (threadIdx.x == 0) fbeta[i] = fpq[i] != 0.0 ? a / fpq[i] : 0.0;
+  if (!arrived_last(counter)) return;
+  static_assert(kFcgKeep <= kK2dThreads / 32, "a warp per kept direction");
+  if (warp < kept) {
+    double a = 0.0;
+    for (int b = lane; b < gridDim.x; b += 32) a += __ldcg(fpart + (size_t)warp * kK2dMaxBlocks + b);
+    for (int d = 16; d > 0; d >>= 1) a += __shfl_down_sync(0xffffffffu, a, d);
+    if (lane == 0) fbeta[warp] = fpq[warp] != 0.0 ? a / fpq[warp] : 0.0;
   }
+  if (threadIdx.x == 0) *counter = 0;
 }
 
 // p = z - sum_i beta_i p_i, written to the new slot (which may be the oldest
-// kept direction: each element is read before it is overwritten)
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pm(int n, const double *__restrict__ z, double *fp,
-                                                        const double *__restrict__ fbeta, const int *flags) {
+// kept direction: each element is read before it is overwritten); partial
+// p . r [A]
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pm(K2dOp o, const double *__restrict__ z, double *fp,
+                                                        const double *__restrict__ fbeta,
+                                                        const double *__restrict__ r, double *pl, double *part,
+                                                        const int *flags) {
+  __shared__ double sh[40];
   if (flags[0]) return;
   const int kept = fcg_kept(flags), slot = fcg_slot(flags);
-  double b[kFcgKeep];
+  double b[kFcgKeep], acc = 0.0;
 #pragma unroll
   for (int i = 0; i < kFcgKeep; i++) b[i] = i < kept ? fbeta[i] : 0.0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < o.n; e += gridDim.x * blockDim.x) {
     double v = z[e];
 #pragma unroll
     for (int i = 0; i < kFcgKeep; i++)
-      if (i < kept) v -= b[i] * fp[(size_t)i * n + e];
-    fp[(size_t)slot * n + e] = v;
+      if (i < kept) v -= b[i] * fp[(size_t)i * o.n + e];
+    fp[(size_t)slot * o.n + e] = v;
+    acc += v * r[e];
+    const int k = e / o.nr;
+    if (e - k * o.nr == o.nr - 1) pl[k] = v;
   }
+  const double t = block_sum(acc, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
-// q = S p for the new slot, partial p . q [B]
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_apply(K2dOp o, const double *fp, double *fq, double *part,
-                                                           const int *flags) {
+// q = S p for the new slot, partial p . q [B]; the last block:
+// alpha = (p . r) / (p . q), p . q kept for the slot
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_apply(K2dOp o, const double *fp, double *fq,
+                                                           const double *__restrict__ pl, double *sc, double *part,
+                                                           double *fpq, unsigned *counter, const int *flags) {
   __shared__ double sh[40];
   if (flags[0]) return;
   const int slot = fcg_slot(flags);
   const double *x = fp + (size_t)slot * o.n;
   double *y = fq + (size_t)slot * o.n;
-  const double mean = last_row_mean(o, x, sh);
+  const double mean = row_mean(o, pl, sh);
   double acc = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x) {
     const double v = apply_S_at(o, x, i, mean);
@@ -630,81 +707,45 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_apply(K2dOp o, const doub
   }
   const double t = block_sum(acc, sh);
   if (threadIdx.x == 0) part[kK2dMaxBlocks + blockIdx.x] = t;
-}
-
-// partial p . r [A] of the new slot
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pr(int n, const double *__restrict__ fp,
-                                                        const double *__restrict__ r, double *part, const int *flags) {
-  __shared__ double sh[40];
-  if (flags[0]) return;
-  const double *p = fp + (size_t)fcg_slot(flags) * n;
-  double acc = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc += p[i] * r[i];
-  const double t = block_sum(acc, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
-// alpha = (p . r) / (p . q); p . q kept for the slot
-__global__ void __launch_bounds__(1024) k2d_fcg_alpha(const double *part, int nb, double *sc, double *fpq,
-                                                    const int *flags) {
-  __shared__ double sh[40];
-  if (flags[0]) return;
-  const double pr = sum_part(part, nb, sh);
-  const double pq = sum_part(part + kK2dMaxBlocks, nb, sh);
+  if (!arrived_last(counter)) return;
+  const double pr = sum_part_l2(part, gridDim.x, sh), pq = sum_part_l2(part + kK2dMaxBlocks, gridDim.x, sh);
   if (threadIdx.x == 0) {
     sc[SC_ALPHA] = pq != 0.0 ? pr / pq : 0.0;
-    fpq[fcg_slot(flags)] = pq;
+    fpq[slot] = pq;
+    *counter = 0;
   }
 }
 
-// x += alpha p; r -= alpha q; partial r.r [A]
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_xrm(int n, double *__restrict__ x, double *__restrict__ r,
-                                                         const double *__restrict__ fp, const double *__restrict__ fq,
-                                                         const double *sc, double *part, const int *flags) {
+// x += alpha p; r -= alpha q; partial r.r [C]; the next iteration's row of z0;
+// the last block: the norm and the convergence and iteration-cap flags
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_xrm(K2dOp o, double omega, double *__restrict__ x,
+                                                         double *__restrict__ r, const double *__restrict__ fp,
+                                                         const double *__restrict__ fq, double *z0l, double *sc,
+                                                         double *part, unsigned *counter, int *flags) {
   __shared__ double sh[40];
   if (flags[0]) return;
-  const size_t so = (size_t)fcg_slot(flags) * n;
+  const size_t so = (size_t)fcg_slot(flags) * o.n;
   const double al = sc[SC_ALPHA];
   double rr = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x) {
     x[i] += al * fp[so + i];
     const double ri = r[i] - al * fq[so + i];
     r[i] = ri;
     rr += ri * ri;
+    const int k = i / o.nr;
+    if (i - k * o.nr == o.nr - 1) z0l[k] = omega * o.dinv[i] * ri;
   }
   const double t = block_sum(rr, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
-// ---- the preconditioner's damped-Jacobi steps -----------------------------------
-// z0 = omega D^-1 r (D^-1 = dinv), t = r - S z0
-__global__ void __launch_bounds__(kK2dThreads) k2d_jac_pre(int n, double omega, const double *__restrict__ dinv,
-                                                         const double *__restrict__ r, double *__restrict__ z0,
-                                                         const int *flags) {
-  if (flags[0]) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) z0[i] = omega * dinv[i] * r[i];
-}
-__global__ void __launch_bounds__(kK2dThreads) k2d_resid(K2dOp o, const double *__restrict__ x,
-                                                       const double *__restrict__ r, double *__restrict__ t,
-                                                       const int *flags) {
-  __shared__ double sh[40];
-  if (flags[0]) return;
-  const double mean = last_row_mean(o, x, sh);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x)
-    t[i] = r[i] - apply_S_at(o, x, i, mean);
-}
-// z += z0 (the network's correction on top of the pre-smoothing)
-__global__ void __launch_bounds__(kK2dThreads) k2d_addv(int n, double *__restrict__ z, const double *__restrict__ z0,
-                                                      const int *flags) {
-  if (flags[0]) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) z[i] += z0[i];
-}
-// z += omega D^-1 t (t = r - S z, the post-smoothing)
-__global__ void __launch_bounds__(kK2dThreads) k2d_jac_post(int n, double omega, const double *__restrict__ dinv,
-                                                          const double *__restrict__ t, double *__restrict__ z,
-                                                          const int *flags) {
-  if (flags[0]) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) z[i] += omega * dinv[i] * t[i];
+  if (threadIdx.x == 0) part[2 * kK2dMaxBlocks + blockIdx.x] = t;
+  if (!arrived_last(counter)) return;
+  const double a = sum_part_l2(part + 2 * kK2dMaxBlocks, gridDim.x, sh);
+  if (threadIdx.x == 0) {
+    sc[SC_RR] = a;
+    flags[1] += 1;
+    if (a <= sc[SC_TOL2] * sc[SC_BB]) flags[0] = 1;
+    if (!flags[0] && flags[1] >= flags[2]) flags[0] = 2;  // iteration cap: stop as not converged
+    *counter = 0;
+  }
 }
 
 // ---- direct solve -----------------------------------------------------------
@@ -984,8 +1025,8 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
   if (cudaMalloc(&k->part, sizeof(double) * PT_N * kK2dMaxBlocks) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->sc, sizeof(double) * SC_N) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->flags, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMalloc(&k->cnt, sizeof(unsigned) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMemset(k->cnt, 0, sizeof(unsigned) * 4) != cudaSuccess) return fail(VR_ERR_CUDA);
+  if (cudaMalloc(&k->cnt, sizeof(unsigned) * 8) != cudaSuccess) return fail(VR_ERR_OOM);
+  if (cudaMemset(k->cnt, 0, sizeof(unsigned) * 8) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaMalloc(&k->dct_f, sizeof(double) * cf.size()) != cudaSuccess) return fail(VR_ERR_OOM);
   if (!ci.empty() && cudaMalloc(&k->dct_i, sizeof(double) * ci.size()) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->tlo, sizeof(double) * nr) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -1022,7 +1063,7 @@ extern "C" int vr_k2d_destroy(vr_k2d *k) {
   for (double *v : k->vec)
     if (v) cudaFree(v);
   double *ps[] = {k->coef, k->part, k->sc, k->dct_f, k->dct_i, k->tlo, k->tup, k->tib, k->tmp,
-                  k->fp, k->fq, k->fpq, k->fbeta, k->fpart};
+                  k->fp, k->fq, k->fpq, k->fbeta, k->fpart, k->frow};
   for (double *p : ps)
     if (p) cudaFree(p);
   if (k->flags) cudaFree(k->flags);
@@ -1271,46 +1312,29 @@ static cudaError_t enq_bicg(vr_k2d *k, int) {
 // Everything stays on the device, so chunks of iterations, the network's
 // launches included, are captured as graphs like the other methods.
 static cudaError_t enqueue_fcg_iter(vr_k2d *k) {
-  const K2dOp o = op_of(k);
-  const int gb = k2d_grid(k);
-  double *P = k->part;
-  double *x = k->vec[V_X], *r = k->vec[V_R], *z = k->vec[V_Z];
   // z = M r: with omega > 0 the network is the middle of a two-level step,
   //   z0 = omega D^-1 r;  z = z0 + N(r - S z0);  z += omega D^-1 (r - S z)
   // (damped-Jacobi steps before and after the network's correction, so the
   // rough error components the network does not resolve are damped); without
   // a network only the two Jacobi steps remain (the method the network is
   // compared against)
+  const K2dOp o = op_of(k);
+  const int gb = k->nb_cg;
   const double om = k->omega;
-  double *z0 = k->vec[V_S], *t = k->vec[V_T];
-  const double *rin = r;
-  if (om > 0.0) {
-    k2d_jac_pre<<<gb, kK2dThreads, 0, k->stream>>>(o.n, om, o.dinv, r, z0, k->flags);
-    k2d_resid<<<gb, kK2dThreads, 0, k->stream>>>(o, z0, r, t, k->flags);
-    rin = t;
-  }
+  double *P = k->part, *x = k->vec[V_X], *r = k->vec[V_R], *z = k->vec[V_Z], *t = k->vec[V_T];
+  double *z0l = k->frow, *dhl = z0l + k->nz, *pl = dhl + k->nz;
+  float *yl = reinterpret_cast<float *>(pl + k->nz);
+  const float *y = nullptr;
   if (k->net) {
-    k2d_dscaled<<<gb, kK2dThreads, 0, k->stream>>>(o.n, rin, k2d_dhalf(k), P, k->flags);
-    k2d_scalar<<<1, 1024, 0, k->stream>>>(SO_SS, P, gb, k->sc, k->flags);
-    if (unet_precondition(k->net, rin, z, k2d_dhalf(k), k->sc + SC_SS, k->flags, k->stream) != VR_OK)
+    k2d_fcg_pre<<<gb, kK2dThreads, 0, k->stream>>>(o, om, r, z0l, t, k2d_dhalf(k), k->sc, P, k->cnt + 4, k->flags);
+    if (unet_correct(k->net, t, k2d_dhalf(k), k->sc + SC_SS, k->flags, yl, &y, k->stream) != VR_OK)
       return cudaErrorLaunchFailure;
-    if (om > 0.0) k2d_addv<<<gb, kK2dThreads, 0, k->stream>>>(o.n, z, z0, k->flags);
-  } else {
-    cudaMemcpyAsync(z, z0, sizeof(double) * o.n, cudaMemcpyDeviceToDevice, k->stream);
   }
-  if (om > 0.0) {
-    k2d_resid<<<gb, kK2dThreads, 0, k->stream>>>(o, z, r, t, k->flags);
-    k2d_jac_post<<<gb, kK2dThreads, 0, k->stream>>>(o.n, om, o.dinv, t, z, k->flags);
-  }
-  // orthogonalise z against the kept directions in S's inner product
-  k2d_fcg_zq<<<gb, kK2dThreads, 0, k->stream>>>(o.n, z, k->fq, k->fpart, k->flags);
-  k2d_fcg_betas<<<1, 1024, 0, k->stream>>>(k->fpart, gb, k->fpq, k->fbeta, k->flags);
-  k2d_fcg_pm<<<gb, kK2dThreads, 0, k->stream>>>(o.n, z, k->fp, k->fbeta, k->flags);
-  k2d_fcg_apply<<<gb, kK2dThreads, 0, k->stream>>>(o, k->fp, k->fq, P, k->flags);
-  k2d_fcg_pr<<<gb, kK2dThreads, 0, k->stream>>>(o.n, k->fp, r, P, k->flags);
-  k2d_fcg_alpha<<<1, 1024, 0, k->stream>>>(P, gb, k->sc, k->fpq, k->flags);
-  k2d_fcg_xrm<<<gb, kK2dThreads, 0, k->stream>>>(o.n, x, r, k->fp, k->fq, k->sc, P, k->flags);
-  k2d_scalar<<<1, 1024, 0, k->stream>>>(SO_FCG_CONV, P, gb, k->sc, k->flags);
+  k2d_fcg_post<<<gb, kK2dThreads, 0, k->stream>>>(o, om, r, y, yl, k2d_dhalf(k), dhl, z0l, z, k->fq, k->sc, k->fpart,
+                                                k->fpq, k->fbeta, k->cnt + 5, k->flags);
+  k2d_fcg_pm<<<gb, kK2dThreads, 0, k->stream>>>(o, z, k->fp, k->fbeta, r, pl, P, k->flags);
+  k2d_fcg_apply<<<gb, kK2dThreads, 0, k->stream>>>(o, k->fp, k->fq, pl, k->sc, P, k->fpq, k->cnt + 6, k->flags);
+  k2d_fcg_xrm<<<gb, kK2dThreads, 0, k->stream>>>(o, om, x, r, k->fp, k->fq, z0l, k->sc, P, k->cnt + 7, k->flags);
   return cudaGetLastError();
 }
 static cudaError_t enq_fcg(vr_k2d *k, int) { return enqueue_fcg_iter(k); }
@@ -1438,11 +1462,15 @@ extern "C" int vr_k2d_solve_dev(vr_k2d *k, int32_t method, const double *f, doub
       if (cudaMalloc(&k->fp, kb) != cudaSuccess || cudaMalloc(&k->fq, kb) != cudaSuccess ||
           cudaMalloc(&k->fpq, sizeof(double) * kFcgKeep) != cudaSuccess ||
           cudaMalloc(&k->fbeta, sizeof(double) * kFcgKeep) != cudaSuccess ||
+          cudaMalloc(&k->frow, sizeof(double) * 4 * k->nz) != cudaSuccess ||
           cudaMalloc(&k->fpart, sizeof(double) * kFcgKeep * kK2dMaxBlocks) != cudaSuccess)
         return k2d_err(k, VR_ERR_OOM, "flexible CG directions");
     }
     k2d_init_dots<<<gb, kK2dThreads, 0, k->stream>>>(o, 0, B, R, nullptr, P);
     k2d_scalar<<<1, 1024, 0, k->stream>>>(SO_CG_INIT, P, gb, k->sc, k->flags);
+    K2D_CUDA(k, cudaGetLastError());
+    k2d_fcg_first<<<(k->nz + kK2dThreads - 1) / kK2dThreads, kK2dThreads, 0, k->stream>>>(o, k->omega, R, k2d_dhalf(k),
+                                                                                          k->frow, k->frow + k->nz);
     K2D_CUDA(k, cudaGetLastError());
     // the graph bakes in whether the network runs: one slot per form
     const vr_unet *keep = k->net;

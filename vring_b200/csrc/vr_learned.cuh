@@ -8,11 +8,12 @@
 
 namespace vr {
 
-// z = s D N(D r / s), D = dscale (per cell, may be NULL for 1) and
-// s = sqrt(*ss / n) with ss = sum (D r)^2 read on the device; r and z device
-// arrays of nr*nz doubles; does nothing once flags[0] is set
-int unet_precondition(const vr_unet *u, const double *r, double *z, const double *dscale, const double *ss,
-                      const int *flags, cudaStream_t s);
+// y = N(D t / s), D = dscale (per cell) and s = sqrt(*ss / n) with
+// ss = sum (D t)^2 read on the device; t a device array of nr*nz doubles, *y
+// the network's own output array, yl (may be null) a copy of its last radial
+// row (nz values).  The input is left alone once flags[0] is set.
+int unet_correct(const vr_unet *u, const double *t, const double *dscale, const double *ss, const int *flags, float *yl,
+                 const float **y, cudaStream_t s);
 
 // grid of a network (nr, nz)
 void unet_dims(const vr_unet *u, int *nr, int *nz);

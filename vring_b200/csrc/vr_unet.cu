@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *__restric
   uint8_t *wst = sm + conv_halo_bytes<CINP>();  // [tap][cc][n] 16-byte chunks
   __shared__ uint64_t bar;
   __shared__ uint32_t tbase;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == 0) {
     tmem_alloc(&tbase, NCOLS);
     tmem_relinquish();
@@ -225,30 +225,39 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *__restric
     mbar_init_fence();
   }
   const int j0 = blockIdx.x * kConvTR, k0 = blockIdx.y * kConvTZ;
-  // the halo, pixels (j0 - 1 .. j0 + 8, k0 - 1 .. k0 + 16): consecutive
-  // threads take consecutive chunks of a pixel, then the next pixel in r
-  const int ctot = skip ? cin + cskip : cin, H2 = H / F;
-  for (int e = tid; e < HR * HZ * CC; e += 128) {
-    const int cc = e % CC, pix = e / CC, hr = pix % HR, hz = pix / HR;
-    const int j = j0 + hr - 1, k = k0 + hz - 1, ci = cc * 8;
-    const bool live = j >= 0 && j < H && k >= 0 && k < W && ci < ctot;
-    uint8_t *dst = halo + (size_t)((hz * CC + cc) * HR + hr) * 16;
-    const __nv_bfloat16 *src = in;
-    if (live) {
-      if (!skip)
-        src = in + ((size_t)j + (size_t)H * k) * cin + ci;
-      else if (ci < cin)
-        src = in + ((size_t)(j / F) + (size_t)H2 * (k / F)) * cin + ci;
-      else
-        src = skip + ((size_t)j + (size_t)H * k) * cskip + (ci - cin);
-    }
-    if ((ctot & 7) == 0) {
-      cp_async16(dst, src, live ? 16u : 0u);
-    } else {
-      __align__(16) __nv_bfloat16 v[8];
+  // the halo, pixels (j0 - 1 .. j0 + 8, k0 - 1 .. k0 + 16), a warp per row of
+  // constant k: a lane keeps its pixel and chunk of the row (consecutive lanes
+  // take consecutive chunks of a pixel, then the next pixel in r), so a row
+  // costs it a pointer, a bounds test and the copy
+  const int ctot = skip ? cin + cskip : cin;
+  if (cin > 1) {
 #pragma unroll
-      for (int q = 0; q < 8; q++) v[q] = (live && ci + q < cin) ? src[q] : __float2bfloat16_rn(0.f);
-      *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(v);
+    for (int p0 = 0; p0 < HR * CC; p0 += 32) {
+      const int p = p0 + lane, cc = p % CC, hr = p / CC, j = j0 + hr - 1, ci = cc * 8;
+      const bool mine = p < HR * CC, jlive = mine && j >= 0 && j < H && ci < ctot;
+      const bool full = !skip || ci >= cin;  // at this level's resolution
+      const int sh = full ? 0 : F >> 1;      // F = 2, 4: shift by 1, 2
+      const __nv_bfloat16 *src = full ? (skip ? skip + (size_t)j * cskip + (ci - cin) : in + (size_t)j * cin + ci)
+                                      : in + (size_t)(j >> sh) * cin + ci;
+      const size_t row = full ? (size_t)H * (skip ? cskip : cin) : (size_t)(H >> sh) * cin;
+      uint8_t *dst = halo + (size_t)(cc * HR + hr) * 16;
+      if (mine)
+#pragma unroll
+        for (int hz0 = 0; hz0 < HZ; hz0 += 4) {
+          const int hz = hz0 + warp, k = k0 + hz - 1;
+          const bool live = jlive && k >= 0 && k < W;
+          if (hz < HZ) cp_async16(dst + (size_t)hz * (CC * HR * 16), live ? src + row * (k >> sh) : in, live ? 16u : 0u);
+        }
+    }
+  } else {  // one channel: the first of a pixel's chunks, zeros beside it
+    for (int e = tid; e < HR * HZ; e += 128) {
+      const int hr = e % HR, hz = e / HR, j = j0 + hr - 1, k = k0 + hz - 1;
+      const bool live = j >= 0 && j < H && k >= 0 && k < W;
+      const unsigned v = live ? (unsigned)__bfloat16_as_ushort(in[(size_t)j + (size_t)H * k]) : 0u;
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++)
+        *reinterpret_cast<uint4 *>(halo + (size_t)((hz * CC + cc) * HR + hr) * 16) =
+            make_uint4(cc == 0 ? v : 0u, 0u, 0u, 0u);
     }
   }
   // the packed weights are already in the staged order
@@ -641,32 +650,49 @@ __global__ void __launch_bounds__(384) k_dgrad3(const float *__restrict__ gout, 
 }
 
 // F x F average pooling (children summed in FP32, r fastest, then scaled by
-// 1 / F^2) and its gradient
-__global__ void k_pool(const __nv_bfloat16 *__restrict__ in, int H, int W, int c, int F,
-                       __nv_bfloat16 *__restrict__ out) {
-  const int H2 = H / F, W2 = W / F;
-  const size_t n = (size_t)H2 * W2 * c;
+// 1 / F^2) and its gradient; eight, then four channels per thread
+template <int F>
+__global__ void k_pool(const __nv_bfloat16 *__restrict__ in, int H, int W, int c, __nv_bfloat16 *__restrict__ out) {
+  const int H2 = H / F, W2 = W / F, c8 = c / 8, n = H2 * W2 * c8;
   const float inv = 1.f / (float)(F * F);
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % c);
-    const size_t p = e / c;
-    const int J = (int)(p % H2), K = (int)(p / H2);
-    float s = 0.f;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int q = e % c8, p = e / c8, J = p % H2, K = p / H2;
+    const uint4 *src = reinterpret_cast<const uint4 *>(in + ((size_t)F * J + (size_t)H * F * K) * c) + q;
+    float s[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] = 0.f;
+#pragma unroll
     for (int dz = 0; dz < F; dz++)
-      for (int dr = 0; dr < F; dr++) s += tof(in[((size_t)F * J + dr + (size_t)H * ((size_t)F * K + dz)) * c + ch]);
-    out[e] = __float2bfloat16_rn(inv * s);
+#pragma unroll
+      for (int dr = 0; dr < F; dr++) {
+        const uint4 u = src[((size_t)H * dz + dr) * c8];
+        const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          s[2 * i] += __uint_as_float(w[i] << 16);
+          s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+        }
+      }
+    __align__(16) __nv_bfloat16 b[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) b[i] = __float2bfloat16_rn(inv * s[i]);
+    *(reinterpret_cast<uint4 *>(out) + e) = *reinterpret_cast<const uint4 *>(b);
   }
 }
 // gin[p][c] += gout[parent(p)][c] / F^2
-__global__ void k_pool_bwd(const float *__restrict__ gout, int H, int W, int c, int F, float *__restrict__ gin) {
-  const size_t n = (size_t)H * W * c;
-  const int H2 = H / F;
+template <int F>
+__global__ void k_pool_bwd(const float *__restrict__ gout, int H, int W, int c, float *__restrict__ gin) {
+  const int H2 = H / F, c4 = c / 4, n = H * W * c4;
   const float inv = 1.f / (float)(F * F);
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % c);
-    const size_t p = e / c;
-    const int j = (int)(p % H), k = (int)(p / H);
-    gin[e] += inv * gout[((size_t)(j / F) + (size_t)H2 * (k / F)) * c + ch];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int q = e % c4, p = e / c4, j = p % H, k = p / H;
+    const float4 g = reinterpret_cast<const float4 *>(gout)[((size_t)(j / F) + (size_t)H2 * (k / F)) * c4 + q];
+    float4 v = reinterpret_cast<float4 *>(gin)[e];
+    v.x += inv * g.x;
+    v.y += inv * g.y;
+    v.z += inv * g.z;
+    v.w += inv * g.w;
+    reinterpret_cast<float4 *>(gin)[e] = v;
   }
 }
 // out[p] = [coarse[parent(p)] (ca channels), skip[p] (cb channels)]
@@ -681,35 +707,54 @@ __global__ void k_upcat(const __nv_bfloat16 *__restrict__ coarse, int ca, const 
     out[e] = ch < ca ? coarse[((size_t)(j / F) + (size_t)H2 * (k / F)) * ca + ch] : skip[p * cb + ch - ca];
   }
 }
-// gradient of k_upcat: gcoarse = sum over the F^2 children, gskip = the skip part
-// (its first contribution)
-__global__ void k_upcat_bwd(const float *__restrict__ gout, int ca, int cb, int H, int W, int F,
-                            float *__restrict__ gcoarse, float *__restrict__ gskip) {
-  const int c = ca + cb, H2 = H / F, W2 = W / F;
-  const size_t nc = (size_t)H2 * W2 * ca;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nc; e += (size_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % ca);
-    const size_t P = e / ca;
-    const int J = (int)(P % H2), K = (int)(P / H2);
-    float s = 0.f;
-    for (int dz = 0; dz < F; dz++)
-      for (int dr = 0; dr < F; dr++) s += gout[((size_t)F * J + dr + (size_t)H * ((size_t)F * K + dz)) * c + ch];
-    gcoarse[e] = s;
-  }
-  const size_t ns = (size_t)H * W * cb;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < ns; e += (size_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % cb);
-    const size_t p = e / cb;
-    gskip[e] = gout[p * c + ca + ch];
+// gradient of k_upcat: gcoarse = sum over the F^2 children (r fastest), gskip =
+// the skip part (its first contribution); a thread takes four channels of a
+// coarse cell, and of its children's skip part
+template <int F>
+__global__ void k_upcat_bwd(const float *__restrict__ gout, int ca, int cb, int H, int W, float *__restrict__ gcoarse,
+                            float *__restrict__ gskip) {
+  const int H2 = H / F, W2 = W / F, c4 = (ca + cb) / 4, a4 = ca / 4, b4 = cb / 4, n = H2 * W2 * c4;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int q = e % c4, P = e / c4, J = P % H2, K = P / H2;
+    const size_t p0 = (size_t)F * J + (size_t)H * F * K;
+    const float4 *src = reinterpret_cast<const float4 *>(gout) + p0 * c4 + q;
+    float4 v[F * F];
+#pragma unroll
+    for (int d = 0; d < F * F; d++) v[d] = src[((size_t)H * (d / F) + d % F) * c4];
+    if (q < a4) {
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int d = 0; d < F * F; d++) {
+        s.x += v[d].x;
+        s.y += v[d].y;
+        s.z += v[d].z;
+        s.w += v[d].w;
+      }
+      reinterpret_cast<float4 *>(gcoarse)[(size_t)P * a4 + q] = s;
+    } else {
+#pragma unroll
+      for (int d = 0; d < F * F; d++)
+        reinterpret_cast<float4 *>(gskip)[(p0 + (size_t)H * (d / F) + d % F) * b4 + (q - a4)] = v[d];
+    }
   }
 }
-// head: y[p] = sum_c in[p][c] w[c]
-__global__ void k_head(const __nv_bfloat16 *__restrict__ in, int P, int c, const float *__restrict__ w,
-                       float *__restrict__ y) {
+// head: y[p] = sum_c in[p][c] w[c], eight channels per load; yl: a copy of the
+// last radial row (or null)
+__global__ void k_head(const __nv_bfloat16 *__restrict__ in, int P, int nr, int c, const float *__restrict__ w,
+                       float *__restrict__ y, float *__restrict__ yl) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
     float s = 0.f;
-    for (int ch = 0; ch < c; ch++) s = fmaf(tof(in[(size_t)p * c + ch]), w[ch], s);
+    for (int ch = 0; ch < c; ch += 8) {
+      const uint4 u = *reinterpret_cast<const uint4 *>(in + (size_t)p * c + ch);
+      const unsigned q[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        s = fmaf(__uint_as_float(q[i] << 16), w[ch + 2 * i], s);
+        s = fmaf(__uint_as_float(q[i] & 0xffff0000u), w[ch + 2 * i + 1], s);
+      }
+    }
     y[p] = s;
+    if (yl && p % nr == nr - 1) yl[p / nr] = s;
   }
 }
 // head gradient: gin[p][c] = gy[p] w[c]; gw[c] += sum_p gy[p] in[p][c]; a
@@ -750,13 +795,9 @@ __global__ void k_in(const double *__restrict__ x, int n, const double *__restri
     xb[i] = __float2bfloat16_rn((float)v);
   }
 }
-// output: z = s D y
-__global__ void k_out(const float *__restrict__ y, int n, const double *__restrict__ ss, double s_host,
-                      const double *__restrict__ dscale, double *__restrict__ z, const int *flags) {
-  if (flags && flags[0]) return;
-  const double s = ss ? sqrt(*ss / n) : s_host;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    z[i] = s * (double)y[i] * (dscale ? dscale[i] : 1.0);
+// output: z = s y
+__global__ void k_out(const float *__restrict__ y, int n, double s, double *__restrict__ z) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) z[i] = s * (double)y[i];
 }
 // weights: bf16 copy and the rounded FP32 copy used by the kernels
 __global__ void k_wprep(const float *__restrict__ w32, size_t n, __nv_bfloat16 *__restrict__ w16,
@@ -1110,7 +1151,7 @@ namespace vr {
 // forward from u->x0 (bf16 input) to u->y (fp32); the tensor-core
 // convolutions (and the weight gradients) read the decoder's concatenations
 // where they lie, only the CUDA-core form copies them
-static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s) {
+static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullptr) {
   const UnetShapes sh = shapes_of(u);
   const vr_unet *x = u;
   cudaError_t e;
@@ -1138,8 +1179,11 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s) {
   };
   auto pool = [&](int src, int dst) {
     HW(sh.lev[src], H, W);
-    const size_t n = (size_t)(H / u->pool) * (W / u->pool) * sh.ch[src];
-    k_pool<<<grid_for(n), 256, 0, s>>>(x->a[src], H, W, sh.ch[src], u->pool, x->a[dst]);
+    const size_t n = (size_t)(H / u->pool) * (W / u->pool) * sh.ch[src] / 8;
+    if (u->pool == 2)
+      k_pool<2><<<grid_for(n), 256, 0, s>>>(x->a[src], H, W, sh.ch[src], x->a[dst]);
+    else
+      k_pool<4><<<grid_for(n), 256, 0, s>>>(x->a[src], H, W, sh.ch[src], x->a[dst]);
     return cudaGetLastError();
   };
   auto upcat = [&](int coarse, int skip, int dst) {
@@ -1163,7 +1207,7 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s) {
     if ((e = upcat(S_D1, S_E0, S_U0)) || (e = conv(12)) || (e = conv(13))) return e;
   }
   const int P0 = u->nr * u->nz;
-  k_head<<<grid_for(P0), 256, 0, s>>>(x->a[S_D0], P0, u->ch[0], u->wk + u->L[14].woff, u->y);
+  k_head<<<grid_for(P0), 256, 0, s>>>(x->a[S_D0], P0, u->nr, u->ch[0], u->wk + u->L[14].woff, u->y, yl);
   return cudaGetLastError();
 }
 
@@ -1199,15 +1243,15 @@ static cudaError_t unet_bwd(const vr_unet *u, bool want_dx, cudaStream_t s) {
   };
   auto upcat_bwd = [&](int coarse, int skip, int dst) {
     HW(sh.lev[skip]);
-    const size_t n = (size_t)H * W * sh.ch[skip];
-    k_upcat_bwd<<<grid_for(n), 256, 0, s>>>(x->g[dst], sh.ch[coarse], sh.ch[skip], H, W, u->pool, x->g[coarse],
-                                            x->g[skip]);
+    const size_t n = (size_t)H * W / (u->pool * u->pool) * sh.ch[dst] / 4;
+    (u->pool == 2 ? k_upcat_bwd<2> : k_upcat_bwd<4>)<<<grid_for(n), 256, 0, s>>>(
+        x->g[dst], sh.ch[coarse], sh.ch[skip], H, W, x->g[coarse], x->g[skip]);
     return cudaGetLastError();
   };
   auto pool_bwd = [&](int src, int dst) {
     HW(sh.lev[src]);
-    const size_t n = (size_t)H * W * sh.ch[src];
-    k_pool_bwd<<<grid_for(n), 256, 0, s>>>(x->g[dst], H, W, sh.ch[src], u->pool, x->g[src]);
+    const size_t n = (size_t)H * W * sh.ch[src] / 4;
+    (u->pool == 2 ? k_pool_bwd<2> : k_pool_bwd<4>)<<<grid_for(n), 256, 0, s>>>(x->g[dst], H, W, sh.ch[src], x->g[src]);
     return cudaGetLastError();
   };
   if ((e = conv_bwd(13)) || (e = conv_bwd(12, S_D1, S_E0)) || (e = upcat_bwd(S_D1, S_E0, S_U0))) return e;
@@ -1225,14 +1269,14 @@ void unet_dims(const vr_unet *u, int *nr, int *nz) {
   *nz = u->nz;
 }
 
-int unet_precondition(const vr_unet *u, const double *r, double *z, const double *dscale, const double *ss,
-                      const int *flags, cudaStream_t s) {
+int unet_correct(const vr_unet *u, const double *t, const double *dscale, const double *ss, const int *flags, float *yl,
+                 const float **y, cudaStream_t s) {
   const int n = u->nr * u->nz;
-  k_in<<<grid_for(n), 256, 0, s>>>(r, n, ss, 0.0, dscale, u->x0, flags);
+  k_in<<<grid_for(n), 256, 0, s>>>(t, n, ss, 0.0, dscale, u->x0, flags);
   if (cudaGetLastError() != cudaSuccess) return VR_ERR_CUDA;
-  if (unet_fwd(u, s) != cudaSuccess) return VR_ERR_CUDA;
-  k_out<<<grid_for(n), 256, 0, s>>>(u->y, n, ss, 0.0, dscale, z, flags);
-  return cudaGetLastError() == cudaSuccess ? VR_OK : VR_ERR_CUDA;
+  if (unet_fwd(u, s, yl) != cudaSuccess) return VR_ERR_CUDA;
+  *y = u->y;
+  return VR_OK;
 }
 
 }  // namespace vr
@@ -1248,7 +1292,7 @@ extern "C" int vr_unet_forward(vr_unet *u, const double *xh, double *yh) {
   k_in<<<grid_for(n), 256, 0, u->stream>>>(u->xs, n, nullptr, s > 0 ? 1.0 / s : 0.0, nullptr, u->x0, nullptr);
   U_CUDA(u, cudaGetLastError());
   U_CUDA(u, unet_fwd(u, u->stream));
-  k_out<<<grid_for(n), 256, 0, u->stream>>>(u->y, n, nullptr, s, nullptr, u->xs, nullptr);
+  k_out<<<grid_for(n), 256, 0, u->stream>>>(u->y, n, s, u->xs);
   U_CUDA(u, cudaGetLastError());
   U_CUDA(u, cudaMemcpyAsync(yh, u->xs, sizeof(double) * n, cudaMemcpyDeviceToHost, u->stream));
   U_CUDA(u, cudaStreamSynchronize(u->stream));
