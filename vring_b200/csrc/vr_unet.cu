@@ -190,6 +190,10 @@ __global__ void __launch_bounds__(256) k_conv3(const __nv_bfloat16 *__restrict__
 // are multiples of 8, so every 16-byte chunk comes from one of them.
 constexpr int kConvTR = 8, kConvTZ = 16;  // pixel patch of a CTA (r x z)
 constexpr int kConvHR = kConvTR + 2, kConvHZ = kConvTZ + 2;
+#ifndef VR_CONV_CTAS
+#define VR_CONV_CTAS 8
+#endif
+constexpr int kConvCtas = VR_CONV_CTAS;  // resident CTAs per SM, at most
 
 template <int CINP>
 __host__ __device__ constexpr int conv_halo_bytes() {
@@ -204,15 +208,16 @@ template <int CINP, int NOUT>
 __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *__restrict__ in, int H, int W, int cin,
                                                 const __nv_bfloat16 *__restrict__ skip, int cskip, int F,
                                                 const __nv_bfloat16 *__restrict__ wpk, int cout,
-                                                __nv_bfloat16 *__restrict__ out, unsigned *status) {
+                                                __nv_bfloat16 *__restrict__ out, unsigned *status, int npr,
+                                                int npatch) {
   static_assert(CINP % 16 == 0 && NOUT % 16 == 0 && NOUT <= 64, "tile shape");
   constexpr int CC = CINP / 8, HR = kConvHR, HZ = kConvHZ;
   constexpr uint32_t NCOLS = NOUT <= 32 ? 32 : 64;
   constexpr uint32_t IDESC = umma_idesc_bf16_f32(128, NOUT);
   extern __shared__ uint8_t smraw[];
   uint8_t *sm = (uint8_t *)(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
-  uint8_t *halo = sm;                           // [hz][cc][hr] 16-byte chunks
-  uint8_t *wst = sm + conv_halo_bytes<CINP>();  // [tap][cc][n] 16-byte chunks
+  uint8_t *wst = sm;                                    // [tap][cc][n] 16-byte chunks
+  uint8_t *halos = sm + conv_wstage_bytes<CINP, NOUT>();  // one or two of [hz][cc][hr] 16-byte chunks
   __shared__ uint64_t bar;
   __shared__ uint32_t tbase;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -224,95 +229,113 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *__restric
     mbar_init(&bar, 1);
     mbar_init_fence();
   }
-  const int j0 = blockIdx.x * kConvTR, k0 = blockIdx.y * kConvTZ;
-  // the halo, pixels (j0 - 1 .. j0 + 8, k0 - 1 .. k0 + 16), a warp per row of
-  // constant k: a lane keeps its pixel and chunk of the row (consecutive lanes
-  // take consecutive chunks of a pixel, then the next pixel in r), so a row
-  // costs it a pointer, a bounds test and the copy
   const int ctot = skip ? cin + cskip : cin;
-  if (cin > 1) {
+  // the halo of a patch, pixels (j0 - 1 .. j0 + 8, k0 - 1 .. k0 + 16), a warp
+  // per row of constant k: a lane keeps its pixel and chunk of the row
+  // (consecutive lanes take consecutive chunks of a pixel, then the next pixel
+  // in r), so a row costs it a pointer, a bounds test and the copy
+  auto fetch = [&](int patch, uint8_t *halo) {
+    const int j0 = (patch % npr) * kConvTR, k0 = (patch / npr) * kConvTZ;
+    if (cin > 1) {
 #pragma unroll
-    for (int p0 = 0; p0 < HR * CC; p0 += 32) {
-      const int p = p0 + lane, cc = p % CC, hr = p / CC, j = j0 + hr - 1, ci = cc * 8;
-      const bool mine = p < HR * CC, jlive = mine && j >= 0 && j < H && ci < ctot;
-      const bool full = !skip || ci >= cin;  // at this level's resolution
-      const int sh = full ? 0 : F >> 1;      // F = 2, 4: shift by 1, 2
-      const __nv_bfloat16 *src = full ? (skip ? skip + (size_t)j * cskip + (ci - cin) : in + (size_t)j * cin + ci)
-                                      : in + (size_t)(j >> sh) * cin + ci;
-      const size_t row = full ? (size_t)H * (skip ? cskip : cin) : (size_t)(H >> sh) * cin;
-      uint8_t *dst = halo + (size_t)(cc * HR + hr) * 16;
-      if (mine)
+      for (int p0 = 0; p0 < HR * CC; p0 += 32) {
+        const int p = p0 + lane, cc = p % CC, hr = p / CC, j = j0 + hr - 1, ci = cc * 8;
+        const bool mine = p < HR * CC, jlive = mine && j >= 0 && j < H && ci < ctot;
+        const bool full = !skip || ci >= cin;  // at this level's resolution
+        const int sh = full ? 0 : F >> 1;      // F = 2, 4: shift by 1, 2
+        const __nv_bfloat16 *src = full ? (skip ? skip + (size_t)j * cskip + (ci - cin) : in + (size_t)j * cin + ci)
+                                        : in + (size_t)(j >> sh) * cin + ci;
+        const size_t row = full ? (size_t)H * (skip ? cskip : cin) : (size_t)(H >> sh) * cin;
+        uint8_t *dst = halo + (size_t)(cc * HR + hr) * 16;
+        if (mine)
 #pragma unroll
-        for (int hz0 = 0; hz0 < HZ; hz0 += 4) {
-          const int hz = hz0 + warp, k = k0 + hz - 1;
-          const bool live = jlive && k >= 0 && k < W;
-          if (hz < HZ) cp_async16(dst + (size_t)hz * (CC * HR * 16), live ? src + row * (k >> sh) : in, live ? 16u : 0u);
-        }
-    }
-  } else {  // one channel: the first of a pixel's chunks, zeros beside it
-    for (int e = tid; e < HR * HZ; e += 128) {
-      const int hr = e % HR, hz = e / HR, j = j0 + hr - 1, k = k0 + hz - 1;
-      const bool live = j >= 0 && j < H && k >= 0 && k < W;
-      const unsigned v = live ? (unsigned)__bfloat16_as_ushort(in[(size_t)j + (size_t)H * k]) : 0u;
+          for (int hz0 = 0; hz0 < HZ; hz0 += 4) {
+            const int hz = hz0 + warp, k = k0 + hz - 1;
+            const bool live = jlive && k >= 0 && k < W;
+            if (hz < HZ)
+              cp_async16(dst + (size_t)hz * (CC * HR * 16), live ? src + row * (k >> sh) : in, live ? 16u : 0u);
+          }
+      }
+    } else {  // one channel: the first of a pixel's chunks, zeros beside it
+      for (int e = tid; e < HR * HZ; e += 128) {
+        const int hr = e % HR, hz = e / HR, j = j0 + hr - 1, k = k0 + hz - 1;
+        const bool live = j >= 0 && j < H && k >= 0 && k < W;
+        const unsigned v = live ? (unsigned)__bfloat16_as_ushort(in[(size_t)j + (size_t)H * k]) : 0u;
 #pragma unroll
-      for (int cc = 0; cc < CC; cc++)
-        *reinterpret_cast<uint4 *>(halo + (size_t)((hz * CC + cc) * HR + hr) * 16) =
-            make_uint4(cc == 0 ? v : 0u, 0u, 0u, 0u);
-    }
-  }
-  // the packed weights are already in the staged order
-  for (int e = tid; e < 9 * CC * NOUT; e += 128) cp_async16(wst + (size_t)e * 16, wpk + (size_t)e * 8, 16u);
-  cp_async_commit();
-  cp_async_wait<0>();
-  fence_proxy_async();  // the halo and weights, before the tensor cores read them
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tbase;
-  if (tid == 0) {
-#pragma unroll 1
-    for (int t = 0; t < 9; t++) {
-      const int dr = t / 3, dz = t % 3;  // tap t: neighbour (j + dr - 1, k + dz - 1)
-#pragma unroll
-      for (int ks = 0; ks < CINP / 16; ks++) {
-        const uint64_t ad = umma_desc_plain(halo + (size_t)((dz * CC + 2 * ks) * HR + dr) * 16, HR * 16, CC * HR * 16);
-        const uint64_t bd = umma_desc_plain(wst + (size_t)((t * CC + 2 * ks) * NOUT) * 16, NOUT * 16, 128);
-        umma_bf16(tmem, ad, bd, IDESC, (t | ks) ? 1u : 0u);
+        for (int cc = 0; cc < CC; cc++)
+          *reinterpret_cast<uint4 *>(halo + (size_t)((hz * CC + cc) * HR + hr) * 16) =
+              make_uint4(cc == 0 ? v : 0u, 0u, 0u, 0u);
       }
     }
-    umma_commit(&bar);
-  }
-  const bool ok = mbar_wait(&bar, 0u);
-  tc_fence_after();
-  const int mr = tid % kConvTR, mz = tid / kConvTR;  // this thread's row of D: pixel (j0 + mr, k0 + mz)
-  const int j = j0 + mr, k = k0 + mz;
-  const bool pin = j < H && k < W;
-  const size_t p = (size_t)j + (size_t)H * k;
+  };
+  // the packed weights are already in the staged order
+  for (int e = tid; e < 9 * CC * NOUT; e += 128) cp_async16(wst + (size_t)e * 16, wpk + (size_t)e * 8, 16u);
+  int patch = blockIdx.x, buf = 0;
+  uint32_t phase = 0;
+  if (patch < npatch) fetch(patch, halos);
+  cp_async_commit();
+  for (; patch < npatch; phase ^= 1, buf ^= 1) {
+    uint8_t *halo = halos + (size_t)buf * conv_halo_bytes<CINP>();
+    cp_async_wait<0>();
+    fence_proxy_async();  // the halo and weights, before the tensor cores read them
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tbase;
+    if (tid == 0) {
+#pragma unroll 1
+      for (int t = 0; t < 9; t++) {
+        const int dr = t / 3, dz = t % 3;  // tap t: neighbour (j + dr - 1, k + dz - 1)
 #pragma unroll
-  for (int c0 = 0; c0 < NOUT; c0 += 16) {
-    float v[16];
-    tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
-    if (pin && ok && c0 < cout) {
-      __nv_bfloat16 *dst = out + p * cout + c0;
-      if (c0 + 16 <= cout) {
+        for (int ks = 0; ks < CINP / 16; ks++) {
+          const uint64_t ad =
+              umma_desc_plain(halo + (size_t)((dz * CC + 2 * ks) * HR + dr) * 16, HR * 16, CC * HR * 16);
+          const uint64_t bd = umma_desc_plain(wst + (size_t)((t * CC + 2 * ks) * NOUT) * 16, NOUT * 16, 128);
+          umma_bf16(tmem, ad, bd, IDESC, (t | ks) ? 1u : 0u);
+        }
+      }
+      umma_commit(&bar);
+    }
+    __syncwarp();
+    // the next patch's halo meanwhile (its buffer's products were waited for)
+    const int next = patch + gridDim.x;
+    if (next < npatch) fetch(next, halos + (size_t)(buf ^ 1) * conv_halo_bytes<CINP>());
+    cp_async_commit();
+    const bool ok = mbar_wait(&bar, phase);
+    tc_fence_after();
+    const int j0 = (patch % npr) * kConvTR, k0 = (patch / npr) * kConvTZ;
+    const int mr = tid % kConvTR, mz = tid / kConvTR;  // this thread's row of D: pixel (j0 + mr, k0 + mz)
+    const int j = j0 + mr, k = k0 + mz;
+    const bool pin = j < H && k < W;
+    const size_t p = (size_t)j + (size_t)H * k;
+#pragma unroll
+    for (int c0 = 0; c0 < NOUT; c0 += 16) {
+      float v[16];
+      tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+      if (pin && ok && c0 < cout) {
+        __nv_bfloat16 *dst = out + p * cout + c0;
         __align__(16) __nv_bfloat16 b[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) b[i] = __float2bfloat16_rn(v[i]);
         reinterpret_cast<uint4 *>(dst)[0] = reinterpret_cast<const uint4 *>(b)[0];
-        reinterpret_cast<uint4 *>(dst)[1] = reinterpret_cast<const uint4 *>(b)[1];
-      } else {
-        for (int i = 0; i < 16 && c0 + i < cout; i++) dst[i] = __float2bfloat16_rn(v[i]);
+        if (c0 + 16 <= cout)  // channel counts are multiples of 8
+          reinterpret_cast<uint4 *>(dst)[1] = reinterpret_cast<const uint4 *>(b)[1];
       }
     }
+    tc_fence_before();
+    // a wait that gave up ends the walk for the whole CTA
+    if (!__syncthreads_and(ok)) {
+      if (tid == 0) atomicOr(status, 1u);
+      // the MMAs may still be reading shared memory and writing tensor memory
+      (void)mbar_wait(&bar, phase);
+      break;
+    }
+    patch = next;
   }
-  if (!ok) {
-    if (tid == 0) atomicOr(status, 1u);
-    // the MMAs may still be reading shared memory and writing tensor memory
-    (void)mbar_wait(&bar, 0u);
-  }
+  cp_async_wait<0>();
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, NCOLS);
+  if (warp == 0) tmem_dealloc(tbase, NCOLS);
 }
 
 // packed tensor-core weights in the order the convolution stages them:
@@ -845,24 +868,28 @@ static cudaError_t conv3(const __nv_bfloat16 *in, int H, int W, int cin, const f
 template <int CINP, int NOUT>
 static cudaError_t conv3_tc_n(const __nv_bfloat16 *in, int H, int W, int cin, const __nv_bfloat16 *skip, int cskip,
                               int F, const __nv_bfloat16 *wpk, int cout, __nv_bfloat16 *out, unsigned *status,
-                              cudaStream_t s) {
-  const size_t sm = 128 + (size_t)conv_halo_bytes<CINP>() + conv_wstage_bytes<CINP, NOUT>();
+                              int nsm, cudaStream_t s) {
+  constexpr int halo = conv_halo_bytes<CINP>(), wst = conv_wstage_bytes<CINP, NOUT>();
+  const int npr = (H + kConvTR - 1) / kConvTR, npatch = npr * ((W + kConvTZ - 1) / kConvTZ);
+  // resident CTAs per SM with two halo buffers; one buffer where no CTA walks
+  const int most = std::max(1, std::min(kConvCtas, (int)((size_t)(220 * 1024) / (128 + wst + 2 * halo + 1024))));
+  const int grid = std::min(npatch, nsm * most);
+  const size_t sm = 128 + (size_t)wst + (size_t)(npatch > grid ? 2 : 1) * halo;
   cudaError_t e = allow_dyn_smem(k_conv3_tc<CINP, NOUT>, sm);
   if (e) return e;
-  dim3 grid((H + kConvTR - 1) / kConvTR, (W + kConvTZ - 1) / kConvTZ);
-  k_conv3_tc<CINP, NOUT><<<grid, 128, sm, s>>>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status);
+  k_conv3_tc<CINP, NOUT><<<grid, 128, sm, s>>>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, npr, npatch);
   return cudaGetLastError();
 }
 
 template <int CINP>
 static cudaError_t conv3_tc_c(const __nv_bfloat16 *in, int H, int W, int cin, const __nv_bfloat16 *skip, int cskip,
                               int F, const __nv_bfloat16 *wpk, int cout, __nv_bfloat16 *out, unsigned *status,
-                              cudaStream_t s) {
+                              int nsm, cudaStream_t s) {
   switch ((cout + 15) / 16) {
-    case 1: return conv3_tc_n<CINP, 16>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, s);
-    case 2: return conv3_tc_n<CINP, 32>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, s);
-    case 3: return conv3_tc_n<CINP, 48>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, s);
-    case 4: return conv3_tc_n<CINP, 64>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, s);
+    case 1: return conv3_tc_n<CINP, 16>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
+    case 2: return conv3_tc_n<CINP, 32>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
+    case 3: return conv3_tc_n<CINP, 48>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
+    case 4: return conv3_tc_n<CINP, 64>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -870,12 +897,12 @@ static cudaError_t conv3_tc_c(const __nv_bfloat16 *in, int H, int W, int cin, co
 // tensor-core 3x3 convolution: cin (+ cskip) up to 128, cout up to 64; with
 // skip, the input is the concatenation of `in` upsampled by F and `skip`
 static cudaError_t conv3_tc(const __nv_bfloat16 *in, int H, int W, int cin, const __nv_bfloat16 *wpk, int cout,
-                            __nv_bfloat16 *out, unsigned *status, cudaStream_t s,
+                            __nv_bfloat16 *out, unsigned *status, int nsm, cudaStream_t s,
                             const __nv_bfloat16 *skip = nullptr, int cskip = 0, int F = 1) {
   if (skip && ((cin & 7) || (cskip & 7))) return cudaErrorInvalidValue;
   const int ctot = cin + (skip ? cskip : 0);
   switch ((ctot + 15) / 16) {
-#define VR_CONV_TC(CP) return conv3_tc_c<CP>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, s)
+#define VR_CONV_TC(CP) return conv3_tc_c<CP>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s)
     case 1: VR_CONV_TC(16);
     case 2: VR_CONV_TC(32);
     case 3: VR_CONV_TC(48);
@@ -1168,14 +1195,14 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullpt
     const __nv_bfloat16 *in = kConvIn[li] < 0 ? u->x0 : x->a[kConvIn[li]];
     if (u->cuda_cores)
       return conv3(in, H, W, L.cin, u->wk + L.woff, L.cout, x->a[kConvOut[li]], s);
-    return conv3_tc(in, H, W, L.cin, u->wpk + u->wpk_off[li], L.cout, x->a[kConvOut[li]], u->status, s);
+    return conv3_tc(in, H, W, L.cin, u->wpk + u->wpk_off[li], L.cout, x->a[kConvOut[li]], u->status, u->nsm, s);
   };
   // the first convolution of a decoder level, on concat(upsample(coarse), skip)
   auto conv_cat = [&](int li, int coarse, int skip) -> cudaError_t {
     const UnetLayer &L = u->L[li];
     HW(L.level, H, W);
     return conv3_tc(x->a[coarse], H, W, sh.ch[coarse], u->wpk + u->wpk_off[li], L.cout, x->a[kConvOut[li]],
-                    u->status, s, x->a[skip], sh.ch[skip], u->pool);
+                    u->status, u->nsm, s, x->a[skip], sh.ch[skip], u->pool);
   };
   auto pool = [&](int src, int dst) {
     HW(sh.lev[src], H, W);
