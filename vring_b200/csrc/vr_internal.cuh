@@ -292,6 +292,15 @@ int vr_part_inflow_step(vr_part *p);
 // the dump of part_tools.F90:444-491 when this step is a dump step
 int vr_part_dump_step(vr_part *p);
 
+// Planes a z-marching CTA walks: 32, or as few as four (the right-hand side's
+// solve batch) while the grid would leave `want` resident CTAs without work.
+// The planes loaded beside its own come from L2 on grids that small.
+inline int march_planes(int row_blocks, int nz, int want) {
+  int zs = 32;
+  while (zs > 4 && row_blocks * ((nz + zs - 1) / zs) < want) zs /= 2;
+  return zs;
+}
+
 // kernel launchers (return cudaError_t of the launch) -----------------------
 cudaError_t launch_hdnbc(vr_ctx *c, const Rk &rk, double corr3s_val, double cor);
 cudaError_t launch_rhs_tsweep(vr_ctx *c, const Rk &rk);

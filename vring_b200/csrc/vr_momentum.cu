@@ -645,8 +645,8 @@ static cudaError_t run_rhs_tsweep(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a)
 
 // ---------------------------------------------------------------------------
 // z-marching form of the fused right-hand side and theta solve.  A CTA owns
-// kMRJ r-rows and up to zs consecutive z-planes and walks them in z.  q1..q3
-// of rows j0-1 .. j0+kMRJ at each plane arrive through a ring of kQRing
+// RJ r-rows and up to zs consecutive z-planes and walks them in z.  q1..q3
+// of rows j0-1 .. j0+RJ at each plane arrive through a ring of kQRing
 // shared-memory slots that TMA fills kQRing-2 planes ahead, so the stencil
 // reads shared memory and every q word crosses HBM once per CTA; each thread
 // prefetches the ru and prg words of its cell one plane ahead into
@@ -654,20 +654,18 @@ static cudaError_t run_rhs_tsweep(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a)
 // the whole walk.
 //
 // The right-hand sides of kTB consecutive planes collect in shared memory;
-// then the warps solve their theta lines 32 / kTL at a time (tsolve_group),
+// then the warps solve their theta lines 32 / TL at a time (tsolve_group),
 // so the CTA pays one solve phase per kTB planes and the short group scans
 // keep the instruction count per unknown low.
 // ---------------------------------------------------------------------------
-constexpr int kMRJ = 2, kQRing = 4, kMarchZ = 32, kTB = 4;
+constexpr int kQRing = 4, kTB = 4;
 
-// Periodic theta solve of one line by a group of kTL consecutive lanes of a
+// Periodic theta solve of one line by a group of TL consecutive lanes of a
 // warp (the arithmetic of tsolve_warp; lane g of the group owns the EG
-// contiguous inner unknowns [g EG, g EG + EG)), so a warp solves 32 / kTL
+// contiguous inner unknowns [g EG, g EG + EG)), so a warp solves 32 / TL
 // lines side by side with short scans.  Groups with on = false touch no
 // memory but take part in the shuffles.
-constexpr int kTL = 8;
-
-template <int EG>
+template <int TL, int EG>
 __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const double *cpp, const double *czz,
                                              const double *rt, double *sl, int gl, bool on) {
   const double A = rt[0];
@@ -693,11 +691,11 @@ __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const do
     }
   }
 #pragma unroll
-  for (int d = 1; d < kTL; d <<= 1) {
-    Aff o{__shfl_up_sync(0xffffffffu, acc.M, d, kTL), __shfl_up_sync(0xffffffffu, acc.C, d, kTL)};
+  for (int d = 1; d < TL; d <<= 1) {
+    Aff o{__shfl_up_sync(0xffffffffu, acc.M, d, TL), __shfl_up_sync(0xffffffffu, acc.C, d, TL)};
     if (gl >= d) acc = aff_then(o, acc);
   }
-  double yin = __shfl_up_sync(0xffffffffu, acc.C, 1, kTL);
+  double yin = __shfl_up_sync(0xffffffffu, acc.C, 1, TL);
   if (gl == 0) yin = 0.0;
 #pragma unroll
   for (int e = 0; e < EG; e++) {
@@ -716,12 +714,12 @@ __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const do
     }
   }
 #pragma unroll
-  for (int d = 1; d < kTL; d <<= 1) {
-    Aff o{__shfl_down_sync(0xffffffffu, acc.M, d, kTL), __shfl_down_sync(0xffffffffu, acc.C, d, kTL)};
-    if (gl + d < kTL) acc = aff_then(o, acc);
+  for (int d = 1; d < TL; d <<= 1) {
+    Aff o{__shfl_down_sync(0xffffffffu, acc.M, d, TL), __shfl_down_sync(0xffffffffu, acc.C, d, TL)};
+    if (gl + d < TL) acc = aff_then(o, acc);
   }
-  double win = __shfl_down_sync(0xffffffffu, acc.C, 1, kTL);
-  if (gl == kTL - 1) win = 0.0;
+  double win = __shfl_down_sync(0xffffffffu, acc.C, 1, TL);
+  if (gl == TL - 1) win = 0.0;
 #pragma unroll
   for (int e = EG - 1; e >= 0; e--) {
     if (e < cnt) {
@@ -731,12 +729,12 @@ __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const do
   }
   // bordering unknown N (step.F90:526-533)
   const int last_lane = (inner - 1) / EG, last_e = (inner - 1) - last_lane * EG;
-  const double w1 = __shfl_sync(0xffffffffu, y[0], 0, kTL);
+  const double w1 = __shfl_sync(0xffffffffu, y[0], 0, TL);
   double wl = 0.0;
 #pragma unroll
   for (int e = 0; e < EG; e++)
     if (e == last_e) wl = y[e];
-  wl = __shfl_sync(0xffffffffu, wl, last_lane, kTL);
+  wl = __shfl_sync(0xffffffffu, wl, last_lane, TL);
   if (on) {
     const double fN = sl[tpad(N - 1)];
     const double xN = (fN - rt[1] * w1 - A * wl) / rt[2];
@@ -748,9 +746,14 @@ __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const do
 }
 
 // NT > 0: the theta extent as a compile-time constant (equal to g.nth), so
-// that the shared-memory offsets, line strides and divisions by it fold
-template <int E, int CPT, class T, int NT>
-__global__ void __launch_bounds__(256, 2)
+// that the shared-memory offsets, line strides and divisions by it fold.
+// RJ rows of up to NTH / RJ cells: short theta lines take more rows, so that
+// a plane still gives every thread a cell (64 x 32 x 128: 44 us with 2 rows of
+// 32 cells in 256 threads and 32 planes per CTA, 21 with 8 rows and 4 planes);
+// lines beyond 128 cells take two rows in 512 threads, one CTA per SM
+// (256 x 128 x 1024, mixed: 1.35 ms by whole lines per warp, 1.08 here).
+template <int RJ, int NTH, int TL, int E, class T, int NT>
+__global__ void __launch_bounds__(NTH, 512 / NTH)
     k_rhs_march(const __grid_constant__ CUtensorMap tq1, const __grid_constant__ CUtensorMap tq2,
                 const __grid_constant__ CUtensorMap tq3, Geo g, Rk rk, RhsArgsT<T> a, TriPer t13, TriPer t2,
                 int zs, unsigned *status) {
@@ -759,24 +762,24 @@ __global__ void __launch_bounds__(256, 2)
   // offsets of the ghosted fields and of prg (I3, IPRG with this N)
   auto i3 = [&](int i, int j, int k) { return (i - 1) + N * (j + g.J3 * k); };
   auto iprg = [&](int i, int j, int k, int m) { return (i - 1) + N * ((j - 1) + g.nr * ((k - 1) + g.nz * (m - 1))); };
-  const int FS = (kMRJ + 2) * N;    // doubles of one field's box
+  const int FS = (RJ + 2) * N;    // doubles of one field's box
   const int FSP = (FS + 15) & ~15;  // box slots start on 128-byte boundaries
   const int SLOT = 3 * FSP;
   double *ring = sm;                           // [slot][field][row j0-1+rr][i]
-  // line stride of the solve buffers: 8 mod 16 doubles, so the 32 / kTL
+  // line stride of the solve buffers: 8 mod 16 doubles, so the 32 / TL
   // groups of a warp fall on disjoint halves of the shared-memory banks
   const int SPL = ((SPN + 15) & ~15) + 8;
   double *lines = ring + kQRing * SLOT;        // [plane of batch][comp][r], each SPL
   // the factorisation of each (fam, r), 3 SPL apart: 3 SPL is 8 mod 16
   // doubles too, so the two groups of a half-warp, which solve rows r = 0, 1
   // of one family, read disjoint halves of the banks
-  double *fac = lines + kTB * 3 * kMRJ * SPL;  // [fam][r][inv, pp, zz], each SPL
-  __shared__ RowCoef rowc[kMRJ];
-  __shared__ double rowt[kMRJ][2][3];  // sub, sup, za2 of each family
+  double *fac = lines + kTB * 3 * RJ * SPL;  // [fam][r][inv, pp, zz], each SPL
+  __shared__ RowCoef rowc[RJ];
+  __shared__ double rowt[RJ][2][3];  // sub, sup, za2 of each family
   __shared__ __align__(8) uint64_t full[kQRing];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nzb = (g.nz + zs - 1) / zs;
-  const int j0 = 1 + (int)(blockIdx.x / nzb) * kMRJ;
+  const int j0 = 1 + (int)(blockIdx.x / nzb) * RJ;
   const int kb = 1 + (int)(blockIdx.x % nzb) * zs;
   const int ke = min(kb + zs, g.nz + 1);  // planes kb .. ke-1 are evaluated
   const int nplanes = ke - kb + 2;        // planes kb-1 .. ke are loaded
@@ -797,44 +800,34 @@ __global__ void __launch_bounds__(256, 2)
     mbar_init_fence();
     for (int pr = 0; pr < kQRing && pr < nplanes; pr++) issue(pr);
   }
-  for (int idx = tid; idx < 2 * kMRJ * N; idx += blockDim.x) {
-    const int i = idx % N, r = (idx / N) % kMRJ, fam = idx / (N * kMRJ), jc = j0 + r;
+  for (int idx = tid; idx < 2 * RJ * N; idx += blockDim.x) {
+    const int i = idx % N, r = (idx / N) % RJ, fam = idx / (N * RJ), jc = j0 + r;
     if (jc > g.nr) continue;
     const double *inv = fam ? t2.inv : t13.inv, *pp = fam ? t2.pp : t13.pp, *zz = fam ? t2.zz : t13.zz;
-    double *f = fac + (size_t)(fam * kMRJ + r) * 3 * SPL;
+    double *f = fac + (size_t)(fam * RJ + r) * 3 * SPL;
     cp_async8(f + tpad(i), inv + (size_t)jc * N + i);
     cp_async8(f + SPL + tpad(i), pp + (size_t)jc * N + i);
     cp_async8(f + 2 * SPL + tpad(i), zz + (size_t)jc * N + i);
   }
-  if (tid < kMRJ && j0 + tid <= g.nr) {
+  if (tid < RJ && j0 + tid <= g.nr) {
     const int jc = j0 + tid;
     rowc[tid] = row_coef(g, jc);
     rowt[tid][0][0] = t13.sub[jc], rowt[tid][0][1] = t13.sup[jc], rowt[tid][0][2] = t13.za2[jc];
     rowt[tid][1][0] = t2.sub[jc], rowt[tid][1][1] = t2.sup[jc], rowt[tid][1][2] = t2.za2[jc];
   }
-  // this thread's cells: (r, i) = divmod(tid + 256 q, N)
-  int ci[CPT], cr[CPT];
-  bool cact[CPT];
-#pragma unroll
-  for (int q = 0; q < CPT; q++) {
-    const int cell = tid + 256 * q;
-    cr[q] = cell / N;
-    ci[q] = cell % N;
-    cact[q] = cell < kMRJ * N && j0 + cr[q] <= g.nr;
-  }
+  // this thread's cell: (r, i) = divmod(tid, N)
+  const int r = tid / N, i = tid - r * N, jc = j0 + r;
+  const bool cact = r < RJ && jc <= g.nr;
   // prefetched in the storage type: a conversion right after the load
   // would wait for it
-  T pru[CPT][3], ppg[CPT][3];
+  T pru[3], ppg[3];
   auto prefetch = [&](int kc) {
+    if (!cact) return;
+    const int o = i3(i + 1, jc, kc);
 #pragma unroll
-    for (int q = 0; q < CPT; q++) {
-      if (!cact[q]) continue;
-      const int jc = j0 + cr[q], o = i3(ci[q] + 1, jc, kc);
-#pragma unroll
-      for (int m = 0; m < 3; m++) {
-        pru[q][m] = __ldg(a.ru[m] + o);
-        ppg[q][m] = __ldg(a.prg + iprg(ci[q] + 1, jc, kc, m + 1));
-      }
+    for (int m = 0; m < 3; m++) {
+      pru[m] = __ldg(a.ru[m] + o);
+      ppg[m] = __ldg(a.prg + iprg(i + 1, jc, kc, m + 1));
     }
   };
   prefetch(kb);
@@ -850,20 +843,15 @@ __global__ void __launch_bounds__(256, 2)
     bool ok = true;
     if (kc == kb) ok = mbar_wait(&full[0], 0u) && mbar_wait(&full[1 % kQRing], 0u);
     ok = ok && mbar_wait(&full[(pr + 1) % kQRing], (unsigned)((pr + 1) / kQRing) & 1u);
-    T cru[CPT][3], cpg[CPT][3];
+    T cru[3], cpg[3];
 #pragma unroll
-    for (int q = 0; q < CPT; q++)
-#pragma unroll
-      for (int m = 0; m < 3; m++) cru[q][m] = pru[q][m], cpg[q][m] = ppg[q][m];
+    for (int m = 0; m < 3; m++) cru[m] = pru[m], cpg[m] = ppg[m];
     if (kc + 1 < ke) prefetch(kc + 1);
     const double *sp = ring + (size_t)((pr - 1) % kQRing) * SLOT;
     const double *sc = ring + (size_t)(pr % kQRing) * SLOT;
     const double *sn = ring + (size_t)((pr + 1) % kQRing) * SLOT;
-    double *lb = lines + (size_t)pb * 3 * kMRJ * SPL;
-#pragma unroll
-    for (int q = 0; q < CPT; q++) {
-      if (!cact[q]) continue;
-      const int i = ci[q], r = cr[q], jc = j0 + r;
+    double *lb = lines + (size_t)pb * 3 * RJ * SPL;
+    if (cact) {
       const int ip = i + 1 < N ? i + 1 : 0, im = i > 0 ? i - 1 : N - 1;
       const int rc = (r + 1) * N, rn = (r + 2) * N, rs = r * N;  // rows jc, jc+1, jc-1
       const int rjm = jc > 1 ? rs : rc;                          // row max(jc-1, 1)
@@ -877,20 +865,20 @@ __global__ void __launch_bounds__(256, 2)
       S.B6 = n2[rc + i], S.B7 = p2[rc + i], S.B8 = c2[rn + im], S.B9 = p2[rn + i];
       S.C1 = c3[rc + i], S.C2 = c3[rc + ip], S.C3 = c3[rc + im], S.C4 = c3[rn + i], S.C5 = c3[rjm + i];
       S.C6 = n3[rc + i], S.C7 = p3[rc + i], S.C8 = n3[rc + im], S.C9 = n3[rs + i];
-      S.ru1 = (double)cru[q][0], S.ru2 = (double)cru[q][1], S.ru3 = (double)cru[q][2];
-      S.pg1 = (double)cpg[q][0], S.pg2 = (double)cpg[q][1], S.pg3 = (double)cpg[q][2];
+      S.ru1 = (double)cru[0], S.ru2 = (double)cru[1], S.ru3 = (double)cru[2];
+      S.pg1 = (double)cpg[0], S.pg2 = (double)cpg[1], S.pg3 = (double)cpg[2];
       RhsCell v;
       rhs_eval(g, rk, jc, kc, S, rowc[r], v);
       const int o = i3(i + 1, jc, kc);
       a.ru[0][o] = (T)v.h1;
-      lb[(size_t)(0 * kMRJ + r) * SPL + tpad(i)] = v.r1;
+      lb[(size_t)(0 * RJ + r) * SPL + tpad(i)] = v.r1;
       if (kc >= 2) {
         a.ru[2][o] = (T)v.h3;
-        lb[(size_t)(2 * kMRJ + r) * SPL + tpad(i)] = v.r3;
+        lb[(size_t)(2 * RJ + r) * SPL + tpad(i)] = v.r3;
       }
       if (jc >= 2) {
         a.ru[1][o] = (T)v.h2;
-        lb[(size_t)(1 * kMRJ + r) * SPL + tpad(i)] = v.r2;
+        lb[(size_t)(1 * RJ + r) * SPL + tpad(i)] = v.r2;
       }
     }
     // the plane's lines are written and plane kc-1 has been read by all; a
@@ -904,27 +892,28 @@ __global__ void __launch_bounds__(256, 2)
       issue(pr - 1 + kQRing);
     }
     if (pb == kTB - 1 || kc == ke - 1) {
-      // solve the batch's [plane][comp][r] lines, 32 / kTL per warp
-      constexpr int kGroups = 32 / kTL, kSolveWarps = kTB * 3 * kMRJ / kGroups;
-      static_assert(kTB * 3 * kMRJ % kGroups == 0 && kSolveWarps <= 8, "solve batch does not fit the warps");
+      // solve the batch's [plane][comp][r] lines, 32 / TL per warp at a time
+      constexpr int kGroups = 32 / TL, kLines = kTB * 3 * RJ;
+      static_assert(kLines % kGroups == 0, "a warp's lines are all in the batch or none");
       const int kc0 = kc - pb;
-      if (warp < kSolveWarps) {
-        const int L = warp * kGroups + lane / kTL;
-        const int pl = L / (3 * kMRJ), comp = (L / kMRJ) % 3, r = L % kMRJ, jc = j0 + r, lk = kc0 + pl;
+#pragma unroll 1
+      for (int Lw = warp * kGroups; Lw < kLines; Lw += NTH / 32 * kGroups) {
+        const int L = Lw + lane / TL;
+        const int pl = L / (3 * RJ), comp = (L / RJ) % 3, lr = L % RJ, lj = j0 + lr, lk = kc0 + pl;
         const int fam = comp == 1 ? 1 : 0;
-        const double *f = fac + (size_t)(fam * kMRJ + r) * 3 * SPL;
-        const bool on = lk <= kc && jc <= g.nr && !(comp == 1 && jc < 2) && !(comp == 2 && lk < 2);
-        tsolve_group<(32 / kTL) * E>(N, f, f + SPL, f + 2 * SPL, &rowt[r][fam][0], lines + (size_t)L * SPL,
-                                     lane % kTL, on);
+        const double *f = fac + (size_t)(fam * RJ + lr) * 3 * SPL;
+        const bool on = lk <= kc && lj <= g.nr && !(comp == 1 && lj < 2) && !(comp == 2 && lk < 2);
+        tsolve_group<TL, (32 / TL) * E>(N, f, f + SPL, f + 2 * SPL, &rowt[lr][fam][0], lines + (size_t)L * SPL,
+                                        lane % TL, on);
         __syncwarp();
 #pragma unroll
         for (int gq = 0; gq < kGroups; gq++) {
-          const int L2 = warp * kGroups + gq;
-          const int pl2 = L2 / (3 * kMRJ), comp2 = (L2 / kMRJ) % 3, r2 = L2 % kMRJ, jc2 = j0 + r2, lk2 = kc0 + pl2;
+          const int L2 = Lw + gq;
+          const int pl2 = L2 / (3 * RJ), comp2 = (L2 / RJ) % 3, r2 = L2 % RJ, jc2 = j0 + r2, lk2 = kc0 + pl2;
           if (lk2 > kc || jc2 > g.nr || (comp2 == 1 && jc2 < 2) || (comp2 == 2 && lk2 < 2)) continue;
           double *dst = (comp2 == 0 ? a.qrhs[0] : (comp2 == 1 ? a.qrhs[1] : a.qrhs[2])) + i3(1, jc2, lk2);
           const double *src = lines + (size_t)L2 * SPL;
-          for (int i = lane; i < N; i += 32) dst[i] = src[tpad(i)];
+          for (int e = lane; e < N; e += 32) dst[e] = src[tpad(e)];
         }
       }
       __syncthreads();  // the batch's lines are free again
@@ -938,27 +927,28 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
-template <int E, int CPT, class T, int NT = 0>
+template <int RJ, int NTH, int TL, int E, class T, int NT = 0>
 static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) {
   const Geo &g = c->geo;
-  if ((g.nth & 1) || kMRJ * g.nth > 256 * CPT || g.nth - 1 > 32 * E || (NT > 0 && g.nth != NT))
+  if ((g.nth & 1) || RJ * g.nth > NTH || g.nth - 1 > 32 * E || (NT > 0 && g.nth != NT))
     return cudaErrorNotSupported;
   CUtensorMap tm[3];
   for (int m = 0; m < 3; m++)
-    if (!encode_tmap_f64_3d(&tm[m], c->q[m], g.nth, g.J3, g.K3, g.nth, kMRJ + 2, 1)) return cudaErrorNotSupported;
+    if (!encode_tmap_f64_3d(&tm[m], c->q[m], g.nth, g.J3, g.K3, g.nth, RJ + 2, 1)) return cudaErrorNotSupported;
   const int SPN = tpad(g.nth) + 1;
-  const int FS = (kMRJ + 2) * g.nth, FSP = (FS + 15) & ~15;
+  const int FS = (RJ + 2) * g.nth, FSP = (FS + 15) & ~15;
   const int SPL = ((SPN + 15) & ~15) + 8;
-  const size_t sm = sizeof(double) * ((size_t)kQRing * 3 * FSP + kTB * 3 * kMRJ * SPL + 2 * kMRJ * 3 * SPL);
-  if (sm > 110 * 1024) return cudaErrorNotSupported;  // two CTAs per SM
-  auto kern = k_rhs_march<E, CPT, T, NT>;
+  const size_t sm = sizeof(double) * ((size_t)kQRing * 3 * FSP + kTB * 3 * RJ * SPL + 2 * RJ * 3 * SPL);
+  constexpr int ctas = 512 / NTH;  // per SM
+  if (sm > (220 / ctas) * 1024) return cudaErrorNotSupported;
+  auto kern = k_rhs_march<RJ, NTH, TL, E, T, NT>;
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
   const TriPer &t13 = c->ttri[c->irk][0], &t2 = c->ttri[c->irk][1];
-  const int zs = kMarchZ;
-  const int grid = ((g.nr + kMRJ - 1) / kMRJ) * ((g.nz + zs - 1) / zs);
+  const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, ctas * c->nsm);
+  const int grid = rows * ((g.nz + zs - 1) / zs);
   LaunchScope ls(c, PK_RHS);
-  kern<<<grid, 256, sm, c->stream>>>(tm[0], tm[1], tm[2], g, rk, a, t13, t2, zs, c->d_status);
+  kern<<<grid, NTH, sm, c->stream>>>(tm[0], tm[1], tm[2], g, rk, a, t13, t2, zs, c->d_status);
   return cudaGetLastError();
 }
 
@@ -975,14 +965,17 @@ static cudaError_t launch_rhs_tsweep_t(vr_ctx *c, const Rk &rk) {
   a.prg = reinterpret_cast<const T *>(c->prg);
   const int E = (g.nth - 1 + 31) / 32;
   cudaError_t me = cudaErrorNotSupported;
-  if (E <= 1)
-    me = run_rhs_march<1, 1, T>(c, rk, a);
-  else if (E <= 2)
-    me = run_rhs_march<2, 1, T>(c, rk, a);
+  // rows per CTA: as many as its threads have cells for
+  if (g.nth <= 32)
+    me = run_rhs_march<8, 256, 8, 1, T>(c, rk, a);
+  else if (g.nth <= 64)
+    me = run_rhs_march<4, 256, 8, 2, T>(c, rk, a);
   else if (g.nth == 128)
-    me = run_rhs_march<4, 1, T, 128>(c, rk, a);
-  else if (E <= 4)
-    me = run_rhs_march<4, 1, T>(c, rk, a);
+    me = run_rhs_march<2, 256, 8, 4, T, 128>(c, rk, a);
+  else if (g.nth <= 128)
+    me = run_rhs_march<2, 256, 8, 4, T>(c, rk, a);
+  else if (g.nth <= 256)
+    me = run_rhs_march<2, 512, 16, 8, T>(c, rk, a);
   if (me != cudaErrorNotSupported) return me;
   if (E <= 1) return run_rhs_tsweep<1, T>(c, rk, a);
   if (E <= 2) return run_rhs_tsweep<2, T>(c, rk, a);

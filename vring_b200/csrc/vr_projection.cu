@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(128) k_uppres_r(Geo g, double be, const double
 }
 
 // ---------------------------------------------------------------------------
-// z-marching form of uppres.  A CTA owns kUpRJ r-rows and up to zs planes
-// and walks them in z; dph of rows j0-2 .. j0+kUpRJ at each plane arrives
+// z-marching form of uppres.  A CTA owns RJ r-rows and up to zs planes
+// and walks them in z; dph of rows j0-2 .. j0+RJ at each plane arrives
 // through a ring of kUpRing shared-memory slots filled by TMA three planes
 // ahead (plane kc+1 is read through the north-ghost map, so the slot of
 // plane nz+1 holds plane nz; rows and planes below 0 read as zero and are
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(128) k_uppres_r(Geo g, double be, const double
 // thread of row nr the slip ghosts of row nrc, and the CTA holding plane nz
 // takes one more step for the north ghost plane nzc (dph read there through
 // the north-ghost map, i.e. plane nz, already in the ring).
-constexpr int kUpRJ = 2, kUpRing = 7, kUpZ = 32;
+constexpr int kUpRing = 7;
 
 // The fields upsol reads and writes.
 template <class T>
@@ -277,21 +277,26 @@ struct UpsolArgs {
   double adt;
 };
 
-// NT > 0: the theta extent as a compile-time constant (equal to g_in.nth)
-template <class T, bool UPSOL, int NT>
-__global__ void __launch_bounds__(256, 2)
+// NT > 0: the theta extent as a compile-time constant (equal to g_in.nth).
+// RJ rows of up to NTH / RJ cells: short theta lines take more rows, so that a
+// plane gives every thread a cell (64 x 32 x 128: 31 us with 2 rows of 32
+// cells in 256 threads and 32 planes per CTA, 13 with 8 rows and 4 planes);
+// lines beyond 128 cells take two rows in 512 threads (256 x 128 x 1024,
+// mixed: 0.97 ms as two kernels, 0.70 here).
+template <class T, bool UPSOL, int RJ, int NTH, int NT>
+__global__ void __launch_bounds__(NTH, 512 / NTH)
     k_uppres_march(const __grid_constant__ CUtensorMap tdph, Geo g_in, double be, T *__restrict__ prg,
                    T *__restrict__ pres, double *__restrict__ dphw, int zs, unsigned *status, UpsolArgs<T> us) {
   extern __shared__ __align__(128) double sm[];
   Geo g = g_in;
   if constexpr (NT > 0) g.nth = NT;
   const int N = g.nth;
-  constexpr int RR = kUpRJ + 3;  // rows j0-2 .. j0+kUpRJ
+  constexpr int RR = RJ + 3;  // rows j0-2 .. j0+RJ
   const int SLOT = (RR * N + 15) & ~15;
   __shared__ __align__(8) uint64_t full[kUpRing];
   const int tid = threadIdx.x;
   const int nzb = (g.nz + zs - 1) / zs;
-  const int j0 = 1 + (int)(blockIdx.x / nzb) * kUpRJ;
+  const int j0 = 1 + (int)(blockIdx.x / nzb) * RJ;
   const int kb = 1 + (int)(blockIdx.x % nzb) * zs;
   const int ke = min(kb + zs, g.nz + 1);  // planes kb .. ke-1 are updated
   const int nplanes = ke - kb + 3;        // planes kb-2 .. ke are loaded
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(256, 2)
     for (int pr = 0; pr < kUpRing && pr < nplanes; pr++) issue(pr);
   }
   const int r = tid / N, i = tid % N, jc = j0 + r;
-  const bool act = tid < kUpRJ * N && jc <= g.nr;
+  const bool act = tid < RJ * N && jc <= g.nr;
   const int ip = i + 1 < N ? i + 1 : 0, im = i > 0 ? i - 1 : N - 1, imm = im > 0 ? im - 1 : N - 1;
   UpRow m{};
   if (act) m = up_row(g, jc);
@@ -419,31 +424,35 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
-template <class T, bool UPSOL, int NT = 0>
+template <class T, bool UPSOL, int RJ, int NTH, int NT = 0>
 static cudaError_t run_uppres_march_n(vr_ctx *c, double be, double adt) {
   const Geo &g = c->geo;
-  if ((g.nth & 1) || kUpRJ * g.nth > 256 || (NT > 0 && g.nth != NT)) return cudaErrorNotSupported;
+  if ((g.nth & 1) || RJ * g.nth > NTH || (NT > 0 && g.nth != NT)) return cudaErrorNotSupported;
   CUtensorMap tm;
-  if (!encode_tmap_f64_3d(&tm, c->dph, g.nth, g.nr + 2, g.nz + 2, g.nth, kUpRJ + 3, 1))
+  if (!encode_tmap_f64_3d(&tm, c->dph, g.nth, g.nr + 2, g.nz + 2, g.nth, RJ + 3, 1))
     return cudaErrorNotSupported;
-  const int SLOT = ((kUpRJ + 3) * g.nth + 15) & ~15;
+  const int SLOT = ((RJ + 3) * g.nth + 15) & ~15;
   const size_t sm = sizeof(double) * (size_t)kUpRing * SLOT;
-  auto kern = k_uppres_march<T, UPSOL, NT>;
+  auto kern = k_uppres_march<T, UPSOL, RJ, NTH, NT>;
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
-  const int zs = kUpZ;
-  const int grid = ((g.nr + kUpRJ - 1) / kUpRJ) * ((g.nz + zs - 1) / zs);
+  const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, 512 / NTH * c->nsm);
+  const int grid = rows * ((g.nz + zs - 1) / zs);
   UpsolArgs<T> us{reinterpret_cast<const T *>(c->dq[0]), reinterpret_cast<const T *>(c->dq[1]),
                   reinterpret_cast<const T *>(c->dq[2]), c->q[0], c->q[1], c->q[2], adt};
-  kern<<<grid, 256, sm, c->stream>>>(tm, g, be, reinterpret_cast<T *>(c->prg), reinterpret_cast<T *>(c->pres),
+  kern<<<grid, NTH, sm, c->stream>>>(tm, g, be, reinterpret_cast<T *>(c->prg), reinterpret_cast<T *>(c->pres),
                                       c->dph, zs, c->d_status, us);
   return cudaGetLastError();
 }
 
 template <class T, bool UPSOL>
 static cudaError_t run_uppres_march(vr_ctx *c, double be, double adt) {
-  if (c->geo.nth == 128) return run_uppres_march_n<T, UPSOL, 128>(c, be, adt);
-  return run_uppres_march_n<T, UPSOL>(c, be, adt);
+  const int n = c->geo.nth;
+  if (n == 128) return run_uppres_march_n<T, UPSOL, 2, 256, 128>(c, be, adt);
+  if (n <= 32) return run_uppres_march_n<T, UPSOL, 8, 256>(c, be, adt);
+  if (n <= 64) return run_uppres_march_n<T, UPSOL, 4, 256>(c, be, adt);
+  if (n <= 128) return run_uppres_march_n<T, UPSOL, 2, 256>(c, be, adt);
+  return run_uppres_march_n<T, UPSOL, 2, 512>(c, be, adt);
 }
 
 cudaError_t launch_uppres(vr_ctx *c, const Rk &rk) {
