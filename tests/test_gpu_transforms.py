@@ -9,7 +9,7 @@ Poisson solve."""
 import numpy as np
 import pytest
 
-from parity_util import make_pair, prep, seed_random
+from parity_util import assert_field_close, make_pair, prep, seed_random
 
 pytestmark = pytest.mark.gpu
 
@@ -34,6 +34,27 @@ def test_folded_lengths_match_oracle(grid):
     r = orc.field("dph")[:, 1:nr + 1, 1:nz + 1]
     assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
     assert np.array_equal(gpu.get("rhs"), rhs)  # the right-hand side is an input
+
+
+# z of 1024: tiles of 8 slots streamed (theta a multiple of 8; more tiles than
+# SMs, so that the buffers rotate), else whole columns per warp; z lines of
+# 1025 positions in 64 chunks (even theta) or the shared-memory sweep
+@pytest.mark.parametrize("grid", [(8, 5, 1024), (24, 4, 1024), (256, 16, 1024), (12, 4, 1024), (5, 4, 1024)],
+                         ids=lambda g: "x".join(map(str, g)))
+def test_long_z_lines_match_oracle(grid):
+    nth, nr, nz = grid
+    orc, gpu = make_pair(nth, nr, nz)
+    seed_random(orc, gpu, ["rhs", "q1", "q2", "q3", "ru1", "ru2", "ru3", "prg", "dq1", "dq2", "dq3"], seed=9, scale=0.1)
+    prep(orc, gpu)
+    orc.laplace_solve()
+    gpu.laplace_solve()
+    g = gpu.get("dph")[:, 1:nr + 1, 1:nz + 1]
+    r = orc.field("dph")[:, 1:nr + 1, 1:nz + 1]
+    assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
+    orc.step()
+    gpu.step()
+    for n in ("dq1", "dq2", "dq3"):
+        assert_field_close(gpu, orc, n)
 
 
 def test_folded_columns_above_two_ctas_per_sm():

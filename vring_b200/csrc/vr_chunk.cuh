@@ -23,10 +23,31 @@ namespace vr {
 // In-place exclusive scan of the NCH chunk maps of each line held in
 // sM/sC[chunk][line]; forward (chunk 0 first) or backward (last chunk
 // first).  Every warp scans 32 / NCH lines, NCH lanes per line.  On return
-// sC[chunk][line] is the recurrence value entering the chunk.
+// sC[chunk][line] is the recurrence value entering the chunk.  With 64 chunks a
+// warp scans one line, two adjacent chunks per lane.
 template <bool FORWARD, int NCH, int LPT = 32>
 __device__ __forceinline__ void chain_chunks(double (*sM)[LPT + 1], double (*sC)[LPT + 1], int warp, int lane) {
-  constexpr int LPW = 32 / NCH;  // lines per warp
+  if constexpr (NCH == 64) {
+    if (warp >= LPT) return;
+    const int c0 = 2 * lane, c1 = c0 + 1;
+    const double M0 = sM[c0][warp], C0 = sC[c0][warp], M1 = sM[c1][warp], C1 = sC[c1][warp];
+    double M = M0 * M1, C = FORWARD ? C1 + M1 * C0 : C0 + M0 * C1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const double om = FORWARD ? __shfl_up_sync(0xffffffffu, M, d) : __shfl_down_sync(0xffffffffu, M, d);
+      const double oc = FORWARD ? __shfl_up_sync(0xffffffffu, C, d) : __shfl_down_sync(0xffffffffu, C, d);
+      if (FORWARD ? lane >= d : lane + d < 32) {
+        C = C + M * oc;
+        M = M * om;
+      }
+    }
+    double in = FORWARD ? __shfl_up_sync(0xffffffffu, C, 1) : __shfl_down_sync(0xffffffffu, C, 1);
+    if (FORWARD ? lane == 0 : lane == 31) in = 0.0;
+    sC[c0][warp] = FORWARD ? in : C1 + M1 * in;
+    sC[c1][warp] = FORWARD ? C0 + M0 * in : in;
+    return;
+  }
+  constexpr int LPW = NCH <= 32 ? 32 / NCH : 1;  // lines per warp
   const int ch = lane % NCH, line = warp * LPW + lane / NCH;
   if (line >= LPT) return;  // warps beyond the tile's lines
   double M = sM[ch][line], C = sC[ch][line];
@@ -178,6 +199,10 @@ __global__ void __launch_bounds__(32 * NCH, NCH == 16 ? 2 : 1) k_chunk(P p) {
 struct TmaTile {
   int nbox, br, ldim;
 };
+template <int NP, class P>
+__host__ __device__ constexpr bool chunk_tab_dyn() {
+  return !P::kLineIB && NP > 544;
+}
 
 template <int LPT, int NCH, int MAXCL, int S, int MINB, class P>
 __global__ void __launch_bounds__(LPT *NCH, MINB)
@@ -190,9 +215,14 @@ __global__ void __launch_bounds__(LPT *NCH, MINB)
   // chunk maps of the forward and the backward substitution (separate, so
   // that one tile needs four CTA barriers)
   __shared__ double sM[NCH][LPT + 1], sC[NCH][LPT + 1], sMb[NCH][LPT + 1], sCb[NCH][LPT + 1];
-  __shared__ double2 sAB[kLine ? 1 : NP];  // (a, ib) per position
-  __shared__ double sMf[kLine ? 1 : NP];   // -a ib
-  __shared__ double sU[kLine ? 1 : NP];    // c ib
+  // (a, ib), -a ib and c ib per position; behind the stages where they would
+  // pass the 48 KB of static shared memory
+  constexpr bool kTabDyn = chunk_tab_dyn<NP, P>();
+  __shared__ double2 sAB_[kLine || kTabDyn ? 1 : NP];
+  __shared__ double sMf_[kLine || kTabDyn ? 1 : NP], sU_[kLine || kTabDyn ? 1 : NP];
+  double *const tab = stage + (size_t)S * tt.nbox * tt.br * LPT;
+  double2 *const sAB = kTabDyn ? reinterpret_cast<double2 *>(tab) : sAB_;
+  double *const sMf = kTabDyn ? tab + 2 * NP : sMf_, *const sU = kTabDyn ? tab + 3 * NP : sU_;
   __shared__ double sA[kLine ? NP : 1], sCc[kLine ? NP : 1];
   __shared__ __align__(8) uint64_t full[S];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -411,7 +441,8 @@ cudaError_t run_chunk_tma(P p, const void *base, int d0, int d1, int d2, int ldi
                 "tile rows must tile 128-byte boundaries");
   tt.br = (tt.br + kRowAlign - 1) / kRowAlign * kRowAlign;
   if (tt.br > 256 || ((size_t)tt.br * LPT * 8) % 128) return cudaErrorNotSupported;
-  const size_t dyn = sizeof(double) * (size_t)S * tt.nbox * tt.br * LPT;
+  const size_t dyn = sizeof(double) * ((size_t)S * tt.nbox * tt.br * LPT +
+                                       (chunk_tab_dyn<NCH * MAXCL, P>() ? (size_t)4 * NCH * MAXCL : 0));
   CUtensorMap tm;
   if (!encode_tmap_f64_3d(&tm, base, d0, d1, d2, LPT, ldim == 1 ? tt.br : 1, ldim == 2 ? tt.br : 1))
     return cudaErrorNotSupported;

@@ -12,7 +12,7 @@
 #include <utility>
 #include <vector>
 
-#include "vr_fold.cuh"
+#include "vr_lin.cuh"
 #include "vr_internal.cuh"
 
 using vr::Geo;
@@ -476,16 +476,6 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
     }
   }
   size_t o_twt = blob.add(twt), o_twz = blob.add(twz);
-  const bool th_fold = !fft_theta_length(N), z_fold = !fft_z_length(d.nz);
-  size_t o_fold[4] = {};
-  for (int kind = 0; kind < 2; kind++) {
-    if (!(kind == kFoldZ ? z_fold : th_fold)) continue;
-    std::vector<double> f, i;
-    fold_tables(kind, kind == kFoldZ ? d.nz : N, f, i);
-    o_fold[2 * kind] = blob.add(f);
-    o_fold[2 * kind + 1] = blob.add(i);
-  }
-
   c->dcoef_len = blob.v.size();
   if (cudaMalloc(&c->dcoef, sizeof(double) * c->dcoef_len) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMemcpy(c->dcoef, blob.v.data(), sizeof(double) * c->dcoef_len, cudaMemcpyHostToDevice) !=
@@ -514,9 +504,18 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
   c->pois_ib = D + o_pib;
   c->tw_th = D + o_twt;
   c->tw_z = D + o_twz;
-  for (int i = 0; i < 2; i++) {
-    c->fold_z[i] = z_fold ? D + o_fold[2 * kFoldZ + i] : nullptr;
-    c->fold_th[i] = th_fold ? D + o_fold[2 * kFoldTh + i] : nullptr;
+  {  // tables of the lengths without an FFT
+    const bool th = !fft_length(N), z = !fft_length(d.nz);
+    size_t len[4] = {}, total = 0;
+    for (int kind = 0; kind < 4; kind++)
+      if (lin_theta(kind) ? th : z) total += len[kind] = lin_table_len(kind, lin_theta(kind) ? N : d.nz);
+    if (total && cudaMalloc(&c->lin_tab, sizeof(double) * total) != cudaSuccess) return fail(VR_ERR_OOM);
+    double *t = c->lin_tab;
+    for (int kind = 0; kind < 4; t += len[kind++])
+      if (len[kind]) {
+        if (lin_table(kind, lin_theta(kind) ? N : d.nz, t, c->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
+        (lin_theta(kind) ? c->lin_th : c->lin_z)[kind & 1] = t;
+      }
   }
   // host copies for the hdnbc scalars
   c->h_rc = new double[m.rc.size()];
@@ -549,7 +548,7 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
     if (cudaMemsetAsync(*o.p, 0, o.w * o.n, c->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
     c->state.emplace_back(*o.p, o.w * o.n);
   }
-  if (z_fold && cudaMalloc(&c->spec2, sizeof(double) * nrs) != cudaSuccess) return fail(VR_ERR_OOM);
+  if (c->lin_z[0] && cudaMalloc(&c->spec2, sizeof(double) * nrs) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&c->d_count, sizeof(unsigned long long) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMemsetAsync(c->d_count, 0, sizeof(unsigned long long) * 4, c->stream) != cudaSuccess)
     return fail(VR_ERR_CUDA);
@@ -567,7 +566,7 @@ extern "C" int vr_destroy(vr_ctx *c) {
   for (int i = 0; i < 4; i++)
     if (c->graph_ok[i]) cudaGraphExecDestroy(c->graph[i]);
   double *ptrs[] = {c->q[0], c->q[1], c->q[2], c->dq[0], c->dq[1], c->dq[2], c->ru[0], c->ru[1],
-                    c->ru[2], c->qrhs[0], c->qrhs[1], c->qrhs[2], c->pres, c->prg, c->rhs, c->spec, c->spec2,
+                    c->ru[2], c->qrhs[0], c->qrhs[1], c->qrhs[2], c->pres, c->prg, c->rhs, c->spec, c->spec2, c->lin_tab,
                     c->dph, c->csort, c->dq3no, c->corr3n, c->corr3s, c->tconv, c->dcoef, c->d_red};
   for (double *p : ptrs)
     if (p) cudaFree(p);

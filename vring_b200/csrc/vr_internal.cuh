@@ -148,6 +148,7 @@ struct vr_ctx {
   double *q[3], *dq[3], *ru[3], *qrhs[3];
   double *prg, *pres, *rhs, *dph, *spec;
   double *spec2;  // second spectral buffer (z lengths without an FFT), or null
+  double *lin_tab;  // the memory behind lin_th and lin_z
   double *csort, *dq3no, *corr3n, *corr3s, *tconv;
   // device coefficient storage (one allocation) and family tables
   double *dcoef;
@@ -157,7 +158,7 @@ struct vr_ctx {
   const double *pois_ib;                   // (nth/2+1, nr, nz) -> [kz][j][mm]
   const double *pois_a, *pois_c;           // aa/cc with aa(1)=0, cc(nr)=0
   const double *tw_th;                     // theta twiddles (cos, sin) 2*nth
-  const double *fold_th[2], *fold_z[2];    // forward, inverse tables of lengths without an FFT (vr_fold.cuh), or null
+  const double *lin_th[2], *lin_z[2];      // forward, inverse tables of lengths without an FFT (vr_lin.cuh), or null
   const double *tw_z;                      // z twiddles for FFT (cos,sin) n and DCT shifts
   // host-side copies needed for hdnbc scalars
   double *h_rc, *h_rm, *h_da, *h_qc;
@@ -315,8 +316,7 @@ cudaError_t launch_divq(vr_ctx *c, const Rk &rk);
 // poisson_takes_dq
 cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk = nullptr);
 bool poisson_takes_dq(const vr_ctx *c);
-bool fft_theta_length(int n);
-bool fft_z_length(int n);
+bool fft_length(int n);
 // the z transform of ncol columns outside a context (twz: cos, sin of
 // 2 pi n / nz, then of pi k / (2 nz)); lengths dct_columns_length takes
 bool dct_columns_length(int n);

@@ -39,7 +39,7 @@
 #include <string>
 #include <vector>
 
-#include "vr_fold.cuh"
+#include "vr_lin.cuh"
 #include "vr_internal.cuh"
 #include "vr_learned.cuh"
 
@@ -66,7 +66,7 @@ enum K2dScal {
 enum K2dPart { PT_A = 0, PT_B, PT_C, PT_D, PT_N };
 // flags: [0] done, [1] iterations, [2] iteration cap, [3] a resident kernel's wait gave up
 // how the direct solve's z transforms run
-enum K2dZ { K2D_Z_FFT = 0, K2D_Z_FOLD, K2D_Z_GEMM };
+enum K2dZ { K2D_Z_FFT = 0, K2D_Z_LIN, K2D_Z_GEMM };
 }  // namespace vr
 
 #include "vr_krylov_res.cuh"
@@ -90,9 +90,9 @@ struct vr_k2d {
   unsigned long long *res_mem = nullptr;
   size_t res_words = 0;
   unsigned res_epoch = 1;
-  // direct solve: the z transforms' tables (dct_f, dct_i: folded matrices, or
-  // nz x nz ones, row-major [kz][k] and [k][kz], for long lines; or the FFT's
-  // twiddles in dct_f alone) and the radial Thomas factorisation per z mode
+  // direct solve: the z transforms' tables (dct_f, dct_i: those of vr_lin.cuh,
+  // or nz x nz matrices, row-major [kz][k] and [k][kz], for long lines; or the
+  // FFT's twiddles in dct_f alone) and the radial Thomas factorisation per z mode
   int zform = 0;  // K2D_Z_*
   double *dct_f = nullptr, *dct_i = nullptr, *tlo = nullptr, *tup = nullptr, *tib = nullptr;
   double *tmp = nullptr;
@@ -974,8 +974,8 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
       coef[4 * nr + (size_t)nr * nz + j + (size_t)nr * kk] = 1.0 / std::sqrt(dg);
     }
   // z transforms of the direct solve: DCT-II scaled 1/(2 nz) (REDFT10) and
-  // DCT-III (REDFT01), by FFT, as folded products, or as full products where
-  // the folded form's columns do not fit shared memory
+  // DCT-III (REDFT01), by FFT, as products from shared memory, or as tiled
+  // products where a column does not fit it
   const double pi = std::acos(-1.0);
   std::vector<double> cf, ci;
   if (dct_columns_length(nz)) {
@@ -987,9 +987,8 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
       cf[2 * nz + 2 * q] = std::cos(pi * q / (2.0 * nz));
       cf[2 * nz + 2 * q + 1] = std::sin(pi * q / (2.0 * nz));
     }
-  } else if (fold_fits(nz)) {
-    k->zform = K2D_Z_FOLD;
-    fold_tables(kFoldZ, nz, cf, ci);
+  } else if (lin_fits(nz)) {
+    k->zform = K2D_Z_LIN;
   } else {
     k->zform = K2D_Z_GEMM;
     cf.resize((size_t)nz * nz);
@@ -1027,8 +1026,12 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
   if (cudaMalloc(&k->flags, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->cnt, sizeof(unsigned) * 8) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMemset(k->cnt, 0, sizeof(unsigned) * 8) != cudaSuccess) return fail(VR_ERR_CUDA);
-  if (cudaMalloc(&k->dct_f, sizeof(double) * cf.size()) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (!ci.empty() && cudaMalloc(&k->dct_i, sizeof(double) * ci.size()) != cudaSuccess) return fail(VR_ERR_OOM);
+  const bool lin = k->zform == K2D_Z_LIN;
+  const size_t nf = lin ? lin_table_len(kLinZFwd, nz) : cf.size(), ni = lin ? lin_table_len(kLinZInv, nz) : ci.size();
+  if (cudaMalloc(&k->dct_f, sizeof(double) * nf) != cudaSuccess) return fail(VR_ERR_OOM);
+  if (ni && cudaMalloc(&k->dct_i, sizeof(double) * ni) != cudaSuccess) return fail(VR_ERR_OOM);
+  if (lin && (lin_table(kLinZFwd, nz, k->dct_f, k->stream) || lin_table(kLinZInv, nz, k->dct_i, k->stream)))
+    return fail(VR_ERR_CUDA);
   if (cudaMalloc(&k->tlo, sizeof(double) * nr) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->tup, sizeof(double) * nr) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->tib, sizeof(double) * ib.size()) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -1128,9 +1131,9 @@ static cudaError_t k2d_direct_dev(vr_k2d *k, const double *f, double *x) {
   // fh(j, kz) = sum_k f(j, k) cf[kz][k], or x(j, k) = sum_kz sol(j, kz) ci[k][kz]
   auto transform = [&](const double *in, double *out, bool fwd) {
     if (k->zform == K2D_Z_FFT) return dct_columns(in, out, nr, nz, fwd ? 1 : -1, k->dct_f, k->stream);
-    if (k->zform == K2D_Z_FOLD)
-      return fwd ? fold_run<kFoldZ, +1>(in, out, k->dct_f, nz, nr, 0, k->nsm, k->stream)
-                 : fold_run<kFoldZ, -1>(in, out, k->dct_i, nz, nr, 0, k->nsm, k->stream);
+    if (k->zform == K2D_Z_LIN)
+      return fwd ? lin_run<kLinZFwd>(in, out, k->dct_f, nz, nr, 0, k->nsm, k->stream)
+                 : lin_run<kLinZInv>(in, out, k->dct_i, nz, nr, 0, k->nsm, k->stream);
     k2d_gemm_abt<<<dim3((nr + 63) / 64, (nz + 63) / 64), 256, 0, k->stream>>>(nr, nz, nz, in,
                                                                             fwd ? k->dct_f : k->dct_i, out);
     return cudaGetLastError();

@@ -1296,6 +1296,25 @@ static cudaError_t dispatch_linesweep(vr_ctx *c, const SweepArgsT<T> &s, const C
     if (e != cudaErrorNotSupported) return e;
     return launch_chunk(p, p.nbx * nm2, c->stream);
   }
+  // up to 1088 positions: 8-line tiles as 64 chunks, one CTA per SM (two
+  // stages of 1026 rows of 64 bytes fill 131 KB).  The z lines of
+  // 256 x 128 x 1024 (1025 positions): 460 us per sweep through the
+  // shared-memory tile below, LONGZ here
+  if (s.n <= 64 * 17 && !(s.nth & 1) && !c->mixed) {
+    MomLine<T> p;
+    p.s = s;
+    p.a = cf.a;
+    p.c = cf.c;
+    p.ib = cf.ib;
+    p.n = s.n;
+    const Geo &g = c->geo;
+    const bool along_r = s.se == g.nth;
+    LaunchScope ls(c, along_r ? PK_RSWEEP : PK_ZSWEEP);
+    const cudaError_t e = run_chunk_tma<8, 64, 17, 2, 1>(p, s.in, g.nth, g.J3, g.K3, along_r ? 1 : 2, nm2, c->nsm,
+                                                         c->d_status, c->stream);
+    if (e != cudaErrorNotSupported) return e;
+    c->nlaunch--;  // nothing was launched
+  }
   if (s.n <= 640) return run_linesweep<16, 16, T>(c, s, cf, nm2);
   if (s.n <= 1600) return run_linesweep<8, 32, T>(c, s, cf, nm2);
   return run_linesweep<4, 64, T>(c, s, cf, nm2);

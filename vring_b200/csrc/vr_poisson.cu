@@ -5,8 +5,8 @@
 //   r:     one tridiagonal solve per (theta mode, z mode) (poisson_solve.F90:270-323)
 //   back:  DCT-III along z, inverse packed DFT along theta, copied into dph.
 //
-// Power-of-two lengths from 32 run FFTs (twiddles computed on the host in
-// double); the other lengths are folded matrix products (vr_fold.cuh).  The radial
+// Power-of-two lengths run FFTs (twiddles computed on the host in double); the
+// other lengths are matrix products (vr_lin.cuh).  The radial
 // factorisation depends only on (theta mode, z mode) and is built once at
 // vr_create; the solve streams the right-hand side through a shared-memory
 // tile and runs the two substitutions chunk-parallel (see vr_momentum.cu).
@@ -15,7 +15,7 @@
 
 #include "vr_chunk.cuh"
 #include "vr_fft.cuh"
-#include "vr_fold.cuh"
+#include "vr_lin.cuh"
 #include "vr_internal.cuh"
 
 namespace vr {
@@ -50,6 +50,75 @@ __device__ void smem_fft(double *re, double *im, int n, int lpb, const double *_
       im[i1] = ai + ti;
     }
     __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// theta transforms of 4, 8 and 16 contiguous values
+// ---------------------------------------------------------------------------
+__global__ void k_fft_fwd(const double *__restrict__ in, double *__restrict__ out, int N, int logn,
+                          int lpb, int nlines, const double *__restrict__ tw) {
+  extern __shared__ double sm[];
+  double *re = sm, *im = sm + lpb * N;
+  int line0 = blockIdx.x * lpb;
+  int nl = min(lpb, nlines - line0);
+  for (int idx = threadIdx.x; idx < lpb * N; idx += blockDim.x) {
+    int l = idx / N, n = idx % N;
+    double v = l < nl ? in[(size_t)(line0 + l) * N + n] : 0.0;
+    re[l * N + brev(n, logn)] = v;
+    im[l * N + brev(n, logn)] = 0.0;
+  }
+  __syncthreads();
+  smem_fft(re, im, N, lpb, tw, -1);
+  for (int idx = threadIdx.x; idx < nl * N; idx += blockDim.x) {
+    int l = idx / N, s = idx % N;  // output slot s (0-based)
+    double v;
+    if (s == 0) {
+      v = re[l * N] / N;
+    } else if (s & 1) {  // a_k, k = (s+1)/2
+      int k = (s + 1) >> 1;
+      v = 2.0 * re[l * N + k] / N;
+    } else {  // b_k, k = s/2 (k < N/2)
+      int k = s >> 1;
+      v = -2.0 * im[l * N + k] / N;
+    }
+    out[(size_t)(line0 + l) * N + s] = v;
+  }
+}
+
+// inverse: packed -> values; writes into dph(i, j, k) (j = 1..nr, k = 1..nz)
+__global__ void k_fft_bwd(const double *__restrict__ in, double *__restrict__ dph, Geo g, int logn, int lpb,
+                          int nlines, const double *__restrict__ tw) {
+  extern __shared__ double sm[];
+  const int N = g.nth;
+  double *re = sm, *im = sm + lpb * N;
+  int line0 = blockIdx.x * lpb;
+  int nl = min(lpb, nlines - line0);
+  for (int idx = threadIdx.x; idx < lpb * N; idx += blockDim.x) {
+    int l = idx / N, k = idx % N;
+    double fr = 0.0, fi = 0.0;
+    if (l < nl) {
+      const double *p = in + (size_t)(line0 + l) * N;
+      int kk = k <= N / 2 ? k : N - k;  // Hermitian extension
+      if (kk == 0) {
+        fr = p[0];
+      } else {
+        fr = p[2 * kk - 1] / 2.0;
+        fi = (2 * kk < N) ? -1.0 * p[2 * kk] / 2.0 : 0.0;
+      }
+      if (k > N / 2) fi = -fi;
+      if (2 * kk == N) fi = 0.0;
+    }
+    re[l * N + brev(k, logn)] = fr;
+    im[l * N + brev(k, logn)] = fi;
+  }
+  __syncthreads();
+  smem_fft(re, im, N, lpb, tw, +1);
+  for (int idx = threadIdx.x; idx < nl * N; idx += blockDim.x) {
+    int l = idx / N, n = idx % N;
+    int L = line0 + l;  // L = (j-1) + nr*(k-1)
+    int j = 1 + L % g.nr, k = 1 + L / g.nr;
+    dph[IDP(g, n + 1, j, k)] = re[l * N + n];
   }
 }
 
@@ -821,13 +890,14 @@ __device__ __forceinline__ int pfft_r2(int k2, int a, int c) {
   return 64 * k2 + 8 * c + (a ^ (((k2 & 3) << 1) | (c & 1)));
 }
 
-// Forward DFT of x[u + 64 q] held in re/im[q] by thread u of pair `pair`;
-// column `pair` of the swizzled tile b is the scratch (its rows no longer
-// needed: the caller has synchronised the pair after its last read).  On
-// return slot brev3(d) holds X[k2 + 8 c + 64 d] (k2 = pfft_k2(u), c =
-// pfft_c(u)); the scratch is still being read until the pair synchronises.
+// Forward DFT of x[u + 64 q] held in re/im[q] by thread u of a group of 64;
+// at(r), r = 0 .. 511, is its scratch column (its rows no longer needed: the
+// caller has synchronised the group after its last read), sync() its barrier.
+// On return slot brev3(d) holds X[k2 + 8 c + 64 d] (k2 = pfft_k2(u), c =
+// pfft_c(u)); the scratch is still being read until the group synchronises.
 // tw1[(k2 - 1) 64 + n1] = W_512^{n1 k2}, tw2[(c - 1) 8 + a] = W_64^{a c}.
-__device__ __forceinline__ void pair_fft512(double (&re)[8], double (&im)[8], double2 *b, int pair, int u,
+template <class At, class Sync>
+__device__ __forceinline__ void pair_fft512(double (&re)[8], double (&im)[8], const At &at, const Sync &sync, int u,
                                             const double2 *tw1, const double2 *tw2) {
   constexpr int N = 512;
   // 8-point DFTs over n2, then W_512^{n1 k2}; entry (n1, k2) at row 64 k2 + n1
@@ -837,35 +907,35 @@ __device__ __forceinline__ void pair_fft512(double (&re)[8], double (&im)[8], do
     const int rg = brev_c(k2, 3);
     double yr = re[rg], yi = im[rg];
     if (k2) tw_mul(yr, yi, tw1[(k2 - 1) * 64 + u]);
-    *swz_pair(b, 64 * k2 + u, pair) = make_double2(yr, yi);
+    *at(64 * k2 + u) = make_double2(yr, yi);
   }
-  pair_sync(pair);
+  sync();
   // thread (k2, a) = (u / 8, u % 8): 8-point DFTs over b of Y'[a + 8 b][k2]
   {
     const int k2 = u >> 3, a = u & 7;
 #pragma unroll
     for (int bb = 0; bb < 8; bb++) {
-      const double2 v = *swz_pair(b, 64 * k2 + a + 8 * bb, pair);
+      const double2 v = *at(64 * k2 + a + 8 * bb);
       re[bb] = v.x;
       im[bb] = v.y;
     }
     reg_dif<8, N, 0, 8>(re, im);
-    pair_sync(pair);  // every entry of the first transpose has been read
+    sync();  // every entry of the first transpose has been read
 #pragma unroll
     for (int c = 0; c < 8; c++) {
       const int rg = brev_c(c, 3);
       double yr = re[rg], yi = im[rg];
       if (c) tw_mul(yr, yi, tw2[(c - 1) * 8 + a]);
-      *swz_pair(b, pfft_r2(k2, a, c), pair) = make_double2(yr, yi);
+      *at(pfft_r2(k2, a, c)) = make_double2(yr, yi);
     }
   }
-  pair_sync(pair);
+  sync();
   // thread (k2, c): 8-point DFTs over a
   {
     const int k2 = pfft_k2(u), c = pfft_c(u);
 #pragma unroll
     for (int a = 0; a < 8; a++) {
-      const double2 v = *swz_pair(b, pfft_r2(k2, a, c), pair);
+      const double2 v = *at(pfft_r2(k2, a, c));
       re[a] = v.x;
       im[a] = v.y;
     }
@@ -933,6 +1003,8 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
       break;
     }
     double2 *const b = buf(s);
+    auto at = [&](int r) { return swz_pair(b, r, pair); };
+    auto sync = [&] { pair_sync(pair); };
     double re[8], im[8];
     if (DIR > 0) {
       // z_n = v^a_n + i v^b_n for n = u + 64 q; the lanes with u & 4 read
@@ -948,7 +1020,7 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
         im[q + 4] = sw ? vA.y : vB.y;
       }
       pair_sync(pair);
-      pair_fft512(re, im, b, pair, u, tw1, tw2);
+      pair_fft512(re, im, at, sync, u, tw1, tw2);
       refill(s);
       pair_sync(pair);
 #pragma unroll
@@ -988,7 +1060,7 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
         im[q] = -(vai + vbr);  // -Im W (inverse as conj(DFT(conj W)))
       }
       pair_sync(pair);
-      pair_fft512(re, im, b, pair, u, tw1, tw2);
+      pair_fft512(re, im, at, sync, u, tw1, tw2);
       refill(s);
       pair_sync(pair);
       // slot brev3(d) holds conj(w_m), m = k2 + 8 cc + 64 d; the lanes with
@@ -1009,6 +1081,180 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
       const int t = bx + s * gx, i0 = (t % nti) * kDctTileCols, j = t / nti;
       tma_store_3d(&tm, i0, j, 0, b);
       tma_store_3d(&tm, i0, j, 256, b + 256 * 8);
+      bulk_commit();
+    }
+  }
+  if (tid == 0) {
+    if (failed) {
+      atomicOr(status, 1u);
+      // the loads already issued (tiles s, s + 1) land before the CTA leaves
+      for (int t = s; t < min(nmine, s + kDctBufs - 1); t++) mbar_wait(&full[t % kDctBufs], (t / kDctBufs) & 1);
+    }
+    bulk_wait_all();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same for length 1024, on tiles of 8 slots (64-byte rows, 64B-swizzled:
+// chunk p of row r at p ^ ((r >> 1) & 3), so that again eight rows distinct
+// modulo 8 are eight bank groups).  128 threads transform a column pair as
+//   X[2 m + h] = DFT_512(x_n + x_{n+512})[m]                 (h = 0)
+//                DFT_512((x_n - x_{n+512}) W_1024^n)[m]      (h = 1):
+// each group of 64 reads all 1024 entries, keeps its half of the butterfly and
+// runs the 512-point transform in its half of the column's rows.  The forward
+// output goes through rows m ^ ((m >> 4) & 1) (eight distinct rows modulo 8
+// per quarter warp); the inverse stores its rows 2-way.
+// 256 x 128 x 1024 (us per transform): 272 with 1024 points per warp and the
+// bit-reversed scatter (k_dct_w), DCT1024 here.
+// ---------------------------------------------------------------------------
+constexpr int kDct2Cols = 8, kDct2N = 1024;
+
+__device__ __forceinline__ int mk_row2(int n) { return n < 512 ? 2 * n : 2047 - 2 * n; }
+__device__ __forceinline__ int pfft_p2(int m) { return m ^ ((m >> 4) & 1); }
+
+template <int DIR>
+__global__ void __launch_bounds__(512, 1) k_dct2_tma(const __grid_constant__ CUtensorMap tm, int nti, int ntiles,
+                                                     const double *__restrict__ twz, unsigned *status) {
+  constexpr int N = kDct2N;
+  static_assert(kDct2Cols * kDct2N * 8 == kDctTileBytes, "the same buffers");
+  extern __shared__ unsigned char dct_dsm[];
+  __shared__ __align__(8) uint64_t full[kDctBufs];
+  double2 *const buf0 = reinterpret_cast<double2 *>(((uintptr_t)dct_dsm + 1023) & ~(uintptr_t)1023);
+  double2 *const tw1 = buf0 + kDctBufs * (kDctTileBytes / 16);  // [k2 - 1][n1]: W_512^{n1 k2}
+  double2 *const tw2 = tw1 + 7 * 64;                              // [c - 1][a]: W_64^{a c}
+  double2 *const tw0 = tw2 + 7 * 8;                               // [n]: W_1024^n, n < 512
+  double2 *const shl = tw0 + 512;                                 // [k]: e^{i pi k / 2048}
+  const int tid = threadIdx.x, pair = tid >> 7, U = tid & 127, h = U >> 6, u = U & 63;
+  const int bx = blockIdx.x, gx = gridDim.x;
+  const int nmine = ntiles > bx ? (ntiles - 1 - bx) / gx + 1 : 0;
+  auto buf = [&](int s) { return buf0 + (size_t)(s % kDctBufs) * (kDctTileBytes / 16); };
+  auto issue_load = [&](int s) {
+    const int t = bx + s * gx, i0 = (t % nti) * kDct2Cols, j = t / nti;
+    uint64_t *bar = &full[s % kDctBufs];
+    mbar_expect_tx(bar, kDctTileBytes);
+    for (int q = 0; q < 4; q++) tma_load_3d(buf(s) + q * 256 * 4, &tm, i0, j, 256 * q, bar);
+  };
+  if (tid == 0) {
+    for (int bf = 0; bf < kDctBufs; bf++) mbar_init(&full[bf], 1);
+    mbar_init_fence();
+    for (int s = 0; s < min(nmine, kDctBufs - 1); s++) issue_load(s);
+  }
+  auto tw = [&](int p) { return make_double2(__ldg(twz + 2 * p), -__ldg(twz + 2 * p + 1)); };  // W_1024^p
+  for (int i = tid; i < 7 * 64; i += 512) tw1[i] = tw(2 * (i & 63) * (i / 64 + 1));
+  for (int i = tid; i < 7 * 8; i += 512) tw2[i] = tw(16 * (i & 7) * (i / 8 + 1));
+  for (int i = tid; i < 512; i += 512) tw0[i] = tw(i);
+  for (int i = tid; i < N; i += 512) shl[i] = make_double2(__ldg(twz + 2 * N + 2 * i), __ldg(twz + 2 * N + 2 * i + 1));
+  __syncthreads();
+  auto refill = [&](int s) {
+    if (tid == 0 && s + kDctBufs - 1 < nmine) {
+      bulk_wait_read<0>();
+      issue_load(s + kDctBufs - 1);
+    }
+  };
+  auto half_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * pair + h) : "memory"); };
+  auto col_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(9 + pair) : "memory"); };
+  const int k2 = pfft_k2(u), cc = pfft_c(u);
+  int s = 0;
+  bool failed = false;
+  for (; s < nmine; s++) {
+    const bool ok = mbar_wait(&full[s % kDctBufs], (s / kDctBufs) & 1);
+    if (!__syncthreads_and(ok)) {
+      failed = true;
+      break;
+    }
+    double2 *const b = buf(s);
+    auto row = [&](int r) { return b + r * 4 + (pair ^ ((r >> 1) & 3)); };
+    auto at = [&](int r) { return row(512 * h + r); };
+    double re[8], im[8];
+    // this group's half of the butterfly of entries n = u + 64 q (a) and n + 512 (c)
+    auto butterfly = [&](int q, double2 a, double2 c) {
+      if (h == 0) {
+        re[q] = a.x + c.x;
+        im[q] = a.y + c.y;
+      } else {
+        double dr = a.x - c.x, di = a.y - c.y;
+        tw_mul(dr, di, tw0[u + 64 * q]);
+        re[q] = dr;
+        im[q] = di;
+      }
+    };
+    if (DIR > 0) {
+      // entry n lies in an even row, entry n + 512 in an odd one: the lanes
+      // with u & 4 read theirs the other way round, so that each quarter warp
+      // meets both
+      const bool sw = (u >> 2) & 1;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int n = u + 64 * q;
+        const double2 v0 = *row(mk_row2(sw ? n + 512 : n)), v1 = *row(mk_row2(sw ? n : n + 512));
+        butterfly(q, sw ? v1 : v0, sw ? v0 : v1);
+      }
+      col_sync();
+      pair_fft512(re, im, at, half_sync, u, tw1, tw2);
+      refill(s);
+      col_sync();
+#pragma unroll
+      for (int d = 0; d < 8; d++) {
+        const int rg = brev_c(d, 3);
+        *row(pfft_p2(2 * (k2 + 8 * cc + 64 * d) + h)) = make_double2(re[rg], im[rg]);
+      }
+      col_sync();
+      // y_k = 2 Re(e^{-i pi k/(2N)} V_k) / (2N)
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int k = U + 128 * q, km = (N - k) & (N - 1);
+        const double2 z = *row(pfft_p2(k)), mz = *row(pfft_p2(km));
+        const double zr = z.x, zi = z.y, mr = mz.x, mi = mz.y;
+        const double var_ = 0.5 * (zr + mr), vai = 0.5 * (zi - mi);  // V^a = (Z_k + conj Z_{N-k}) / 2
+        const double vbr = 0.5 * (zi + mi), vbi = -0.5 * (zr - mr);  // V^b = -i (Z_k - conj Z_{N-k}) / 2
+        const double2 cs = shl[k];
+        re[q] = 2.0 * (var_ * cs.x + vai * cs.y) / (2.0 * N * 1);
+        im[q] = 2.0 * (vbr * cs.x + vbi * cs.y) / (2.0 * N * 1);
+      }
+      col_sync();
+#pragma unroll
+      for (int q = 0; q < 8; q++) *row(U + 128 * q) = make_double2(re[q], im[q]);
+    } else {
+      // W_k = V^a_k + i V^b_k, V_k = e^{i pi k/(2N)} (X_k - i X_{N-k}) / 2
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int k = U + 128 * q;
+        const double2 cs = shl[k];
+        const double c = cs.x, sn = cs.y;
+        const double2 x = *row(k), y = *row((N - k) & (N - 1));
+        const double xa = x.x / 2.0, xb = x.y / 2.0;
+        const double ya = k == 0 ? 0.0 : -y.x / 2.0, yb = k == 0 ? 0.0 : -y.y / 2.0;
+        const double var_ = xa * c - ya * sn, vai = xa * sn + ya * c;
+        const double vbr = xb * c - yb * sn, vbi = xb * sn + yb * c;
+        re[q] = var_ - vbi;    // Re W
+        im[q] = -(vai + vbr);  // -Im W (inverse as conj(DFT(conj W)))
+      }
+      col_sync();
+#pragma unroll
+      for (int q = 0; q < 8; q++) *row(U + 128 * q) = make_double2(re[q], im[q]);
+      col_sync();
+#pragma unroll
+      for (int q = 0; q < 8; q++) butterfly(q, *row(u + 64 * q), *row(u + 64 * q + 512));
+      col_sync();
+      pair_fft512(re, im, at, half_sync, u, tw1, tw2);
+      refill(s);
+      col_sync();
+      // slot brev3(d) holds conj(w_m), m = 2 (k2 + 8 cc + 64 d) + h; the lanes
+      // with odd cc write slot d ^ 4 first (odd rows beside the others' even ones)
+      const bool sw = cc & 1;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int ra = brev_c(j, 3), rb = brev_c(j ^ 4, 3);
+        const double wr = sw ? re[rb] : re[ra], wi = sw ? im[rb] : im[ra];
+        const int m = 2 * (k2 + 8 * cc + 64 * (sw ? j ^ 4 : j)) + h;
+        *row(mk_row2(m)) = make_double2(2.0 * wr, -2.0 * wi);
+      }
+    }
+    fence_proxy_async();  // the tile's shared-memory writes, before the TMA store reads them
+    __syncthreads();
+    if (tid == 0) {
+      const int t = bx + s * gx, i0 = (t % nti) * kDct2Cols, j = t / nti;
+      for (int q = 0; q < 4; q++) tma_store_3d(&tm, i0, j, 256 * q, b + q * 256 * 4);
       bulk_commit();
     }
   }
@@ -1524,9 +1770,9 @@ static cudaError_t run_dct(vr_ctx *c, int dir) {
   return cudaGetLastError();
 }
 
-// the theta transforms' side of the spectrum: the folded z transforms are not
-// in place, so theirs is the second buffer
-static double *theta_spec(vr_ctx *c) { return c->fold_z[0] ? c->spec2 : c->spec; }
+// the theta transforms' side of the spectrum: the z products are not in place,
+// so theirs is the second buffer
+static double *theta_spec(vr_ctx *c) { return c->lin_z[0] ? c->spec2 : c->spec; }
 
 template <int E>
 static cudaError_t run_fft_w(vr_ctx *c, int dir) {
@@ -1646,7 +1892,7 @@ static cudaError_t run_dct_tma(vr_ctx *c, int dir) {
   const Geo &g = c->geo;
   if (g.nz != kDctN || g.nth % kDctTileCols) return cudaErrorNotSupported;
   CUtensorMap tm;
-  if (!encode_tmap_f64_3d(&tm, c->spec, g.nth, g.nr, g.nz, kDctTileCols, 1, 256, true)) return cudaErrorNotSupported;
+  if (!encode_tmap_f64_3d(&tm, c->spec, g.nth, g.nr, g.nz, kDctTileCols, 1, 256, 128)) return cudaErrorNotSupported;
   const int nti = g.nth / kDctTileCols, ntiles = nti * g.nr;
   const size_t sm = (size_t)kDctBufs * kDctTileBytes + (7 * 64 + 7 * 8 + kDctN) * 16 + 1024;
   auto kern = dir > 0 ? k_dct_tma<1> : k_dct_tma<-1>;
@@ -1658,8 +1904,30 @@ static cudaError_t run_dct_tma(vr_ctx *c, int dir) {
   return cudaGetLastError();
 }
 
+// the same for 1024 points
+static cudaError_t run_dct2_tma(vr_ctx *c, int dir) {
+  const Geo &g = c->geo;
+  if (g.nz != kDct2N || g.nth % kDct2Cols) return cudaErrorNotSupported;
+  CUtensorMap tm;
+  if (!encode_tmap_f64_3d(&tm, c->spec, g.nth, g.nr, g.nz, kDct2Cols, 1, 256, 64)) return cudaErrorNotSupported;
+  const int nti = g.nth / kDct2Cols, ntiles = nti * g.nr;
+  const size_t sm = (size_t)kDctBufs * kDctTileBytes + (7 * 64 + 7 * 8 + 512 + kDct2N) * 16 + 1024;
+  auto kern = dir > 0 ? k_dct2_tma<1> : k_dct2_tma<-1>;
+  cudaError_t e = allow_dyn_smem(kern, sm);
+  if (e) return e;
+  LaunchScope ls(c, PK_DCT);
+  kern<<<std::min(ntiles, c->nsm), 512, sm, c->stream>>>(tm, nti, ntiles, c->tw_z, c->d_status);
+  return cudaGetLastError();
+}
+
 static cudaError_t dct_warp_dispatch(vr_ctx *c, int dir, bool *done) {
   *done = true;
+  // (double precision only: the mixed form keeps the rounding of k_dct_w, a
+  // change of which its float fields would show at 3e-7 a few steps later)
+  if (c->geo.nz == kDct2N && !c->mixed) {
+    cudaError_t e = run_dct2_tma(c, dir);
+    if (e != cudaErrorNotSupported) return e;
+  }
   if (c->geo.nz == kDctN) {
     cudaError_t e = run_dct_tma(c, dir);
     if (e != cudaErrorNotSupported) return e;
@@ -1711,27 +1979,26 @@ static cudaError_t run_slab_bwd(vr_ctx *c, const CUtensorMap &tm) {
 static bool slab_tmap(vr_ctx *c, CUtensorMap *tm) {
   const Geo &g = c->geo;
   if (!c->slab_transforms || g.nth != kClSlab || g.nz != kDctN) return false;
-  return encode_tmap_f64_3d(tm, c->spec, g.nth, g.nr, g.nz, kDctTileCols, 1, 256, true);
+  return encode_tmap_f64_3d(tm, c->spec, g.nth, g.nr, g.nz, kDctTileCols, 1, 256, 128);
 }
 
 static cudaError_t radial_solves(vr_ctx *c);
 
-// the lengths with an FFT of their own (2048 along z: radix 2 in shared memory)
-bool fft_theta_length(int n) { return is_pow2(n) && n >= 32 && n <= 1024; }
-bool fft_z_length(int n) { return is_pow2(n) && n >= 32 && n <= 2048; }
+// the lengths with an FFT
+bool fft_length(int n) { return is_pow2(n); }
 
 // the z transforms of every (slot, r) column
 static cudaError_t run_z(vr_ctx *c, int dir) {
   const Geo &g = c->geo;
-  if (c->fold_z[0]) {
+  if (c->lin_z[0]) {
     const int M = g.nth * g.nr;
     LaunchScope ls(c, PK_DCT);
-    return dir > 0 ? fold_run<kFoldZ, +1>(c->spec2, c->spec, c->fold_z[0], g.nz, M, 0, c->nsm, c->stream)
-                   : fold_run<kFoldZ, -1>(c->spec, c->spec2, c->fold_z[1], g.nz, M, 0, c->nsm, c->stream);
+    return dir > 0 ? lin_run<kLinZFwd>(c->spec2, c->spec, c->lin_z[0], g.nz, M, 0, c->nsm, c->stream)
+                   : lin_run<kLinZInv>(c->spec, c->spec2, c->lin_z[1], g.nz, M, 0, c->nsm, c->stream);
   }
   bool done = false;
   cudaError_t e = dct_warp_dispatch(c, dir, &done);
-  return done || e ? e : run_dct<4>(c, dir);
+  return done || e ? e : g.nz <= 1024 ? run_dct<8>(c, dir) : run_dct<4>(c, dir);
 }
 
 cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk) {
@@ -1747,22 +2014,33 @@ cudaError_t launch_poisson(vr_ctx *c, const Rk *div_rk) {
   }
   // theta forward: rhs (or divq of dq) -> spectrum
   bool done = false;
-  if (c->fold_th[0]) {
+  const int lpb = N >= 1024 ? 1 : 1024 / N;  // lines per CTA of the short FFTs
+  const size_t sm = sizeof(double) * 2 * lpb * N;
+  if (c->lin_th[0]) {
     LaunchScope ls(c, PK_FFT);
-    e = fold_run<kFoldTh, +1>(c->rhs, theta_spec(c), c->fold_th[0], N, nlines, 0, c->nsm, c->stream);
-  } else {
-    e = fft_warp_dispatch(c, +1, &done, div_rk);
+    e = lin_run<kLinThFwd>(c->rhs, theta_spec(c), c->lin_th[0], N, nlines, 0, c->nsm, c->stream);
+  } else if (!(e = fft_warp_dispatch(c, +1, &done, div_rk)) && !done) {
+    if ((e = allow_dyn_smem(k_fft_fwd, sm))) return e;
+    LaunchScope ls(c, PK_FFT);
+    k_fft_fwd<<<(nlines + lpb - 1) / lpb, 256, sm, c->stream>>>(c->rhs, theta_spec(c), N, ilog2(N), lpb, nlines,
+                                                                c->tw_th);
+    e = cudaGetLastError();
   }
   if (e) return e;
   if ((e = run_z(c, +1))) return e;
   if ((e = radial_solves(c))) return e;
   if ((e = run_z(c, -1))) return e;
   // theta backward -> dph
-  if (c->fold_th[0]) {
+  if (c->lin_th[0]) {
     LaunchScope ls(c, PK_FFT);
-    return fold_run<kFoldTh, -1>(theta_spec(c), c->dph, c->fold_th[1], N, nlines, g.nr, c->nsm, c->stream);
+    return lin_run<kLinThInv>(theta_spec(c), c->dph, c->lin_th[1], N, nlines, g.nr, c->nsm, c->stream);
   }
-  return fft_warp_dispatch(c, -1, &done);
+  if ((e = fft_warp_dispatch(c, -1, &done)) || done) return e;
+  if ((e = allow_dyn_smem(k_fft_bwd, sm))) return e;
+  LaunchScope ls(c, PK_FFT);
+  k_fft_bwd<<<(nlines + lpb - 1) / lpb, 256, sm, c->stream>>>(theta_spec(c), c->dph, g, ilog2(N), lpb, nlines,
+                                                              c->tw_th);
+  return cudaGetLastError();
 }
 
 // the radial tridiagonal lines of every (theta mode, z mode)

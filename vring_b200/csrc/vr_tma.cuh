@@ -98,12 +98,13 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 
 // Host: a tensor map of a column-major FP64 array (d0, d1, d2) with boxes of
 // (b0, b1, b2) elements; out-of-range elements of a box read as zero.  With
-// swizzle128 the box rows (b0 * 8 = 128 bytes) land in shared memory with
+// swizzle 128 the box rows (b0 * 8 = 128 bytes) land in shared memory with
 // their 16-byte chunks permuted, chunk c of row r at c ^ (r & 7) (the buffer
-// 1024-byte aligned).  False when the driver entry point is missing or the
+// 1024-byte aligned); with swizzle 64 (64-byte rows) chunk c of row r at
+// c ^ ((r >> 1) & 3).  False when the driver entry point is missing or the
 // driver rejects the map (base not 16-byte aligned, d0 * 8 not a multiple of
 // 16, box too large).
 bool encode_tmap_f64_3d(CUtensorMap *tm, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, unsigned b0,
-                        unsigned b1, unsigned b2, bool swizzle128 = false);
+                        unsigned b1, unsigned b2, int swizzle = 0);
 
 }  // namespace vr
