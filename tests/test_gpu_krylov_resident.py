@@ -1,5 +1,5 @@
-"""CG, Jacobi CG and BiCGSTAB at the grid shapes where the resident kernels'
-split changes: segments per CTA, idle threads, a partly filled last CTA, one to
+"""CG and Jacobi CG at the grid shapes where the resident kernel's split
+changes: segments per CTA, idle threads, a partly filled last CTA, one to
 eight planes per thread, and the grids that do not fit (streaming kernels).
 
 Tolerance: the error of an answer with relative residual tol is at most the
@@ -18,13 +18,8 @@ SHAPES = [(4, 4), (5, 9), (31, 70), (64, 148), (100, 1023), (255, 33), (256, 300
           (512, 1036), (512, 1184), (512, 1185), (513, 24)]
 
 
-# BiCGSTAB breaks down (in every order of its sums) where the cells are much
-# finer in r than in z
-CASES = [(m, s) for s in SHAPES for m in ("cg", "pcg", "bicgstab")
-         if m != "bicgstab" or s not in ((511, 20), (512, 7), (513, 24))]
-
-
-@pytest.mark.parametrize("method,shape", CASES, ids=lambda v: v if isinstance(v, str) else "%dx%d" % v)
+@pytest.mark.parametrize("method", ["cg", "pcg"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda v: "%dx%d" % v)
 def test_shapes_converge_to_the_direct_solve(method, shape):
     import vring_b200 as V
     nr, nz = shape
@@ -40,7 +35,7 @@ def test_shapes_converge_to_the_direct_solve(method, shape):
     assert it2 == it and np.array_equal(x, y)
 
 
-@pytest.mark.parametrize("method", ["pcg", "bicgstab"])
+@pytest.mark.parametrize("method", ["cg", "pcg"])
 def test_iterations_carry_over_launches_and_caps(method):
     """A solve stopped at a cap and restarted from its answer still converges,
     and a cap on either side of a launch's 512 iterations is met exactly."""

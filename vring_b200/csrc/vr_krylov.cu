@@ -24,8 +24,8 @@
 // kernel reads -- by the block that finishes last (a ticket counter after a
 // memory fence) in the iteration kernels, which also take the scalar steps
 // there, and by a one-block kernel in the setup.
-// Grids whose vectors fit the chip run CG and BiCGSTAB in resident kernels
-// (vr_krylov_res.cuh).  The others stream them:
+// Grids whose vectors fit the chip run CG in a resident kernel
+// (vr_krylov_res.cuh).  Otherwise the vectors are streamed:
 // CG runs two kernels per iteration and BiCGSTAB three: each operator
 // application forms the vector it applies (the new direction, or s) as it
 // reads it.  Iterations are issued in chunks
@@ -59,7 +59,7 @@ constexpr int kFcgKeep = 8;          // directions the flexible CG keeps (trunca
 enum K2dScal {
   SC_ALPHA = 0, SC_BETA, SC_RZ, SC_BB, SC_RR, SC_RHO, SC_OMEGA, SC_TOL2, SC_RHO_NEW, SC_SS,
   SC_PMEAN,  // CG, BiCGSTAB: mean over z of the next direction's last radial row
-  SC_SMEAN,  // BiCGSTAB: the same for s (between resident launches: for r)
+  SC_SMEAN,  // BiCGSTAB: the same for s
   SC_N
 };
 // partial-sum slots
@@ -74,7 +74,7 @@ enum K2dZ { K2D_Z_FFT = 0, K2D_Z_LIN, K2D_Z_GEMM };
 struct vr_k2d {
   int nr = 0, nz = 0, n = 0, dev = 0, nb = 0, nsm = 148;
   cudaStream_t stream = nullptr;
-  double *coef = nullptr;  // aw, ae, az, vol (per j), per cell 1/diag(S) and diag(S)^-1/2, then 1/vol (per j)
+  double *coef = nullptr;  // aw, ae, az, vol (per j), per cell 1/diag(S) and diag(S)^-1/2
   double gam = 0.0;
   double *vec[12] = {};
   double *part = nullptr;   // PT_N x kK2dMaxBlocks
@@ -84,8 +84,9 @@ struct vr_k2d {
   int cg_parity = 0;        // direction buffer of the next CG iteration being captured
   int bi_parity = 0;        // p and v buffers of the next BiCGSTAB iteration being captured
   int nb_cg = 1;            // grid of the CG iteration kernels
-  // resident CG and BiCGSTAB: planes per thread (0: the grid does not fit),
-  // segments and CTAs, the exchanges' memory and the next exchange's number
+  // resident CG: planes per thread (0: the grid does not fit), segments and
+  // CTAs, the exchanges' memory (allocated by the first solve that needs it)
+  // and the next exchange's number
   int res_c = 0, res_nseg = 0, res_ctas = 0;
   unsigned long long *res_mem = nullptr;
   size_t res_words = 0;
@@ -491,7 +492,6 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_bi_first(K2dOp o, const doubl
                                                           const double *v, double *sc) {
   __shared__ double sh[40];
   bi_next(o, r, p, v, sc, sh);
-  if (threadIdx.x == 0) sc[SC_SMEAN] = sc[SC_PMEAN];  // p = v = 0: r's own mean
 }
 
 // third: x += alpha p + omega s; r = s - omega t; partials rh.r [A], r.r [B];
@@ -958,13 +958,12 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
     ae[j - 1] = f[j] * dz / h;
   }
   k->gam = 2.0 * f[nr] * dz / dr[nr - 1];
-  std::vector<double> coef((size_t)5 * nr + 2 * (size_t)nr * nz);
+  std::vector<double> coef((size_t)4 * nr + 2 * (size_t)nr * nz);
   for (int j = 0; j < nr; j++) {
     coef[j] = aw[j];
     coef[nr + j] = ae[j];
     coef[2 * nr + j] = az[j];
     coef[3 * nr + j] = vol[j];
-    coef[4 * nr + 2 * (size_t)nr * nz + j] = 1.0 / vol[j];
   }
   for (int kk = 0; kk < nz; kk++)
     for (int j = 0; j < nr; j++) {
@@ -1046,13 +1045,7 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
       return fail(VR_ERR_CUDA);
   if (cudaMemset(k->part, 0, sizeof(double) * PT_N * kK2dMaxBlocks) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaMemset(k->flags, 0, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_CUDA);
-  if (res_shape(nr, nz, nsm, &k->res_c, &k->res_nseg, &k->res_ctas)) {
-    k->res_words = (size_t)k->res_ctas * (2 * kResCopies * kResSlotWords + 2 * 2 * 2 * (size_t)nr);
-    if (cudaMalloc(&k->res_mem, sizeof(unsigned long long) * k->res_words) != cudaSuccess) return fail(VR_ERR_OOM);
-    if (cudaMemset(k->res_mem, 0, sizeof(unsigned long long) * k->res_words) != cudaSuccess) return fail(VR_ERR_CUDA);
-  } else {
-    k->res_c = 0;
-  }
+  if (!res_shape(nr, nz, nsm, &k->res_c, &k->res_nseg, &k->res_ctas)) k->res_c = 0;
   *out = k;
   return VR_OK;
 }
@@ -1228,15 +1221,13 @@ static int run_chunks(vr_k2d *k, int slot, cudaError_t (*enq)(vr_k2d *, int), in
   return VR_OK;
 }
 
-// launches of kResIters resident iterations (CG, Jacobi CG: jacobi 0, 1;
-// BiCGSTAB: -1) until converged or maxit; cudaErrorNotSupported when the
-// cooperative launch is not possible here (nothing has run then)
+// one launch of kResIters resident CG iterations; cudaErrorNotSupported when
+// the cooperative launch is not possible here (nothing has run then)
 template <int C>
-static cudaError_t res_launch(vr_k2d *k, int jacobi, ResArg a) {
-  void (*kern)(ResArg) = jacobi < 0 ? k2d_bi_res<C> : jacobi ? k2d_cg_res<C, true> : k2d_cg_res<C, false>;
+static cudaError_t res_launch(vr_k2d *k, bool jacobi, ResArg a) {
+  void (*kern)(ResArg) = jacobi ? k2d_cg_res<C, true> : k2d_cg_res<C, false>;
   const int threads = (k->res_nseg * k->nr + 31) / 32 * 32;
-  const size_t sm = sizeof(double) * ((((size_t)k->res_nseg * C * k->nr + 3) & ~(size_t)1) +
-                                      (jacobi < 0 ? (size_t)2 * C * threads : 0));
+  const size_t sm = sizeof(double) * ((size_t)k->res_nseg * C * k->nr + 2);
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
   void *args[] = {&a};
@@ -1247,19 +1238,18 @@ static cudaError_t res_launch(vr_k2d *k, int jacobi, ResArg a) {
   }
   return e;
 }
-static cudaError_t res_chunk(vr_k2d *k, int jacobi) {
-  // the exchange numbers of a launch are all different and never 0 again
-  const unsigned need = 3u * kResIters;
+static cudaError_t res_chunk(vr_k2d *k, bool jacobi) {
+  // the exchange numbers of all launches differ, and none is 0
+  const unsigned need = 2u * kResIters;
   if (k->res_epoch > 0xffffffffu - need) {
     cudaError_t e = cudaMemsetAsync(k->res_mem, 0, sizeof(unsigned long long) * k->res_words, k->stream);
     if (e) return e;
     k->res_epoch = 1;
   }
   const K2dOp o = op_of(k);
-  ResArg a{o.nr, o.nz, k->res_nseg, o.aw, o.ae, o.az, k->coef + 4 * k->nr + 2 * (size_t)k->n, o.dinv, o.gam,
-           k->vec[V_X], k->vec[V_R], k->vec[V_P], k->vec[V_V], k->vec[V_RH], k->sc, k->flags, k->res_mem,
-           k->res_mem + (size_t)2 * kResCopies * k->res_ctas * kResSlotWords, k->res_epoch};
-  k->res_epoch += need + (need & 1);  // an even number: a launch starts on the other slots than the one before it ended on
+  ResArg a{o.nr, o.nz, k->res_nseg, o.aw, o.ae, o.az, o.dinv, o.gam, k->vec[V_X], k->vec[V_R], k->vec[V_P], k->sc,
+           k->flags, k->res_mem, k->res_mem + (size_t)2 * kResCopies * k->res_ctas * kResSlotWords, k->res_epoch};
+  k->res_epoch += need;
   switch (k->res_c) {
     case 1: return res_launch<1>(k, jacobi, a);
     case 2: return res_launch<2>(k, jacobi, a);
@@ -1272,9 +1262,15 @@ static cudaError_t res_chunk(vr_k2d *k, int jacobi) {
     default: return cudaErrorNotSupported;
   }
 }
-static int run_resident(vr_k2d *k, int jacobi, int maxit, int *iters, bool *ran) {
+static int run_resident(vr_k2d *k, bool jacobi, int maxit, int *iters, bool *ran) {
   int h[4] = {0, 0, 0, 0};
   *ran = false;
+  if (!k->res_mem) {
+    k->res_words = (size_t)k->res_ctas * (2 * kResCopies * kResSlotWords + 2 * 2 * (size_t)k->nr);
+    if (cudaMalloc(&k->res_mem, sizeof(unsigned long long) * k->res_words) != cudaSuccess)
+      return k2d_err(k, VR_ERR_OOM, "resident krylov");
+    K2D_CUDA(k, cudaMemsetAsync(k->res_mem, 0, sizeof(unsigned long long) * k->res_words, k->stream));
+  }
   for (int done = 0; done < maxit; done += kResIters) {
     const cudaError_t e = res_chunk(k, jacobi);
     if (e == cudaErrorNotSupported && !*ran) return VR_OK;
@@ -1283,10 +1279,6 @@ static int run_resident(vr_k2d *k, int jacobi, int maxit, int *iters, bool *ran)
     K2D_CUDA(k, cudaMemcpyAsync(h, k->flags, sizeof(h), cudaMemcpyDeviceToHost, k->stream));
     K2D_CUDA(k, cudaStreamSynchronize(k->stream));
     if (h[3]) return k2d_err(k, VR_ERR_TIMEOUT, "resident krylov: a bounded wait between CTAs gave up");
-    if (h[0] == 3) {
-      *ran = false;
-      return VR_OK;
-    }
     if (h[0] || h[1] >= maxit) break;
   }
   *iters = h[1];
@@ -1435,30 +1427,15 @@ extern "C" int vr_k2d_solve_dev(vr_k2d *k, int32_t method, const double *f, doub
     if (k->res_c) rc = run_resident(k, jac, maxit, &it, &ran);
     if (!rc && !ran) rc = run_chunks(k, jac, enq_cg, jac, maxit, &it);
   } else if (method == VR_KRYLOV_BICGSTAB) {
-    bool ran = false;
-    for (int form = k->res_c ? 0 : 1; form < 2 && !ran && !rc; form++) {
-      if (form == 1 && k->res_c) {
-        // the resident kernel broke down (or cannot run): from the start again
-        K2D_CUDA(k, cudaMemcpyAsync(k->flags, hf, sizeof(hf), cudaMemcpyHostToDevice, k->stream));
-        K2D_CUDA(k, cudaMemcpyAsync(X, x, bytes, cudaMemcpyDeviceToDevice, k->stream));
-        k2d_apply<<<gb, kK2dThreads, 0, k->stream>>>(o, X, R, 1, nullptr, nullptr, nullptr);
-        k2d_axpby<<<gb, kK2dThreads, 0, k->stream>>>(k->n, 1.0, B, -1.0, R, R);
-      }
-      K2D_CUDA(k, cudaMemcpyAsync(k->vec[V_RH], R, bytes, cudaMemcpyDeviceToDevice, k->stream));
-      K2D_CUDA(k, cudaMemsetAsync(Pv, 0, bytes, k->stream));
-      K2D_CUDA(k, cudaMemsetAsync(k->vec[V_V], 0, bytes, k->stream));
-      // partials: b.b [A], rh.r = r.r [B], r.r [C]
-      k2d_init_dots<<<gb, kK2dThreads, 0, k->stream>>>(o, 0, B, R, nullptr, P);
-      k2d_scalar<<<1, 1024, 0, k->stream>>>(SO_BI_INIT, P, gb, k->sc, k->flags);
-      k2d_bi_first<<<1, kK2dThreads, 0, k->stream>>>(o, R, Pv, k->vec[V_V], k->sc);
-      K2D_CUDA(k, cudaGetLastError());
-      if (form == 0) {
-        rc = run_resident(k, -1, maxit, &it, &ran);
-      } else {
-        rc = run_chunks(k, 2, enq_bicg, 0, maxit, &it);
-        ran = true;
-      }
-    }
+    K2D_CUDA(k, cudaMemcpyAsync(k->vec[V_RH], R, bytes, cudaMemcpyDeviceToDevice, k->stream));
+    K2D_CUDA(k, cudaMemsetAsync(Pv, 0, bytes, k->stream));
+    K2D_CUDA(k, cudaMemsetAsync(k->vec[V_V], 0, bytes, k->stream));
+    // partials: b.b [A], rh.r = r.r [B], r.r [C]
+    k2d_init_dots<<<gb, kK2dThreads, 0, k->stream>>>(o, 0, B, R, nullptr, P);
+    k2d_scalar<<<1, 1024, 0, k->stream>>>(SO_BI_INIT, P, gb, k->sc, k->flags);
+    k2d_bi_first<<<1, kK2dThreads, 0, k->stream>>>(o, R, Pv, k->vec[V_V], k->sc);
+    K2D_CUDA(k, cudaGetLastError());
+    rc = run_chunks(k, 2, enq_bicg, 0, maxit, &it);
   } else {
     if (!k->fp) {
       const size_t kb = sizeof(double) * kFcgKeep * (size_t)k->n;

@@ -1,9 +1,8 @@
-// vr_krylov_res.cuh -- CG and BiCGSTAB on the axisymmetric operator with every
-// vector resident on the chip (included by vr_krylov.cu).
+// vr_krylov_res.cuh -- CG on the axisymmetric operator with every vector
+// resident on the chip (included by vr_krylov.cu).
 //
-// An iteration moves 40 to 70 MB through L2 when its kernels stream the
-// vectors, yet all of them at 512 x 1024 are 20 to 30 MB, less than the
-// registers of the chip.  So one cooperative kernel runs many iterations with
+// An iteration moves 40 MB through L2 when its kernels stream the vectors, yet
+// all of them at 512 x 1024 are 20 MB, less than the registers of the chip.  So one cooperative kernel runs many iterations with
 // the vectors in registers: a CTA owns nseg x C consecutive z planes, a thread
 // one radial index j of C of them (nseg = 512 / nr segments side by side).
 // Radial neighbours come from a shared-memory copy of the CTA's planes, z
@@ -26,9 +25,11 @@
 // leaves, the others then run into their own limits, and the host reports
 // VR_ERR_TIMEOUT.  The launch is cooperative, so all CTAs are resident.
 //
-// us per iteration at 512 x 1024, streaming kernels / resident:
-// Jacobi CG 20.2 / 6.3, BiCGSTAB 35.9 / 10.4 (128 x 256: 12.1 / 4.6 and 18.6 /
-// 7.4).  An exchange of one double per CTA between 148 CTAs takes 1.4 us
+// us per iteration of Jacobi CG, streaming kernels / resident: 20.2 / 6.3 at
+// 512 x 1024, 12.1 / 4.6 at 128 x 256.  (BiCGSTAB the same way took 10.4 for
+// 35.9, but its iterates depend on the order of the sums: two orders, both
+// converged to 1e-12, answer 1e-9 apart, and it breaks down in one and not in
+// the other, so it keeps the streaming kernels and their order.)  An exchange of one double per CTA between 148 CTAs takes 1.4 us
 // beyond the sums inside the CTA (0.25): one 128-byte line per CTA, the slots
 // packed side by side take 3.2 (the lines are then written by eight CTAs
 // while all read them), one CTA that adds and broadcasts 1.9, a counter with
@@ -48,14 +49,13 @@ constexpr int kResMaxCtas = 256;  // a CTA's first 256 threads read one slot eac
 
 struct ResArg {
   int nr, nz, nseg;
-  const double *aw, *ae, *az, *ivol, *dinv;
+  const double *aw, *ae, *az, *dinv;
   double gam;
-  double *x, *r, *p, *v;
-  const double *rh;
+  double *x, *r, *p;
   double *sc;
   int *flags;
   unsigned long long *slots;  // [2][kResCopies][CTAs][kResSlotWords]
-  unsigned long long *ends;   // [2 kinds][CTAs][bottom, top][nr][2]
+  unsigned long long *ends;   // [CTAs][bottom, top][nr][2]
   unsigned epoch;             // number of the launch's first exchange
 };
 
@@ -228,22 +228,22 @@ struct ResCell {
       y[c] = s;
     }
   }
-  // the CTA's end planes of u, and the neighbours'; kind: which vector
-  __device__ unsigned long long *end_slot(const ResArg &a, int kind, int cta, int top) const {
-    return a.ends + 2 * ((((size_t)kind * gridDim.x + cta) * 2 + top) * a.nr + j);
+  // the CTA's end planes of u, and the neighbours'
+  __device__ unsigned long long *end_slot(const ResArg &a, int cta, int top) const {
+    return a.ends + 2 * (((size_t)cta * 2 + top) * a.nr + j);
   }
-  __device__ void put_ends(const ResArg &a, int kind, const double (&u)[C], unsigned tag) const {
-    if (first && blockIdx.x > 0) put_tagged(end_slot(a, kind, blockIdx.x, 0), u[0], tag);
-    if (last && blockIdx.x + 1 < gridDim.x) put_tagged(end_slot(a, kind, blockIdx.x, 1), u[C - 1], tag);
+  __device__ void put_ends(const ResArg &a, const double (&u)[C], unsigned tag) const {
+    if (first && blockIdx.x > 0) put_tagged(end_slot(a, blockIdx.x, 0), u[0], tag);
+    if (last && blockIdx.x + 1 < gridDim.x) put_tagged(end_slot(a, blockIdx.x, 1), u[C - 1], tag);
   }
   // the neighbours' end planes; read after the sums of their exchange are in,
   // when they have as good as arrived: spinning on them meanwhile would put
   // every thread of the chip on L2 beside the sums
-  __device__ bool get_ends(const ResArg &a, int kind, double &lo, double &hi, unsigned tag) const {
+  __device__ bool get_ends(const ResArg &a, double &lo, double &hi, unsigned tag) const {
     const bool wlo = first && blockIdx.x > 0, whi = last && blockIdx.x + 1 < gridDim.x;
     if (!wlo && !whi) return true;
-    const unsigned long long *pl = end_slot(a, kind, wlo ? blockIdx.x - 1 : blockIdx.x + 1, wlo ? 1 : 0);
-    const unsigned long long *ph = whi ? end_slot(a, kind, blockIdx.x + 1, 0) : pl;
+    const unsigned long long *pl = end_slot(a, wlo ? blockIdx.x - 1 : blockIdx.x + 1, wlo ? 1 : 0);
+    const unsigned long long *ph = whi ? end_slot(a, blockIdx.x + 1, 0) : pl;
     double vl = 0.0, vh = 0.0;
     const bool ok = wait_tagged([&] {
       unsigned long long wl[2], wh[2];
@@ -327,9 +327,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k2d_cg_res(const ResArg a) {
         s2[3] += p[c];
       }
     }
-    e.put_ends(a, 0, z, tag);
+    e.put_ends(a, z, tag);
     if (!grid_sum(s2, a, tag, sh)) return;
-    ok = e.get_ends(a, 0, zlo, zhi, tag++);
+    ok = e.get_ends(a, zlo, zhi, tag++);
     be = s2[0] / rz;
     rz = s2[0];
     rr = s2[1];
@@ -349,126 +349,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k2d_cg_res(const ResArg a) {
     a.sc[SC_PMEAN] = pmean;
     a.sc[SC_RZ] = rz;
     a.sc[SC_RR] = rr;
-    a.flags[1] = it;
-    a.flags[0] = done;
-  }
-}
-
-// Up to kResIters BiCGSTAB iterations on K x = f from the state (x, r, p, v,
-// SC_BETA, SC_OMEGA, SC_RHO_NEW, SC_PMEAN, SC_SMEAN = mean of r's last row);
-// the steps are those of k2d_bi_pv, k2d_bi_st and k2d_bi_xr3.  BiCGSTAB can
-// break down (rh . v or omega vanish in rounding, in one order of the sums and
-// not in another: 1 to 3 of 60 seeded grids); the launch then stops with
-// flags[0] = 3 and the host runs the streaming kernels from the start.
-template <int C>
-__global__ void __launch_bounds__(kResThreads, 1) k2d_bi_res(const ResArg a) {
-  extern __shared__ double planes[];
-  __shared__ ResShared sh;
-  if (a.flags[0]) return;
-  const ResCell<C> e(a, planes);
-  // x and rh, read once or twice per iteration, in shared memory (this
-  // thread's own words): six vectors of seven planes do not fit 128 registers
-  double *xs = planes + (((size_t)a.nseg * C * a.nr + 3) & ~(size_t)1) + threadIdx.x, *rhs_ = xs + C * blockDim.x;
-  const int ld = blockDim.x;
-  double r[C], p[C], v[C], t[C], plo, phi, vlo, vhi, rlo, rhi;
-  e.load(a, a.x, t);
-#pragma unroll
-  for (int c = 0; c < C; c++) xs[c * ld] = t[c];
-  e.load(a, a.rh, t);
-#pragma unroll
-  for (int c = 0; c < C; c++) rhs_[c * ld] = t[c];
-  e.load(a, a.r, r);
-  e.load(a, a.p, p);
-  e.load(a, a.v, v);
-  e.load_ends(a, a.p, plo, phi);
-  e.load_ends(a, a.v, vlo, vhi);
-  e.load_ends(a, a.r, rlo, rhi);
-  const double iv = a.ivol[e.j];
-  double be = a.sc[SC_BETA], om = a.sc[SC_OMEGA], rho = a.sc[SC_RHO], rho_new = a.sc[SC_RHO_NEW];
-  double pmean = a.sc[SC_PMEAN], rmean = a.sc[SC_SMEAN], rr = 0.0, al = 0.0;
-  const double stop = a.sc[SC_TOL2] * a.sc[SC_BB];
-  int it = a.flags[1], done = 0;
-  const int cap = a.flags[2];
-  unsigned tag = a.epoch;
-  bool ok = true;
-  if (threadIdx.x == 0) planes[0] = planes[1 + (size_t)a.nseg * C * a.nr] = 0.0;
-  for (int n = 0; n < kResIters && !done; n++) {
-#pragma unroll
-    for (int c = 0; c < C; c++) p[c] = r[c] + be * (p[c] - om * v[c]);
-    plo = rlo + be * (plo - om * vlo);
-    phi = rhi + be * (phi - om * vhi);
-    e.put(a, p);
-    if (!__syncthreads_and(ok)) return give_up(a);
-    e.apply(a, p, plo, phi, pmean, v);
-    double s1[2] = {0.0, 0.0};
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      v[c] *= iv;
-      s1[0] += rhs_[c * ld] * v[c];
-      if (e.wall) s1[1] += v[c];
-    }
-    e.put_ends(a, 0, v, tag);
-    if (!grid_sum(s1, a, tag, sh)) return;
-    ok = e.get_ends(a, 0, vlo, vhi, tag++);
-    rho = rho_new;
-    al = rho / s1[0];
-#pragma unroll
-    for (int c = 0; c < C; c++) r[c] -= al * v[c];  // s
-    const double slo = rlo - al * vlo, shi = rhi - al * vhi;
-    e.put(a, r);
-    if (!__syncthreads_and(ok)) return give_up(a);
-    e.apply(a, r, slo, shi, rmean - al * (s1[1] / a.nz), t);
-    double s2[2] = {0.0, 0.0};
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      t[c] *= iv;
-      s2[0] += r[c] * t[c];
-      s2[1] += t[c] * t[c];
-    }
-    if (!grid_sum(s2, a, tag++, sh)) return;
-    om = s2[1] != 0.0 ? s2[0] / s2[1] : 0.0;
-    double s3[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      xs[c * ld] += al * p[c] + om * r[c];
-      r[c] -= om * t[c];
-      s3[0] += rhs_[c * ld] * r[c];
-      s3[1] += r[c] * r[c];
-      if (e.wall) {
-        s3[2] += r[c];
-        s3[3] += p[c];
-      }
-    }
-    e.put_ends(a, 1, r, tag);
-    if (!grid_sum(s3, a, tag, sh)) return;
-    ok = e.get_ends(a, 1, rlo, rhi, tag++);
-    rho_new = s3[0];
-    rr = s3[1];
-    it++;
-    if (rr <= stop)
-      done = 1;
-    else if (it >= cap)
-      done = 2;
-    if (!isfinite(rr)) done = 3;  // broken down
-    be = (rho_new / rho) * (al / om);
-    rmean = s3[2] / a.nz;
-    pmean = (s3[2] + be * (s3[3] - om * s1[1])) / a.nz;
-  }
-#pragma unroll
-  for (int c = 0; c < C; c++) t[c] = xs[c * ld];
-  e.store(a, a.x, t);
-  e.store(a, a.r, r);
-  e.store(a, a.p, p);
-  e.store(a, a.v, v);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.sc[SC_ALPHA] = al;
-    a.sc[SC_OMEGA] = om;
-    a.sc[SC_RHO] = rho;
-    a.sc[SC_RHO_NEW] = rho_new;
-    a.sc[SC_RR] = rr;
-    a.sc[SC_BETA] = be;
-    a.sc[SC_PMEAN] = pmean;
-    a.sc[SC_SMEAN] = rmean;
     a.flags[1] = it;
     a.flags[0] = done;
   }
