@@ -245,6 +245,7 @@ __global__ void __launch_bounds__(LPT *NCH, MINB)
     }
   };
   if (smem_u32(stage) & 127u) {  // TMA destinations need 128-byte alignment
+    pdl_wait();
     if (tid == 0) atomicOr(status, 2u);
     return;
   }
@@ -266,6 +267,7 @@ __global__ void __launch_bounds__(LPT *NCH, MINB)
     }
   }
   __syncthreads();
+  pdl_wait();  // up to here: the factorisation
   if (tid == 0)
     for (int k = 0; k < S; k++) {
       const int tile = blockIdx.x + k * gridDim.x;
@@ -453,8 +455,7 @@ cudaError_t run_chunk_tma(P p, const void *base, int d0, int d1, int d2, int ldi
   p.nbx = (p.nth_lines() + LPT - 1) / LPT;
   const int ntiles = p.nbx * nm2;
   const int grid = ntiles < MINB * nsm ? ntiles : MINB * nsm;
-  kern<<<grid, LPT * NCH, dyn, st>>>(tm, p, ntiles, tt, status);
-  return cudaGetLastError();
+  return launch_pdl(kern, grid, LPT * NCH, dyn, st, tm, p, ntiles, tt, status);
 }
 
 // chunk length bucket: the smallest compiled MAXCL with 32 * MAXCL >= n

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(512) k_lin(const LinArg a) {
   double *st0 = sm + (((size_t)N * LD + 1) & ~(size_t)1), *st = st0 + (size_t)warp * 2 * SUB * KC * 16;  // stages
   double *so = st0 + (size_t)nw * 2 * SUB * KC * 16;  // theta: [N][LD] results
   const int c0 = blockIdx.x * NC, nc = min(NC, a.M - c0);
+  pdl_wait();
   if (!TH) {
     for (int k = warp; k < N; k += nw)
       for (int c = lane; c < NC; c += 32)
@@ -251,8 +252,7 @@ static cudaError_t lin_launch(const LinArg &a, int nw, int gy, cudaStream_t s) {
   const size_t sm = lin_smem(a.N, NCL, CPL, nw, a.staged != 0);
   cudaError_t e = allow_dyn_smem(k_lin<KIND, NCL, CPL>, sm);
   if (e) return e;
-  k_lin<KIND, NCL, CPL><<<dim3((a.M + NC - 1) / NC, gy), nw * 32, sm, s>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(k_lin<KIND, NCL, CPL>, dim3((a.M + NC - 1) / NC, gy), nw * 32, sm, s, a);
 }
 
 // One transform of M columns (z: entry k of column c at in[c + M k]; theta:

@@ -31,11 +31,12 @@ __device__ __forceinline__ double ld(const double *p) { return __ldg(p); }
 // ---------------------------------------------------------------------------
 // hdnbc (momentum_terms_swirl.F90:177-296), one thread per (ic, jc<=nrc)
 // ---------------------------------------------------------------------------
-__global__ void k_hdnbc(Geo g, Rk rk, double cs, double cor, const double *__restrict__ q3,
+__global__ void k_hdnbc(Geo g, Rk rk, double cs, double cor, const double *q3,
                         double *csort, double *tconv, double *corr3n, double *dq3no,
                         double *corr3s) {
   int ic = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   int jc = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+  pdl_wait();
   if (ic > g.nth || jc > g.nrc) return;
   int o = I2O(g, ic, jc);
   corr3s[o] = (jc <= g.nr && g.rc[jc] <= (double)0.4999f) ? cs : 0.0;
@@ -57,9 +58,8 @@ cudaError_t launch_hdnbc(vr_ctx *c, const Rk &rk, double cs, double cor) {
   const Geo &g = c->geo;
   dim3 b(32, 4), gr((g.nth + 31) / 32, (g.nrc + 3) / 4);
   LaunchScope ls(c, PK_HDNBC);
-  k_hdnbc<<<gr, b, 0, c->stream>>>(g, rk, cs, cor, c->q[2], c->csort, c->tconv, c->corr3n, c->dq3no,
-                                   c->corr3s);
-  return cudaGetLastError();
+  return launch_pdl(k_hdnbc, gr, b, 0, c->stream, g, rk, cs, cor, c->q[2], c->csort, c->tconv, c->corr3n, c->dq3no,
+                    c->corr3s);
 }
 
 // ---------------------------------------------------------------------------
@@ -176,7 +176,7 @@ struct RhsArgsT {
   QV q;
   const double *__restrict__ dqh[3];  // H when not inlined
   T *ru[3];
-  const T *__restrict__ prg;
+  const T *prg;
   double *qrhs[3];
 };
 using RhsArgs = RhsArgsT<double>;
@@ -784,6 +784,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
   const int ke = min(kb + zs, g.nz + 1);  // planes kb .. ke-1 are evaluated
   const int nplanes = ke - kb + 2;        // planes kb-1 .. ke are loaded
   if (smem_u32(sm) & 127u) {
+    pdl_wait();
     if (tid == 0) atomicOr(status, 2u);
     return;
   }
@@ -795,11 +796,6 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     tma_load_3d(dst + FSP, &tq2, 0, j0 - 1, kc, &full[sl]);
     tma_load_3d(dst + 2 * FSP, &tq3, 0, j0 - 1, kc, &full[sl]);
   };
-  if (tid == 0) {
-    for (int sl = 0; sl < kQRing; sl++) mbar_init(&full[sl], 1);
-    mbar_init_fence();
-    for (int pr = 0; pr < kQRing && pr < nplanes; pr++) issue(pr);
-  }
   for (int idx = tid; idx < 2 * RJ * N; idx += blockDim.x) {
     const int i = idx % N, r = (idx / N) % RJ, fam = idx / (N * RJ), jc = j0 + r;
     if (jc > g.nr) continue;
@@ -826,10 +822,17 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     const int o = i3(i + 1, jc, kc);
 #pragma unroll
     for (int m = 0; m < 3; m++) {
-      pru[m] = __ldg(a.ru[m] + o);
-      ppg[m] = __ldg(a.prg + iprg(i + 1, jc, kc, m + 1));
+      pru[m] = a.ru[m][o];
+      ppg[m] = a.prg[iprg(i + 1, jc, kc, m + 1)];
     }
   };
+  if (tid == 0) {
+    for (int sl = 0; sl < kQRing; sl++) mbar_init(&full[sl], 1);
+    mbar_init_fence();
+  }
+  pdl_wait();  // up to here: constant tables
+  if (tid == 0)
+    for (int pr = 0; pr < kQRing && pr < nplanes; pr++) issue(pr);
   prefetch(kb);
   cp_async_wait_all();
   __syncthreads();
@@ -948,8 +951,7 @@ static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) 
   const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, ctas * c->nsm);
   const int grid = rows * ((g.nz + zs - 1) / zs);
   LaunchScope ls(c, PK_RHS);
-  kern<<<grid, NTH, sm, c->stream>>>(tm[0], tm[1], tm[2], g, rk, a, t13, t2, zs, c->d_status);
-  return cudaGetLastError();
+  return launch_pdl(kern, grid, NTH, sm, c->stream, tm[0], tm[1], tm[2], g, rk, a, t13, t2, zs, c->d_status);
 }
 
 template <class T>

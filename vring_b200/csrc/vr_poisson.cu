@@ -467,7 +467,7 @@ struct DivSrc {
 };
 
 template <int T, class TQ = double, bool DIV = false>
-__global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_fwd_s(const double *__restrict__ in, double *__restrict__ out,
+__global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_fwd_s(const double *in, double *out,
                                                    int nlines, const double *__restrict__ tw, DivSrc<TQ> dv) {
   constexpr int N = 16 * T, NPB = 128 / T, PS = fft_pair_stride(T);
   extern __shared__ double2 smv[];
@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_fwd_s(const double *__
   double2 *sc = smv + 15 * T + (size_t)pl * PS;
   load_lane_twiddles<T>(twl, tw);
   __syncthreads();
+  pdl_wait();
   const int la = (blockIdx.x * NPB + pl) * 2;
   if (la >= nlines) return;  // no CTA barrier follows; the pair's group leaves together
   const unsigned gm = T >= 32 ? 0xffffffffu : (((1u << T) - 1u) << ((tid & 31) / T * T));
@@ -494,11 +495,11 @@ __global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_fwd_s(const double *__
 #pragma unroll
     for (int m = 0; m < 16; m++) {
       const int i = t + T * m, ip = i + 1 < N ? i + 1 : 0;
-      re[m] = divq_of(g, dv.inv_adt, (double)__ldg(a1 + ip), (double)__ldg(a1 + i), (double)__ldg(a2 + i + sj),
-                      (double)__ldg(a2 + i), (double)__ldg(a3 + i + sk), (double)__ldg(a3 + i), irma);
-      im[m] = hasb ? divq_of(g, dv.inv_adt, (double)__ldg(b1 + ip), (double)__ldg(b1 + i),
-                             (double)__ldg(b2 + i + sj), (double)__ldg(b2 + i), (double)__ldg(b3 + i + sk),
-                             (double)__ldg(b3 + i), irmb)
+      re[m] = divq_of(g, dv.inv_adt, (double)a1[ip], (double)a1[i], (double)a2[i + sj],
+                      (double)a2[i], (double)a3[i + sk], (double)a3[i], irma);
+      im[m] = hasb ? divq_of(g, dv.inv_adt, (double)b1[ip], (double)b1[i],
+                             (double)b2[i + sj], (double)b2[i], (double)b3[i + sk],
+                             (double)b3[i], irmb)
                    : 0.0;
     }
   } else {
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_fwd_s(const double *__
 }
 
 template <int T>
-__global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_bwd_s(const double *__restrict__ in, double *__restrict__ dph, Geo g,
+__global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_bwd_s(const double *in, double *dph, Geo g,
                                                    int nlines, const double *__restrict__ tw) {
   constexpr int N = 16 * T, NPB = 128 / T, PS = fft_pair_stride(T);
   extern __shared__ double2 smv[];
@@ -548,6 +549,7 @@ __global__ void __launch_bounds__(128, VR_FFT_MINB) k_fft_bwd_s(const double *__
   double2 *sc = smv + 15 * T + (size_t)pl * PS;
   load_lane_twiddles<T>(twl, tw);
   __syncthreads();
+  pdl_wait();
   const int la = (blockIdx.x * NPB + pl) * 2;
   if (la >= nlines) return;  // no CTA barrier follows; the pair's group leaves together
   const unsigned gm = T >= 32 ? 0xffffffffu : (((1u << T) - 1u) << ((tid & 31) / T * T));
@@ -714,6 +716,7 @@ __global__ void __launch_bounds__(LT * 16) k_dct_w(const double *in, double *out
   const size_t s2 = (size_t)g.nth * g.nr;
   const double *base = in + i0 + (size_t)g.nth * j;
   double *dest = out + i0 + (size_t)g.nth * j;  // in place when in == out: the CTA holds its whole columns
+  pdl_wait();
   for (int idx = threadIdx.x; idx < N * LT; idx += LT * 16) {
     int k = idx / LT, l = idx % LT;
     if (l < nl)
@@ -969,11 +972,9 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
     tma_load_3d(buf(s), &tm, i0, j, 0, bar);
     tma_load_3d(buf(s) + 256 * 8, &tm, i0, j, 256, bar);
   };
-  // the first tiles start loading while the CTA stages its twiddles
   if (tid == 0) {
     for (int bf = 0; bf < kDctBufs; bf++) mbar_init(&full[bf], 1);
     mbar_init_fence();
-    for (int s = 0; s < min(nmine, kDctBufs - 1); s++) issue_load(s);
   }
   for (int i = tid; i < 7 * 64; i += 512) {
     const int p = (i & 63) * (i / 64 + 1);
@@ -984,6 +985,9 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
     tw2[i] = make_double2(__ldg(twz + 2 * p), -__ldg(twz + 2 * p + 1));
   }
   for (int i = tid; i < N; i += 512) shl[i] = make_double2(__ldg(twz + 2 * N + 2 * i), __ldg(twz + 2 * N + 2 * i + 1));
+  pdl_wait();  // up to here: twiddles
+  if (tid == 0)
+    for (int s = 0; s < min(nmine, kDctBufs - 1); s++) issue_load(s);
   __syncthreads();
   // tile s + 2 loads into the buffer of tile s - 1 once that tile's store
   // has read it out; thread 0 refills it halfway through tile s
@@ -1137,13 +1141,15 @@ __global__ void __launch_bounds__(512, 1) k_dct2_tma(const __grid_constant__ CUt
   if (tid == 0) {
     for (int bf = 0; bf < kDctBufs; bf++) mbar_init(&full[bf], 1);
     mbar_init_fence();
-    for (int s = 0; s < min(nmine, kDctBufs - 1); s++) issue_load(s);
   }
   auto tw = [&](int p) { return make_double2(__ldg(twz + 2 * p), -__ldg(twz + 2 * p + 1)); };  // W_1024^p
   for (int i = tid; i < 7 * 64; i += 512) tw1[i] = tw(2 * (i & 63) * (i / 64 + 1));
   for (int i = tid; i < 7 * 8; i += 512) tw2[i] = tw(16 * (i & 7) * (i / 8 + 1));
   for (int i = tid; i < 512; i += 512) tw0[i] = tw(i);
   for (int i = tid; i < N; i += 512) shl[i] = make_double2(__ldg(twz + 2 * N + 2 * i), __ldg(twz + 2 * N + 2 * i + 1));
+  pdl_wait();  // up to here: twiddles
+  if (tid == 0)
+    for (int s = 0; s < min(nmine, kDctBufs - 1); s++) issue_load(s);
   __syncthreads();
   auto refill = [&](int s) {
     if (tid == 0 && s + kDctBufs - 1 < nmine) {
@@ -1809,19 +1815,20 @@ static cudaError_t run_fft_s(vr_ctx *c, int dir, const Rk *div_rk = nullptr) {
       if ((e = allow_dyn_smem(kern, sm))) return e;
       DivSrc<float> dv{g, inv_adt, reinterpret_cast<const float *>(c->dq[0]),
                        reinterpret_cast<const float *>(c->dq[1]), reinterpret_cast<const float *>(c->dq[2])};
-      kern<<<blocks, 128, sm, c->stream>>>(nullptr, theta_spec(c), nlines, c->tw_th, dv);
+      return launch_pdl(kern, blocks, 128, sm, c->stream, nullptr, theta_spec(c), nlines, c->tw_th, dv);
     } else {
       auto kern = k_fft_fwd_s<T, double, true>;
       if ((e = allow_dyn_smem(kern, sm))) return e;
       DivSrc<double> dv{g, inv_adt, c->dq[0], c->dq[1], c->dq[2]};
-      kern<<<blocks, 128, sm, c->stream>>>(nullptr, theta_spec(c), nlines, c->tw_th, dv);
+      return launch_pdl(kern, blocks, 128, sm, c->stream, nullptr, theta_spec(c), nlines, c->tw_th, dv);
     }
   } else if (dir > 0) {
     if ((e = allow_dyn_smem(k_fft_fwd_s<T>, sm))) return e;
-    k_fft_fwd_s<T><<<blocks, 128, sm, c->stream>>>(c->rhs, theta_spec(c), nlines, c->tw_th, DivSrc<double>{});
+    return launch_pdl(k_fft_fwd_s<T, double, false>, blocks, 128, sm, c->stream, c->rhs, theta_spec(c), nlines, c->tw_th,
+                      DivSrc<double>{});
   } else {
     if ((e = allow_dyn_smem(k_fft_bwd_s<T>, sm))) return e;
-    k_fft_bwd_s<T><<<blocks, 128, sm, c->stream>>>(theta_spec(c), c->dph, g, nlines, c->tw_th);
+    return launch_pdl(k_fft_bwd_s<T>, blocks, 128, sm, c->stream, theta_spec(c), c->dph, g, nlines, c->tw_th);
   }
   return cudaGetLastError();
 }
@@ -1852,8 +1859,8 @@ static cudaError_t run_dct_w(vr_ctx *c, int dir) {
   cudaError_t e = allow_dyn_smem(k_dct_w<E, LT>, sm);
   if (e) return e;
   LaunchScope ls(c, PK_DCT);
-  k_dct_w<E, LT><<<dim3((g.nth + LT - 1) / LT, g.nr), LT * 16, sm, c->stream>>>(c->spec, c->spec, g, dir, c->tw_z);
-  return cudaGetLastError();
+  return launch_pdl(k_dct_w<E, LT>, dim3((g.nth + LT - 1) / LT, g.nr), LT * 16, sm, c->stream, c->spec, c->spec, g, dir,
+                    c->tw_z);
 }
 
 // The z transform of ncol columns (entry k of column c at in[c + ncol k]) for
@@ -1900,8 +1907,7 @@ static cudaError_t run_dct_tma(vr_ctx *c, int dir) {
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
   LaunchScope ls(c, PK_DCT);
-  kern<<<std::min(ntiles, c->nsm), threads, sm, c->stream>>>(tm, nti, ntiles, c->tw_z, c->d_status);
-  return cudaGetLastError();
+  return launch_pdl(kern, std::min(ntiles, c->nsm), threads, sm, c->stream, tm, nti, ntiles, c->tw_z, c->d_status);
 }
 
 // the same for 1024 points
@@ -1916,8 +1922,7 @@ static cudaError_t run_dct2_tma(vr_ctx *c, int dir) {
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
   LaunchScope ls(c, PK_DCT);
-  kern<<<std::min(ntiles, c->nsm), 512, sm, c->stream>>>(tm, nti, ntiles, c->tw_z, c->d_status);
-  return cudaGetLastError();
+  return launch_pdl(kern, std::min(ntiles, c->nsm), 512, sm, c->stream, tm, nti, ntiles, c->tw_z, c->d_status);
 }
 
 static cudaError_t dct_warp_dispatch(vr_ctx *c, int dir, bool *done) {

@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
   const int ke = min(kb + zs, g.nz + 1);  // planes kb .. ke-1 are updated
   const int nplanes = ke - kb + 3;        // planes kb-2 .. ke are loaded
   if (smem_u32(sm) & 127u) {
+    pdl_wait();
     if (tid == 0) atomicOr(status, 2u);
     return;
   }
@@ -314,13 +315,15 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
   if (tid == 0) {
     for (int sl = 0; sl < kUpRing; sl++) mbar_init(&full[sl], 1);
     mbar_init_fence();
-    for (int pr = 0; pr < kUpRing && pr < nplanes; pr++) issue(pr);
   }
   const int r = tid / N, i = tid % N, jc = j0 + r;
   const bool act = tid < RJ * N && jc <= g.nr;
   const int ip = i + 1 < N ? i + 1 : 0, im = i > 0 ? i - 1 : N - 1, imm = im > 0 ? im - 1 : N - 1;
   UpRow m{};
   if (act) m = up_row(g, jc);
+  pdl_wait();  // up to here: the row's coefficients
+  if (tid == 0)
+    for (int pr = 0; pr < kUpRing && pr < nplanes; pr++) issue(pr);
   // prefetched in the storage type: a conversion right after the load
   // would wait for it
   T pp1 = T(0), pp2 = T(0), pp3 = T(0), pps = T(0);
@@ -335,9 +338,9 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     }
     if constexpr (UPSOL) {
       const int o = I3(g, i + 1, jc, kc);
-      pd1 = __ldg(us.dq1 + o);
-      pd2 = __ldg(us.dq2 + o);
-      pd3 = __ldg(us.dq3 + o);
+      pd1 = us.dq1[o];
+      pd2 = us.dq2[o];
+      pd3 = us.dq3[o];
     }
   };
   prefetch(kb);
@@ -353,8 +356,8 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     if (jc == g.nr) us.q2[o + g.nth] = 0.0;
     if (kc == 1) {
       us.q3[o] = d3;  // imposed south value, rows 0 .. nrc
-      if (jc == 1) us.q3[o - g.nth] = (double)__ldg(us.dq3 + o - g.nth);
-      if (jc == g.nr) us.q3[o + g.nth] = (double)__ldg(us.dq3 + o + g.nth);
+      if (jc == 1) us.q3[o - g.nth] = (double)us.dq3[o - g.nth];
+      if (jc == g.nr) us.q3[o + g.nth] = (double)us.dq3[o + g.nth];
     } else {
       const double v3 = d3 - us.adt * g.dx3 * (Pc[rc + i] - Pl[rc + i]);
       us.q3[o] = v3;
@@ -440,9 +443,8 @@ static cudaError_t run_uppres_march_n(vr_ctx *c, double be, double adt) {
   const int grid = rows * ((g.nz + zs - 1) / zs);
   UpsolArgs<T> us{reinterpret_cast<const T *>(c->dq[0]), reinterpret_cast<const T *>(c->dq[1]),
                   reinterpret_cast<const T *>(c->dq[2]), c->q[0], c->q[1], c->q[2], adt};
-  kern<<<grid, NTH, sm, c->stream>>>(tm, g, be, reinterpret_cast<T *>(c->prg), reinterpret_cast<T *>(c->pres),
-                                      c->dph, zs, c->d_status, us);
-  return cudaGetLastError();
+  return launch_pdl(kern, grid, NTH, sm, c->stream, tm, g, be, reinterpret_cast<T *>(c->prg),
+                    reinterpret_cast<T *>(c->pres), c->dph, zs, c->d_status, us);
 }
 
 template <class T, bool UPSOL>
