@@ -34,6 +34,24 @@ def test_fused_substep(grid, irk):
         assert_field_close(gpu, orc, n, rel=1e-11)
 
 
+@pytest.mark.parametrize("grid", GRIDS + [(9, 6, 10)], ids=lambda g: "x".join(map(str, g)))
+def test_step_with_given_explicit_terms(grid):
+    """vr_step on arbitrary H in dq1..3: the walk that reads them (odd theta
+    extents go through the separate kernels)."""
+    orc, gpu = make_pair(*grid, wth="modified")
+    _state(orc, gpu, grid, 5)
+    rng = np.random.default_rng(6)
+    for n in ("dq1", "dq2", "dq3"):
+        a = orc.field(n)
+        a[...] = 0.1 * rng.uniform(-1.0, 1.0, size=a.shape)
+    copy_to_gpu(orc, gpu, ["dq1", "dq2", "dq3"])
+    prep(orc, gpu, 2, 2e-3, 0)
+    orc.step()
+    gpu.step()
+    for n in ("dq1", "dq2", "dq3", "ru1", "ru2", "ru3"):
+        assert_field_close(gpu, orc, n, rel=1e-11)
+
+
 @pytest.mark.parametrize("grid", [(32, 12, 40), (64, 9, 36), (256, 6, 32)], ids=lambda g: "x".join(map(str, g)))
 def test_mixed_form_follows_fp64(grid):
     """One step of the mixed form against FP64 on a ring: the fields are stored

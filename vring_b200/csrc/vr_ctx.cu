@@ -969,8 +969,14 @@ extern "C" int vr_step(vr_ctx *c) {
   if (!c) return VR_ERR_ARG;
   if (c->mixed) return set_err(c, VR_ERR_STATE, "vr_step: the mixed form runs through vr_substep/vr_iterate only");
   VR_CUDA(c, cudaSetDevice(c->dev));
-  VR_CUDA(c, launch_rhs(c, rk_of(c), false));
-  VR_CUDA(c, sweeps(c));
+  const cudaError_t e = launch_rhs_tsweep(c, rk_of(c), true);
+  if (e == cudaErrorNotSupported) {
+    (void)cudaGetLastError();
+    VR_CUDA(c, launch_rhs(c, rk_of(c), false));
+  } else {
+    VR_CUDA(c, e);
+  }
+  VR_CUDA(c, sweeps(c, e == cudaSuccess));
   return VR_OK;
 }
 

@@ -174,7 +174,7 @@ cudaError_t launch_hdnl(vr_ctx *c, int comp) {
 template <class T>
 struct RhsArgsT {
   QV q;
-  const double *__restrict__ dqh[3];  // H when not inlined
+  const double *dqh[3];  // H when not inlined
   T *ru[3];
   const T *prg;
   double *qrhs[3];
@@ -291,7 +291,8 @@ __device__ __forceinline__ RowCoef row_coef(const Geo &g, int jc) {
 }
 
 // hdnl1-3 and the RK right-hand sides of one cell from its samples and the
-// coefficients m of its row
+// coefficients m of its row; HIN: H comes in as out.h1 .. h3 instead
+template <bool HIN = false>
 __device__ __forceinline__ void rhs_eval(const Geo &g, const Rk &rk, int jc, int kc, const RhsSamples &S,
                                          const RowCoef &m, RhsCell &out) {
   const double A1 = S.A1, A2 = S.A2, A3 = S.A3, A4 = S.A4, A5 = S.A5, A6 = S.A6, A7 = S.A7, A8 = S.A8, A9 = S.A9;
@@ -300,8 +301,9 @@ __device__ __forceinline__ void rhs_eval(const Geo &g, const Rk &rk, int jc, int
   const double ru1 = S.ru1, ru2 = S.ru2, ru3 = S.ru3, pg1 = S.pg1, pg2 = S.pg2, pg3 = S.pg3;
   const double are = rk.alm / g.re;
   const bool do3 = kc >= 2, do2 = jc >= 2;
-  double h1, h2 = 0.0, h3 = 0.0, r1, r2 = 0.0, r3 = 0.0;
-  {  // hdnl1 (momentum_terms_swirl.F90:29-68)
+  double h1 = 0.0, h2 = 0.0, h3 = 0.0, r1, r2 = 0.0, r3 = 0.0;
+  if constexpr (HIN) h1 = out.h1, h2 = out.h2, h3 = out.h3;
+  if constexpr (!HIN) {  // hdnl1 (momentum_terms_swirl.F90:29-68)
     const double q1c = A1, q1p = A2, q1m = A3;
     double qnn = q1p + q1c, qss = q1m + q1c;
     const double h11 = (qnn * qnn - qss * qss) * m.h1d11;
@@ -328,7 +330,7 @@ __device__ __forceinline__ void rhs_eval(const Geo &g, const Rk &rk, int jc, int
     r1 = (rk.gam * h1 + rk.rom * ru1 - rk.alm * pg1 + are * (d11 + d33 + d22)) * g.dt;
   }
   if (do3) {
-    {  // hdnl3 (momentum_terms_swirl.F90:150-171)
+    if constexpr (!HIN) {  // hdnl3 (momentum_terms_swirl.F90:150-171)
       const double q3c = C1;
       double qnn = (C4 + q3c) * (B4 + B9);
       double qss = (C5 + q3c) * (B1 + B7);
@@ -351,7 +353,7 @@ __device__ __forceinline__ void rhs_eval(const Geo &g, const Rk &rk, int jc, int
     r3 = (rk.gam * h3 + rk.rom * ru3 - rk.alm * pg3 + are * (d11 + d33 + d22)) * g.dt;
   }
   if (do2) {
-    {  // hdnl2 (momentum_terms_swirl.F90:94-128)
+    if constexpr (!HIN) {  // hdnl2 (momentum_terms_swirl.F90:94-128)
       const double q1p = A2, q1pm = A8, q1c = A1, q1cm = A5, q2c = B1;
       double qnn = (q1p + q1pm) * (B2 + q2c);
       double qss = (q1c + q1cm) * (q2c + B3);
@@ -752,7 +754,11 @@ __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const do
 // 32 cells in 256 threads and 32 planes per CTA, 21 with 8 rows and 4 planes);
 // lines beyond 128 cells take two rows in 512 threads, one CTA per SM
 // (256 x 128 x 1024, mixed: 1.35 ms by whole lines per warp, 1.08 here).
-template <int RJ, int NTH, int TL, int E, class T, int NT>
+// HIN: the explicit terms are read from dqh (vr_hdnl1..3 wrote them) and only
+// the right-hand sides and theta solves remain, in the same walk (vr_step,
+// 64 x 128 x 256, cold: right-hand sides 63 us and three theta sweeps of 20 us,
+// 92 here).
+template <int RJ, int NTH, int TL, int E, class T, int NT, bool HIN>
 __global__ void __launch_bounds__(NTH, 512 / NTH)
     k_rhs_march(const __grid_constant__ CUtensorMap tq1, const __grid_constant__ CUtensorMap tq2,
                 const __grid_constant__ CUtensorMap tq3, Geo g, Rk rk, RhsArgsT<T> a, TriPer t13, TriPer t2,
@@ -817,6 +823,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
   // prefetched in the storage type: a conversion right after the load
   // would wait for it
   T pru[3], ppg[3];
+  double ph[3];  // HIN
   auto prefetch = [&](int kc) {
     if (!cact) return;
     const int o = i3(i + 1, jc, kc);
@@ -824,6 +831,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     for (int m = 0; m < 3; m++) {
       pru[m] = a.ru[m][o];
       ppg[m] = a.prg[iprg(i + 1, jc, kc, m + 1)];
+      if constexpr (HIN) ph[m] = a.dqh[m][o];
     }
   };
   if (tid == 0) {
@@ -849,6 +857,8 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     T cru[3], cpg[3];
 #pragma unroll
     for (int m = 0; m < 3; m++) cru[m] = pru[m], cpg[m] = ppg[m];
+    RhsCell v;
+    if constexpr (HIN) v.h1 = ph[0], v.h2 = ph[1], v.h3 = ph[2];
     if (kc + 1 < ke) prefetch(kc + 1);
     const double *sp = ring + (size_t)((pr - 1) % kQRing) * SLOT;
     const double *sc = ring + (size_t)(pr % kQRing) * SLOT;
@@ -870,8 +880,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
       S.C6 = n3[rc + i], S.C7 = p3[rc + i], S.C8 = n3[rc + im], S.C9 = n3[rs + i];
       S.ru1 = (double)cru[0], S.ru2 = (double)cru[1], S.ru3 = (double)cru[2];
       S.pg1 = (double)cpg[0], S.pg2 = (double)cpg[1], S.pg3 = (double)cpg[2];
-      RhsCell v;
-      rhs_eval(g, rk, jc, kc, S, rowc[r], v);
+      rhs_eval<HIN>(g, rk, jc, kc, S, rowc[r], v);
       const int o = i3(i + 1, jc, kc);
       a.ru[0][o] = (T)v.h1;
       lb[(size_t)(0 * RJ + r) * SPL + tpad(i)] = v.r1;
@@ -930,7 +939,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
   }
 }
 
-template <int RJ, int NTH, int TL, int E, class T, int NT = 0>
+template <int RJ, int NTH, int TL, int E, class T, int NT = 0, bool HIN = false>
 static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) {
   const Geo &g = c->geo;
   if ((g.nth & 1) || RJ * g.nth > NTH || g.nth - 1 > 32 * E || (NT > 0 && g.nth != NT))
@@ -944,7 +953,7 @@ static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) 
   const size_t sm = sizeof(double) * ((size_t)kQRing * 3 * FSP + kTB * 3 * RJ * SPL + 2 * RJ * 3 * SPL);
   constexpr int ctas = 512 / NTH;  // per SM
   if (sm > (220 / ctas) * 1024) return cudaErrorNotSupported;
-  auto kern = k_rhs_march<RJ, NTH, TL, E, T, NT>;
+  auto kern = k_rhs_march<RJ, NTH, TL, E, T, NT, HIN>;
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
   const TriPer &t13 = c->ttri[c->irk][0], &t2 = c->ttri[c->irk][1];
@@ -954,7 +963,7 @@ static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) 
   return launch_pdl(kern, grid, NTH, sm, c->stream, tm[0], tm[1], tm[2], g, rk, a, t13, t2, zs, c->d_status);
 }
 
-template <class T>
+template <class T, bool HIN>
 static cudaError_t launch_rhs_tsweep_t(vr_ctx *c, const Rk &rk) {
   const Geo &g = c->geo;
   RhsArgsT<T> a;
@@ -969,16 +978,16 @@ static cudaError_t launch_rhs_tsweep_t(vr_ctx *c, const Rk &rk) {
   cudaError_t me = cudaErrorNotSupported;
   // rows per CTA: as many as its threads have cells for
   if (g.nth <= 32)
-    me = run_rhs_march<8, 256, 8, 1, T>(c, rk, a);
+    me = run_rhs_march<8, 256, 8, 1, T, 0, HIN>(c, rk, a);
   else if (g.nth <= 64)
-    me = run_rhs_march<4, 256, 8, 2, T>(c, rk, a);
+    me = run_rhs_march<4, 256, 8, 2, T, 0, HIN>(c, rk, a);
   else if (g.nth == 128)
-    me = run_rhs_march<2, 256, 8, 4, T, 128>(c, rk, a);
+    me = run_rhs_march<2, 256, 8, 4, T, 128, HIN>(c, rk, a);
   else if (g.nth <= 128)
-    me = run_rhs_march<2, 256, 8, 4, T>(c, rk, a);
+    me = run_rhs_march<2, 256, 8, 4, T, 0, HIN>(c, rk, a);
   else if (g.nth <= 256)
-    me = run_rhs_march<2, 512, 16, 8, T>(c, rk, a);
-  if (me != cudaErrorNotSupported) return me;
+    me = run_rhs_march<2, 512, 16, 8, T, 0, HIN>(c, rk, a);
+  if (HIN || me != cudaErrorNotSupported) return me;
   if (E <= 1) return run_rhs_tsweep<1, T>(c, rk, a);
   if (E <= 2) return run_rhs_tsweep<2, T>(c, rk, a);
   if (E <= 4) return run_rhs_tsweep<4, T>(c, rk, a);
@@ -987,9 +996,12 @@ static cudaError_t launch_rhs_tsweep_t(vr_ctx *c, const Rk &rk) {
 }
 
 // the fused momentum right-hand side and theta sweep; cudaErrorNotSupported
-// for theta lines longer than 257 (then rhs and theta sweep run apart)
-cudaError_t launch_rhs_tsweep(vr_ctx *c, const Rk &rk) {
-  return c->mixed ? launch_rhs_tsweep_t<float>(c, rk) : launch_rhs_tsweep_t<double>(c, rk);
+// for theta lines longer than 257 (then rhs and theta sweep run apart).
+// h_given (FP64): the explicit terms are in dq; also not supported for odd
+// theta extents, whose rows TMA cannot address
+cudaError_t launch_rhs_tsweep(vr_ctx *c, const Rk &rk, bool h_given) {
+  if (h_given) return c->mixed ? cudaErrorNotSupported : launch_rhs_tsweep_t<double, true>(c, rk);
+  return c->mixed ? launch_rhs_tsweep_t<float, false>(c, rk) : launch_rhs_tsweep_t<double, false>(c, rk);
 }
 
 template <int E>
