@@ -1,4 +1,4 @@
-"""The folded transforms (lengths without an FFT) and the axisymmetric direct
+"""The transforms by products (lengths without an FFT), long sweep lines and the axisymmetric direct
 solve, at the lengths where a tile, a coefficient stage or the choice of form
 ends.
 
@@ -13,7 +13,7 @@ from parity_util import assert_field_close, make_pair, prep, seed_random
 
 pytestmark = pytest.mark.gpu
 
-# (ntheta, nr, nz): theta 3 .. 16 and odd, even and long folded lines; z around
+# (ntheta, nr, nz): theta 3 .. 16 and odd, even and long lines; z around
 # the stage of 16 steps (2 x 16 positions), groups of 8 and 16 outputs, the
 # longest z; column counts below and above a CTA's 32
 GRIDS = [(3, 5, 6), (4, 4, 4), (5, 33, 8), (7, 9, 15), (8, 6, 16), (15, 13, 31), (16, 7, 33), (17, 5, 34), (31, 4, 35),
@@ -38,7 +38,7 @@ def test_folded_lengths_match_oracle(grid):
 
 # z of 1024: tiles of 8 slots streamed (theta a multiple of 8; more tiles than
 # SMs, so that the buffers rotate), else whole columns per warp; z lines of
-# 1025 positions in 64 chunks (even theta) or the shared-memory sweep
+# 1025 positions in registers (even theta) or the shared-memory sweep
 @pytest.mark.parametrize("grid", [(8, 5, 1024), (24, 4, 1024), (256, 16, 1024), (12, 4, 1024), (5, 4, 1024)],
                          ids=lambda g: "x".join(map(str, g)))
 def test_long_z_lines_match_oracle(grid):
@@ -57,8 +57,23 @@ def test_long_z_lines_match_oracle(grid):
         assert_field_close(gpu, orc, n)
 
 
+# r lines where the register form begins and ends (641 .. 1088 positions, q2
+# has one less), where its chunks are full (1024) and where its last chunks are
+# empty (673 = 30 x 22 + 13 in 32 chunks of 22)
+@pytest.mark.parametrize("grid", [(4, 640, 4), (4, 641, 4), (6, 673, 4), (4, 1024, 4), (10, 1088, 4), (4, 1089, 4),
+                                  (5, 700, 4), (64, 700, 40)], ids=lambda g: "x".join(map(str, g)))
+def test_long_r_lines_match_oracle(grid):
+    orc, gpu = make_pair(*grid)
+    seed_random(orc, gpu, ["q1", "q2", "q3", "ru1", "ru2", "ru3", "prg", "dq1", "dq2", "dq3"], seed=10, scale=0.1)
+    prep(orc, gpu)
+    orc.step()
+    gpu.step()
+    for n in ("dq1", "dq2", "dq3"):
+        assert_field_close(gpu, orc, n)
+
+
 def test_folded_columns_above_two_ctas_per_sm():
-    # 64-column CTAs: theta 64 by FFT, z folded, nth * nr / 64 >= 2 * 148
+    # 64-column CTAs: theta 64 by FFT, z by products, nth * nr / 64 >= 2 * 148
     nth, nr, nz = 64, 300, 20
     orc, gpu = make_pair(nth, nr, nz)
     seed_random(orc, gpu, ["rhs"], seed=8)
@@ -93,7 +108,7 @@ def _direct(faces, nz, zmax, f):
     return fh @ C
 
 
-# z: FFT (32 .. 1024), folded (other lengths up to 1453), full products above;
+# z: FFT (32 .. 1024), products by k_lin (other lengths up to 1453), full products above;
 # r: below a lane's 16 positions, around a segment of 512
 @pytest.mark.parametrize("nr,nz", [(4, 4), (5, 7), (16, 16), (17, 31), (33, 32), (100, 33), (511, 64), (512, 97),
                                    (513, 128), (64, 180), (30, 256), (40, 512), (1025, 40), (512, 1024), (20, 1000),

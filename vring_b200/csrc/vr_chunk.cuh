@@ -23,31 +23,10 @@ namespace vr {
 // In-place exclusive scan of the NCH chunk maps of each line held in
 // sM/sC[chunk][line]; forward (chunk 0 first) or backward (last chunk
 // first).  Every warp scans 32 / NCH lines, NCH lanes per line.  On return
-// sC[chunk][line] is the recurrence value entering the chunk.  With 64 chunks a
-// warp scans one line, two adjacent chunks per lane.
+// sC[chunk][line] is the recurrence value entering the chunk.
 template <bool FORWARD, int NCH, int LPT = 32>
 __device__ __forceinline__ void chain_chunks(double (*sM)[LPT + 1], double (*sC)[LPT + 1], int warp, int lane) {
-  if constexpr (NCH == 64) {
-    if (warp >= LPT) return;
-    const int c0 = 2 * lane, c1 = c0 + 1;
-    const double M0 = sM[c0][warp], C0 = sC[c0][warp], M1 = sM[c1][warp], C1 = sC[c1][warp];
-    double M = M0 * M1, C = FORWARD ? C1 + M1 * C0 : C0 + M0 * C1;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const double om = FORWARD ? __shfl_up_sync(0xffffffffu, M, d) : __shfl_down_sync(0xffffffffu, M, d);
-      const double oc = FORWARD ? __shfl_up_sync(0xffffffffu, C, d) : __shfl_down_sync(0xffffffffu, C, d);
-      if (FORWARD ? lane >= d : lane + d < 32) {
-        C = C + M * oc;
-        M = M * om;
-      }
-    }
-    double in = FORWARD ? __shfl_up_sync(0xffffffffu, C, 1) : __shfl_down_sync(0xffffffffu, C, 1);
-    if (FORWARD ? lane == 0 : lane == 31) in = 0.0;
-    sC[c0][warp] = FORWARD ? in : C1 + M1 * in;
-    sC[c1][warp] = FORWARD ? C0 + M0 * in : in;
-    return;
-  }
-  constexpr int LPW = NCH <= 32 ? 32 / NCH : 1;  // lines per warp
+  constexpr int LPW = 32 / NCH;  // lines per warp
   const int ch = lane % NCH, line = warp * LPW + lane / NCH;
   if (line >= LPT) return;  // warps beyond the tile's lines
   double M = sM[ch][line], C = sC[ch][line];
@@ -199,11 +178,6 @@ __global__ void __launch_bounds__(32 * NCH, NCH == 16 ? 2 : 1) k_chunk(P p) {
 struct TmaTile {
   int nbox, br, ldim;
 };
-template <int NP, class P>
-__host__ __device__ constexpr bool chunk_tab_dyn() {
-  return !P::kLineIB && NP > 544;
-}
-
 template <int LPT, int NCH, int MAXCL, int S, int MINB, class P>
 __global__ void __launch_bounds__(LPT *NCH, MINB)
     k_chunk_tma(const __grid_constant__ CUtensorMap tm, P p, int ntiles, TmaTile tt, unsigned *status) {
@@ -215,14 +189,9 @@ __global__ void __launch_bounds__(LPT *NCH, MINB)
   // chunk maps of the forward and the backward substitution (separate, so
   // that one tile needs four CTA barriers)
   __shared__ double sM[NCH][LPT + 1], sC[NCH][LPT + 1], sMb[NCH][LPT + 1], sCb[NCH][LPT + 1];
-  // (a, ib), -a ib and c ib per position; behind the stages where they would
-  // pass the 48 KB of static shared memory
-  constexpr bool kTabDyn = chunk_tab_dyn<NP, P>();
-  __shared__ double2 sAB_[kLine || kTabDyn ? 1 : NP];
-  __shared__ double sMf_[kLine || kTabDyn ? 1 : NP], sU_[kLine || kTabDyn ? 1 : NP];
-  double *const tab = stage + (size_t)S * tt.nbox * tt.br * LPT;
-  double2 *const sAB = kTabDyn ? reinterpret_cast<double2 *>(tab) : sAB_;
-  double *const sMf = kTabDyn ? tab + 2 * NP : sMf_, *const sU = kTabDyn ? tab + 3 * NP : sU_;
+  __shared__ double2 sAB[kLine ? 1 : NP];  // (a, ib) per position
+  __shared__ double sMf[kLine ? 1 : NP];   // -a ib
+  __shared__ double sU[kLine ? 1 : NP];    // c ib
   __shared__ double sA[kLine ? NP : 1], sCc[kLine ? NP : 1];
   __shared__ __align__(8) uint64_t full[S];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -443,8 +412,7 @@ cudaError_t run_chunk_tma(P p, const void *base, int d0, int d1, int d2, int ldi
                 "tile rows must tile 128-byte boundaries");
   tt.br = (tt.br + kRowAlign - 1) / kRowAlign * kRowAlign;
   if (tt.br > 256 || ((size_t)tt.br * LPT * 8) % 128) return cudaErrorNotSupported;
-  const size_t dyn = sizeof(double) * ((size_t)S * tt.nbox * tt.br * LPT +
-                                       (chunk_tab_dyn<NCH * MAXCL, P>() ? (size_t)4 * NCH * MAXCL : 0));
+  const size_t dyn = sizeof(double) * (size_t)S * tt.nbox * tt.br * LPT;
   CUtensorMap tm;
   if (!encode_tmap_f64_3d(&tm, base, d0, d1, d2, LPT, ldim == 1 ? tt.br : 1, ldim == 2 ? tt.br : 1))
     return cudaErrorNotSupported;
@@ -456,6 +424,227 @@ cudaError_t run_chunk_tma(P p, const void *base, int d0, int d1, int d2, int ldi
   const int ntiles = p.nbx * nm2;
   const int grid = ntiles < MINB * nsm ? ntiles : MINB * nsm;
   return launch_pdl(kern, grid, LPT * NCH, dyn, st, tm, p, ntiles, tt, status);
+}
+
+// ---------------------------------------------------------------------------
+// Long lines: 32 chunks of CL = ceil(n / 32) <= MAXCL positions held in
+// registers, 8 lines (64-byte rows) in 256 threads, two CTAs per SM.  One TMA
+// stage is enough: a tile leaves it for registers at once, and the next tile
+// loads while this one is substituted and stored.  The partition, the
+// products and the order of the chain over the chunks (one thread per line,
+// first chunk to last) are those of the shared-memory tile form, so the
+// results have its bits.  Bound by memory once two CTAs overlap their
+// substitutions (a serial chain of 4 CL + 64 dependent steps) with each
+// other's loads: z lines of 256 x 128 x 1024, mixed form, 460 -> 206 us per
+// sweep.
+// ---------------------------------------------------------------------------
+template <bool FORWARD, int LPT>
+__device__ __forceinline__ void chain_serial(double (*sM)[LPT + 1], double (*sC)[LPT + 1], int line) {
+  double y = 0.0;
+#pragma unroll
+  for (int b = 0; b < 32; b += 8) {
+    double m[8], cc[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int k = FORWARD ? b + q : 31 - b - q;
+      m[q] = sM[k][line];
+      cc[q] = sC[k][line];
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int k = FORWARD ? b + q : 31 - b - q;
+      sC[k][line] = y;  // what enters chunk k
+      y = cc[q] + m[q] * y;
+    }
+  }
+}
+
+template <int MAXCL, class P>
+__global__ void __launch_bounds__(256, 2)
+    k_chunk_long(const __grid_constant__ CUtensorMap tm, P p, int ntiles, TmaTile tt, unsigned *status) {
+  constexpr int LPT = 8, NCH = 32, NP = NCH * (MAXCL + 1), HALF = MAXCL / 2;
+  using OutT = typename P::OutT;
+  extern __shared__ __align__(128) double stage[];
+  __shared__ double sM[NCH][LPT + 1], sC[NCH][LPT + 1];  // a thread writes and reads its own entry only
+  __shared__ __align__(8) uint64_t full;
+  const int slen = tt.nbox * tt.br * LPT;  // doubles of the stage
+  // (a, ib), -a ib and c ib per position, one entry of skew per chunk: the
+  // four chunks of a warp read different banks also when CL is a power of two
+  double2 *const sAB = reinterpret_cast<double2 *>(stage + slen);
+  double *const sMf = stage + slen + 2 * NP, *const sU = sMf + NP;
+  const int tid = threadIdx.x, line = tid % LPT, c = tid / LPT;
+  const int n = p.n, CL = (n + NCH - 1) / NCH, e0 = c * CL, k0 = c * (CL + 1);
+  const int cnt = max(0, min(CL, n - e0));
+  const bool has_last = cnt > 0 && e0 + cnt == n;
+  auto issue = [&](int tile) {
+    P q = p;
+    q.set_tile(tile);
+    int x, y, z;
+    q.tma_xyz(x, y, z);
+    mbar_expect_tx(&full, (unsigned)slen * 8u);
+    for (int b = 0; b < tt.nbox; b++) {
+      const int o = b * tt.br;
+      tma_load_3d(stage + (size_t)o * LPT, &tm, x, y + (tt.ldim == 1 ? o : 0), z + (tt.ldim == 2 ? o : 0), &full);
+    }
+  };
+  if (smem_u32(stage) & 127u) {  // TMA destinations need 128-byte alignment
+    pdl_wait();
+    if (tid == 0) atomicOr(status, 2u);
+    return;
+  }
+  if (tid == 0) {
+    mbar_init(&full, 1);
+    mbar_init_fence();
+  }
+  for (int e = tid; e < n; e += 256) {
+    const double a = p.a_ptr()[e], ib = p.ib[e];
+    const int o = e + e / CL;
+    sAB[o] = make_double2(a, ib);
+    sMf[o] = -a * ib;
+    sU[o] = p.c_ptr()[e] * ib;
+  }
+  __syncthreads();
+  pdl_wait();  // up to here: the factorisation
+  if (tid == 0) issue(blockIdx.x);
+
+  bool failed = false;
+  int k = 0;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
+    p.set_tile(tile);
+    const bool ok = mbar_wait(&full, (unsigned)k & 1u);
+    const double *buf = stage + (size_t)e0 * LPT + line;
+    const bool act = p.line_active(line);
+    double v[MAXCL];
+    // boundary right-hand sides of rows 0 and n-1
+    const bool lo = act && c == 0 && p.bc_lo_on(), hi = act && has_last && p.bc_hi_on();
+    const double lv = lo ? p.bc_lo_val(line) : 0.0, hv = hi ? p.bc_hi_val(line) : 0.0;
+    const int hit = hi ? cnt - 1 : MAXCL;
+#pragma unroll
+    for (int t = 0; t < MAXCL; t++) {
+      const double f = t < cnt ? buf[t * LPT] : 0.0;
+      v[t] = t == hit ? hv : f;
+    }
+    if (lo) v[0] = lv;
+    // forward: chunk map with zero input
+    double M = 1.0, C = 0.0;
+#pragma unroll
+    for (int t = 0; t < MAXCL; t++)
+      if (t < cnt) {
+        const double2 ab = sAB[k0 + t];
+        C = (v[t] - ab.x * C) * ab.y;
+        M = sMf[k0 + t] * M;
+      }
+    sM[c][line] = M;
+    sC[c][line] = C;
+    // every thread has read the stage and written its map; a failed wait
+    // ends the walk for the whole CTA
+    if (__syncthreads_or(!ok)) {
+      failed = true;
+      break;
+    }
+    if (tid == 0 && tile + gridDim.x < ntiles) {
+      fence_proxy_async();
+      issue(tile + gridDim.x);
+    }
+    if (c == 0) chain_serial<true, LPT>(sM, sC, line);
+    __syncthreads();
+    double y = sC[c][line];
+#pragma unroll
+    for (int t = 0; t < MAXCL; t++)
+      if (t < cnt) {
+        const double2 ab = sAB[k0 + t];
+        y = (v[t] - ab.x * y) * ab.y;
+        v[t] = y;
+      }
+    // backward
+    M = 1.0;
+    C = 0.0;
+#pragma unroll
+    for (int t = MAXCL - 1; t >= 0; t--)
+      if (t < cnt) {
+        const double u = sU[k0 + t];
+        C = v[t] - u * C;
+        M = -u * M;
+      }
+    sM[c][line] = M;
+    sC[c][line] = C;
+    // half of the added field arrives during the chain and the substitution
+    const bool hadd = p.has_add() && act;
+    const int st = p.stride();
+    double ad[MAXCL - HALF];
+    const double *ap = hadd ? p.add_ptr(line, e0) : nullptr;
+    if (hadd) {
+#pragma unroll
+      for (int t = HALF; t < MAXCL; t++) ad[t - HALF] = t < cnt ? ap[t * st] : 0.0;
+    }
+    __syncthreads();
+    if (c == 0) chain_serial<false, LPT>(sM, sC, line);
+    __syncthreads();
+    double x = sC[c][line];
+#pragma unroll
+    for (int t = MAXCL - 1; t >= 0; t--)
+      if (t < cnt) {
+        x = v[t] - sU[k0 + t] * x;
+        v[t] = x;
+      }
+    if (!act) continue;
+    if (hadd) {
+#pragma unroll
+      for (int t = HALF; t < MAXCL; t++) v[t] = ad[t - HALF] + v[t];
+#pragma unroll
+      for (int t = 0; t < HALF; t++) ad[t] = t < cnt ? ap[t * st] : 0.0;
+#pragma unroll
+      for (int t = 0; t < HALF; t++) v[t] = ad[t] + v[t];
+    }
+    OutT *op = p.out_ptr(line, e0);
+    const int edge = p.edges() && has_last ? cnt - 1 : MAXCL;
+#pragma unroll
+    for (int t = 0; t < MAXCL; t++)
+      if (t < cnt) {
+        op[t * st] = (OutT)v[t];
+        if (t == edge) p.edge_hi(line, v[t]);  // the row after the last position
+      }
+    if (p.ghost_copy()) {  // slip ghost one row past the line's row
+      const int go = p.ghost_off();
+      const double sl = p.slip();
+#pragma unroll
+      for (int t = 0; t < MAXCL; t++)
+        if (t < cnt) op[t * st + go] = (OutT)(sl * v[t]);
+    }
+    if (p.edges() && c == 0) p.edge_lo(line);  // the row before the first
+  }
+  if (failed) {
+    // record the timeout; the load it waited for may still land before the
+    // CTA's shared memory goes away (again a bounded wait)
+    if (tid == 0) {
+      atomicOr(status, 1u);
+      (void)mbar_wait(&full, (unsigned)k & 1u);
+    }
+    __syncthreads();
+  }
+}
+
+template <int MAXCL, class P>
+cudaError_t run_chunk_long(P p, const void *base, int d0, int d1, int d2, int ldim, int nm2, int nsm,
+                           unsigned *status, cudaStream_t st) {
+  if (p.n < 1 || p.n > 32 * MAXCL || (d0 & 1)) return cudaErrorNotSupported;
+  TmaTile tt;
+  tt.ldim = ldim;
+  tt.nbox = (p.n + 255) / 256;
+  tt.br = (p.n + tt.nbox - 1) / tt.nbox;
+  tt.br = (tt.br + 1) & ~1;  // boxes of 64-byte rows start on 128-byte boundaries
+  if (tt.br > 256) return cudaErrorNotSupported;
+  const size_t dyn = sizeof(double) * ((size_t)tt.nbox * tt.br * 8 + 4 * 32 * (MAXCL + 1));
+  CUtensorMap tm;
+  if (!encode_tmap_f64_3d(&tm, base, d0, d1, d2, 8, ldim == 1 ? tt.br : 1, ldim == 2 ? tt.br : 1))
+    return cudaErrorNotSupported;
+  auto kern = k_chunk_long<MAXCL, P>;
+  cudaError_t e = allow_dyn_smem(kern, dyn);
+  if (e) return e;
+  p.lpt = 8;
+  p.nbx = (p.nth_lines() + 7) / 8;
+  const int ntiles = p.nbx * nm2, grid = std::min(ntiles, 2 * nsm);
+  return launch_pdl(kern, grid, 256, dyn, st, tm, p, ntiles, tt, status);
 }
 
 // chunk length bucket: the smallest compiled MAXCL with 32 * MAXCL >= n

@@ -1310,11 +1310,13 @@ static cudaError_t dispatch_linesweep(vr_ctx *c, const SweepArgsT<T> &s, const C
     if (e != cudaErrorNotSupported) return e;
     return launch_chunk(p, p.nbx * nm2, c->stream);
   }
-  // up to 1088 positions: 8-line tiles as 64 chunks, one CTA per SM (two
-  // stages of 1026 rows of 64 bytes fill 131 KB).  The z lines of
-  // 256 x 128 x 1024 (1025 positions): 460 us per sweep through the
-  // shared-memory tile below, LONGZ here
-  if (s.n <= 64 * 17 && !(s.nth & 1) && !c->mixed) {
+  // 641 .. 1088 positions: 32 chunks of up to 34 in registers.  The z lines
+  // of 256 x 128 x 1024 (1025 positions), per sweep: 460 us through the
+  // shared-memory tile below, 206 here, 223 as 64 chunks of 17 in one CTA per
+  // SM.  Up to 640 positions the tile is cut into 16 chunks, which would not
+  // fit the registers, and the mixed form, whose float fields grow any
+  // rounding, keeps its bits only with the same cut.
+  if (s.n > 640 && s.n <= 32 * 34 && !(s.nth & 1)) {
     MomLine<T> p;
     p.s = s;
     p.a = cf.a;
@@ -1324,8 +1326,8 @@ static cudaError_t dispatch_linesweep(vr_ctx *c, const SweepArgsT<T> &s, const C
     const Geo &g = c->geo;
     const bool along_r = s.se == g.nth;
     LaunchScope ls(c, along_r ? PK_RSWEEP : PK_ZSWEEP);
-    const cudaError_t e = run_chunk_tma<8, 64, 17, 2, 1>(p, s.in, g.nth, g.J3, g.K3, along_r ? 1 : 2, nm2, c->nsm,
-                                                         c->d_status, c->stream);
+    const cudaError_t e = run_chunk_long<34>(p, s.in, g.nth, g.J3, g.K3, along_r ? 1 : 2, nm2, c->nsm, c->d_status,
+                                             c->stream);
     if (e != cudaErrorNotSupported) return e;
     c->nlaunch--;  // nothing was launched
   }
