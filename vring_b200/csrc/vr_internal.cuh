@@ -12,6 +12,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <stdint.h>
 
@@ -326,13 +328,23 @@ int vr_part_inflow_step(vr_part *p);
 // the dump of part_tools.F90:444-491 when this step is a dump step
 int vr_part_dump_step(vr_part *p);
 
-// Planes a z-marching CTA walks: 32, or as few as four (the right-hand side's
-// solve batch) while the grid would leave `want` resident CTAs without work.
-// The planes loaded beside its own come from L2 on grids that small.
-inline int march_planes(int row_blocks, int nz, int want) {
-  int zs = 32;
-  while (zs > 4 && row_blocks * ((nz + zs - 1) / zs) < want) zs /= 2;
-  return zs;
+// Planes a z-marching CTA walks, up to 64: the division of nz whose waves of
+// `slots` resident CTAs take least, counting a plane as one, the planes loaded
+// beside a CTA's own and its set-up as three, and (batch > 0) the theta solves
+// of up to `batch` planes as one and a half.  Against 32 planes, halved while the
+// grid leaves SMs idle (us per launch, right-hand side): 64 x 128 x 256 100 ->
+// 87, 128 x 256 x 512 513 -> 480 and 256 x 128 x 1024 mixed 1087 -> 1042 (with
+// the larger solve batch).
+inline int march_planes(int row_blocks, int nz, int slots, int batch) {
+  int best = nz, best_cost = INT_MAX;
+  for (int nb = (nz + 63) / 64; nb <= std::max(1, nz / 4); nb++) {
+    const int zs = (nz + nb - 1) / nb, n = (nz + zs - 1) / zs;
+    if (n != nb) continue;
+    const int waves = (int)(((long long)row_blocks * n + slots - 1) / slots);
+    const int cost = waves * (2 * (zs + 3) + (batch ? 3 * ((zs + batch - 1) / batch) : 0));
+    if (cost < best_cost) best_cost = cost, best = zs;
+  }
+  return best;
 }
 
 // kernel launchers (return cudaError_t of the launch) -----------------------

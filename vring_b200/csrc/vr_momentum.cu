@@ -660,7 +660,12 @@ static cudaError_t run_rhs_tsweep(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a)
 // so the CTA pays one solve phase per kTB planes and the short group scans
 // keep the instruction count per unknown low.
 // ---------------------------------------------------------------------------
-constexpr int kQRing = 4, kTB = 4;
+constexpr int kQRing = 4;
+// Planes per solve batch.  A warp takes 32 / TL lines at once: four planes of
+// 2 or 4 rows are 3/4 of a round of the CTA's warps (or 3/2), five are 15/16
+// (15/8) in the same time; four planes of 8 rows fill their rounds.  128 x 256
+// x 512, with the division of z by march_planes: 513 -> 480 us.
+constexpr int rhs_batch(int rj) { return rj == 8 ? 4 : 5; }
 
 // Periodic theta solve of one line by a group of TL consecutive lanes of a
 // warp (the arithmetic of tsolve_warp; lane g of the group owns the EG
@@ -763,6 +768,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     k_rhs_march(const __grid_constant__ CUtensorMap tq1, const __grid_constant__ CUtensorMap tq2,
                 const __grid_constant__ CUtensorMap tq3, Geo g, Rk rk, RhsArgsT<T> a, TriPer t13, TriPer t2,
                 int zs, unsigned *status) {
+  constexpr int kTB = rhs_batch(RJ);
   extern __shared__ __align__(128) double sm[];
   const int N = NT > 0 ? NT : g.nth, SPN = tpad(N) + 1;
   // offsets of the ghosted fields and of prg (I3, IPRG with this N)
@@ -906,15 +912,14 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
     if (pb == kTB - 1 || kc == ke - 1) {
       // solve the batch's [plane][comp][r] lines, 32 / TL per warp at a time
       constexpr int kGroups = 32 / TL, kLines = kTB * 3 * RJ;
-      static_assert(kLines % kGroups == 0, "a warp's lines are all in the batch or none");
       const int kc0 = kc - pb;
 #pragma unroll 1
       for (int Lw = warp * kGroups; Lw < kLines; Lw += NTH / 32 * kGroups) {
-        const int L = Lw + lane / TL;
+        const int L = min(Lw + lane / TL, kLines);  // kLines: past the batch
         const int pl = L / (3 * RJ), comp = (L / RJ) % 3, lr = L % RJ, lj = j0 + lr, lk = kc0 + pl;
         const int fam = comp == 1 ? 1 : 0;
         const double *f = fac + (size_t)(fam * RJ + lr) * 3 * SPL;
-        const bool on = lk <= kc && lj <= g.nr && !(comp == 1 && lj < 2) && !(comp == 2 && lk < 2);
+        const bool on = L < kLines && lk <= kc && lj <= g.nr && !(comp == 1 && lj < 2) && !(comp == 2 && lk < 2);
         tsolve_group<TL, (32 / TL) * E>(N, f, f + SPL, f + 2 * SPL, &rowt[lr][fam][0], lines + (size_t)L * SPL,
                                         lane % TL, on);
         __syncwarp();
@@ -922,7 +927,7 @@ __global__ void __launch_bounds__(NTH, 512 / NTH)
         for (int gq = 0; gq < kGroups; gq++) {
           const int L2 = Lw + gq;
           const int pl2 = L2 / (3 * RJ), comp2 = (L2 / RJ) % 3, r2 = L2 % RJ, jc2 = j0 + r2, lk2 = kc0 + pl2;
-          if (lk2 > kc || jc2 > g.nr || (comp2 == 1 && jc2 < 2) || (comp2 == 2 && lk2 < 2)) continue;
+          if (L2 >= kLines || lk2 > kc || jc2 > g.nr || (comp2 == 1 && jc2 < 2) || (comp2 == 2 && lk2 < 2)) continue;
           double *dst = (comp2 == 0 ? a.qrhs[0] : (comp2 == 1 ? a.qrhs[1] : a.qrhs[2])) + i3(1, jc2, lk2);
           const double *src = lines + (size_t)L2 * SPL;
           for (int e = lane; e < N; e += 32) dst[e] = src[tpad(e)];
@@ -950,6 +955,7 @@ static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) 
   const int SPN = tpad(g.nth) + 1;
   const int FS = (RJ + 2) * g.nth, FSP = (FS + 15) & ~15;
   const int SPL = ((SPN + 15) & ~15) + 8;
+  constexpr int kTB = rhs_batch(RJ);
   const size_t sm = sizeof(double) * ((size_t)kQRing * 3 * FSP + kTB * 3 * RJ * SPL + 2 * RJ * 3 * SPL);
   constexpr int ctas = 512 / NTH;  // per SM
   if (sm > (220 / ctas) * 1024) return cudaErrorNotSupported;
@@ -957,7 +963,7 @@ static cudaError_t run_rhs_march(vr_ctx *c, const Rk &rk, const RhsArgsT<T> &a) 
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
   const TriPer &t13 = c->ttri[c->irk][0], &t2 = c->ttri[c->irk][1];
-  const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, ctas * c->nsm);
+  const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, ctas * c->nsm, kTB);
   const int grid = rows * ((g.nz + zs - 1) / zs);
   LaunchScope ls(c, PK_RHS);
   return launch_pdl(kern, grid, NTH, sm, c->stream, tm[0], tm[1], tm[2], g, rk, a, t13, t2, zs, c->d_status);

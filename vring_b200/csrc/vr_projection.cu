@@ -439,7 +439,7 @@ static cudaError_t run_uppres_march_n(vr_ctx *c, double be, double adt) {
   auto kern = k_uppres_march<T, UPSOL, RJ, NTH, NT>;
   cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
-  const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, 512 / NTH * c->nsm);
+  const int rows = (g.nr + RJ - 1) / RJ, zs = march_planes(rows, g.nz, 512 / NTH * c->nsm, 0);
   const int grid = rows * ((g.nz + zs - 1) / zs);
   UpsolArgs<T> us{reinterpret_cast<const T *>(c->dq[0]), reinterpret_cast<const T *>(c->dq[1]),
                   reinterpret_cast<const T *>(c->dq[2]), c->q[0], c->q[1], c->q[2], adt};
