@@ -276,8 +276,11 @@ struct ResCell {
 // Up to kResIters CG iterations from the state (x, r, p, SC_BETA, SC_PMEAN,
 // SC_RZ) that the setup or the previous launch left; the steps are those of
 // k2d_cg_pq and k2d_cg_xr.  JAC: z = r / diag(S), else z = r.
+// The argument stays in constant memory: a struct this small is otherwise held
+// in registers over the loop, and the vectors spill (9.8 us per iteration at
+// 512 x 1024 for 6.2).
 template <int C, bool JAC>
-__global__ void __launch_bounds__(kResThreads, 1) k2d_cg_res(const ResArg a) {
+__global__ void __launch_bounds__(kResThreads, 1) k2d_cg_res(const __grid_constant__ ResArg a) {
   extern __shared__ double planes[];
   __shared__ ResShared sh;
   if (a.flags[0]) return;
