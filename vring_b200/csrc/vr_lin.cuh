@@ -14,11 +14,13 @@
 // holding CPL columns x 16 sums: one shared load of the column's value and
 // eight 16-byte loads of coefficients, which all lanes share, feed 16 CPL
 // multiply-adds.  The coefficients ([group of 16 outputs][step][16]) stream
-// from L2 through a two-stage asynchronous ring of each warp's own.  What
-// bounds it is the FP64 pipe with CPL = 2 (12 shared-memory wavefronts per 16
-// issue cycles of multiply-adds) and the shared loads with CPL = 1 (10 per 8).
-// At 100 x 48 x 180 (us per transform): a sine and a cosine per term, one line
-// per CTA, z 756 and theta 272; this form LINZ and LINTH.
+// from L2 through a two-stage asynchronous ring of each warp's own, and a
+// step's words are in registers before the step before it is done (a step's
+// loads and products one after the other: 38 us for 33 below).
+// What bounds it with CPL = 2 is the latency of those loads at two warps per
+// scheduler (the FP64 pipe would take 12 us), with CPL = 1 the shared-memory
+// pipe.  48 x 100 x 180 (theta x r x z; us per transform): a sine and a cosine
+// per term, one line per CTA, z 756 and theta 272; here 33 and 17.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -86,6 +88,7 @@ struct LinArg {
   int nr;        // theta inverse: lines of a dph plane
   int ngroups;   // groups of 16 outputs
   int staged;    // theta: the results leave through shared memory
+  int pairs;     // z: the columns come two at a time (M even, in aligned)
 };
 
 // line L of the theta transforms' output
@@ -98,11 +101,16 @@ __device__ __forceinline__ size_t lin_line(const LinArg &a, int L) {
 
 constexpr int kLinKC = 16;  // steps per coefficient stage
 
+// row of the tile: the theta form writes it along its lines, one word to a
+// row, so an odd length spreads the banks; the z form's rows come in 16-byte
+// pieces
+__host__ __device__ constexpr int lin_ld(bool theta, int nc) { return theta ? nc + 1 : nc; }
+
 // NCL lanes along the columns, CPL columns per lane, SUB = 32 / NCL output
 // groups per warp
 template <int KIND, int NCL, int CPL>
 __global__ void __launch_bounds__(512) k_lin(const LinArg a) {
-  constexpr int NC = NCL * CPL, LD = NC + 1, SUB = 32 / NCL, KC = kLinKC, first = lin_first(KIND);
+  constexpr int NC = NCL * CPL, LD = lin_ld(lin_theta(KIND), NC), SUB = 32 / NCL, KC = kLinKC, first = lin_first(KIND);
   constexpr bool TH = lin_theta(KIND);
   extern __shared__ double sm[];
   const int N = a.N, steps = N - first;
@@ -113,12 +121,19 @@ __global__ void __launch_bounds__(512) k_lin(const LinArg a) {
   const int c0 = blockIdx.x * NC, nc = min(NC, a.M - c0);
   pdl_wait();
   if (!TH) {
-    for (int k = warp; k < N; k += nw)
-      for (int c = lane; c < NC; c += 32)
-        if (c < nc)
-          cp_async8(x + (size_t)k * LD + c, a.in + (size_t)a.M * k + c0 + c);
-        else
-          x[(size_t)k * LD + c] = 0.0;
+    if (a.pairs) {
+      for (int e = threadIdx.x; e < N * (NC / 2); e += blockDim.x) {
+        const int k = e / (NC / 2), c = 2 * (e % (NC / 2));
+        cp_async16(x + (size_t)k * LD + c, c < nc ? a.in + (size_t)a.M * k + c0 + c : a.in, c < nc ? 16u : 0u);
+      }
+    } else {
+      for (int k = warp; k < N; k += nw)
+        for (int c = lane; c < NC; c += 32)
+          if (c < nc)
+            cp_async8(x + (size_t)k * LD + c, a.in + (size_t)a.M * k + c0 + c);
+          else
+            x[(size_t)k * LD + c] = 0.0;
+    }
   } else {
     for (int l = warp; l < NC; l += nw)
       for (int n = lane; n < N; n += 32)
@@ -195,17 +210,28 @@ __global__ void __launch_bounds__(512) k_lin(const LinArg a) {
             for (int o = 0; o < 16; o++) acc[c][o] = fma(xs[k * LD + 32 * c], wc[o], acc[c][o]);
         }
       } else {
-#pragma unroll 4
-        for (int k = 0; k < k1; k++) {
-          double w[16];
-          coef(cf + k * 16, w);
+        // the next step's words load during this step's products
+        double w[2][16], v[2][CPL];
+        auto fetch = [&](int k, int b) {
+          coef(cf + k * 16, w[b]);
 #pragma unroll
-          for (int c = 0; c < CPL; c++) {
-            const double v = xs[k * LD + 32 * c];
+          for (int c = 0; c < CPL; c++) v[b][c] = xs[k * LD + 32 * c];
+        };
+        auto mul = [&](int b) {
 #pragma unroll
-            for (int o = 0; o < 16; o++) acc[c][o] = fma(w[o], v, acc[c][o]);
-          }
+          for (int c = 0; c < CPL; c++)
+#pragma unroll
+            for (int o = 0; o < 16; o++) acc[c][o] = fma(w[b][o], v[b][c], acc[c][o]);
+        };
+        fetch(0, 0);
+        int k = 0;
+        for (; k + 1 < k1; k += 2) {
+          fetch(k + 1, 1);
+          mul(0);
+          fetch(min(k + 2, k1 - 1), 0);
+          mul(1);
         }
+        if (k < k1) mul(0);
       }
       __syncwarp();  // the stage is refilled next
     }
@@ -238,18 +264,18 @@ __global__ void __launch_bounds__(512) k_lin(const LinArg a) {
 }
 
 // shared memory of a CTA of nw warps
-inline size_t lin_smem(int N, int ncl, int cpl, int nw, bool staged) {
-  const size_t ld = (size_t)ncl * cpl + 1, x = ((size_t)N * ld + 1) & ~(size_t)1;
+inline size_t lin_smem(bool theta, int N, int ncl, int cpl, int nw, bool staged) {
+  const size_t ld = lin_ld(theta, ncl * cpl), x = ((size_t)N * ld + 1) & ~(size_t)1;
   return sizeof(double) * (x + (size_t)nw * 2 * (32 / ncl) * kLinKC * 16 + (staged ? x : 0));
 }
 constexpr size_t kLinSmemMax = 225 * 1024;
 // longest line a CTA's shared memory holds (16 columns, 4 warps)
-inline bool lin_fits(int N) { return lin_smem(N, 16, 1, 4, false) <= kLinSmemMax; }
+inline bool lin_fits(int N) { return lin_smem(true, N, 16, 1, 4, false) <= kLinSmemMax; }
 
 template <int KIND, int NCL, int CPL>
 static cudaError_t lin_launch(const LinArg &a, int nw, int gy, cudaStream_t s) {
   constexpr int NC = NCL * CPL;
-  const size_t sm = lin_smem(a.N, NCL, CPL, nw, a.staged != 0);
+  const size_t sm = lin_smem(lin_theta(KIND), a.N, NCL, CPL, nw, a.staged != 0);
   cudaError_t e = allow_dyn_smem(k_lin<KIND, NCL, CPL>, sm);
   if (e) return e;
   return launch_pdl(k_lin<KIND, NCL, CPL>, dim3((a.M + NC - 1) / NC, gy), nw * 32, sm, s, a);
@@ -257,26 +283,43 @@ static cudaError_t lin_launch(const LinArg &a, int nw, int gy, cudaStream_t s) {
 
 // One transform of M columns (z: entry k of column c at in[c + M k]; theta:
 // line L at in + L N, the inverse into dph of nr rows).  in != out.
-// Columns per CTA: 64 where those CTAs still give every SM two, else 32 (a
-// column pair shares the loads of its coefficients, but half the CTAs of a
-// small grid would leave SMs idle); 16 where 32 columns of the line do not
-// fit.  The z form also splits the output groups over blockIdx.y until there
-// are two CTAs per SM; the theta form, whose lines leave through shared
-// memory whole, does not (past 726 positions, where a second tile does not
-// fit, they leave directly).
+// The z form takes two columns per lane, which halves the loads of
+// coefficients (the one-column form is bound by them: 80 % of the shared-memory
+// pipe), where that leaves every scheduler a warp's 16 outputs of a tile; 16
+// columns where 32 of the line do not fit.  Its output groups are split over
+// blockIdx.y: four warps of one group each where two such CTAs fit an SM, else
+// all the groups one CTA has warps for, and further while SMs would get
+// nothing.  The theta form's lines leave through shared memory whole, so one
+// CTA takes all groups, by a multiple of four warps (past 726 positions, where
+// a second tile does not fit, they leave directly).
+// us per transform before (z split only until two CTAs per SM, one column per
+// lane below 2 x 64 columns per SM) and so: z of 48 x 100 x 180 44 / 33, of
+// 100 x 64 x 200 70 / 61, of 90 x 128 x 288 210 / 158, of 12 x 64 x 320 39 /
+// 25; theta of 100 x 64 x 200 45 / 43; a whole axisymmetric direct solve of
+// 512 x 1000 427 / 199, of 128 x 300 82 / 55.
 template <int KIND>
 static cudaError_t lin_run(const double *in, double *out, const double *tab, int N, int M, int nr, int nsm,
                            cudaStream_t s) {
-  LinArg a{in, out, tab, N, M, nr, (N + 15) / 16, lin_theta(KIND)};
+  constexpr bool TH = lin_theta(KIND);
+  constexpr int kMaxWarps = 12;
+  LinArg a{in, out, tab, N, M, nr, (N + 15) / 16, TH, !(M & 1) && !((uintptr_t)in & 15)};
   auto shape = [&](int ncl, int cpl, int &nw, int &gy) {
     const int sub = 32 / ncl, nb = (M + ncl * cpl - 1) / (ncl * cpl), gw = (a.ngroups + sub - 1) / sub;
-    gy = !lin_theta(KIND) ? std::min(std::max(1, (2 * nsm + nb - 1) / nb), (gw + 3) / 4) : 1;
-    nw = std::max(4, std::min(12, (gw + gy - 1) / gy));
-    while (nw > 4 && lin_smem(N, ncl, cpl, nw, a.staged) > kLinSmemMax) nw--;
-    return lin_smem(N, ncl, cpl, nw, a.staged) <= kLinSmemMax;
+    gy = 1;
+    if (TH) {
+      nw = std::min(kMaxWarps, (gw + 3) / 4 * 4);
+    } else {
+      gy = (gw + 3) / 4;
+      if (2 * (lin_smem(TH, N, ncl, cpl, 4, false) + 1024) > 227 * 1024) gy = (gw + kMaxWarps - 1) / kMaxWarps;
+      gy = std::max(gy, std::min(gw, nsm / nb));
+      nw = std::max(4, (gw + gy - 1) / gy);
+    }
+    while (nw > 4 && lin_smem(TH, N, ncl, cpl, nw, a.staged) > kLinSmemMax) nw--;
+    return lin_smem(TH, N, ncl, cpl, nw, a.staged) <= kLinSmemMax;
   };
   int nw, gy;
-  if ((M + 63) / 64 >= 2 * nsm && shape(32, 2, nw, gy)) return lin_launch<KIND, 32, 2>(a, nw, gy, s);
+  if constexpr (!TH)
+    if ((M + 63) / 64 * a.ngroups >= 4 * nsm && shape(32, 2, nw, gy)) return lin_launch<KIND, 32, 2>(a, nw, gy, s);
   if (shape(32, 1, nw, gy)) return lin_launch<KIND, 32, 1>(a, nw, gy, s);
   if (shape(16, 1, nw, gy)) return lin_launch<KIND, 16, 1>(a, nw, gy, s);
   a.staged = 0;

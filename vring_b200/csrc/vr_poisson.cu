@@ -1109,7 +1109,7 @@ __global__ void __launch_bounds__(512, 1) k_dct_tma(const __grid_constant__ CUte
 // output goes through rows m ^ ((m >> 4) & 1) (eight distinct rows modulo 8
 // per quarter warp); the inverse stores its rows 2-way.
 // 256 x 128 x 1024 (us per transform): 272 with 1024 points per warp and the
-// bit-reversed scatter (k_dct_w), DCT1024 here.
+// bit-reversed scatter (k_dct_w), 146 here.
 // ---------------------------------------------------------------------------
 constexpr int kDct2Cols = 8, kDct2N = 1024;
 
