@@ -85,6 +85,21 @@ def test_folded_columns_above_two_ctas_per_sm():
     assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
 
 
+# two columns per lane (enough output groups for every scheduler), with an odd
+# number of columns, a last tile partly filled and groups beyond the line
+@pytest.mark.parametrize("grid", [(63, 301, 20), (47, 121, 100), (48, 100, 180)], ids=lambda g: "x".join(map(str, g)))
+def test_two_columns_per_lane(grid):
+    nth, nr, nz = grid
+    orc, gpu = make_pair(nth, nr, nz)
+    seed_random(orc, gpu, ["rhs"], seed=11)
+    prep(orc, gpu)
+    orc.laplace_solve()
+    gpu.laplace_solve()
+    g = gpu.get("dph")[:, 1:nr + 1, 1:nz + 1]
+    r = orc.field("dph")[:, 1:nr + 1, 1:nz + 1]
+    assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
+
+
 def _direct(faces, nz, zmax, f):
     """The direct solve in plain numpy: z cosine products, a Thomas solve per mode."""
     nr = faces.size - 1

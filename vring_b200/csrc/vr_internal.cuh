@@ -102,19 +102,22 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Programmatic dependent launch of a substep's kernels: a kernel may start
 // while the one before it in the stream still runs, sets up what depends on
 // constant tables only, and then waits (pdl_wait) until that kernel has
-// finished and its writes are visible.  No kernel lets its successor start
-// before its own CTAs exit (with griddepcontrol.launch_dependents after the
-// wait, the successor's CTAs fill the SMs that are free at that moment several
-// deep and leave the others idle: a 64x32x128 step of 0.31 ms becomes 0.36).
+// finished and its writes are visible.  The successor starts as CTAs of the
+// kernel before it exit, or, where that one calls pdl_trigger after its own
+// pdl_wait, beside it: that pays only for grids that leave SMs free.  (In the
+// substep the successor's CTAs fill the SMs that are free at that moment
+// several deep and leave the others idle: a 32x64x128 step of 0.31 ms becomes
+// 0.36.)
 // So whatever ran before the previous kernel is complete when a kernel starts,
 // and only the previous kernel's own writes have to wait for pdl_wait.  A
 // kernel launched by launch_pdl calls pdl_wait in every thread, also one that
 // returns on an error, and reads what the previous kernel may write by TMA,
 // cp.async or plain loads: not through __ldg or a const __restrict__
 // parameter, which the compiler may take for constant over the whole kernel
-// and load early.  Against plain launches: a 64x32x128 ring, 10 steps with
-// read-back, 3.57 -> 3.51 ms; 100x48x180 with inflow, launch by launch,
-// 5.93 -> 5.84; 128x64x256 routine by routine, 4 steps, 4.95 -> 4.65.
+// and load early.  Against plain launches (theta x r x z): 32x64x128, 10 steps
+// with read-back, 3.57 -> 3.51 ms; 48x100x180 with inflow, launch by launch,
+// 5.93 -> 5.84; 64x128x256 routine by routine, 4 steps, 4.95 -> 4.65.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>

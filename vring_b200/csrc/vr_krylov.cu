@@ -545,8 +545,8 @@ __device__ __forceinline__ int fcg_slot(const int *flags) { return flags[1] % kF
 // also kept side by side (row arrays of nz), so that every block of the next
 // kernel takes their mean from a few KB instead of one word per plane.  The
 // separate steps took 14 kernels of 2 blocks per SM: 0.11 of the 0.35 ms of a
-// learned iteration at 512 x 1024; these take FCGUS.
-__device__ __forceinline__ double row_mean(const K2dOp &o, const double *__restrict__ row, double *sh) {
+// learned iteration at 512 x 1024; these 0.09 (cold).
+__device__ __forceinline__ double row_mean(const K2dOp &o, const double *row, double *sh) {
   double v = 0.0;
   for (int k = threadIdx.x; k < o.nz; k += blockDim.x) v += row[k];
   const double s = block_sum(v, sh);
@@ -568,11 +568,12 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_first(K2dOp o, double ome
 
 // the network's input t = r - S z0, z0 = omega D^-1 r; the last block: the sum
 // of (D^-1/2 t)^2, its scale
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pre(K2dOp o, double omega, const double *__restrict__ r,
-                                                         const double *__restrict__ z0l, double *__restrict__ t,
-                                                         const double *__restrict__ dh, double *sc, double *part,
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pre(K2dOp o, double omega, const double *r,
+                                                         const double *z0l, double *__restrict__ t,
+                                                         const double *dh, double *sc, double *part,
                                                          unsigned *counter, const int *flags) {
   __shared__ double sh[40];
+  pdl_wait();
   if (flags[0]) return;
   const double mean = row_mean(o, z0l, sh);
   auto z0 = [&](int e) { return omega * o.dinv[e] * r[e]; };
@@ -596,15 +597,16 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pre(K2dOp o, double omega
 // z = N + z0 (N = s D^-1/2 y, the network's correction; y null: none), with
 // omega > 0 also z += omega D^-1 (r - S z); partials of z . q_i for the kept
 // directions; the last block: beta_i = (z . q_i) / (p_i . q_i)
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_post(K2dOp o, double omega, const double *__restrict__ r,
-                                                          const float *__restrict__ y, const float *__restrict__ yl,
-                                                          const double *__restrict__ dh,
-                                                          const double *__restrict__ dhl,
-                                                          const double *__restrict__ z0l, double *__restrict__ z,
-                                                          const double *__restrict__ fq, const double *sc,
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_post(K2dOp o, double omega, const double *r,
+                                                          const float *y, const float *yl,
+                                                          const double *dh,
+                                                          const double *dhl,
+                                                          const double *z0l, double *__restrict__ z,
+                                                          const double *fq, const double *sc,
                                                           double *fpart, const double *fpq, double *fbeta,
                                                           unsigned *counter, const int *flags) {
   __shared__ double sh[40];
+  pdl_wait();
   if (flags[0]) return;
   const int kept = fcg_kept(flags);
   const double s = y ? sqrt(sc[SC_SS] / o.n) : 0.0;
@@ -664,11 +666,12 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_post(K2dOp o, double omeg
 // p = z - sum_i beta_i p_i, written to the new slot (which may be the oldest
 // kept direction: each element is read before it is overwritten); partial
 // p . r [A]
-__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pm(K2dOp o, const double *__restrict__ z, double *fp,
-                                                        const double *__restrict__ fbeta,
-                                                        const double *__restrict__ r, double *pl, double *part,
+__global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pm(K2dOp o, const double *z, double *fp,
+                                                        const double *fbeta,
+                                                        const double *r, double *pl, double *part,
                                                         const int *flags) {
   __shared__ double sh[40];
+  pdl_wait();
   if (flags[0]) return;
   const int kept = fcg_kept(flags), slot = fcg_slot(flags);
   double b[kFcgKeep], acc = 0.0;
@@ -691,9 +694,10 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_pm(K2dOp o, const double 
 // q = S p for the new slot, partial p . q [B]; the last block:
 // alpha = (p . r) / (p . q), p . q kept for the slot
 __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_apply(K2dOp o, const double *fp, double *fq,
-                                                           const double *__restrict__ pl, double *sc, double *part,
+                                                           const double *pl, double *sc, double *part,
                                                            double *fpq, unsigned *counter, const int *flags) {
   __shared__ double sh[40];
+  pdl_wait();
   if (flags[0]) return;
   const int slot = fcg_slot(flags);
   const double *x = fp + (size_t)slot * o.n;
@@ -719,10 +723,11 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_apply(K2dOp o, const doub
 // x += alpha p; r -= alpha q; partial r.r [C]; the next iteration's row of z0;
 // the last block: the norm and the convergence and iteration-cap flags
 __global__ void __launch_bounds__(kK2dThreads) k2d_fcg_xrm(K2dOp o, double omega, double *__restrict__ x,
-                                                         double *__restrict__ r, const double *__restrict__ fp,
-                                                         const double *__restrict__ fq, double *z0l, double *sc,
+                                                         double *__restrict__ r, const double *fp,
+                                                         const double *fq, double *z0l, double *sc,
                                                          double *part, unsigned *counter, int *flags) {
   __shared__ double sh[40];
+  pdl_wait();
   if (flags[0]) return;
   const size_t so = (size_t)fcg_slot(flags) * o.n;
   const double al = sc[SC_ALPHA];
@@ -1320,17 +1325,25 @@ static cudaError_t enqueue_fcg_iter(vr_k2d *k) {
   double *z0l = k->frow, *dhl = z0l + k->nz, *pl = dhl + k->nz;
   float *yl = reinterpret_cast<float *>(pl + k->nz);
   const float *y = nullptr;
+  cudaError_t e;
   if (k->net) {
-    k2d_fcg_pre<<<gb, kK2dThreads, 0, k->stream>>>(o, om, r, z0l, t, k2d_dhalf(k), k->sc, P, k->cnt + 4, k->flags);
+    if ((e = launch_pdl(k2d_fcg_pre, gb, kK2dThreads, 0, k->stream, o, om, r, z0l, t, k2d_dhalf(k), k->sc, P, k->cnt + 4,
+                        k->flags)))
+      return e;
     if (unet_correct(k->net, t, k2d_dhalf(k), k->sc + SC_SS, k->flags, yl, &y, k->stream) != VR_OK)
       return cudaErrorLaunchFailure;
   }
-  k2d_fcg_post<<<gb, kK2dThreads, 0, k->stream>>>(o, om, r, y, yl, k2d_dhalf(k), dhl, z0l, z, k->fq, k->sc, k->fpart,
-                                                k->fpq, k->fbeta, k->cnt + 5, k->flags);
-  k2d_fcg_pm<<<gb, kK2dThreads, 0, k->stream>>>(o, z, k->fp, k->fbeta, r, pl, P, k->flags);
-  k2d_fcg_apply<<<gb, kK2dThreads, 0, k->stream>>>(o, k->fp, k->fq, pl, k->sc, P, k->fpq, k->cnt + 6, k->flags);
-  k2d_fcg_xrm<<<gb, kK2dThreads, 0, k->stream>>>(o, om, x, r, k->fp, k->fq, z0l, k->sc, P, k->cnt + 7, k->flags);
-  return cudaGetLastError();
+  if ((e = launch_pdl(k2d_fcg_post, gb, kK2dThreads, 0, k->stream, o, om, r, y, yl, k2d_dhalf(k), dhl, z0l, z, k->fq,
+                      k->sc, k->fpart, k->fpq, k->fbeta, k->cnt + 5, k->flags)))
+    return e;
+  if ((e = launch_pdl(k2d_fcg_pm, gb, kK2dThreads, 0, k->stream, o, z, k->fp, k->fbeta, r, pl, P, k->flags))) return e;
+  if ((e = launch_pdl(k2d_fcg_apply, gb, kK2dThreads, 0, k->stream, o, k->fp, k->fq, pl, k->sc, P, k->fpq, k->cnt + 6,
+                      k->flags)))
+    return e;
+  if ((e = launch_pdl(k2d_fcg_xrm, gb, kK2dThreads, 0, k->stream, o, om, x, r, k->fp, k->fq, z0l, k->sc, P, k->cnt + 7,
+                      k->flags)))
+    return e;
+  return cudaSuccess;
 }
 static cudaError_t enq_fcg(vr_k2d *k, int) { return enqueue_fcg_iter(k); }
 

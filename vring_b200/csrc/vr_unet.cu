@@ -194,6 +194,11 @@ constexpr int kConvHR = kConvTR + 2, kConvHZ = kConvTZ + 2;
 #define VR_CONV_CTAS 8
 #endif
 constexpr int kConvCtas = VR_CONV_CTAS;  // resident CTAs per SM, at most
+// Grids of at most this many CTAs leave SMs free: their successor starts beside
+// them and stages its weights meanwhile (pdl_trigger).  The coarse levels are
+// chains of such kernels, 6 us each of which a third is staging: a learned
+// solve at 512 x 1024 131 -> 117 ms, together with the other kernels' launches.
+constexpr int kTriggerCtas = 148;
 
 template <int CINP>
 __host__ __device__ constexpr int conv_halo_bytes() {
@@ -205,8 +210,8 @@ __host__ __device__ constexpr int conv_wstage_bytes() {
 }
 
 template <int CINP, int NOUT>
-__global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *__restrict__ in, int H, int W, int cin,
-                                                const __nv_bfloat16 *__restrict__ skip, int cskip, int F,
+__global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *in, int H, int W, int cin,
+                                                const __nv_bfloat16 *skip, int cskip, int F,
                                                 const __nv_bfloat16 *__restrict__ wpk, int cout,
                                                 __nv_bfloat16 *__restrict__ out, unsigned *status, int npr,
                                                 int npatch) {
@@ -270,6 +275,8 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *__restric
   };
   // the packed weights are already in the staged order
   for (int e = tid; e < 9 * CC * NOUT; e += 128) cp_async16(wst + (size_t)e * 16, wpk + (size_t)e * 8, 16u);
+  pdl_wait();  // up to here: tensor memory and the weights
+  if (gridDim.x <= kTriggerCtas) pdl_trigger();
   int patch = blockIdx.x, buf = 0;
   uint32_t phase = 0;
   if (patch < npatch) fetch(patch, halos);
@@ -675,7 +682,9 @@ __global__ void __launch_bounds__(384) k_dgrad3(const float *__restrict__ gout, 
 // F x F average pooling (children summed in FP32, r fastest, then scaled by
 // 1 / F^2) and its gradient; eight, then four channels per thread
 template <int F>
-__global__ void k_pool(const __nv_bfloat16 *__restrict__ in, int H, int W, int c, __nv_bfloat16 *__restrict__ out) {
+__global__ void k_pool(const __nv_bfloat16 *in, int H, int W, int c, __nv_bfloat16 *__restrict__ out) {
+  pdl_wait();
+  if (gridDim.x <= kTriggerCtas) pdl_trigger();
   const int H2 = H / F, W2 = W / F, c8 = c / 8, n = H2 * W2 * c8;
   const float inv = 1.f / (float)(F * F);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
@@ -763,8 +772,9 @@ __global__ void k_upcat_bwd(const float *__restrict__ gout, int ca, int cb, int 
 }
 // head: y[p] = sum_c in[p][c] w[c], eight channels per load; yl: a copy of the
 // last radial row (or null)
-__global__ void k_head(const __nv_bfloat16 *__restrict__ in, int P, int nr, int c, const float *__restrict__ w,
+__global__ void k_head(const __nv_bfloat16 *in, int P, int nr, int c, const float *__restrict__ w,
                        float *__restrict__ y, float *__restrict__ yl) {
+  pdl_wait();
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
     float s = 0.f;
     for (int ch = 0; ch < c; ch += 8) {
@@ -809,8 +819,9 @@ __global__ void __launch_bounds__(256) k_head_bwd(const __nv_bfloat16 *__restric
 }
 // input: x[p] * D[p] / s -> bf16 (D = dscale or 1; s = sqrt(*ss / n) when ss is
 // given, else 1 / inv_host)
-__global__ void k_in(const double *__restrict__ x, int n, const double *__restrict__ ss, double inv_host,
-                     const double *__restrict__ dscale, __nv_bfloat16 *__restrict__ xb, const int *flags) {
+__global__ void k_in(const double *x, int n, const double *ss, double inv_host, const double *dscale,
+                     __nv_bfloat16 *__restrict__ xb, const int *flags) {
+  pdl_wait();
   if (flags && flags[0]) return;
   const double inv = ss ? (*ss > 0 ? 1.0 / sqrt(*ss / n) : 0.0) : inv_host;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -877,8 +888,8 @@ static cudaError_t conv3_tc_n(const __nv_bfloat16 *in, int H, int W, int cin, co
   const size_t sm = 128 + (size_t)wst + (size_t)(npatch > grid ? 2 : 1) * halo;
   cudaError_t e = allow_dyn_smem(k_conv3_tc<CINP, NOUT>, sm);
   if (e) return e;
-  k_conv3_tc<CINP, NOUT><<<grid, 128, sm, s>>>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, npr, npatch);
-  return cudaGetLastError();
+  return launch_pdl(k_conv3_tc<CINP, NOUT>, grid, 128, sm, s, in, H, W, cin, skip, cskip, F, wpk, cout, out, status, npr,
+                    npatch);
 }
 
 template <int CINP>
@@ -1207,11 +1218,8 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullpt
   auto pool = [&](int src, int dst) {
     HW(sh.lev[src], H, W);
     const size_t n = (size_t)(H / u->pool) * (W / u->pool) * sh.ch[src] / 8;
-    if (u->pool == 2)
-      k_pool<2><<<grid_for(n), 256, 0, s>>>(x->a[src], H, W, sh.ch[src], x->a[dst]);
-    else
-      k_pool<4><<<grid_for(n), 256, 0, s>>>(x->a[src], H, W, sh.ch[src], x->a[dst]);
-    return cudaGetLastError();
+    return launch_pdl(u->pool == 2 ? k_pool<2> : k_pool<4>, grid_for(n), 256, 0, s, x->a[src], H, W, sh.ch[src],
+                      x->a[dst]);
   };
   auto upcat = [&](int coarse, int skip, int dst) {
     HW(sh.lev[skip], H, W);
@@ -1234,8 +1242,7 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullpt
     if ((e = upcat(S_D1, S_E0, S_U0)) || (e = conv(12)) || (e = conv(13))) return e;
   }
   const int P0 = u->nr * u->nz;
-  k_head<<<grid_for(P0), 256, 0, s>>>(x->a[S_D0], P0, u->nr, u->ch[0], u->wk + u->L[14].woff, u->y, yl);
-  return cudaGetLastError();
+  return launch_pdl(k_head, grid_for(P0), 256, 0, s, x->a[S_D0], P0, u->nr, u->ch[0], u->wk + u->L[14].woff, u->y, yl);
 }
 
 // backward from u->gy; accumulates parameter gradients into u->gw and, with
@@ -1299,8 +1306,7 @@ void unet_dims(const vr_unet *u, int *nr, int *nz) {
 int unet_correct(const vr_unet *u, const double *t, const double *dscale, const double *ss, const int *flags, float *yl,
                  const float **y, cudaStream_t s) {
   const int n = u->nr * u->nz;
-  k_in<<<grid_for(n), 256, 0, s>>>(t, n, ss, 0.0, dscale, u->x0, flags);
-  if (cudaGetLastError() != cudaSuccess) return VR_ERR_CUDA;
+  if (launch_pdl(k_in, grid_for(n), 256, 0, s, t, n, ss, 0.0, dscale, u->x0, flags)) return VR_ERR_CUDA;
   if (unet_fwd(u, s, yl) != cudaSuccess) return VR_ERR_CUDA;
   *y = u->y;
   return VR_OK;
