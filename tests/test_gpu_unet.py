@@ -65,6 +65,22 @@ def test_tensor_core_forward_matches_cuda_core_forward_and_oracle(grid):
     cc.close()
 
 
+# the pooling and the head in the convolutions' epilogues: a level smaller than
+# a patch, patches cut in r or z, several patches per CTA, channel counts that
+# are no multiple of 16
+@pytest.mark.parametrize("nr,nz,ch,pool", [(8, 8, (8, 8, 8, 8), 2), (24, 40, (24, 16, 40, 8), 2),
+                                           (64, 192, (8, 16, 24, 64), 4), (192, 64, (48, 32, 16, 16), 4),
+                                           (576, 512, (8, 8, 8, 8), 4)])
+def test_forward_at_patch_edges(nr, nz, ch, pool):
+    import vring_b200 as V
+    from oracle import unet_ref as U
+    net = V.UNet(nr, nz, ch, seed=3, pool=pool)
+    x = np.random.default_rng(2).standard_normal((nr, nz))
+    s = np.sqrt(np.mean(x ** 2))
+    assert _rel(net.forward(x), s * U.forward(net.get_params(), ch, x / s, F=pool)) <= 5e-3
+    net.close()
+
+
 @pytest.mark.parametrize("pool", [2, 4])
 def test_gradients_match_oracle(pool):
     import vring_b200 as V

@@ -209,12 +209,55 @@ __host__ __device__ constexpr int conv_wstage_bytes() {
   return 9 * CINP * NOUT * 2;
 }
 
-template <int CINP, int NOUT>
+// What follows a level's last convolution is taken in its epilogue (EPI), from
+// the rounded values and in the order of the separate kernels, so with their
+// bits:
+//   kEpiHead: the 1 x 1 head y = sum_c out_c w_c (k_head); yl: a copy of the
+//     last radial row (or null).  out may be null: only the training reads it.
+//   kEpiPool: the F x F average pooling (k_pool), through the halo the products
+//     have done with; a patch holds whole cells, since F divides 8.
+// A learned solve at 512 x 1024 spares four launches and a 17 MB tensor written
+// and read again per iteration: 0.29 -> 0.28 ms per iteration.
+enum ConvEpiKind { kEpiNone = 0, kEpiHead, kEpiPool };
+struct ConvEpi {
+  const float *w;
+  float *y, *yl;
+  __nv_bfloat16 *pooled;
+  int F;
+};
+
+// sum of the F x F pixels from src on (pitches dr, dz in 16-byte chunks), r
+// fastest, times 1 / F^2
+template <int F>
+__device__ __forceinline__ uint4 pool_chunk(const uint4 *src, size_t dr, size_t dz) {
+  float s[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) s[i] = 0.f;
+#pragma unroll
+  for (int z = 0; z < F; z++)
+#pragma unroll
+    for (int r = 0; r < F; r++) {
+      const uint4 u = src[dz * z + dr * r];
+      const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        s[2 * i] += __uint_as_float(w[i] << 16);
+        s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+      }
+    }
+  const float inv = 1.f / (float)(F * F);
+  __align__(16) __nv_bfloat16 b[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) b[i] = __float2bfloat16_rn(inv * s[i]);
+  return *reinterpret_cast<const uint4 *>(b);
+}
+
+template <int CINP, int NOUT, int EPI>
 __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *in, int H, int W, int cin,
                                                 const __nv_bfloat16 *skip, int cskip, int F,
                                                 const __nv_bfloat16 *__restrict__ wpk, int cout,
                                                 __nv_bfloat16 *__restrict__ out, unsigned *status, int npr,
-                                                int npatch) {
+                                                int npatch, ConvEpi epi) {
   static_assert(CINP % 16 == 0 && NOUT % 16 == 0 && NOUT <= 64, "tile shape");
   constexpr int CC = CINP / 8, HR = kConvHR, HZ = kConvHZ;
   constexpr uint32_t NCOLS = NOUT <= 32 ? 32 : 64;
@@ -315,6 +358,7 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *in, int H
     const int j = j0 + mr, k = k0 + mz;
     const bool pin = j < H && k < W;
     const size_t p = (size_t)j + (size_t)H * k;
+    float hs = 0.f;
 #pragma unroll
     for (int c0 = 0; c0 < NOUT; c0 += 16) {
       float v[16];
@@ -324,9 +368,38 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *in, int H
         __align__(16) __nv_bfloat16 b[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) b[i] = __float2bfloat16_rn(v[i]);
-        reinterpret_cast<uint4 *>(dst)[0] = reinterpret_cast<const uint4 *>(b)[0];
-        if (c0 + 16 <= cout)  // channel counts are multiples of 8
-          reinterpret_cast<uint4 *>(dst)[1] = reinterpret_cast<const uint4 *>(b)[1];
+        if (EPI != kEpiHead || out) {
+          reinterpret_cast<uint4 *>(dst)[0] = reinterpret_cast<const uint4 *>(b)[0];
+          if (c0 + 16 <= cout)  // channel counts are multiples of 8
+            reinterpret_cast<uint4 *>(dst)[1] = reinterpret_cast<const uint4 *>(b)[1];
+        }
+        if constexpr (EPI == kEpiHead) {
+#pragma unroll
+          for (int i = 0; i < 16; i++)
+            if (c0 + i < cout) hs = fmaf(__bfloat162float(b[i]), __ldg(epi.w + c0 + i), hs);
+        }
+        if constexpr (EPI == kEpiPool) {
+          uint4 *px = reinterpret_cast<uint4 *>(halo) + (tid * cout + c0) / 8;
+          px[0] = reinterpret_cast<const uint4 *>(b)[0];
+          if (c0 + 16 <= cout) px[1] = reinterpret_cast<const uint4 *>(b)[1];
+        }
+      }
+    }
+    if constexpr (EPI == kEpiHead)
+      if (pin && ok) {
+        epi.y[p] = hs;
+        if (epi.yl && j == H - 1) epi.yl[k] = hs;
+      }
+    if constexpr (EPI == kEpiPool) {
+      static_assert(CINP == NOUT && conv_halo_bytes<CINP>() >= 128 * NOUT * 2, "the patch fits its halo");
+      __syncthreads();
+      const int F = epi.F, c8 = cout / 8, nj = kConvTR / F, nk = kConvTZ / F, H2 = H / F, W2 = W / F;
+      for (int e = tid; e < nj * nk * c8; e += 128) {
+        const int q = e % c8, J = e / c8 % nj, K = e / c8 / nj, gj = j0 / F + J, gk = k0 / F + K;
+        if (gj >= H2 || gk >= W2) continue;
+        const uint4 *src = reinterpret_cast<const uint4 *>(halo) + (size_t)(F * J + kConvTR * F * K) * c8 + q;
+        reinterpret_cast<uint4 *>(epi.pooled)[((size_t)gj + (size_t)H2 * gk) * c8 + q] =
+            F == 2 ? pool_chunk<2>(src, c8, kConvTR * c8) : pool_chunk<4>(src, c8, kConvTR * c8);
       }
     }
     tc_fence_before();
@@ -686,29 +759,10 @@ __global__ void k_pool(const __nv_bfloat16 *in, int H, int W, int c, __nv_bfloat
   pdl_wait();
   if (gridDim.x <= kTriggerCtas) pdl_trigger();
   const int H2 = H / F, W2 = W / F, c8 = c / 8, n = H2 * W2 * c8;
-  const float inv = 1.f / (float)(F * F);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int q = e % c8, p = e / c8, J = p % H2, K = p / H2;
     const uint4 *src = reinterpret_cast<const uint4 *>(in + ((size_t)F * J + (size_t)H * F * K) * c) + q;
-    float s[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) s[i] = 0.f;
-#pragma unroll
-    for (int dz = 0; dz < F; dz++)
-#pragma unroll
-      for (int dr = 0; dr < F; dr++) {
-        const uint4 u = src[((size_t)H * dz + dr) * c8];
-        const unsigned w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          s[2 * i] += __uint_as_float(w[i] << 16);
-          s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
-        }
-      }
-    __align__(16) __nv_bfloat16 b[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) b[i] = __float2bfloat16_rn(inv * s[i]);
-    *(reinterpret_cast<uint4 *>(out) + e) = *reinterpret_cast<const uint4 *>(b);
+    reinterpret_cast<uint4 *>(out)[e] = pool_chunk<F>(src, c8, (size_t)H * c8);
   }
 }
 // gin[p][c] += gout[parent(p)][c] / F^2
@@ -879,28 +933,34 @@ static cudaError_t conv3(const __nv_bfloat16 *in, int H, int W, int cin, const f
 template <int CINP, int NOUT>
 static cudaError_t conv3_tc_n(const __nv_bfloat16 *in, int H, int W, int cin, const __nv_bfloat16 *skip, int cskip,
                               int F, const __nv_bfloat16 *wpk, int cout, __nv_bfloat16 *out, unsigned *status,
-                              int nsm, cudaStream_t s) {
+                              int nsm, cudaStream_t s, ConvEpi epi) {
   constexpr int halo = conv_halo_bytes<CINP>(), wst = conv_wstage_bytes<CINP, NOUT>();
   const int npr = (H + kConvTR - 1) / kConvTR, npatch = npr * ((W + kConvTZ - 1) / kConvTZ);
   // resident CTAs per SM with two halo buffers; one buffer where no CTA walks
   const int most = std::max(1, std::min(kConvCtas, (int)((size_t)(220 * 1024) / (128 + wst + 2 * halo + 1024))));
   const int grid = std::min(npatch, nsm * most);
   const size_t sm = 128 + (size_t)wst + (size_t)(npatch > grid ? 2 : 1) * halo;
-  cudaError_t e = allow_dyn_smem(k_conv3_tc<CINP, NOUT>, sm);
+  auto kern = k_conv3_tc<CINP, NOUT, kEpiNone>;
+  if (epi.w || epi.pooled) {  // as many channels in as out
+    if constexpr (CINP == NOUT)
+      kern = epi.w ? k_conv3_tc<CINP, NOUT, kEpiHead> : k_conv3_tc<CINP, NOUT, kEpiPool>;
+    else
+      return cudaErrorInvalidValue;
+  }
+  cudaError_t e = allow_dyn_smem(kern, sm);
   if (e) return e;
-  return launch_pdl(k_conv3_tc<CINP, NOUT>, grid, 128, sm, s, in, H, W, cin, skip, cskip, F, wpk, cout, out, status, npr,
-                    npatch);
+  return launch_pdl(kern, grid, 128, sm, s, in, H, W, cin, skip, cskip, F, wpk, cout, out, status, npr, npatch, epi);
 }
 
 template <int CINP>
 static cudaError_t conv3_tc_c(const __nv_bfloat16 *in, int H, int W, int cin, const __nv_bfloat16 *skip, int cskip,
                               int F, const __nv_bfloat16 *wpk, int cout, __nv_bfloat16 *out, unsigned *status,
-                              int nsm, cudaStream_t s) {
+                              int nsm, cudaStream_t s, ConvEpi epi) {
   switch ((cout + 15) / 16) {
-    case 1: return conv3_tc_n<CINP, 16>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
-    case 2: return conv3_tc_n<CINP, 32>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
-    case 3: return conv3_tc_n<CINP, 48>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
-    case 4: return conv3_tc_n<CINP, 64>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s);
+    case 1: return conv3_tc_n<CINP, 16>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s, epi);
+    case 2: return conv3_tc_n<CINP, 32>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s, epi);
+    case 3: return conv3_tc_n<CINP, 48>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s, epi);
+    case 4: return conv3_tc_n<CINP, 64>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s, epi);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -909,11 +969,11 @@ static cudaError_t conv3_tc_c(const __nv_bfloat16 *in, int H, int W, int cin, co
 // skip, the input is the concatenation of `in` upsampled by F and `skip`
 static cudaError_t conv3_tc(const __nv_bfloat16 *in, int H, int W, int cin, const __nv_bfloat16 *wpk, int cout,
                             __nv_bfloat16 *out, unsigned *status, int nsm, cudaStream_t s,
-                            const __nv_bfloat16 *skip = nullptr, int cskip = 0, int F = 1) {
+                            const __nv_bfloat16 *skip = nullptr, int cskip = 0, int F = 1, ConvEpi epi = {}) {
   if (skip && ((cin & 7) || (cskip & 7))) return cudaErrorInvalidValue;
   const int ctot = cin + (skip ? cskip : 0);
   switch ((ctot + 15) / 16) {
-#define VR_CONV_TC(CP) return conv3_tc_c<CP>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s)
+#define VR_CONV_TC(CP) return conv3_tc_c<CP>(in, H, W, cin, skip, cskip, F, wpk, cout, out, status, nsm, s, epi)
     case 1: VR_CONV_TC(16);
     case 2: VR_CONV_TC(32);
     case 3: VR_CONV_TC(48);
@@ -1189,7 +1249,7 @@ namespace vr {
 // forward from u->x0 (bf16 input) to u->y (fp32); the tensor-core
 // convolutions (and the weight gradients) read the decoder's concatenations
 // where they lie, only the CUDA-core form copies them
-static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullptr) {
+static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullptr, bool keep = true) {
   const UnetShapes sh = shapes_of(u);
   const vr_unet *x = u;
   cudaError_t e;
@@ -1200,13 +1260,14 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullpt
   };
   int H, W;
   const bool fuse = !u->cuda_cores;
-  auto conv = [&](int li) -> cudaError_t {
+  auto conv = [&](int li, int pooled = -1) -> cudaError_t {
     const UnetLayer &L = u->L[li];
     HW(L.level, H, W);
     const __nv_bfloat16 *in = kConvIn[li] < 0 ? u->x0 : x->a[kConvIn[li]];
     if (u->cuda_cores)
       return conv3(in, H, W, L.cin, u->wk + L.woff, L.cout, x->a[kConvOut[li]], s);
-    return conv3_tc(in, H, W, L.cin, u->wpk + u->wpk_off[li], L.cout, x->a[kConvOut[li]], u->status, u->nsm, s);
+    return conv3_tc(in, H, W, L.cin, u->wpk + u->wpk_off[li], L.cout, x->a[kConvOut[li]], u->status, u->nsm, s,
+                    nullptr, 0, 1, ConvEpi{nullptr, nullptr, nullptr, pooled < 0 ? nullptr : x->a[pooled], u->pool});
   };
   // the first convolution of a decoder level, on concat(upsample(coarse), skip)
   auto conv_cat = [&](int li, int coarse, int skip) -> cudaError_t {
@@ -1228,14 +1289,19 @@ static cudaError_t unet_fwd(const vr_unet *u, cudaStream_t s, float *yl = nullpt
                                         x->a[dst]);
     return cudaGetLastError();
   };
-  if ((e = conv(0)) || (e = conv(1)) || (e = pool(S_E0, S_P1))) return e;
-  if ((e = conv(2)) || (e = conv(3)) || (e = pool(S_E1, S_P2))) return e;
-  if ((e = conv(4)) || (e = conv(5)) || (e = pool(S_E2, S_P3))) return e;
+  const int skips[3] = {S_E0, S_E1, S_E2}, pooled[3] = {S_P1, S_P2, S_P3};
+  for (int l = 0; l < 3; l++) {
+    if ((e = conv(2 * l)) || (e = conv(2 * l + 1, pooled[l]))) return e;
+    if (!fuse && (e = pool(skips[l], pooled[l]))) return e;
+  }
   if ((e = conv(6)) || (e = conv(7))) return e;
   if (fuse) {
     if ((e = conv_cat(8, S_B3, S_E2)) || (e = conv(9))) return e;
     if ((e = conv_cat(10, S_D2, S_E1)) || (e = conv(11))) return e;
-    if ((e = conv_cat(12, S_D1, S_E0)) || (e = conv(13))) return e;
+    if ((e = conv_cat(12, S_D1, S_E0))) return e;
+    const UnetLayer &L = u->L[13];
+    return conv3_tc(x->a[S_D0A], u->nr, u->nz, L.cin, u->wpk + u->wpk_off[13], L.cout, keep ? x->a[S_D0] : nullptr,
+                    u->status, u->nsm, s, nullptr, 0, 1, ConvEpi{u->wk + u->L[14].woff, u->y, yl, nullptr, 1});
   } else {
     if ((e = upcat(S_B3, S_E2, S_U2)) || (e = conv(8)) || (e = conv(9))) return e;
     if ((e = upcat(S_D2, S_E1, S_U1)) || (e = conv(10)) || (e = conv(11))) return e;
@@ -1307,7 +1373,7 @@ int unet_correct(const vr_unet *u, const double *t, const double *dscale, const 
                  const float **y, cudaStream_t s) {
   const int n = u->nr * u->nz;
   if (launch_pdl(k_in, grid_for(n), 256, 0, s, t, n, ss, 0.0, dscale, u->x0, flags)) return VR_ERR_CUDA;
-  if (unet_fwd(u, s, yl) != cudaSuccess) return VR_ERR_CUDA;
+  if (unet_fwd(u, s, yl, false) != cudaSuccess) return VR_ERR_CUDA;
   *y = u->y;
   return VR_OK;
 }
