@@ -755,10 +755,10 @@ __device__ __forceinline__ void tsolve_group(int N, const double *cinv, const do
 // NT > 0: the theta extent as a compile-time constant (equal to g.nth), so
 // that the shared-memory offsets, line strides and divisions by it fold.
 // RJ rows of up to NTH / RJ cells: short theta lines take more rows, so that
-// a plane still gives every thread a cell (64 x 32 x 128: 44 us with 2 rows of
+// a plane still gives every thread a cell (32 x 64 x 128: 44 us with 2 rows of
 // 32 cells in 256 threads and 32 planes per CTA, 21 with 8 rows and 4 planes);
 // lines beyond 128 cells take two rows in 512 threads, one CTA per SM
-// (256 x 128 x 1024, mixed: 1.35 ms by whole lines per warp, 1.08 here).
+// (256 x 128 x 1024, mixed: 1.35 ms by whole lines per warp, 1.04 here).
 // HIN: the explicit terms are read from dqh (vr_hdnl1..3 wrote them) and only
 // the right-hand sides and theta solves remain, in the same walk (vr_step,
 // 64 x 128 x 256, cold: right-hand sides 63 us and three theta sweeps of 20 us,

@@ -279,7 +279,7 @@ struct UpsolArgs {
 
 // NT > 0: the theta extent as a compile-time constant (equal to g_in.nth).
 // RJ rows of up to NTH / RJ cells: short theta lines take more rows, so that a
-// plane gives every thread a cell (64 x 32 x 128: 31 us with 2 rows of 32
+// plane gives every thread a cell (32 x 64 x 128: 31 us with 2 rows of 32
 // cells in 256 threads and 32 planes per CTA, 13 with 8 rows and 4 planes);
 // lines beyond 128 cells take two rows in 512 threads (256 x 128 x 1024,
 // mixed: 0.97 ms as two kernels, 0.70 here).

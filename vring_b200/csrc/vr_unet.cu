@@ -217,7 +217,7 @@ __host__ __device__ constexpr int conv_wstage_bytes() {
 //   kEpiPool: the F x F average pooling (k_pool), through the halo the products
 //     have done with; a patch holds whole cells, since F divides 8.
 // A learned solve at 512 x 1024 spares four launches and a 17 MB tensor written
-// and read again per iteration: 0.29 -> 0.28 ms per iteration.
+// and read again per iteration: 0.225 -> 0.216 ms per iteration.
 enum ConvEpiKind { kEpiNone = 0, kEpiHead, kEpiPool };
 struct ConvEpi {
   const float *w;
