@@ -20,12 +20,15 @@ namespace vr {
 // division per step alone 10 us.  The chain is therefore taken apart:
 // - beta is carried as a ratio u(k) / u(k-1) of the leading minors,
 //   u(k) = bb(k) u(k-1) - cc(k-1) aa(k) u(k-2), one fused multiply-add per
-//   step on the critical path and no division.  The ratio of the two stored
-//   numbers is the beta that the next step continues from, so the rounding of
-//   a step enters as it does in the recurrence above; the pair is scaled by a
-//   power of two per step (exact), so the minors neither overflow nor vanish.
+//   step on the critical path and no division.  The pair is scaled by the
+//   power of two of u(k-1) (exact) before each step, so that u(k) is about
+//   beta(k): the numbers formed are those of the recurrence above, in range
+//   where its are.  The rounding error of u(k) goes along, to be taken out of
+//   the ratio where it divides; the next step continues from the rounded one,
+//   as the recurrence does.
 // - the divisions 1 / beta(k) of a tile are independent of each other and run
-//   on all 32 lanes of a warp of their own.
+//   on all lanes of kThomDiv warps of their own, to twice the precision (ib + lo),
+//   so that a multiplication by them rounds once, as a division would.
 // - three warps work on three consecutive tiles of KT positions at a time:
 //   the minors of one, the divisions of the one before, gamm of the one
 //   before that, while a fourth brings the next tile from memory (8-byte
@@ -35,31 +38,85 @@ namespace vr {
 // The positions past n of the last tile, and systems past nbatch, are rows of
 // the identity.  aa(1) and cc(n) are not used: they are taken as 0.
 //
+// A system with a pivot beyond 2^+-480 (inside, a product cc aa that loses bits
+// is far below the rounding of u(k)), a cc / beta that is not 0 but below
+// 2^-960, infinities or NaN is solved again by the plain recurrence
+// (thomas_plain), one thread per system.
+//
 // 257 x 1024 (us per call): one thread per system with its loads a system
-// apart 241, this form 18.4.
+// apart 241; this form 18.4, with one dividing warp 22.5.  Error against 64
+// bits there, of the largest entry: recurrence 1.1e-16, here 9.6e-17 (a
+// multiplication by the rounded 1 / beta of the rounded minors: 1.2e-16).
 constexpr int kThomKT = 16;    // positions per tile
 constexpr int kThomRing = 6;   // tiles in flight
+constexpr int kThomArr = 6;    // arrays of a tile
+constexpr int kThomDiv = 4;    // warps that divide
+constexpr int kThomThreads = 32 * (3 + kThomDiv);
 
-// 2^-e of x = m 2^e, 1 <= |m| < 2 (0 for an infinity or a NaN: the product is then no number either)
+__device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// 2^-e of x = m 2^e, 1 <= |m| < 2, for |x| below 2^1023
 __device__ __forceinline__ double pow2_inv(double x) {
-  const int e = (__double2hiint(x) >> 20) & 0x7ff;
-  return __hiloint2double(max(2046 - e, 0) << 20, 0);
+  return __hiloint2double(0x7fe00000 - (__double2hiint(x) & 0x7ff00000), 0);
+}
+// whether |x| lies outside 2^-E .. 2^E (0, infinities and NaN do)
+template <int E>
+__device__ __forceinline__ bool off_range(double x) {
+  return 2u * (unsigned)__double2hiint(x) - ((1023u - E) << 21) > (2u * E) << 21;
+}
+// the exponent by which a factor is scaled, -1022 .. 1022 (0 for infinities and NaN)
+__device__ __forceinline__ int scale_exp(double x) {
+  const int e = exp_field(x);
+  return e == 0x7ff ? 0 : min(max(e - 1023, -1022), 1022);
+}
+__device__ __forceinline__ double scaled(double x, int e) { return x * __hiloint2double((1023 - e) << 20, 0); }
+
+// x y / d without overflow or underflow on the way
+__device__ __forceinline__ double mul_div(double x, double y, double d) {
+  const int ex = scale_exp(x), ey = scale_exp(y), ed = scale_exp(d);
+  return scalbn(scaled(x, ex) * scaled(y, ey) / scaled(d, ed), ex + ey - ed);
+}
+
+// One system by the recurrence as it stands, for any scale of its rows: beta
+// is kept in sol until the substitution overwrites it, gamm in its scratch.
+__device__ __noinline__ void thomas_plain(const double *r, double *sol, const double *a, const double *d,
+                                          const double *c, double *gm, int n) {
+  double beta = d[0], g = r[0] / beta;
+  sol[0] = beta;
+  gm[0] = g;
+  for (int k = 1; k < n; k++) {
+    beta = d[k] - mul_div(c[k - 1], a[k], beta);
+    const int e = max(scale_exp(beta), scale_exp(a[k]));
+    g = fma(-scaled(a[k], e), g, scaled(r[k], e)) / scaled(beta, e);
+    sol[k] = beta;
+    gm[k] = g;
+  }
+  double x = g;
+  sol[n - 1] = x;
+  for (int k = n - 2; k >= 0; k--) {
+    x = gm[k] - mul_div(c[k], x, sol[k]);
+    sol[k] = x;
+  }
 }
 
 template <int S>
-__global__ void __launch_bounds__(128) k_thomas(const double *__restrict__ rhs, double *sol,
+__global__ void __launch_bounds__(kThomThreads) k_thomas(const double *__restrict__ rhs, double *sol,
                                               const double *__restrict__ aa, const double *__restrict__ bb,
                                               const double *__restrict__ cc, double *gamm, int n, int nbatch) {
   constexpr int KT = kThomKT, LD = S + 1, AR = KT * LD, R = kThomRing;
-  constexpr int TR = 0, TA = 1, TB = 2, TC = 3, TX = 4;  // arrays of a tile: rhs, aa, bb, cc, u(k-1)
+  // arrays of a tile: rhs then gamm, aa, bb then u(k) then 1/beta, cc then cc/beta, u(k-1), the error of u(k) then
+  // that of 1/beta
+  constexpr int TR = 0, TA = 1, TB = 2, TC = 3, TX = 4, TE = 5;
   extern __shared__ double sm[];
+  __shared__ unsigned again;  // systems for thomas_plain
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s0 = blockIdx.x * S, ns = min(S, nbatch - s0);
   const int nt = (n + KT - 1) / KT;
-  auto tile = [&](int t, int arr) { return sm + ((size_t)(t % R) * 5 + arr) * AR; };
+  auto tile = [&](int t, int arr) { return sm + ((size_t)(t % R) * kThomArr + arr) * AR; };
   const size_t base = (size_t)s0 * n;
-  double x = 1.0, y = 1.0, cprev = 0.0;  // warp 1: u(k-1), u(k-2), cc(k-1)
-  double g = 0.0;                        // warp 3: gamm(k-1)
+  double x = 1.0, y = 0.0, cprev = 0.0;  // warp 1: u(k-1), u(k-2) by the scale of u(k-1), cc(k-1)
+  double g = 0.0;                        // warp 2: gamm(k-1)
+  bool bad = false;                      // of system lane % S
+  if (threadIdx.x == 0) again = 0;
   for (int i = 0; i < nt + 5; i++) {
     if (warp == 0) {
       if (i < nt) {
@@ -100,45 +157,56 @@ __global__ void __launch_bounds__(128) k_thomas(const double *__restrict__ rhs, 
       const int t = i - 2;
       if (t >= 0 && t < nt && lane < S) {
         const double *a = tile(t, TA) + lane, *c = tile(t, TC) + lane;
-        double *b = tile(t, TB) + lane, *xo = tile(t, TX) + lane;
+        double *b = tile(t, TB) + lane, *xo = tile(t, TX) + lane, *eo = tile(t, TE) + lane;
 #pragma unroll
         for (int kk = 0; kk < KT; kk++) {
-          const double s = pow2_inv(y), p = (cprev * a[kk * LD]) * s;
+          const double ak = a[kk * LD], bk = b[kk * LD], p = cprev * ak;
           cprev = c[kk * LD];
-          const double z = fma(b[kk * LD] * s, x, -(p * y));
+          const double s = pow2_inv(x), v = (p * y) * s;
           y = x * s;
-          b[kk * LD] = z;
+          x = fma(bk, y, -v);
+          bad |= off_range<480>(x);
+          b[kk * LD] = x;
           xo[kk * LD] = y;
-          x = z;
+          eo[kk * LD] = fma(bk, y, -x) - v;
         }
       }
-    } else if (warp == 2) {
+    } else if (warp >= 3) {
       const int t = i - 3;
       if (t >= 0 && t < nt) {
-        const double *b = tile(t, TB);
-        double *c = tile(t, TC), *xo = tile(t, TX);
+        double *b = tile(t, TB), *c = tile(t, TC), *eo = tile(t, TE);
+        const double *xo = tile(t, TX);
 #pragma unroll
-        for (int e = lane; e < KT * S; e += 32) {
+        for (int e = threadIdx.x - 96; e < KT * S; e += 32 * kThomDiv) {
           const int o = (e / S) * LD + e % S;
-          const double ib = xo[o] / b[o];
-          xo[o] = ib;
-          c[o] = c[o] * ib;
+          // 1 / beta = ib + lo of beta = (u(k) + its error) / u(k-1); the last
+          // factor, 1 / u(k-1) of a number in [1, 2), needs few bits
+          const double u = xo[o], z = b[o], ib = u / z;
+          const double lo = (fma(-z, ib, u) - ib * eo[o]) * ib * (double)__frcp_rn((float)u);
+          const double ck = c[o], f0 = ck * ib, f = f0 + fma(ck, lo, fma(ck, ib, -f0));
+          bad |= off_range<960>(f) && ck != 0.0;
+          b[o] = ib;
+          eo[o] = lo;
+          c[o] = f;
         }
       }
     } else {
       const int t = i - 4;
       if (t >= 0 && t < nt && lane < S) {
-        const double *a = tile(t, TA) + lane, *xo = tile(t, TX) + lane;
+        const double *a = tile(t, TA) + lane, *ib = tile(t, TB) + lane, *lo = tile(t, TE) + lane;
         double *r = tile(t, TR) + lane;
 #pragma unroll
         for (int kk = 0; kk < KT; kk++) {
-          g = fma(-a[kk * LD], g, r[kk * LD]) * xo[kk * LD];
+          const double v = fma(-a[kk * LD], g, r[kk * LD]);
+          g = fma(v, ib[kk * LD], v * lo[kk * LD]);
           r[kk * LD] = g;
         }
       }
     }
     __syncthreads();
   }
+  if (warp == 2) bad = exp_field(g) == 0x7ff;  // an infinity or a NaN lasts to the end of its system
+  if (bad) atomicOr(&again, 1u << (lane % S));
   // back substitution, last tile first: arrays 0 gamm, 1 cc/beta, 2 the solution
   double xn = 0.0;
   for (int i = 0; i < nt + 3; i++) {
@@ -184,6 +252,10 @@ __global__ void __launch_bounds__(128) k_thomas(const double *__restrict__ rhs, 
     }
     __syncthreads();
   }
+  if (threadIdx.x < ns && (again >> threadIdx.x & 1)) {
+    const size_t o = base + (size_t)threadIdx.x * n;
+    thomas_plain(rhs + o, sol + o, aa + o, bb + o, cc + o, gamm + o, n);
+  }
 }
 
 // S systems per CTA: 8 keeps a batch of up to 2 x 148 x 8 systems on CTAs of
@@ -191,7 +263,7 @@ __global__ void __launch_bounds__(128) k_thomas(const double *__restrict__ rhs, 
 // nothing there); larger batches are bound by throughput and take 16.
 static const void *thomas_kernel(int nbatch, int *s, size_t *smem) {
   *s = nbatch <= 2 * 148 * 8 ? 8 : 16;
-  *smem = sizeof(double) * kThomRing * 5 * kThomKT * (*s + 1);
+  *smem = sizeof(double) * kThomRing * kThomArr * kThomKT * (*s + 1);
   return *s == 8 ? (const void *)k_thomas<8> : (const void *)k_thomas<16>;
 }
 
@@ -206,7 +278,7 @@ static cudaError_t launch_thomas(const double *rhs, double *sol, const double *a
   if (e) return e;
   void *args[] = {(void *)&rhs, (void *)&sol, (void *)&aa, (void *)&bb, (void *)&cc, (void *)&gamm,
                   (void *)&n, (void *)&nbatch};
-  return cudaLaunchKernel(kern, dim3((nbatch + s - 1) / s), dim3(128), args, smem, st);
+  return cudaLaunchKernel(kern, dim3((nbatch + s - 1) / s), dim3(kThomThreads), args, smem, st);
 }
 
 cudaError_t launch_thomas_batched(const double *rhs, double *sol, const double *aa, const double *bb,
