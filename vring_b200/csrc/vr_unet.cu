@@ -319,7 +319,14 @@ __global__ void __launch_bounds__(128) k_conv3_tc(const __nv_bfloat16 *in, int H
   // the packed weights are already in the staged order
   for (int e = tid; e < 9 * CC * NOUT; e += 128) cp_async16(wst + (size_t)e * 16, wpk + (size_t)e * 8, 16u);
   pdl_wait();  // up to here: tensor memory and the weights
-  if (gridDim.x <= kTriggerCtas) pdl_trigger();
+  if (gridDim.x <= kTriggerCtas) {
+    // A CTA counts as soon as one of its threads triggers, and the successor's
+    // CTAs, which wait for this grid to end, take tensor memory as they start:
+    // all of an SM's while this CTA's warp 0 still asks for its own would
+    // leave both waiting.  So not before every warp knows that it has it.
+    __syncthreads();
+    pdl_trigger();
+  }
   int patch = blockIdx.x, buf = 0;
   uint32_t phase = 0;
   if (patch < npatch) fetch(patch, halos);
