@@ -450,7 +450,10 @@ VR_API int vr_unet_backward(vr_unet *u, const double *x, const double *g, float 
 VR_API int vr_unet_train_step(vr_unet *u, vr_k2d *k, const double *e_dev, int32_t nb, float lr, double *loss);
 /* diag(S) of the symmetric form (host, nr*nz) */
 VR_API int vr_k2d_diag(const vr_k2d *k, double *d);
-/* make the network the preconditioner of VR_KRYLOV_FCG_LEARNED (NULL clears) */
+/* make the network the preconditioner of VR_KRYLOV_FCG_LEARNED (NULL clears).
+ * The solver holds it: a network destroyed meanwhile keeps working as the
+ * preconditioner, and its memory goes when the solver is given another one (or
+ * NULL) or is destroyed. */
 VR_API int vr_k2d_set_preconditioner(vr_k2d *k, const vr_unet *u);
 /* The flexible CG's preconditioner is z0 = w D^-1 r, z = z0 + N(r - S z0),
  * z += w D^-1 (r - S z) (D the diagonal of S, N the network): a two-level step

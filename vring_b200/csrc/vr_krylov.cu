@@ -1070,6 +1070,7 @@ extern "C" int vr_k2d_destroy(vr_k2d *k) {
   if (k->flags) cudaFree(k->flags);
   if (k->cnt) cudaFree(k->cnt);
   if (k->res_mem) cudaFree(k->res_mem);
+  if (k->net) unet_drop(k->net);
   if (k->stream) cudaStreamDestroy(k->stream);
   delete k;
   return VR_OK;
@@ -1366,10 +1367,13 @@ extern "C" int vr_k2d_set_preconditioner(vr_k2d *k, const vr_unet *net) {
     unet_dims(net, &nr, &nz);
     if (nr != k->nr || nz != k->nz) return k2d_err(k, VR_ERR_ARG, "network and operator grids differ");
   }
-  if (k->net != net && k->graph_ok[3]) {
+  if (k->net == net) return VR_OK;
+  if (k->graph_ok[3]) {
     cudaGraphExecDestroy(k->graph[3]);
     k->graph_ok[3] = false;
   }
+  if (net) unet_hold(net);
+  if (k->net) unet_drop(k->net);
   k->net = net;
   return VR_OK;
 }

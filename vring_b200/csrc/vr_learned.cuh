@@ -15,6 +15,12 @@ namespace vr {
 int unet_correct(const vr_unet *u, const double *t, const double *dscale, const double *ss, const int *flags, float *yl,
                  const float **y, cudaStream_t s);
 
+// A solver holds the network that it is given: its captured iterations have the
+// network's buffers in them.  A destroyed network's memory, and with it its
+// address, is free for another one only after the last holder has dropped it.
+void unet_hold(const vr_unet *u);
+void unet_drop(const vr_unet *u);
+
 // grid of a network (nr, nz)
 void unet_dims(const vr_unet *u, int *nr, int *nz);
 

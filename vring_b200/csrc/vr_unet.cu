@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -45,6 +46,7 @@ struct UnetLayer {
 }  // namespace vr
 
 struct vr_unet {
+  std::atomic<int> refs{1};  // the caller, and every solver whose preconditioner it is
   int nr = 0, nz = 0, dev = 0, nsm = 148;
   int ch[4] = {};
   int pool = 2;  // pooling factor between levels
@@ -1204,8 +1206,7 @@ extern "C" int vr_unet_create(const vr_unet_desc *d, uint64_t seed, vr_unet **ou
   return VR_OK;
 }
 
-extern "C" int vr_unet_destroy(vr_unet *u) {
-  if (!u) return VR_OK;
+static void unet_free(vr_unet *u) {
   cudaSetDevice(u->dev);
   if (u->stream) cudaStreamSynchronize(u->stream);
   for (int i = 0; i < S_NSLOT; i++) {
@@ -1224,6 +1225,20 @@ extern "C" int vr_unet_destroy(vr_unet *u) {
   if (u->dscal) cudaFree(u->dscal);
   if (u->stream) cudaStreamDestroy(u->stream);
   delete u;
+}
+
+namespace vr {
+
+void unet_hold(const vr_unet *u) { const_cast<vr_unet *>(u)->refs.fetch_add(1, std::memory_order_relaxed); }
+void unet_drop(const vr_unet *u) {
+  vr_unet *x = const_cast<vr_unet *>(u);
+  if (x->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) unet_free(x);
+}
+
+}  // namespace vr
+
+extern "C" int vr_unet_destroy(vr_unet *u) {
+  if (u) unet_drop(u);
   return VR_OK;
 }
 
