@@ -448,6 +448,14 @@ VR_API int vr_unet_backward(vr_unet *u, const double *x, const double *g, float 
  * L before the step (may be NULL).  The flexible CG applies the network the
  * same way: z = s D N(D r / s). */
 VR_API int vr_unet_train_step(vr_unet *u, vr_k2d *k, const double *e_dev, int32_t nb, float lr, double *loss);
+/* A convolution's tensor-core wait is bounded.  When one gives up, the forward,
+ * the backward, the training step (which then leaves the weights alone) or the
+ * learned solve that it belongs to returns VR_ERR_TIMEOUT, and its outputs are
+ * not valid; the network stays usable.  The self-test makes such a wait run
+ * out after limit_ns nanoseconds (1e3 .. 1e9) on a barrier that nothing
+ * completes and returns VR_ERR_TIMEOUT as designed; the next of those calls
+ * reports it too. */
+VR_API int vr_unet_wait_selftest(vr_unet *u, int64_t limit_ns);
 /* diag(S) of the symmetric form (host, nr*nz) */
 VR_API int vr_k2d_diag(const vr_k2d *k, double *d);
 /* make the network the preconditioner of VR_KRYLOV_FCG_LEARNED (NULL clears).

@@ -159,6 +159,7 @@ def lib():
         L.vr_unet_last_error.restype = C.c_char_p
         L.vr_unet_last_error.argtypes = [vp]
         L.vr_unet_nparams.argtypes = [vp, C.POINTER(i64)]
+        L.vr_unet_wait_selftest.argtypes = [vp, i64]
         L.vr_unet_get_params.argtypes = [vp, vp]
         L.vr_unet_set_params.argtypes = [vp, vp]
         L.vr_unet_forward.argtypes = [vp, vp, vp]
@@ -659,6 +660,11 @@ class UNet:
         dx = np.empty_like(x)
         self._chk(lib().vr_unet_backward(self._h, _p(x), _p(g), _p(dw), _p(dx)), "unet_backward")
         return dw, dx
+
+    def wait_selftest(self, limit_ns: int = 10_000_000) -> int:
+        """Run a kernel whose bounded wait must run out; returns the status code
+        (VR_ERR_TIMEOUT = 5), which the next call on the network reports too."""
+        return lib().vr_unet_wait_selftest(self._h, int(limit_ns))
 
     def train_step(self, k2d: K2d, e_ptr: int, nb: int, lr: float) -> float:
         """One Adam step on nb device-resident errors (nb x nr*nz doubles);

@@ -1485,7 +1485,15 @@ extern "C" int vr_k2d_solve_dev(vr_k2d *k, int32_t method, const double *f, doub
   double hs[SC_N];
   K2D_CUDA(k, cudaMemcpyAsync(x, X, bytes, cudaMemcpyDeviceToDevice, k->stream));
   K2D_CUDA(k, cudaMemcpyAsync(hs, k->sc, sizeof(hs), cudaMemcpyDeviceToHost, k->stream));
+  const bool learned = method == VR_KRYLOV_FCG_LEARNED;
+  unsigned st = 0;
+  if (learned) K2D_CUDA(k, unet_read_status(k->net, &st, k->stream));
   K2D_CUDA(k, cudaStreamSynchronize(k->stream));
+  if (st) {
+    K2D_CUDA(k, unet_clear_status(k->net, k->stream));
+    K2D_CUDA(k, cudaStreamSynchronize(k->stream));
+    return k2d_err(k, VR_ERR_TIMEOUT, "learned krylov: a bounded wait of a convolution gave up");
+  }
   if (iters) *iters = it;
   if (relres) *relres = hs[SC_BB] > 0 ? std::sqrt(hs[SC_RR] / hs[SC_BB]) : 0.0;
   return VR_OK;

@@ -21,6 +21,11 @@ int unet_correct(const vr_unet *u, const double *t, const double *dscale, const 
 void unet_hold(const vr_unet *u);
 void unet_drop(const vr_unet *u);
 
+// the word that a convolution sets when its bounded tensor-core wait gives up
+// (its outputs are then not valid); the caller synchronises the stream
+cudaError_t unet_read_status(const vr_unet *u, unsigned *st, cudaStream_t s);
+cudaError_t unet_clear_status(const vr_unet *u, cudaStream_t s);
+
 // grid of a network (nr, nz)
 void unet_dims(const vr_unet *u, int *nr, int *nz);
 

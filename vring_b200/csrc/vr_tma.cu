@@ -29,6 +29,11 @@ __global__ void k_wait_selftest(unsigned long long limit_ns, unsigned *status) {
   if (!__any_sync(0xffffffffu, ok) && threadIdx.x == 0) atomicOr(status, 1u);
 }
 
+cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned *status, cudaStream_t s) {
+  k_wait_selftest<<<1, 32, 0, s>>>(limit_ns, status);
+  return cudaGetLastError();
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
@@ -74,8 +79,7 @@ extern "C" int vr_wait_selftest(vr_ctx *c, int64_t limit_ns) {
   using namespace vr;
   if (!c || limit_ns < 1000 || limit_ns > 1000000000) return VR_ERR_ARG;
   VR_CUDA(c, cudaSetDevice(c->dev));
-  k_wait_selftest<<<1, 32, 0, c->stream>>>((unsigned long long)limit_ns, c->d_status);
-  VR_LAUNCH_CHECK(c);
+  VR_CUDA(c, launch_wait_selftest((unsigned long long)limit_ns, c->d_status, c->stream));
   unsigned st = 0;
   VR_CUDA(c, cudaMemcpyAsync(&st, c->d_status, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
   VR_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -96,6 +96,10 @@ __device__ __forceinline__ void bulk_wait_read() {
 // until every bulk group of this thread has completed
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Host: one warp that waits limit_ns on an mbarrier nothing completes and then
+// sets bit 0 of the status word
+cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned *status, cudaStream_t s);
+
 // Host: a tensor map of a column-major FP64 array (d0, d1, d2) with boxes of
 // (b0, b1, b2) elements; out-of-range elements of a box read as zero.  With
 // swizzle 128 the box rows (b0 * 8 = 128 bytes) land in shared memory with

@@ -32,6 +32,7 @@
 
 #include "vr_internal.cuh"
 #include "vr_learned.cuh"
+#include "vr_tma.cuh"
 #include "vr_umma.cuh"
 
 namespace vr {
@@ -906,8 +907,11 @@ __global__ void k_wprep(const float *__restrict__ w32, size_t n, __nv_bfloat16 *
   }
 }
 // Adam (Kingma & Ba 2015) on the FP32 master weights, gradient scaled by gs
+// (no step on the gradient of a forward pass that gave up)
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       size_t n, float lr, float gs, float b1, float b2, float c1, float c2, float eps) {
+                       size_t n, float lr, float gs, float b1, float b2, float c1, float c2, float eps,
+                       const unsigned *status) {
+  if (*status) return;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const float gi = g[i] * gs;
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -1391,6 +1395,13 @@ void unet_dims(const vr_unet *u, int *nr, int *nz) {
   *nz = u->nz;
 }
 
+cudaError_t unet_read_status(const vr_unet *u, unsigned *st, cudaStream_t s) {
+  return cudaMemcpyAsync(st, u->status, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+}
+cudaError_t unet_clear_status(const vr_unet *u, cudaStream_t s) {
+  return cudaMemsetAsync(u->status, 0, sizeof(unsigned), s);
+}
+
 int unet_correct(const vr_unet *u, const double *t, const double *dscale, const double *ss, const int *flags, float *yl,
                  const float **y, cudaStream_t s) {
   const int n = u->nr * u->nz;
@@ -1401,6 +1412,27 @@ int unet_correct(const vr_unet *u, const double *t, const double *dscale, const 
 }
 
 }  // namespace vr
+
+// waits for the stream; reports, once, a tensor-core wait that gave up
+static int unet_finish(vr_unet *u) {
+  unsigned st = 0;
+  U_CUDA(u, unet_read_status(u, &st, u->stream));
+  U_CUDA(u, cudaStreamSynchronize(u->stream));
+  if (!st) return VR_OK;
+  U_CUDA(u, unet_clear_status(u, u->stream));
+  U_CUDA(u, cudaStreamSynchronize(u->stream));
+  return unet_err(u, VR_ERR_TIMEOUT, "a bounded wait of a convolution gave up");
+}
+
+extern "C" int vr_unet_wait_selftest(vr_unet *u, int64_t limit_ns) {
+  if (!u || limit_ns < 1000 || limit_ns > 1000000000) return VR_ERR_ARG;
+  U_CUDA(u, cudaSetDevice(u->dev));
+  U_CUDA(u, launch_wait_selftest((unsigned long long)limit_ns, u->status, u->stream));
+  unsigned st = 0;
+  U_CUDA(u, unet_read_status(u, &st, u->stream));
+  U_CUDA(u, cudaStreamSynchronize(u->stream));
+  return st ? VR_ERR_TIMEOUT : VR_OK;
+}
 
 extern "C" int vr_unet_forward(vr_unet *u, const double *xh, double *yh) {
   if (!u || !xh || !yh) return VR_ERR_ARG;
@@ -1416,8 +1448,7 @@ extern "C" int vr_unet_forward(vr_unet *u, const double *xh, double *yh) {
   k_out<<<grid_for(n), 256, 0, u->stream>>>(u->y, n, s, u->xs);
   U_CUDA(u, cudaGetLastError());
   U_CUDA(u, cudaMemcpyAsync(yh, u->xs, sizeof(double) * n, cudaMemcpyDeviceToHost, u->stream));
-  U_CUDA(u, cudaStreamSynchronize(u->stream));
-  return VR_OK;
+  return unet_finish(u);
 }
 
 __global__ static void k_f2d(const float *a, double *b, int n) {
@@ -1444,8 +1475,7 @@ extern "C" int vr_unet_backward(vr_unet *u, const double *xh, const double *gh, 
     k_f2d<<<grid_for(n), 256, 0, u->stream>>>(u->gx0, u->xs, n);
     U_CUDA(u, cudaMemcpyAsync(dx, u->xs, sizeof(double) * n, cudaMemcpyDeviceToHost, u->stream));
   }
-  U_CUDA(u, cudaStreamSynchronize(u->stream));
-  return VR_OK;
+  return unet_finish(u);
 }
 
 extern "C" int vr_unet_train_step(vr_unet *u, vr_k2d *k, const double *e_dev, int32_t nb, float lr, double *loss) {
@@ -1474,11 +1504,13 @@ extern "C" int vr_unet_train_step(vr_unet *u, vr_k2d *k, const double *e_dev, in
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)u->adam_t), c2 = 1.f - std::pow(b2, (float)u->adam_t);
   k_adam<<<grid_for(u->nparam), 256, 0, s>>>(u->w32, u->gw, u->m1, u->m2, u->nparam, lr, 1.f / nb, b1, b2, c1, c2,
-                                            1e-8f);
+                                            1e-8f, u->status);
   U_CUDA(u, unet_prep_weights(u, s));
   double h = 0.0;
   U_CUDA(u, cudaMemcpyAsync(&h, u->dscal, sizeof(double), cudaMemcpyDeviceToHost, s));
-  U_CUDA(u, cudaStreamSynchronize(s));
+  const int rc = unet_finish(u);
+  if (rc == VR_ERR_TIMEOUT) u->adam_t--;  // no step was made
+  if (rc) return rc;
   if (loss) *loss = h / nb;
   return VR_OK;
 }
