@@ -970,8 +970,7 @@ extern "C" int vr_step(vr_ctx *c) {
   if (c->mixed) return set_err(c, VR_ERR_STATE, "vr_step: the mixed form runs through vr_substep/vr_iterate only");
   VR_CUDA(c, cudaSetDevice(c->dev));
   const cudaError_t e = launch_rhs_tsweep(c, rk_of(c), true);
-  if (e == cudaErrorNotSupported) {
-    (void)cudaGetLastError();
+  if (e == cudaErrorNotSupported) {  // a grid that is not its, not an error of a call
     VR_CUDA(c, launch_rhs(c, rk_of(c), false));
   } else {
     VR_CUDA(c, e);
