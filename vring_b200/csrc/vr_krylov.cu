@@ -85,8 +85,7 @@ struct vr_k2d {
   int bi_parity = 0;        // p and v buffers of the next BiCGSTAB iteration being captured
   int nb_cg = 1;            // grid of the CG iteration kernels
   // resident CG: planes per thread (0: the grid does not fit), segments and
-  // CTAs, the exchanges' memory (allocated by the first solve that needs it)
-  // and the next exchange's number
+  // CTAs, the exchanges' memory and the next exchange's number
   int res_c = 0, res_nseg = 0, res_ctas = 0;
   unsigned long long *res_mem = nullptr;
   size_t res_words = 0;
@@ -1051,6 +1050,17 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
   if (cudaMemset(k->part, 0, sizeof(double) * PT_N * kK2dMaxBlocks) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaMemset(k->flags, 0, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (!res_shape(nr, nz, nsm, &k->res_c, &k->res_nseg, &k->res_ctas)) k->res_c = 0;
+  if (k->res_c) {  // made here, so that a solve allocates nothing; without it CG streams its vectors
+    k->res_words = (size_t)k->res_ctas * (2 * kResCopies * kResSlotWords + 2 * 2 * (size_t)nr);
+    const size_t bytes = sizeof(unsigned long long) * k->res_words;
+    if (cudaMalloc(&k->res_mem, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      k->res_mem = nullptr;
+      k->res_c = 0;
+    } else if (cudaMemsetAsync(k->res_mem, 0, bytes, k->stream) != cudaSuccess) {
+      return fail(VR_ERR_CUDA);
+    }
+  }
   *out = k;
   return VR_OK;
 }
@@ -1271,12 +1281,6 @@ static cudaError_t res_chunk(vr_k2d *k, bool jacobi) {
 static int run_resident(vr_k2d *k, bool jacobi, int maxit, int *iters, bool *ran) {
   int h[4] = {0, 0, 0, 0};
   *ran = false;
-  if (!k->res_mem) {
-    k->res_words = (size_t)k->res_ctas * (2 * kResCopies * kResSlotWords + 2 * 2 * (size_t)k->nr);
-    if (cudaMalloc(&k->res_mem, sizeof(unsigned long long) * k->res_words) != cudaSuccess)
-      return k2d_err(k, VR_ERR_OOM, "resident krylov");
-    K2D_CUDA(k, cudaMemsetAsync(k->res_mem, 0, sizeof(unsigned long long) * k->res_words, k->stream));
-  }
   for (int done = 0; done < maxit; done += kResIters) {
     const cudaError_t e = res_chunk(k, jacobi);
     if (e == cudaErrorNotSupported && !*ran) return VR_OK;
