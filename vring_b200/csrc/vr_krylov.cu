@@ -1406,6 +1406,30 @@ __global__ void __launch_bounds__(kK2dThreads) k2d_init_dots(K2dOp o, int jacobi
   if (threadIdx.x == 0) part[2 * kK2dMaxBlocks + blockIdx.x] = t;
 }
 
+// the flexible CG's buffers, all of them or none; the refusal is this call's
+// answer and does not stay pending on the thread
+static bool fcg_alloc(vr_k2d *k) {
+  if (k->fp) return true;
+  const size_t kb = (size_t)kFcgKeep * k->n;
+  struct {
+    double **p;
+    size_t n;
+  } want[] = {{&k->fp, kb},       {&k->fq, kb},
+              {&k->fpq, kFcgKeep}, {&k->fbeta, kFcgKeep},
+              {&k->frow, (size_t)4 * k->nz}, {&k->fpart, (size_t)kFcgKeep * kK2dMaxBlocks}};
+  for (auto &w : want)
+    if (cudaMalloc(w.p, sizeof(double) * w.n) != cudaSuccess) {
+      (void)cudaGetLastError();
+      *w.p = nullptr;
+      for (auto &v : want) {
+        if (*v.p) cudaFree(*v.p);
+        *v.p = nullptr;
+      }
+      return false;
+    }
+  return true;
+}
+
 // solve K x = f on device arrays of nr*nz doubles (r fastest); x holds the
 // initial guess on entry and the solution on return
 extern "C" int vr_k2d_solve_dev(vr_k2d *k, int32_t method, const double *f, double *x, double tol, int32_t maxit,
@@ -1458,15 +1482,7 @@ extern "C" int vr_k2d_solve_dev(vr_k2d *k, int32_t method, const double *f, doub
     K2D_CUDA(k, cudaGetLastError());
     rc = run_chunks(k, 2, enq_bicg, 0, maxit, &it);
   } else {
-    if (!k->fp) {
-      const size_t kb = sizeof(double) * kFcgKeep * (size_t)k->n;
-      if (cudaMalloc(&k->fp, kb) != cudaSuccess || cudaMalloc(&k->fq, kb) != cudaSuccess ||
-          cudaMalloc(&k->fpq, sizeof(double) * kFcgKeep) != cudaSuccess ||
-          cudaMalloc(&k->fbeta, sizeof(double) * kFcgKeep) != cudaSuccess ||
-          cudaMalloc(&k->frow, sizeof(double) * 4 * k->nz) != cudaSuccess ||
-          cudaMalloc(&k->fpart, sizeof(double) * kFcgKeep * kK2dMaxBlocks) != cudaSuccess)
-        return k2d_err(k, VR_ERR_OOM, "flexible CG directions");
-    }
+    if (!fcg_alloc(k)) return k2d_err(k, VR_ERR_OOM, "flexible CG directions");
     k2d_init_dots<<<gb, kK2dThreads, 0, k->stream>>>(o, 0, B, R, nullptr, P);
     k2d_scalar<<<1, 1024, 0, k->stream>>>(SO_CG_INIT, P, gb, k->sc, k->flags);
     K2D_CUDA(k, cudaGetLastError());
