@@ -548,7 +548,6 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
     if (cudaMemsetAsync(*o.p, 0, o.w * o.n, c->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
     c->state.emplace_back(*o.p, o.w * o.n);
   }
-  if (c->lin_z[0] && cudaMalloc(&c->spec2, sizeof(double) * nrs) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&c->d_count, sizeof(unsigned long long) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMemsetAsync(c->d_count, 0, sizeof(unsigned long long) * 4, c->stream) != cudaSuccess)
     return fail(VR_ERR_CUDA);
@@ -566,7 +565,7 @@ extern "C" int vr_destroy(vr_ctx *c) {
   for (int i = 0; i < 4; i++)
     if (c->graph_ok[i]) cudaGraphExecDestroy(c->graph[i]);
   double *ptrs[] = {c->q[0], c->q[1], c->q[2], c->dq[0], c->dq[1], c->dq[2], c->ru[0], c->ru[1],
-                    c->ru[2], c->qrhs[0], c->qrhs[1], c->qrhs[2], c->pres, c->prg, c->rhs, c->spec, c->spec2, c->lin_tab,
+                    c->ru[2], c->qrhs[0], c->qrhs[1], c->qrhs[2], c->pres, c->prg, c->rhs, c->spec, c->lin_tab,
                     c->dph, c->csort, c->dq3no, c->corr3n, c->corr3s, c->tconv, c->dcoef, c->d_red};
   for (double *p : ptrs)
     if (p) cudaFree(p);

@@ -185,7 +185,6 @@ struct vr_ctx {
   // device fields
   double *q[3], *dq[3], *ru[3], *qrhs[3];
   double *prg, *pres, *rhs, *dph, *spec;
-  double *spec2;  // second spectral buffer (z lengths without an FFT), or null
   double *lin_tab;  // the memory behind lin_th and lin_z
   double *csort, *dq3no, *corr3n, *corr3s, *tconv;
   // device coefficient storage (one allocation) and family tables

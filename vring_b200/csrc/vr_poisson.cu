@@ -1776,9 +1776,10 @@ static cudaError_t run_dct(vr_ctx *c, int dir) {
   return cudaGetLastError();
 }
 
-// the theta transforms' side of the spectrum: the z products are not in place,
-// so theirs is the second buffer
-static double *theta_spec(vr_ctx *c) { return c->lin_z[0] ? c->spec2 : c->spec; }
+// The theta transforms' side of the spectrum.  The z products are not in place;
+// theirs is q1's work array of the sweeps, which is written anew in every step
+// before it is read.
+static double *theta_spec(vr_ctx *c) { return c->lin_z[0] ? c->qrhs[0] : c->spec; }
 
 template <int E>
 static cudaError_t run_fft_w(vr_ctx *c, int dir) {
@@ -1998,8 +1999,8 @@ static cudaError_t run_z(vr_ctx *c, int dir) {
   if (c->lin_z[0]) {
     const int M = g.nth * g.nr;
     LaunchScope ls(c, PK_DCT);
-    return dir > 0 ? lin_run<kLinZFwd>(c->spec2, c->spec, c->lin_z[0], g.nz, M, 0, c->nsm, c->stream)
-                   : lin_run<kLinZInv>(c->spec, c->spec2, c->lin_z[1], g.nz, M, 0, c->nsm, c->stream);
+    return dir > 0 ? lin_run<kLinZFwd>(theta_spec(c), c->spec, c->lin_z[0], g.nz, M, 0, c->nsm, c->stream)
+                   : lin_run<kLinZInv>(c->spec, theta_spec(c), c->lin_z[1], g.nz, M, 0, c->nsm, c->stream);
   }
   bool done = false;
   cudaError_t e = dct_warp_dispatch(c, dir, &done);
