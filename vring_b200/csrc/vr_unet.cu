@@ -949,9 +949,11 @@ static cudaError_t conv3_tc_n(const __nv_bfloat16 *in, int H, int W, int cin, co
                               int nsm, cudaStream_t s, ConvEpi epi) {
   constexpr int halo = conv_halo_bytes<CINP>(), wst = conv_wstage_bytes<CINP, NOUT>();
   const int npr = (H + kConvTR - 1) / kConvTR, npatch = npr * ((W + kConvTZ - 1) / kConvTZ);
-  // resident CTAs per SM with two halo buffers; one buffer where no CTA walks
-  const int most = std::max(1, std::min(kConvCtas, (int)((size_t)(220 * 1024) / (128 + wst + 2 * halo + 1024))));
-  const int grid = std::min(npatch, nsm * most);
+  // resident CTAs per SM with two halo buffers; one buffer where no CTA walks,
+  // and a CTA per patch where two do not fit beside the weights (128 channels
+  // to 64: 148 + 2 x 46 KB)
+  constexpr int most = std::min(kConvCtas, 220 * 1024 / (128 + wst + 2 * halo + 1024));
+  const int grid = most ? std::min(npatch, nsm * most) : npatch;
   const size_t sm = 128 + (size_t)wst + (size_t)(npatch > grid ? 2 : 1) * halo;
   auto kern = k_conv3_tc<CINP, NOUT, kEpiNone>;
   if (epi.w || epi.pooled) {  // as many channels in as out
