@@ -1184,7 +1184,7 @@ extern "C" int vr_unet_create(const vr_unet_desc *d, uint64_t seed, vr_unet **ou
   }
   if (cudaMalloc(&u->wpk, sizeof(__nv_bfloat16) * npk) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&u->status, sizeof(unsigned)) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMemset(u->status, 0, sizeof(unsigned)) != cudaSuccess) return fail(VR_ERR_CUDA);
+  if (cudaMemsetAsync(u->status, 0, sizeof(unsigned), u->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
   u->cuda_cores = (d->flags & VR_UNET_CUDA_CORES) != 0;
   if (cudaMalloc(&u->x0, sizeof(__nv_bfloat16) * P0) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&u->y, sizeof(float) * P0) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -1202,10 +1202,13 @@ extern "C" int vr_unet_create(const vr_unet_desc *d, uint64_t seed, vr_unet **ou
     if (cudaMalloc(&x->g[i], sizeof(float) * n) != cudaSuccess) return fail(VR_ERR_OOM);
   }
   if (cudaMalloc(&x->gx0, sizeof(float) * P0) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMemcpy(u->w32, w.data(), sizeof(float) * u->nparam, cudaMemcpyHostToDevice) != cudaSuccess)
+  // on the stream that goes on to use them: cudaMemcpy from pageable memory and
+  // cudaMemset may return before the device has the bytes, in the order of the
+  // legacy stream, which this one does not wait for
+  if (cudaMemcpyAsync(u->w32, w.data(), sizeof(float) * u->nparam, cudaMemcpyHostToDevice, u->stream) != cudaSuccess ||
+      cudaMemsetAsync(u->m1, 0, sizeof(float) * u->nparam, u->stream) != cudaSuccess ||
+      cudaMemsetAsync(u->m2, 0, sizeof(float) * u->nparam, u->stream) != cudaSuccess)
     return fail(VR_ERR_CUDA);
-  if (cudaMemset(u->m1, 0, sizeof(float) * u->nparam) != cudaSuccess) return fail(VR_ERR_CUDA);
-  if (cudaMemset(u->m2, 0, sizeof(float) * u->nparam) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (unet_prep_weights(u, u->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
   if (cudaStreamSynchronize(u->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
   *out = u;
