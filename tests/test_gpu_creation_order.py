@@ -16,3 +16,21 @@ def test_networks_run_with_their_weights_from_the_first_call():
         y = kept[-1].forward(x)
         first = y if first is None else first
         assert np.abs(y).max() > 0 and np.array_equal(y, first)
+
+
+def test_axisymmetric_solvers_run_with_their_coefficients_from_the_first_call():
+    import torch
+    import vring_b200 as V
+    from vring_b200.learned import tanh_faces
+    faces = tanh_faces(512)
+    f = torch.randn((1024, 512), dtype=torch.float64, device="cuda")
+    x = torch.zeros_like(f)
+    torch.cuda.synchronize()
+    kept, first = [], None
+    for _ in range(12):
+        kept.append(V.K2d(faces, 1024, 15.0))
+        kept[-1].direct_dev(f.data_ptr(), x.data_ptr())
+        y = x.clone()
+        torch.cuda.synchronize()
+        first = y if first is None else first
+        assert torch.equal(y, first) and bool(torch.isfinite(y).all())

@@ -1028,7 +1028,9 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
   if (cudaMalloc(&k->sc, sizeof(double) * SC_N) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->flags, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_OOM);
   if (cudaMalloc(&k->cnt, sizeof(unsigned) * 8) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMemset(k->cnt, 0, sizeof(unsigned) * 8) != cudaSuccess) return fail(VR_ERR_CUDA);
+  // copies and fills on the solver's stream, which does not wait for the legacy
+  // one that cudaMemcpy and cudaMemset are ordered on (both may return early)
+  if (cudaMemsetAsync(k->cnt, 0, sizeof(unsigned) * 8, k->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
   const bool lin = k->zform == K2D_Z_LIN;
   const size_t nf = lin ? lin_table_len(kLinZFwd, nz) : cf.size(), ni = lin ? lin_table_len(kLinZInv, nz) : ci.size();
   if (cudaMalloc(&k->dct_f, sizeof(double) * nf) != cudaSuccess) return fail(VR_ERR_OOM);
@@ -1044,11 +1046,12 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
     const std::vector<double> *h;
   } up_[] = {{k->coef, &coef}, {k->dct_f, &cf}, {k->dct_i, &ci}, {k->tlo, &lo}, {k->tup, &up}, {k->tib, &ib}};
   for (auto &u : up_)
-    if (!u.h->empty() &&
-        cudaMemcpy(u.d, u.h->data(), sizeof(double) * u.h->size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (!u.h->empty() && cudaMemcpyAsync(u.d, u.h->data(), sizeof(double) * u.h->size(), cudaMemcpyHostToDevice,
+                                         k->stream) != cudaSuccess)
       return fail(VR_ERR_CUDA);
-  if (cudaMemset(k->part, 0, sizeof(double) * PT_N * kK2dMaxBlocks) != cudaSuccess) return fail(VR_ERR_CUDA);
-  if (cudaMemset(k->flags, 0, sizeof(int) * 4) != cudaSuccess) return fail(VR_ERR_CUDA);
+  if (cudaMemsetAsync(k->part, 0, sizeof(double) * PT_N * kK2dMaxBlocks, k->stream) != cudaSuccess ||
+      cudaMemsetAsync(k->flags, 0, sizeof(int) * 4, k->stream) != cudaSuccess)
+    return fail(VR_ERR_CUDA);
   if (!res_shape(nr, nz, nsm, &k->res_c, &k->res_nseg, &k->res_ctas)) k->res_c = 0;
   if (k->res_c) {  // made here, so that a solve allocates nothing; without it CG streams its vectors
     k->res_words = (size_t)k->res_ctas * (2 * kResCopies * kResSlotWords + 2 * 2 * (size_t)nr);
@@ -1061,6 +1064,8 @@ extern "C" int vr_k2d_create(const vr_k2d_desc *d, vr_k2d **out) {
       return fail(VR_ERR_CUDA);
     }
   }
+  // a network's training reads the coefficients on a stream of its own
+  if (cudaStreamSynchronize(k->stream) != cudaSuccess) return fail(VR_ERR_CUDA);
   *out = k;
   return VR_OK;
 }
