@@ -187,7 +187,8 @@ extern "C" int vr_analysis(vr_ctx *c, int32_t anlstp, double out[13], const char
     if (cudaMalloc(&c->ana_zm, sizeof(double) * zm.size()) != cudaSuccess ||
         cudaMalloc(&c->ana_part, sizeof(double) * (8 * (size_t)nb + 10)) != cudaSuccess)
       return set_err(c, VR_ERR_OOM, "analysis buffers");
-    VR_CUDA(c, cudaMemcpy(c->ana_zm, zm.data(), sizeof(double) * zm.size(), cudaMemcpyHostToDevice));
+    VR_CUDA(c, cudaMemcpyAsync(c->ana_zm, zm.data(), sizeof(double) * zm.size(), cudaMemcpyHostToDevice, c->stream));
+    VR_CUDA(c, cudaStreamSynchronize(c->stream));  // a later call may run on another stream
   }
   {
     LaunchScope ls(c, PK_DIAG);

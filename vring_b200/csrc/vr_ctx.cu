@@ -478,7 +478,9 @@ extern "C" int vr_create(const vr_desc *desc, vr_ctx **out) {
   size_t o_twt = blob.add(twt), o_twz = blob.add(twz);
   c->dcoef_len = blob.v.size();
   if (cudaMalloc(&c->dcoef, sizeof(double) * c->dcoef_len) != cudaSuccess) return fail(VR_ERR_OOM);
-  if (cudaMemcpy(c->dcoef, blob.v.data(), sizeof(double) * c->dcoef_len, cudaMemcpyHostToDevice) !=
+  // on the context's stream: it does not wait for the legacy one, and cudaMemcpy
+  // from pageable memory may return before the device has the values
+  if (cudaMemcpyAsync(c->dcoef, blob.v.data(), sizeof(double) * c->dcoef_len, cudaMemcpyHostToDevice, c->stream) !=
       cudaSuccess)
     return fail(VR_ERR_CUDA);
   const double *D = c->dcoef;
