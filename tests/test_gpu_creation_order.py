@@ -34,3 +34,28 @@ def test_axisymmetric_solvers_run_with_their_coefficients_from_the_first_call():
         torch.cuda.synchronize()
         first = y if first is None else first
         assert torch.equal(y, first) and bool(torch.isfinite(y).all())
+
+
+def test_particles_are_advanced_from_the_state_they_were_given():
+    import vring_b200 as V
+    from vring_b200.synthetic import annulus_particles, ring_fields
+    n = 20000
+    u = np.zeros((n, 117), order="F")
+    u[:, 0], u[:, 1], u[:, 2] = annulus_particles(n, 0.5, 1.5, 2.0, 4.0, seed=1)
+    v = np.zeros((n, 3), order="F")
+    v[:, 2] = np.arange(1, n + 1)
+    r = V.Run(32, 24, 64, 4.0, 12.0, 1e-3, 1000.0, 1.0, 1.0)
+    for name, a in zip(("q1", "q2", "q3"), ring_fields(32, 24, 64, 4.0, 12.0, noise=1e-4, seed=5)):
+        r.set(name, a)
+    kept, first = [], None
+    for _ in range(8):
+        p = V.Part(r, 8, n, 1)
+        kept.append(p)
+        p.set_state(u, v, None, n)
+        p.iter_part(1)
+        got = p.state()[0]
+        first = got if first is None else first
+        assert np.array_equal(got, first) and not np.array_equal(got[:, :3], u[:, :3])
+    for p in kept:
+        p.close()
+    r.close()

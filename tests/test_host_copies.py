@@ -14,7 +14,8 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vring_b200", "csrc")
 
 
-@pytest.mark.parametrize("name", ["vr_unet.cu", "vr_krylov.cu", "vr_ctx.cu", "vr_analysis.cu"])
+@pytest.mark.parametrize("name", ["vr_unet.cu", "vr_krylov.cu", "vr_ctx.cu", "vr_analysis.cu",
+                                  "vr_particles.cu"])
 def test_no_copy_to_the_device_or_fill_on_the_legacy_stream(name):
     src = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
     found = re.findall(r"\bcudaMemset\([^;]*;", src) + \

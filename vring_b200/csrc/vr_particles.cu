@@ -1002,7 +1002,10 @@ static int vr_part_mesh_init(vr_ctx *c) {
   part_coef(g.dtheta, g.dr, g.dz, C);
   std::memcpy(h.data() + nmesh, &C, sizeof(C));
   if (cudaMalloc(&c->part_mesh, sizeof(double) * h.size()) != cudaSuccess) return VR_ERR_OOM;
-  if (cudaMemcpy(c->part_mesh, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+  // (a class may be advanced on another stream than this: it has arrived on return)
+  if (cudaMemcpyAsync(c->part_mesh, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, c->stream) !=
+          cudaSuccess ||
+      cudaStreamSynchronize(c->stream) != cudaSuccess)
     return VR_ERR_CUDA;
   return VR_OK;
 }
@@ -1048,12 +1051,12 @@ extern "C" int vr_part_create(vr_ctx *c, int32_t id, int32_t naloc, int32_t mode
     vr_part_destroy(p);
     return set_err(c, VR_ERR_OOM, "particle arrays");
   }
-  cudaMemset(p->u, 0, nu * sizeof(double));
-  cudaMemset(p->v, 0, nv * sizeof(double));
-  cudaMemset(p->isfre, 0, naloc * sizeof(int));
-  cudaMemset(p->gone, 0xff, naloc * sizeof(int));
-  cudaMemset(p->d_nremoved, 0, 3 * sizeof(int));
-  cudaMemset(p->d_key, 0, naloc * sizeof(int));
+  cudaMemsetAsync(p->u, 0, nu * sizeof(double), c->stream);
+  cudaMemsetAsync(p->v, 0, nv * sizeof(double), c->stream);
+  cudaMemsetAsync(p->isfre, 0, naloc * sizeof(int), c->stream);
+  cudaMemsetAsync(p->gone, 0xff, naloc * sizeof(int), c->stream);
+  cudaMemsetAsync(p->d_nremoved, 0, 3 * sizeof(int), c->stream);
+  cudaMemsetAsync(p->d_key, 0, naloc * sizeof(int), c->stream);
   p->ifree.assign(naloc + 2, 0);
   p->h_isfre.assign(naloc + 1, 0);
   p->inflow.assign(c->geo.nr + 2, 0.0);
@@ -1083,6 +1086,22 @@ extern "C" int vr_part_destroy(vr_part *p) {
   cudaFree(p->d_bcnt);
   if (p->d_batch) cudaFree(p->d_batch);
   delete p;
+  return VR_OK;
+}
+
+// The class's state (u, v: may be null) and free marks, no removals pending.
+// On the context's stream, since the legacy one, which cudaMemcpy and
+// cudaMemset are ordered on, is not waited for by the kernels that come next;
+// all of it has arrived on return, also for a class advanced on another stream.
+static int part_upload(vr_part *p, const double *u, const double *v, const int *isfre) {
+  vr_ctx *c = p->ctx;
+  const size_t N = (size_t)p->naloc;
+  if (u) VR_CUDA(c, cudaMemcpyAsync(p->u, u, sizeof(double) * N * 117, cudaMemcpyHostToDevice, c->stream));
+  if (v) VR_CUDA(c, cudaMemcpyAsync(p->v, v, sizeof(double) * N * 3, cudaMemcpyHostToDevice, c->stream));
+  VR_CUDA(c, cudaMemcpyAsync(p->isfre, isfre, sizeof(int) * N, cudaMemcpyHostToDevice, c->stream));
+  VR_CUDA(c, cudaMemsetAsync(p->gone, 0xff, sizeof(int) * N, c->stream));
+  VR_CUDA(c, cudaMemsetAsync(p->d_nremoved, 0, sizeof(int), c->stream));
+  VR_CUDA(c, cudaStreamSynchronize(c->stream));
   return VR_OK;
 }
 
@@ -1117,10 +1136,7 @@ static int part_sync_bookkeeping(vr_part *p) {
   // device isfre follows the host free list
   std::vector<int> isf(p->naloc);
   for (int i = 0; i < p->naloc; i++) isf[i] = p->h_isfre[i + 1];
-  VR_CUDA(c, cudaMemcpy(p->isfre, isf.data(), sizeof(int) * p->naloc, cudaMemcpyHostToDevice));
-  VR_CUDA(c, cudaMemset(p->gone, 0xff, sizeof(int) * p->naloc));
-  VR_CUDA(c, cudaMemset(p->d_nremoved, 0, sizeof(int)));
-  return VR_OK;
+  return part_upload(p, nullptr, nullptr, isf.data());
 }
 
 // injc_part (part_tools.F90:144-197) on the host free list; the device
@@ -1386,14 +1402,10 @@ extern "C" int vr_part_set_state(vr_part *p, const double *u, const double *v, c
   vr_ctx *c = p->ctx;
   VR_CUDA(c, cudaSetDevice(c->dev));
   VR_CUDA(c, cudaStreamSynchronize(c->stream));  // queued steps may still advance this class
-  VR_CUDA(c, cudaMemcpy(p->u, u, sizeof(double) * (size_t)p->naloc * 117, cudaMemcpyHostToDevice));
-  VR_CUDA(c, cudaMemcpy(p->v, v, sizeof(double) * (size_t)p->naloc * 3, cudaMemcpyHostToDevice));
   std::vector<int> isf(p->naloc, 0);
   if (isfre)
     for (int i = 0; i < p->naloc; i++) isf[i] = isfre[i];
-  VR_CUDA(c, cudaMemcpy(p->isfre, isf.data(), sizeof(int) * p->naloc, cudaMemcpyHostToDevice));
-  VR_CUDA(c, cudaMemset(p->gone, 0xff, sizeof(int) * p->naloc));
-  VR_CUDA(c, cudaMemset(p->d_nremoved, 0, sizeof(int)));
+  if (int rc = part_upload(p, u, v, isf.data())) return rc;
   p->nlast = nlast;
   p->nsorted = 0;
   p->nfree = 0;
@@ -1446,7 +1458,7 @@ extern "C" int vr_part_probe(vr_part *p, const double *xyz, int32_t n, double *o
   if (cudaMalloc(&dx, sizeof(double) * 3 * n) || cudaMalloc(&dout, sizeof(double) * 39 * n) ||
       cudaMalloc(&dcell, sizeof(int) * 3 * n))
     rc = VR_ERR_OOM;
-  if (!rc && cudaMemcpy(dx, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice)) rc = VR_ERR_CUDA;
+  if (!rc && cudaMemcpyAsync(dx, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream)) rc = VR_ERR_CUDA;
   if (!rc) {
     auto kern = c->mixed ? k_part_probe<float> : k_part_probe<double>;
     kern<<<(n + kPartPerBlock - 1) / kPartPerBlock, 96, 0, c->stream>>>(P, c->q[0], c->q[1], c->q[2], dx, n, dout, dcell);
@@ -1536,7 +1548,7 @@ extern "C" int vr_part_restart_load(vr_part *p, const char *path) {
   p->nfree = h.nfree;
   p->nids = h.nids;
   p->serial = h.serial;
-  VR_CUDA(c, cudaMemset(p->d_nremoved + 1, 0, 2 * sizeof(int)));  // the deferred counts follow serial's parity
+  VR_CUDA(c, cudaMemsetAsync(p->d_nremoved + 1, 0, 2 * sizeof(int), c->stream));  // the deferred counts follow serial's parity
   p->inflow_on = h.inflow_on != 0;
   p->r0 = h.r0;
   p->rng = h.rng;
@@ -1545,12 +1557,7 @@ extern "C" int vr_part_restart_load(vr_part *p, const char *path) {
   p->inflow = inflow;
   std::vector<int> d_isf(p->naloc);
   for (int i = 0; i < p->naloc; i++) d_isf[i] = isfre[i + 1];
-  VR_CUDA(c, cudaMemcpy(p->u, u.data(), sizeof(double) * u.size(), cudaMemcpyHostToDevice));
-  VR_CUDA(c, cudaMemcpy(p->v, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice));
-  VR_CUDA(c, cudaMemcpy(p->isfre, d_isf.data(), sizeof(int) * d_isf.size(), cudaMemcpyHostToDevice));
-  VR_CUDA(c, cudaMemset(p->gone, 0xff, sizeof(int) * p->naloc));
-  VR_CUDA(c, cudaMemset(p->d_nremoved, 0, sizeof(int)));
-  return VR_OK;
+  return part_upload(p, u.data(), v.data(), d_isf.data());
 }
 
 // ---- particle dumps (part_tools.F90:444-491) ------------------------------
