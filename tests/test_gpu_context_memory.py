@@ -1,4 +1,6 @@
 """A z length without an FFT costs a context its tables and no further field."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -8,6 +10,7 @@ pytestmark = pytest.mark.gpu
 def _taken(nth, nr, nz, precision):
     import torch
     import vring_b200 as V
+    gc.collect()
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
     r = V.Run(nth, nr, nz, 4.0, 12.0, 1e-3, 1000.0, 1.0, 1.0, precision=precision)
