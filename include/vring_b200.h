@@ -302,7 +302,9 @@ VR_API int vr_part_probe(vr_part *part, const double *xyz, int32_t n, double *ou
 
 /* ---- batched tridiagonal solvers (host arrays) --------------------------- */
 /* tripar.F90:120-145 / trithom.F90:6-29: nbatch independent systems of size n,
- * system b at offset b*n in every array; aa(1) and cc(n) are not used. */
+ * system b at offset b*n in every array; aa(1) and cc(n) are not used.  Pivots of
+ * any size: beyond 2^+-480, and with infinities or NaN, a system takes the plain
+ * recurrence, one thread per system. */
 VR_API int vr_solve_lap_thom(const double *rhs, double *sol, const double *aa, const double *bb,
                       const double *cc, int32_t n, int32_t nbatch);
 /* btrithom.F90:5-71: block tridiagonal, n blocks of size m, identity

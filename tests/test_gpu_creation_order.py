@@ -59,3 +59,13 @@ def test_particles_are_advanced_from_the_state_they_were_given():
     for p in kept:
         p.close()
     r.close()
+
+
+@pytest.mark.parametrize("method", ["cg", "pcg"])
+def test_a_second_solver_gives_the_first_ones_bits(method):
+    import vring_b200 as V
+    f = np.random.default_rng(9).standard_normal((100, 150))
+    a, b = (V.K2d(np.linspace(0.0, 4.0, 101), 150, 12.0) for _ in range(2))
+    x, its, _, _ = a.solve(f, method, tol=1e-10, maxit=5000)
+    y, its2, _, _ = b.solve(f, method, tol=1e-10, maxit=5000)
+    assert its == its2 and np.array_equal(x, y)
