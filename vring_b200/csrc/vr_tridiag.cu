@@ -41,7 +41,7 @@ namespace vr {
 // A system with a pivot beyond 2^+-480 (inside, a product cc aa that loses bits
 // is far below the rounding of u(k)), a cc / beta that is not 0 but below
 // 2^-960, infinities or NaN is solved again by the plain recurrence
-// (thomas_plain), one thread per system.
+// (thomas_plain), one thread per system: 275 us at 257 x 1024 if all are such.
 //
 // 257 x 1024 (us per call): one thread per system with its loads a system
 // apart 241; this form 18.4, with one dividing warp 22.5.  Error against 64
